@@ -684,7 +684,7 @@ class Engine:
         while b < n:
             b <<= 1
         cfg = {"bucket": b, "act_ctas_per_sm": 8, "decode_threads": 128, "decode_ctas_per_sm": 16,
-               "mc_ctas_per_sm": 6, "mc_blocks_per_tile": 16}
+               "mc_ctas_per_sm": 6, "mc_blocks_per_tile": 32}
         cfg.update(params)
         self.set_tuning(cfg)
 

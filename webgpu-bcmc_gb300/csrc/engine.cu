@@ -42,11 +42,11 @@ namespace {
 
 constexpr int kEngThreads = 256;
 constexpr uint32_t kEngTile = 1024;  // blocks per active tile (4 per thread)
-// k_bmc tiles: kBlocks active blocks per tile, 16 threads per block (4 cells
-// each); 1536 threads per SM resident whatever the tile (6 CTAs of 16 blocks)
-constexpr int kBmcThreadsPerSm = 1536;
-constexpr int kBmcPerSm = 6;        // CTAs per SM of the default 16-block tile
-constexpr int kBmcMaxPerSm = 12;    // of the 8-block tile: sizes the MC look-back status words
+// k_bmc CTAs of 8, 16 or 32 "tile blocks", 16 threads to each; 1024 threads per
+// SM resident whatever the tile (4 CTAs of 16)
+constexpr int kBmcThreadsPerSm = 1024;
+constexpr int kBmcPerSm = 6;        // CTAs per SM that a configuration may ask for at 16 blocks
+constexpr int kBmcMaxPerSm = 12;    // of the 8-block tile: sizes the MC status words
 constexpr uint32_t kMaxVolumes = 4096;
 
 struct EngVolDev {
@@ -360,35 +360,19 @@ __global__ void __launch_bounds__(kThreads, 640 / kThreads) k_decode_probe(const
 }
 
 // ---------------------------------------------------------------------------
-// k_bmc: the per-query MC kernel (pipeline.cu, k_mc) over a batch's entries
+// k_bmc: the per-query MC kernel (pipeline.cu, k_mc) over a batch's entries:
+// the same warp work (mc_common.cuh), the isovalue, volume and neighbour flags
+// taken from each entry's query, and the emit always shared out over the grid
 // ---------------------------------------------------------------------------
-template <int kBmcBlocks>
-__global__ void __launch_bounds__(16 * kBmcBlocks, kBmcThreadsPerSm / (16 * kBmcBlocks)) k_bmc(BatchArgs a)
+template <int kTileBlocks>
+__global__ void __launch_bounds__(16 * kTileBlocks, kBmcThreadsPerSm / (16 * kTileBlocks)) k_bmc(BatchArgs a)
 {
-    constexpr int kBmcThreads = 16 * kBmcBlocks;
-    constexpr int kBmcCells = 64 * kBmcBlocks;
-    // a block's 5^3 grid; rows 144 floats apart (16 mod 32 banks), so the two
-    // blocks of a warp read their corner rows on complementary banks
-    __shared__ float s_vol[kBmcBlocks][144];
-    __shared__ uint8_t s_rm[kBmcBlocks][32];  // corner-row masks of each block (count_cells)
-    __shared__ uint32_t s_pair[32], s_pair_sw[32];  // 5-bit row mask -> per-cell corner pairs
-    __shared__ __align__(16) uint16_t s_te[256][16];  // c_tri_edges
-    __shared__ __align__(16) uint32_t s_cp[64 * 8];    // c_corner_pack
-    __shared__ __align__(16) uint8_t s_cnt[256];
-    __shared__ __align__(16) uint8_t s_case[kBmcCells];
-    constexpr int kMaskWords = kBmcCells * 15 / 32;  // a tile holds at most 15 vertices per cell
-    __shared__ uint32_t s_cells[kBmcCells];    // the tile's cells with vertices in order: cell | first vertex << 16
-    __shared__ uint32_t s_vmask[kMaskWords];   // bit k: vertex k of the tile is its cell's first
-    __shared__ uint16_t s_vbase[kMaskWords];   // cells with vertices starting before vertex 32w
-    __shared__ uint32_t s_id[kBmcBlocks];
-    __shared__ uint32_t s_qi[kBmcBlocks];
-    __shared__ float s_iso[kBmcBlocks];
-    __shared__ uint32_t s_slot[kBmcBlocks][8];
-    __shared__ uint32_t s_act[kBmcBlocks];
-    __shared__ uint32_t s_warp[kBmcThreads / 32 + 1];
-    __shared__ uint32_t s_stop, s_with, s_pv, s_pb, s_cta_v, s_cta_b, s_rank;
-    __shared__ uint32_t s_gdesc[64];  // ghost_desc of each ghost voxel
-    __shared__ uint8_t s_nb_off[8];
+    constexpr int kThreads = 16 * kTileBlocks, kWarps = kThreads / 32;
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    McShared<kThreads>& sm = *reinterpret_cast<McShared<kThreads>*>(s_dyn);
+    __shared__ uint32_t s_warp[kWarps + 1];
+    __shared__ uint32_t s_ntri[32];  // the triangle counts, ready before the rest of the tables
+    __shared__ uint32_t s_stop, s_with, s_pv, s_pb, s_cta_v, s_cta_b;
 
     EngState* st = a.st;
     const uint32_t A = min(st->num_entries, st->entry_capacity);
@@ -396,207 +380,99 @@ __global__ void __launch_bounds__(16 * kBmcBlocks, kBmcThreadsPerSm / (16 * kBmc
     const uint32_t epoch = st->epoch;
     const uint64_t cap = st->vert_capacity, vbase = st->vert_base;
     const uint32_t slots = a.pool->capacity;
-    const uint32_t t = threadIdx.x;
-    const uint32_t G = gridDim.x;
-    if (t == 0) s_rank = atomicAdd(&st->tiles_mc, 1u);
-    __syncthreads();
-    const uint32_t rank = s_rank;
-    const uint32_t range = div_up(div_up(A, G), kBmcBlocks) * kBmcBlocks;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, jb = lane >> 3;
+    const uint32_t G = gridDim.x, rank = blockIdx.x;
+    // whole batches for every warp: up to kMcBlocks blocks each, or a multiple of a batch
+    const uint32_t share = div_up(A, G);
+    const uint32_t range = align_up(share, share <= kWarps * kMcBlocks ? (uint32_t)kWarps : kMcBlocks);
     const uint32_t start = min(A, rank * range), end = min(A, start + range);
-    // ranks 0 .. worked - 1 own entries; the others take part in no look-back
+    // ranks 0 .. worked - 1 own entries; the others only help with the emit
     const uint32_t worked = div_up(A, range);
-    for (uint32_t i = t; i < 512u; i += kBmcThreads)
-        reinterpret_cast<uint4*>(&s_te[0][0])[i] = reinterpret_cast<const uint4*>(&c_tri_edges.e[0][0])[i];
-    for (uint32_t i = t; i < 128u; i += kBmcThreads)
-        reinterpret_cast<uint4*>(s_cp)[i] = reinterpret_cast<const uint4*>(&c_corner_pack.p[0][0])[i];
-    if (t < 16) reinterpret_cast<uint4*>(s_cnt)[t] = reinterpret_cast<const uint4*>(c_tri.count)[t];
+    mc_shared_begin(sm);
+    if (t < 32) s_ntri[t] = c_mc.rows.ntri[t];
     if (t == 0) s_cta_v = s_cta_b = s_pv = s_pb = 0;
-    if (t < 61) s_gdesc[t] = ghost_desc(c_ghost[t]);
-    if (t < 32) {
-        uint32_t w = 0, ws = 0;
-#pragma unroll
-        for (uint32_t x = 0; x < 4; ++x) {
-            const uint32_t pr = (t >> x) & 3u;
-            w |= pr << (8u * x);
-            ws |= (((pr & 1u) << 1) | (pr >> 1)) << (8u * x);
-        }
-        s_pair[t] = w;
-        s_pair_sw[t] = ws;
-    }
-    if (t < 7) s_nb_off[t] = c_nb_off[t];
-    const uint32_t j = t >> 4, u = t & 15u, ry = u & 3u, rz = u >> 2;
+    const McLane geo = mc_lane(a.cache);
+    McWarpMem& mem = sm.warp[warp];
+    __syncthreads();
 
-    auto load_tile = [&]() -> uint32_t {
-        if (t < kBmcBlocks * 8) {
-            const uint32_t jb = t >> 3, k = t & 7u, id = s_id[jb];
-            uint32_t slot = 0xffffffffu, act = 0;
-            if (id != 0xffffffffu) {
-                const EngQuery* Q = a.queries + s_qi[jb];
-                const EngVolDev& V = a.vols[__ldg(&Q->vol)];
-                const uint3 nb = V.grid.nb;
-                const uint3 bc = block_coords(id, V.grid);
-                const uint32_t bx = bc.x, by = bc.y, bz = bc.z;
-                if (k == kNbSelf) {
-                    slot = (uint32_t)__ldg(V.item_slots + id);
-                    act = (bx + 1 < nb.x ? 0x100u : 0u) | (by + 1 < nb.y ? 0x200u : 0u) |
-                          (bz + 1 < nb.z ? 0x400u : 0u);
-                } else {
-                    const uint32_t o = s_nb_off[k], ox = o & 1u, oy = (o >> 1) & 1u, oz = o >> 2;
-                    if (bx + ox < nb.x && by + oy < nb.y && bz + oz < nb.z) {
-                        const uint32_t nid = id + ox + nb.x * (oy + nb.y * oz);
-                        const uint32_t w = __ldg(a.bitmap + __ldg(&Q->bit0) + (nid >> 5));
-                        act = (w >> (nid & 31u)) & 1u;
-                        slot = (uint32_t)__ldg(V.item_slots + nid);
-                    }
-                }
-            }
-            s_slot[jb][k] = slot;
-            const uint32_t bits = __ballot_sync(0xffffffffu, (act & 1u) != 0u);
-            if (k == kNbSelf) s_act[jb] = ((bits >> (t & 24u)) & 0x7fu) | act;
-        }
-        __syncthreads();
-        const uint32_t id = s_id[j];
-        uint32_t dims = 0;
-        if (id != 0xffffffffu) {
-            const uint32_t act = s_act[j];
-            dims = block_dims_with_ghost(act, (act & 0x100u) != 0u, (act & 0x200u) != 0u, (act & 0x400u) != 0u);
-            const uint32_t slot = s_slot[j][kNbSelf];
-            float4 v4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (slot < slots) v4 = __ldg(reinterpret_cast<const float4*>(a.cache + (uint64_t)slot * 64u) + u);
-            else atomicCAS(&st->error, 0u, 62u);
-            const uint32_t has = ghost_axes(dims);
-            float gv[4];
-            uint32_t gaddr[4];
-#pragma unroll
-            for (uint32_t r = 0; r < 4; ++r) {
-                const uint32_t gi = u + 16u * r;
-                gv[r] = 0.0f;
-                gaddr[r] = 0xffffffffu;
-                if (gi < 61) {
-                    const uint32_t d = s_gdesc[gi];
-                    if ((d & 7u & ~has) == 0u) {
-                        const uint32_t nslot = s_slot[j][d >> 16];
-                        if (nslot < slots) {
-                            gv[r] = __ldg(a.cache + (uint64_t)nslot * 64u + ((d >> 3) & 63u));
-                            gaddr[r] = (d >> 9) & 127u;
-                        } else {
-                            atomicCAS(&st->error, 0u, 63u);
-                        }
-                    }
-                }
-            }
-            float* row = &s_vol[j][5u * (ry + 5u * rz)];
-            row[0] = v4.x;
-            row[1] = v4.y;
-            row[2] = v4.z;
-            row[3] = v4.w;
-#pragma unroll
-            for (uint32_t r = 0; r < 4; ++r)
-                if (gaddr[r] != 0xffffffffu) s_vol[j][gaddr[r]] = gv[r];
-        }
-        __syncthreads();
-        return dims;
-    };
-    // cases and counts of cells 4u..4u+3 (compute_block_has_vertices.comp:28-51):
-    // the 4 corner rows (y, z), (y+1, z), (y, z+1), (y+1, z+1) are tested once each
-    auto count_cells = [&](uint32_t dims, uint32_t nv[4], uint32_t& cs4) -> uint32_t {
-        const uint32_t dx = dims & 15u, dy = (dims >> 4) & 15u, dz = dims >> 8;
-        const bool row_ok = s_id[j] != 0xffffffffu && ry + 1 < dy && rz + 1 < dz;
-        const float iso = s_iso[j];
-        // the 25 corner rows (y, z) of the block's grid, row y + 5z, two per
-        // thread of the block's 16 (one warp half): masks of value <= iso
-#pragma unroll
-        for (uint32_t h = 0; h < 2; ++h) {
-            const uint32_t i = u + 16u * h;
-            if (i < 25u) {
-                const float* p = &s_vol[j][5u * i];
-                uint32_t m = 0;
-#pragma unroll
-                for (uint32_t x = 0; x < 5; ++x) m |= (p[x] <= iso ? 1u : 0u) << x;
-                s_rm[j][i] = (uint8_t)m;
-            }
-        }
-        __syncwarp();
-        const uint32_t r0 = ry + 5u * rz;
-        // the four cases at once, one byte per cell: s_pair[m] puts bits x and
-        // x+1 of a row mask into byte x, s_pair_sw the same pair swapped; the
-        // corner order of the case (compute_vertex_values.comp:48-57) is
-        // (x,y,z) (x+1,y,z) (x+1,y+1,z) (x,y+1,z), then the same at z+1
-        cs4 = s_pair[s_rm[j][r0]] | (s_pair_sw[s_rm[j][r0 + 1u]] << 2) | (s_pair[s_rm[j][r0 + 5u]] << 4) |
-              (s_pair_sw[s_rm[j][r0 + 6u]] << 6);
-        // cells past the grid (the last one when dims.x is 4) or in rows past it: no case
-        cs4 &= row_ok ? (dx == 5u ? 0xffffffffu : 0x00ffffffu) : 0u;
-        uint32_t sum = 0;
-#pragma unroll
-        for (uint32_t x = 0; x < 4; ++x) {
-            nv[x] = s_cnt[(cs4 >> (8u * x)) & 255u];
-            sum += nv[x];
-        }
-        return sum;
+    // lane 8j + o: neighbour o of the block of entry e (of lane 8j)
+    const auto lookup = [&](bool valid, uint32_t e, uint32_t& id, uint32_t& qi, float& iso, uint32_t& slot,
+                            uint32_t& has) {
+        id = valid ? __ldg(a.ent_id + e) : 0u;
+        qi = valid ? __ldg(a.ent_q + e) : 0u;
+        const EngQuery* Q = a.queries + qi;
+        iso = __ldg(&Q->iso);
+        const EngVolDev& V = a.vols[__ldg(&Q->vol)];
+        const uint32_t* bits = a.bitmap + __ldg(&Q->bit0);
+        mc_lookup(valid, id, V.grid, V.item_slots, slots,
+                  [&](uint32_t nid) { return (__ldg(bits + (nid >> 5)) >> (nid & 31u) & 1u) != 0u; }, &st->error, 62u,
+                  63u, slot, has);
     };
 
     // ---- count pass
-    for (uint32_t base = start; base < end; base += kBmcBlocks) {
-        __syncthreads();
-        if (t < kBmcBlocks) {
-            const uint32_t idx = base + t;
-            uint32_t id = 0xffffffffu, qi = 0;
-            if (idx < end) {
-                id = __ldg(a.ent_id + idx);
-                qi = __ldg(a.ent_q + idx);
-            }
-            s_id[t] = id;
-            s_qi[t] = qi;
-            s_iso[t] = __ldg(&a.queries[qi].iso);
-        }
-        __syncthreads();
-        const uint32_t dims = load_tile();
-        uint32_t nv[4], cs4;
-        uint32_t bsum = count_cells(dims, nv, cs4);
+    {
+        const uint32_t batch = min(kMcBlocks, max(range / kWarps, 1u));
+        uint32_t wv = 0, wb = 0;
+        uint32_t cur = 0xffffffffu, cur_v = 0;  // the query being added up (one atomic per warp and run of a query)
+        for (uint32_t base = start + warp * batch; base < end; base += kWarps * batch) {
+            const uint32_t n = min(batch, end - base);
+            uint32_t id, qi, slot, has, mine = 0;
+            float iso;
+            lookup(jb < n, base + jb, id, qi, iso, slot, has);
+            float f[kMcBlocks][4];
+            mc_voxels(geo, slot, n, f);
 #pragma unroll
-        for (int o = 8; o; o >>= 1) bsum += __shfl_xor_sync(0xffffffffu, bsum, o);
-        if (u == 0 && s_id[j] != 0xffffffffu) {
-            a.block_counts[base + j] = bsum;
-            if (bsum) {
-                atomicAdd(&s_cta_v, bsum);
-                atomicAdd(&s_cta_b, 1u);
-                atomicAdd(a.q_nverts + s_qi[j], bsum);
-            }
+            for (uint32_t j = 0; j < kMcBlocks; ++j)
+                if (j < n) {
+                    uint32_t c0, c1;
+                    if (!mc_cases(geo, f[j], __shfl_sync(kFull, iso, 8u * j), __shfl_sync(kFull, has, 8u * j), c0, c1))
+                        continue;
+                    const uint32_t v = 3u * __reduce_add_sync(kFull, mc_tri_count(s_ntri, c0) + mc_tri_count(s_ntri, c1));
+                    if (lane == j) mine = v;
+                    wv += v;
+                    wb += v != 0u ? 1u : 0u;
+                    const uint32_t qj = __shfl_sync(kFull, qi, 8u * j);
+                    if (qj != cur) {
+                        if (cur_v && lane == 0) atomicAdd(a.q_nverts + cur, cur_v);
+                        cur = qj;
+                        cur_v = 0;
+                    }
+                    cur_v += v;
+                }
+            if (lane < n) a.block_counts[base + lane] = mine;
+        }
+        if (lane == 0 && wb) {
+            if (cur_v) atomicAdd(a.q_nverts + cur, cur_v);
+            atomicAdd(&s_cta_v, wv);
+            atomicAdd(&s_cta_b, wb);
         }
     }
     __syncthreads();
-    if (t < 64 && rank < worked) {
-        if (t < 32) {
-            const uint32_t p = warp_lookback(a.status_v, rank, s_cta_v, epoch, &st->error, 61u);
-            if (t == 0) s_pv = p;
-        } else {
-            const uint32_t p = warp_lookback(a.status_b, rank, s_cta_b, epoch, &st->error, 64u);
-            if (t == 32) {
-                s_pb = p;
-                if (rank == worked - 1) st->with_verts = p + s_cta_b;
-            }
-        }
-    }
+    if (rank < worked)
+        cta_prefix_sums<kThreads>(a.status_v, a.status_b, rank, s_cta_v, s_cta_b, epoch, &st->error, 61u, 64u, &s_pv,
+                                  &s_pb);
+    mc_tables_wait();
     __syncthreads();
     // 32-bit prefix: a sequence over 2^32 vertices wraps here; k_bfinish
     // detects it from the 64-bit per-query totals and the host splits
     uint32_t pv = s_pv, pb = s_pb;
+    if (rank == worked - 1 && t == 0) st->with_verts = pb + s_cta_b;
     const bool fits = vbase + pv + s_cta_v <= cap;
     if (!fits && t == 0) atomicOr(&st->vert_overflow, 1u);
     // the range's entries with vertices: list positions and vertex offsets
     if (fits)
-        for (uint32_t b0 = start; b0 < end; b0 += kBmcThreads) {
+        for (uint32_t b0 = start; b0 < end; b0 += kThreads) {
             const uint32_t i = b0 + t;
             const uint32_t c = i < end ? a.block_counts[i] : 0u;  // <= 64 cells x 15 vertices
-            uint32_t tot;
-            const uint32_t ex = cta_exclusive_scan<kBmcThreads>(c | (c ? 1u << 18 : 0u), s_warp, &tot);
+            uint32_t v, w;
+            const uint32_t ex_v = cta_exclusive_scan<kThreads>(c, s_warp, &v);
+            const uint32_t ex_w = cta_exclusive_scan<kThreads>(c ? 1u : 0u, s_warp, &w);
             if (c) {
-                const uint32_t r = pb + (ex >> 18);
-                a.wv_list[r] = i;
-                a.wv_off[r] = pv + (ex & 0x3ffffu);
+                a.wv_list[pb + ex_w] = i;
+                a.wv_off[pb + ex_w] = pv + ex_v;
             }
-            pv += tot & 0x3ffffu;
-            pb += tot >> 18;
+            pv += v;
+            pb += w;
         }
     // grid barrier (the launch is cooperative: every CTA is resident)
     __syncthreads();
@@ -617,63 +493,16 @@ __global__ void __launch_bounds__(16 * kBmcBlocks, kBmcThreadsPerSm / (16 * kBmc
     }
     __syncthreads();
     if (s_stop) return;
-    // emit: tiles of kBmcBlocks consecutive list entries, claimed by whichever CTA is free
-    const uint32_t W = s_with, ntiles = div_up(W, (uint32_t)kBmcBlocks);
-    for (;;) {
-        __syncthreads();
-        if (t == 0) s_rank = atomicAdd(&st->tiles_emit, 1u);
-        for (uint32_t i = t; i < (uint32_t)kMaskWords; i += kBmcThreads) s_vmask[i] = 0u;
-        __syncthreads();
-        const uint32_t tile = s_rank;
-        if (tile >= ntiles) break;
-        const uint32_t first = tile * kBmcBlocks;
-        if (t < kBmcBlocks) {
-            uint32_t id = 0xffffffffu, qi = 0;
-            if (first + t < W) {
-                const uint32_t e = __ldcg(a.wv_list + first + t);
-                id = __ldg(a.ent_id + e);
-                qi = __ldg(a.ent_q + e);
-            }
-            s_id[t] = id;
-            s_qi[t] = qi;
-            s_iso[t] = __ldg(&a.queries[qi].iso);
-        }
-        if (t == 0) s_pv = __ldcg(a.wv_off + first);
-        __syncthreads();
-        const uint32_t dims = load_tile();
-        uint32_t nv[4], cs4;
-        const uint32_t mysum = count_cells(dims, nv, cs4);
-        // the emit's tables (as k_mc's prep_tile): each cell with vertices sets
-        // its start bit, takes its place in s_cells and records, for the one
-        // 32-vertex word whose first vertex falls in its range, the cells
-        // starting before that word
-        const uint32_t ne = (nv[0] != 0u) + (nv[1] != 0u) + (nv[2] != 0u) + (nv[3] != 0u);
-        uint32_t tot;
-        const uint32_t ex = cta_exclusive_scan<kBmcThreads>(mysum | (ne << 16), s_warp, &tot);
-        const uint32_t tile_v = tot & 0xffffu;
-        uint32_t run = ex & 0xffffu, rank = ex >> 16;
-        *reinterpret_cast<uint32_t*>(&s_case[4u * t]) = cs4;
-        if (t == 0) s_vbase[0] = 0;
-#pragma unroll
-        for (uint32_t x = 0; x < 4; ++x) {
-            if (nv[x]) {
-                atomicOr(&s_vmask[run >> 5], 1u << (run & 31u));
-                s_cells[rank] = (4u * t + x) | (run << 16);
-                const uint32_t w = (run + nv[x]) >> 5;
-                if ((w << 5) > run && w < (uint32_t)kMaskWords) s_vbase[w] = (uint16_t)(rank + 1u);
-                ++rank;
-            }
-            run += nv[x];
-        }
-        __syncthreads();
-        uint2* out = a.verts + vbase + s_pv;
-        for (uint32_t k = t; k < tile_v; k += kBmcThreads) {
-            const uint32_t w = k >> 5;
-            const uint32_t r = s_vbase[w] + (uint32_t)__popc(s_vmask[w] & (0xffffffffu >> (31u - (k & 31u)))) - 1u;
-            const uint32_t e = s_cells[r], cell = e & 0xffffu, jb = cell >> 6;
-            out[k] = make_uint2(mc_vertex(s_te[s_case[cell]][k - (e >> 16)], cell & 63u, s_vol[jb], s_cp, s_iso[jb]),
-                                s_id[jb]);
-        }
+    // emit: runs of `per` list entries, warp by warp over the whole grid
+    const uint32_t W = s_with;
+    const uint32_t per = min(kMcBlocks, div_up(W, G * kWarps));
+    for (uint32_t first = (rank * kWarps + warp) * per; first < W; first += G * kWarps * per) {
+        const uint32_t n = min(per, W - first);
+        uint32_t id, qi, slot, has;
+        float iso;
+        lookup(jb < n, jb < n ? __ldcg(a.wv_list + first + jb) : 0u, id, qi, iso, slot, has);
+        McSink<false> sink{a.verts + vbase + __ldcg(a.wv_off + first)};
+        mc_emit(geo, sm.tab, mem, n, id, slot, has, iso, sink);
     }
 }
 
@@ -780,7 +609,7 @@ struct EngConfig {
     int dec_per_sm = 16;     // k_bdecode CTAs per SM
     int mc_per_sm = kBmcPerSm;  // k_bmc CTAs per SM of the 16-block tile (<= its residency, 6); scaled
                                 // by 16 / mc_blocks for the other tiles
-    int mc_blocks = 16;         // k_bmc active blocks per tile (8, 16, 32)
+    int mc_blocks = 32;         // k_bmc "tile blocks", 16 threads each (8, 16, 32)
 };
 
 // The buffers of one batch in flight.  Two lanes let the server keep two
@@ -864,8 +693,10 @@ template <int kB>
 int bmc_resident()
 {
     static const int n = [] {
+        constexpr size_t smem = sizeof(McShared<16 * kB>);
+        allow_smem(k_bmc<kB>, smem);
         int r = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_bmc<kB>, 16 * kB, 0) != cudaSuccess || r < 1) r = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_bmc<kB>, 16 * kB, smem) != cudaSuccess || r < 1) r = 1;
         return r;
     }();
     return n;
@@ -1120,6 +951,14 @@ void eng_enqueue_front(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
     BCMC_CUDA(cudaGetLastError());
 }
 
+template <int kB>
+void bmc_launch(cudaLaunchConfig_t cfg, const BatchArgs& a)
+{
+    cfg.dynamicSmemBytes = sizeof(McShared<16 * kB>);
+    allow_smem(k_bmc<kB>, cfg.dynamicSmemBytes);
+    BCMC_CUDA(cudaLaunchKernelEx(&cfg, k_bmc<kB>, a));
+}
+
 // Phase 2: marching cubes over the batch's entries, per-query results, state out.
 void eng_enqueue_back(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
 {
@@ -1128,16 +967,15 @@ void eng_enqueue_back(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(eng_grid_mc(e));
     cfg.blockDim = dim3(16 * e->cfg.mc_blocks);
-    cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeCooperative;
     attr.val.cooperative = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    if (e->cfg.mc_blocks == 8) BCMC_CUDA(cudaLaunchKernelEx(&cfg, k_bmc<8>, a));
-    else if (e->cfg.mc_blocks == 32) BCMC_CUDA(cudaLaunchKernelEx(&cfg, k_bmc<32>, a));
-    else BCMC_CUDA(cudaLaunchKernelEx(&cfg, k_bmc<16>, a));
+    if (e->cfg.mc_blocks == 8) bmc_launch<8>(cfg, a);
+    else if (e->cfg.mc_blocks == 32) bmc_launch<32>(cfg, a);
+    else bmc_launch<16>(cfg, a);
     k_bfinish<<<1, kFinThreads, 0, s>>>(a);
     count_launches(2);
     BCMC_CUDA(cudaGetLastError());

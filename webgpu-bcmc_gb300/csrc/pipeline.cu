@@ -615,66 +615,43 @@ __global__ void __launch_bounds__(kDecodeNewThreads, 5) k_decode_new(const Query
 }
 
 // ---------------------------------------------------------------------------
-// k_mc: marching cubes over the active blocks, 16 blocks per tile.
+// k_mc: marching cubes over the active blocks.
 // ---------------------------------------------------------------------------
-constexpr int kMcBlocks = 16;
-constexpr int kMcThreads = 256;
-constexpr int kMcCells = 64 * kMcBlocks;  // 4 consecutive cells per thread
-constexpr int kMcPerSm = 6;               // resident CTAs per SM (the grid: one launch, all resident)
-constexpr int kMcMaskWords = kMcCells * 15 / 32;  // a tile holds at most 15 vertices per cell
+constexpr int kMcThreads = 512;
+constexpr int kMcWarps = kMcThreads / 32;
+constexpr int kMcPerSm = 2;  // resident CTAs per SM (the grid: one launch, all resident)
+// Ranges of at most this many blocks per CTA (small queries) are emitted by
+// their own CTA; longer ones go through a grid barrier and an even share-out.
+constexpr uint32_t kMcOwnRange = kMcWarps * kMcBlocks;
 
 // Marching cubes over the active blocks, one cooperative launch (every CTA
-// resident).  Each CTA owns one contiguous range of active blocks:
-//   count pass: per 16-block tile, one parallel round of loads fetches the
-//     active flags and cache slots of every block's 7 +x/+y/+z neighbours and
-//     its own slot, a second round fills each block's 5^3 grid in shared
-//     memory (16 B loads of 4 voxels per thread, ghost voxels alongside); a
-//     thread tests its 4 corner rows once and derives the cases and vertex
-//     counts of its 4 cells; block totals are kept;
-//   one warp-cooperative decoupled look-back per CTA turns the CTA totals into
-//     its global vertex offset and its offset in the blocks-with-vertices list;
-//   the range's entries of that list and their vertex offsets (a CTA scan over
-//     the block totals), then a grid barrier;
-//   emit: tiles of 16 consecutive list entries, claimed from a counter by
-//     whichever CTA is free -- vertex counts differ between ranges by up to
-//     7x, so the emit work is balanced across the grid, not per range --
-//     reloaded (from L2); a CTA scan gives each cell's offset and marks each
-//     cell's first vertex in a bitmask, and the vertices are spread over the
-//     CTA -- thread k takes vertex k of the tile, finds its cell from the
-//     bitmask (a population count below bit k plus the cells started before
-//     its word), its edge's two corners and axis in the (case, vertex) table
-//     -- so lanes stay converged and stores are contiguous.
-// Ranges of at most two tiles (small queries) skip the barrier: each CTA
-// emits its own range's tiles of blocks with vertices.  On the 256^3 CT-like
-// sweep the barrier and the tile claims cost 6-10 us on queries of under
-// 30,000 active blocks and the balance saves up to 48 us on the largest.
+// resident), all of its block work done by single warps (mc_common.cuh).  Each
+// CTA owns one contiguous range of active blocks:
+//   count pass: the warps take up to four blocks at a time, look their
+//     neighbours up, load their grids and count the triangles of their cells
+//     from the corner masks; block totals are kept;
+//   the CTA publishes its totals and adds up those of the CTAs before it: its
+//     vertex offset and its place in the blocks-with-vertices list;
+//   it writes its entries of that list and their vertex offsets, then a grid
+//     barrier;
+//   emit: the list in runs of up to four consecutive entries, warp by warp
+//     over the whole grid -- vertex counts differ between ranges by up to 7x,
+//     so the emit work is shared out by list entry, not by range.  Entries that
+//     follow each other in the list have their vertices one after the other,
+//     so a run needs only its first entry's offset.
+// Short ranges (small queries) skip the barrier: each CTA emits its own
+// entries.
 // Output order = the reference's: active-block order, cell order, table order.
-// kHost: the vertices go to page-locked host memory (a.host_verts); its own
-// instantiation keeps the device path's emit loop free of the alignment shift.
+// kHost: the vertices go to page-locked host memory (a.host_verts).
 template <bool kHost>
 __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McArgs a)
 {
-    // a block's 5^3 grid; rows 144 floats apart (16 mod 32 banks), so the two
-    // blocks of a warp read their corner rows on complementary banks
-    __shared__ float s_vol[kMcBlocks][144];
-    __shared__ uint8_t s_rm[kMcBlocks][32];  // corner-row masks of each block (count_cells)
-    __shared__ uint32_t s_pair[32], s_pair_sw[32];  // 5-bit row mask -> per-cell corner pairs
-    __shared__ __align__(16) uint16_t s_te[256][16];  // c_tri_edges
-    __shared__ __align__(16) uint32_t s_cp[64 * 8];    // c_corner_pack
-    __shared__ __align__(16) uint8_t s_cnt[256];
-    __shared__ __align__(16) uint8_t s_case[kMcCells];
-    __shared__ uint32_t s_cells[kMcCells];          // the tile's cells with vertices in order: cell | first vertex << 16
-    __shared__ uint32_t s_vmask[kMcMaskWords];      // bit k: vertex k of the tile is its cell's first
-    __shared__ uint16_t s_vbase[kMcMaskWords];      // cells with vertices starting before vertex 32w
-    __shared__ uint32_t s_boff[kMcBlocks];          // each block's first vertex in the tile
-    __shared__ uint32_t s_id[kMcBlocks];
-    __shared__ uint32_t s_slot[kMcBlocks][8];
-    __shared__ uint32_t s_act[kMcBlocks];
-    __shared__ uint32_t s_warp[kMcThreads / 32 + 1];
-    __shared__ uint32_t s_idx[kMcBlocks];
-    __shared__ uint32_t s_stop, s_with, s_pv, s_pb, s_cta_v, s_cta_b, s_rank, s_cursor;
-    __shared__ uint32_t s_gdesc[64];  // ghost_desc of each ghost voxel
-    __shared__ uint8_t s_nb_off[8];
+    extern __shared__ __align__(16) unsigned char s_dyn[];
+    McShared<kMcThreads>& sm = *reinterpret_cast<McShared<kMcThreads>*>(s_dyn);
+    __shared__ uint32_t s_warp[kMcWarps + 1];
+    __shared__ uint32_t s_ntri[32];  // the triangle counts, ready before the rest of the tables
+    __shared__ uint32_t s_cnt[kMcOwnRange], s_idx[kMcOwnRange], s_off[kMcOwnRange];  // short ranges
+    __shared__ uint32_t s_stop, s_with, s_pv, s_pb, s_cta_v, s_cta_b;
 
     const uint32_t A = q->num_active;
     if (A == 0 || q->grow_needed) return;
@@ -682,289 +659,104 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     const float iso = q->isovalue;
     const uint32_t cap = q->vert_capacity;
     const uint32_t slots = q->cache_size;
-    const uint3 nb = a.nb;
-    const uint32_t t = threadIdx.x;
-    const uint32_t G = gridDim.x;
-    if (t == 0) s_rank = atomicAdd(&q->tiles_mc, 1u);
-    __syncthreads();
-    const uint32_t rank = s_rank;
-    const uint32_t range = div_up(div_up(A, G), kMcBlocks) * kMcBlocks;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, jb = lane >> 3;
+    const uint32_t G = gridDim.x, rank = blockIdx.x;
+    // whole batches for every warp: 8, 16, 24 or 32 blocks, or a multiple of a batch
+    const uint32_t share = div_up(A, G);
+    const uint32_t range = align_up(share, share <= kMcOwnRange ? (uint32_t)kMcWarps : kMcBlocks);
     const uint32_t start = min(A, rank * range), end = min(A, start + range);
-    // ranks 0 .. worked - 1 own blocks; the others take part in no look-back
-    // (the walk of the last rank, past every predecessor, would end the kernel)
+    // ranks 0 .. worked - 1 own blocks; the others only help with the emit
     const uint32_t worked = div_up(A, range);
-    for (uint32_t i = t; i < 512u; i += kMcThreads)
-        reinterpret_cast<uint4*>(&s_te[0][0])[i] = reinterpret_cast<const uint4*>(&c_tri_edges.e[0][0])[i];
-    if (t < 128) reinterpret_cast<uint4*>(s_cp)[t] = reinterpret_cast<const uint4*>(&c_corner_pack.p[0][0])[t];
-    if (t < 16) reinterpret_cast<uint4*>(s_cnt)[t] = reinterpret_cast<const uint4*>(c_tri.count)[t];
-    if (t == 0) {
-        s_cta_v = s_cta_b = 0;
-        s_pv = s_pb = 0;
-        s_cursor = start;
-    }
-    if (t < 61) s_gdesc[t] = ghost_desc(c_ghost[t]);
-    if (t < 32) {
-        uint32_t w = 0, ws = 0;
-#pragma unroll
-        for (uint32_t x = 0; x < 4; ++x) {
-            const uint32_t pr = (t >> x) & 3u;
-            w |= pr << (8u * x);
-            ws |= (((pr & 1u) << 1) | (pr >> 1)) << (8u * x);
-        }
-        s_pair[t] = w;
-        s_pair_sw[t] = ws;
-    }
-    if (t < 7) s_nb_off[t] = c_nb_off[t];
-    const uint32_t j = t >> 4, u = t & 15u, ry = u & 3u, rz = u >> 2;
-
-    auto load_tile = [&]() -> uint32_t {
-        if (t < kMcBlocks * 8) {
-            const uint32_t jb = t >> 3, k = t & 7u, id = s_id[jb];
-            uint32_t slot = 0xffffffffu, act = 0;
-            if (id != 0xffffffffu) {
-                const uint3 bc = block_coords(id, a.grid);
-                const uint32_t bx = bc.x, by = bc.y, bz = bc.z;
-                if (k == kNbSelf) {
-                    slot = (uint32_t)__ldg(a.item_slots + id);
-                    act = (bx + 1 < nb.x ? 0x100u : 0u) | (by + 1 < nb.y ? 0x200u : 0u) |
-                          (bz + 1 < nb.z ? 0x400u : 0u);
-                } else {
-                    const uint32_t o = s_nb_off[k], ox = o & 1u, oy = (o >> 1) & 1u, oz = o >> 2;
-                    if (bx + ox < nb.x && by + oy < nb.y && bz + oz < nb.z) {
-                        const uint32_t nid = id + ox + nb.x * (oy + nb.y * oz);
-                        act = __ldg(a.active + nid) != 0u ? 1u : 0u;
-                        slot = (uint32_t)__ldg(a.item_slots + nid);
-                    }
-                }
-            }
-            s_slot[jb][k] = slot;
-            const uint32_t bits = __ballot_sync(0xffffffffu, (act & 1u) != 0u);
-            if (k == kNbSelf) s_act[jb] = ((bits >> (t & 24u)) & 0x7fu) | act;
-        }
-        __syncthreads();
-        const uint32_t id = s_id[j];
-        uint32_t dims = 0;
-        if (id != 0xffffffffu) {
-            const uint32_t act = s_act[j];
-            dims = block_dims_with_ghost(act, (act & 0x100u) != 0u, (act & 0x200u) != 0u, (act & 0x400u) != 0u);
-            const uint32_t slot = s_slot[j][kNbSelf];
-            float4 v4 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (slot < slots) v4 = __ldg(reinterpret_cast<const float4*>(a.cache + (uint64_t)slot * 64u) + u);
-            else atomicCAS(&q->error, 0u, 51u);
-            const uint32_t has = ghost_axes(dims);
-            float gv[4];
-            uint32_t gaddr[4];
-#pragma unroll
-            for (uint32_t r = 0; r < 4; ++r) {
-                const uint32_t gi = u + 16u * r;
-                gv[r] = 0.0f;
-                gaddr[r] = 0xffffffffu;
-                if (gi < 61) {
-                    const uint32_t d = s_gdesc[gi];
-                    if ((d & 7u & ~has) == 0u) {
-                        const uint32_t nslot = s_slot[j][d >> 16];
-                        if (nslot < slots) {
-                            gv[r] = __ldg(a.cache + (uint64_t)nslot * 64u + ((d >> 3) & 63u));
-                            gaddr[r] = (d >> 9) & 127u;
-                        } else {
-                            atomicCAS(&q->error, 0u, 52u);
-                        }
-                    }
-                }
-            }
-            float* row = &s_vol[j][5u * (ry + 5u * rz)];
-            row[0] = v4.x;
-            row[1] = v4.y;
-            row[2] = v4.z;
-            row[3] = v4.w;
-#pragma unroll
-            for (uint32_t r = 0; r < 4; ++r)
-                if (gaddr[r] != 0xffffffffu) s_vol[j][gaddr[r]] = gv[r];
-        }
-        __syncthreads();
-        return dims;
-    };
-    // cases and counts of cells 4u..4u+3 (compute_block_has_vertices.comp:28-51):
-    // the 4 corner rows (y, z), (y+1, z), (y, z+1), (y+1, z+1) are tested once each
-    auto count_cells = [&](uint32_t dims, uint32_t nv[4], uint32_t& cs4) -> uint32_t {
-        const uint32_t dx = dims & 15u, dy = (dims >> 4) & 15u, dz = dims >> 8;
-        const bool row_ok = s_id[j] != 0xffffffffu && ry + 1 < dy && rz + 1 < dz;
-        // the 25 corner rows (y, z) of the block's grid, row y + 5z, two per
-        // thread of the block's 16 (one warp half): masks of value <= iso
-#pragma unroll
-        for (uint32_t h = 0; h < 2; ++h) {
-            const uint32_t i = u + 16u * h;
-            if (i < 25u) {
-                const float* p = &s_vol[j][5u * i];
-                uint32_t m = 0;
-#pragma unroll
-                for (uint32_t x = 0; x < 5; ++x) m |= (p[x] <= iso ? 1u : 0u) << x;
-                s_rm[j][i] = (uint8_t)m;
-            }
-        }
-        __syncwarp();
-        const uint32_t r0 = ry + 5u * rz;
-        // the four cases at once, one byte per cell: s_pair[m] puts bits x and
-        // x+1 of a row mask into byte x, s_pair_sw the same pair swapped; the
-        // corner order of the case (compute_vertex_values.comp:48-57) is
-        // (x,y,z) (x+1,y,z) (x+1,y+1,z) (x,y+1,z), then the same at z+1
-        cs4 = s_pair[s_rm[j][r0]] | (s_pair_sw[s_rm[j][r0 + 1u]] << 2) | (s_pair[s_rm[j][r0 + 5u]] << 4) |
-              (s_pair_sw[s_rm[j][r0 + 6u]] << 6);
-        // cells past the grid (the last one when dims.x is 4) or in rows past it: no case
-        cs4 &= row_ok ? (dx == 5u ? 0xffffffffu : 0x00ffffffu) : 0u;
-        uint32_t sum = 0;
-#pragma unroll
-        for (uint32_t x = 0; x < 4; ++x) {
-            nv[x] = s_cnt[(cs4 >> (8u * x)) & 255u];
-            sum += nv[x];
-        }
-        return sum;
-    };
-
-    // a tile's cases and counts into the emit's tables: one CTA scan gives each
-    // thread's first vertex and first rank among the cells with vertices; each
-    // such cell sets its start bit, takes its place in s_cells and, for the one
-    // 32-vertex word whose first vertex falls in its range (it has at most 15),
-    // records the cells starting before that word (s_vmask is zeroed when the
-    // tile is claimed).  Returns the tile's vertex count; ends with a barrier.
-    auto prep_tile = [&](const uint32_t* nv, const uint32_t cs4, const uint32_t mysum) -> uint32_t {
-        const uint32_t ne = (nv[0] != 0u) + (nv[1] != 0u) + (nv[2] != 0u) + (nv[3] != 0u);
-        uint32_t tot;
-        const uint32_t ex = cta_exclusive_scan<kMcThreads>(mysum | (ne << 16), s_warp, &tot);
-        uint32_t run = ex & 0xffffu, rank = ex >> 16;
-        *reinterpret_cast<uint32_t*>(&s_case[4u * t]) = cs4;
-        if ((t & 15u) == 0u) s_boff[t >> 4] = run;
-        if (t == 0) s_vbase[0] = 0;
-#pragma unroll
-        for (uint32_t x = 0; x < 4; ++x) {
-            if (nv[x]) {
-                atomicOr(&s_vmask[run >> 5], 1u << (run & 31u));
-                s_cells[rank] = (4u * t + x) | (run << 16);
-                const uint32_t w = (run + nv[x]) >> 5;
-                if ((w << 5) > run && w < (uint32_t)kMcMaskWords) s_vbase[w] = (uint16_t)(rank + 1u);
-                ++rank;
-            }
-            run += nv[x];
-        }
-        __syncthreads();
-        return tot & 0xffffu;
-    };
-
-    // the vertices of the tile in shared memory (s_vol, s_case, s_cells,
-    // s_vmask, s_vbase, s_id), vertex k of the tile to out[k], out = a.verts + pv
-    auto emit_tile = [&](const uint32_t pv, const uint32_t tile_v) {
-        uint2* out = a.verts + pv;
-        const auto emit = [&](const uint32_t k) {
-            // vertex k's cell: the last cell starting at or before k, counted
-            // through the start bits of k's word
-            const uint32_t w = k >> 5;
-            const uint32_t r = s_vbase[w] + (uint32_t)__popc(s_vmask[w] & (0xffffffffu >> (31u - (k & 31u)))) - 1u;
-            const uint32_t e = s_cells[r], cell = e & 0xffffu, jb = cell >> 6;
-            out[k] = make_uint2(mc_vertex(s_te[s_case[cell]][k - (e >> 16)], cell & 63u, s_vol[jb], s_cp, iso),
-                                s_id[jb]);
-        };
-        if constexpr (kHost) {
-            // into host memory, j = k + shift puts each warp's 32 stores in
-            // one 256 B-aligned window: stores over the host link run ~20 %
-            // faster aligned (device memory gains less than the extra round
-            // costs)
-            const uint32_t shift = (uint32_t)(reinterpret_cast<uintptr_t>(out) >> 3) & 31u;
-            for (uint32_t j = t; j < tile_v + shift; j += kMcThreads)
-                if (j >= shift) emit(j - shift);
-        } else {
-            for (uint32_t k = t; k < tile_v; k += kMcThreads) emit(k);
-        }
-    };
+    mc_shared_begin(sm);
+    if (t < 32) s_ntri[t] = c_mc.rows.ntri[t];
+    if (t == 0) s_cta_v = s_cta_b = s_pv = s_pb = 0;
+    const McLane geo = mc_lane(a.cache);
+    McWarpMem& mem = sm.warp[warp];
+    const auto active = [&](uint32_t nid) { return __ldg(a.active + nid) != 0u; };
+    __syncthreads();
 
     // ---- count pass
-    for (uint32_t base = start; base < end; base += kMcBlocks) {
-        __syncthreads();
-        if (t < kMcBlocks) {
-            const uint32_t idx = base + t;
-            s_id[t] = idx < end ? __ldg(a.active_ids + idx) : 0xffffffffu;
-        }
-        __syncthreads();
-        const uint32_t dims = load_tile();
-        uint32_t nv[4], cs4;
-        uint32_t bsum = count_cells(dims, nv, cs4);
+    {
+        const uint32_t batch = min(kMcBlocks, range / kMcWarps);
+        uint32_t wv = 0, wb = 0;
+        for (uint32_t base = start + warp * batch; base < end; base += kMcWarps * batch) {
+            const uint32_t n = min(batch, end - base);
+            const bool valid = jb < n;
+            const uint32_t id = valid ? __ldg(a.active_ids + base + jb) : 0u;
+            uint32_t slot, has, mine = 0;
+            mc_lookup(valid, id, a.grid, a.item_slots, slots, active, &q->error, 51u, 52u, slot, has);
+            float f[kMcBlocks][4];
+            mc_voxels(geo, slot, n, f);
 #pragma unroll
-        for (int o = 8; o; o >>= 1) bsum += __shfl_xor_sync(0xffffffffu, bsum, o);
-        if (u == 0 && s_id[j] != 0xffffffffu) {
-            a.block_counts[base + j] = bsum;
-            if (bsum) {
-                atomicAdd(&s_cta_v, bsum);
-                atomicAdd(&s_cta_b, 1u);
+            for (uint32_t j = 0; j < kMcBlocks; ++j)
+                if (j < n) {
+                    uint32_t c0, c1;
+                    if (!mc_cases(geo, f[j], iso, __shfl_sync(kFull, has, 8u * j), c0, c1)) continue;
+                    const uint32_t v = 3u * __reduce_add_sync(kFull, mc_tri_count(s_ntri, c0) + mc_tri_count(s_ntri, c1));
+                    if (lane == j) mine = v;
+                    wv += v;
+                    wb += v != 0u ? 1u : 0u;
+                }
+            if (lane < n) {
+                a.block_counts[base + lane] = mine;
+                if (range <= kMcOwnRange) s_cnt[base - start + lane] = mine;
             }
+        }
+        if (lane == 0 && wb) {
+            atomicAdd(&s_cta_v, wv);
+            atomicAdd(&s_cta_b, wb);
         }
     }
     __syncthreads();
-    if (t < 64 && rank < worked) {
-        if (t < 32) {
-            const uint32_t p = warp_lookback(a.status_v, rank, s_cta_v, epoch, &q->error, 40u);
-            if (t == 0) {
-                s_pv = p;
-                if (rank == worked - 1) q->num_verts = p + s_cta_v;
-            }
-        } else {
-            const uint32_t p = warp_lookback(a.status_b, rank, s_cta_b, epoch, &q->error, 41u);
-            if (t == 32) {
-                s_pb = p;
-                if (rank == worked - 1) q->num_with_verts = p + s_cta_b;
-            }
-        }
-    }
+    if (rank < worked)
+        cta_prefix_sums<kMcThreads>(a.status_v, a.status_b, rank, s_cta_v, s_cta_b, epoch, &q->error, 40u, 41u, &s_pv,
+                                    &s_pb);
+    mc_tables_wait();
     __syncthreads();
     uint32_t pv = s_pv, pb = s_pb;
+    if (rank == worked - 1 && t == 0) {
+        q->num_verts = pv + s_cta_v;
+        q->num_with_verts = pb + s_cta_b;
+    }
     const bool fits = (uint64_t)pv + s_cta_v <= cap;
     if (!fits && t == 0) atomicOr(&q->vert_overflow, 1u);
-    if (range <= 2u * kMcBlocks) {
-        // short ranges (small queries): each CTA emits its own range, tiles of
-        // its next 16 blocks that have vertices (a warp ballot over the counts
-        // skips the others); the imbalance costs less here than the barrier
+
+    // a run of n list entries: lane 8j's active block `idx`, the first vertex at `off`
+    const auto emit = [&](const uint32_t idx, const uint32_t n, McSink<kHost>& sink) {
+        const bool valid = jb < n;
+        const uint32_t id = valid ? __ldg(a.active_ids + idx) : 0u;
+        uint32_t slot, has;
+        mc_lookup(valid, id, a.grid, a.item_slots, slots, active, &q->error, 51u, 52u, slot, has);
+        mc_emit(geo, sm.tab, mem, n, id, slot, has, iso, sink);
+    };
+
+    if (range <= kMcOwnRange) {
         if (!fits) return;
-        const uint32_t lane = t & 31u;
-        for (;;) {
-            __syncthreads();
-            for (uint32_t i = t; i < (uint32_t)kMcMaskWords; i += kMcThreads) s_vmask[i] = 0u;
-            if (t < 32) {
-                uint32_t cur = s_cursor, filled = 0;
-                while (filled < kMcBlocks && cur < end) {
-                    const uint32_t i = cur + lane;
-                    const uint32_t c = i < end ? a.block_counts[i] : 0u;
-                    const uint32_t m = __ballot_sync(0xffffffffu, c != 0u);
-                    const uint32_t nz = __popc(m), take = min(nz, kMcBlocks - filled);
-                    const uint32_t r = __popc(m & ((1u << lane) - 1u));
-                    if (c != 0u && r < take) s_idx[filled + r] = i;
-                    if (take < nz) {
-                        uint32_t mm = m;
-                        for (uint32_t k = 0; k < take; ++k) mm &= mm - 1u;
-                        cur += (uint32_t)__ffs(mm) - 1u;
-                    } else {
-                        cur += 32u;
-                    }
-                    filled += take;
+        // the range's blocks with vertices, by one warp
+        if (warp == 0)
+            for (uint32_t i0 = 0; start + i0 < end; i0 += 32u) {
+                const uint32_t i = start + i0 + lane;
+                const uint32_t c = i < end ? s_cnt[i0 + lane] : 0u;
+                const uint32_t inc = warp_inclusive_scan(c);
+                const uint32_t some = __ballot_sync(kFull, c != 0u);
+                const uint32_t r = pb + __popc(some & ((1u << lane) - 1u));
+                if (c) {
+                    s_idx[r - s_pb] = i;
+                    s_off[r - s_pb] = pv + inc - c;
+                    a.with_verts[r] = i;
+                    a.vert_offsets[r] = pv + inc - c;
                 }
-                __syncwarp();
-                if (lane < kMcBlocks) s_id[lane] = lane < filled ? __ldg(a.active_ids + s_idx[lane]) : 0xffffffffu;
-                if (lane == 0) {
-                    s_stop = filled;
-                    s_cursor = min(cur, end);
-                }
+                pv += __shfl_sync(kFull, inc, 31);
+                pb += __popc(some);
             }
-            __syncthreads();
-            const uint32_t n_sel = s_stop;
-            if (n_sel == 0) break;
-            const uint32_t dims = load_tile();
-            uint32_t nv[4], cs4;
-            const uint32_t mysum = count_cells(dims, nv, cs4);
-            const uint32_t tile_v = prep_tile(nv, cs4, mysum);
-            if (t < n_sel) {
-                a.with_verts[pb + t] = s_idx[t];
-                a.vert_offsets[pb + t] = pv + s_boff[t];
-            }
-            emit_tile(pv, tile_v);
-            pv += tile_v;
-            pb += n_sel;
+        __syncthreads();
+        const uint32_t W = s_cta_b, per = div_up(W, (uint32_t)kMcWarps);
+        const uint32_t first = warp * per;
+        if (first < W) {
+            const uint32_t n = min(per, W - first);
+            McSink<kHost> sink{a.verts + s_off[first]};
+            emit(jb < n ? s_idx[first + jb] : 0u, n, sink);
+            sink.finish(mem.out);
         }
         return;
     }
@@ -1002,25 +794,18 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     }
     __syncthreads();
     if (s_stop) return;
-    // emit: tiles of 16 consecutive list entries, claimed by whichever CTA is free
-    const uint32_t W = s_with, ntiles = div_up(W, kMcBlocks);
-    for (;;) {
-        __syncthreads();
-        if (t == 0) s_rank = atomicAdd(&q->tiles_emit, 1u);
-        for (uint32_t i = t; i < (uint32_t)kMcMaskWords; i += kMcThreads) s_vmask[i] = 0u;
-        __syncthreads();
-        const uint32_t tile = s_rank;
-        if (tile >= ntiles) break;
-        const uint32_t first = tile * kMcBlocks;
-        if (t < kMcBlocks)
-            s_id[t] = first + t < W ? __ldg(a.active_ids + __ldcg(a.with_verts + first + t)) : 0xffffffffu;
-        if (t == 0) s_pv = __ldcg(a.vert_offsets + first);
-        __syncthreads();
-        const uint32_t dims = load_tile();
-        uint32_t nv[4], cs4;
-        const uint32_t mysum = count_cells(dims, nv, cs4);
-        const uint32_t tile_v = prep_tile(nv, cs4, mysum);
-        emit_tile(s_pv, tile_v);
+    // emit: runs of `per` entries; into host memory a warp takes four runs one
+    // after the other, which leaves fewer windows of 32 vertices partly filled
+    const uint32_t W = s_with;
+    const uint32_t per = min(kMcBlocks, div_up(W, G * kMcWarps));
+    constexpr uint32_t kRuns = kHost ? 4u : 1u;
+    for (uint32_t first = (rank * kMcWarps + warp) * per * kRuns; first < W; first += G * kMcWarps * per * kRuns) {
+        McSink<kHost> sink{a.verts + __ldcg(a.vert_offsets + first)};
+        for (uint32_t e = first; e < min(W, first + per * kRuns); e += per) {
+            const uint32_t n = min(per, W - e);
+            emit(jb < n ? __ldcg(a.with_verts + e + jb) : 0u, n, sink);
+        }
+        sink.finish(mem.out);
     }
 }
 
@@ -1084,13 +869,21 @@ void decode_new_launch(bcmc_ctx* ctx, const QueryState* q, const DecodeArgs& a, 
     BCMC_CUDA(cudaGetLastError());
 }
 
+static void mc_allow_smem()
+{
+    allow_smem(k_mc<false>, sizeof(McShared<kMcThreads>));
+    allow_smem(k_mc<true>, sizeof(McShared<kMcThreads>));
+}
+
 // CTAs of k_mc resident per SM: the bound of its cooperative grid
 static uint32_t mc_per_sm()
 {
     static const uint32_t n = [] {
+        constexpr size_t smem = sizeof(McShared<kMcThreads>);
         int a = 0, b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_mc<false>, kMcThreads, 0) != cudaSuccess) a = 1;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_mc<true>, kMcThreads, 0) != cudaSuccess) b = 1;
+        mc_allow_smem();
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_mc<false>, kMcThreads, smem) != cudaSuccess) a = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_mc<true>, kMcThreads, smem) != cudaSuccess) b = 1;
         const int m = std::min(std::min(a, b), kMcPerSm);
         return (uint32_t)(m > 0 ? m : 1);
     }();
@@ -1099,11 +892,12 @@ static uint32_t mc_per_sm()
 
 void mc_launch(bcmc_ctx* ctx, QueryState* q, const McArgs& a, uint32_t max_active, cudaStream_t s)
 {
+    mc_allow_smem();  // a setting of the current device
     // cooperative: the kernel's grid barrier needs every CTA resident
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(mc_grid(ctx, max_active));
     cfg.blockDim = dim3(kMcThreads);
-    cfg.dynamicSmemBytes = 0;
+    cfg.dynamicSmemBytes = sizeof(McShared<kMcThreads>);
     cfg.stream = s;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeCooperative;
@@ -1117,11 +911,11 @@ void mc_launch(bcmc_ctx* ctx, QueryState* q, const McArgs& a, uint32_t max_activ
 
 uint32_t active_tiles(uint32_t total) { return div_up(total, kActiveTile); }
 uint32_t slot_tiles(uint32_t slots) { return div_up(slots, kSlotTile); }
-// one CTA per range of active blocks, every CTA resident
+// one CTA per range of active blocks, every CTA resident; at least a block to a warp
 uint32_t mc_grid(bcmc_ctx* ctx, uint32_t max_active)
 {
-    const uint32_t r = (uint32_t)ctx->num_sms * mc_per_sm(), tiles = div_up(max_active ? max_active : 1, kMcBlocks);
-    return tiles < r ? tiles : r;
+    const uint32_t r = (uint32_t)ctx->num_sms * mc_per_sm(), most = div_up(max_active ? max_active : 1, (uint32_t)kMcWarps);
+    return most < r ? most : r;
 }
 
 }  // namespace bcmc
