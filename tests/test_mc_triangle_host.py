@@ -1,4 +1,4 @@
-"""The MC kernels' triangle table and division-free vertex (csrc/mc_triangle.cuh),
+"""The MC kernels' case table and division-free vertex (csrc/mc_triangle.cuh),
 compiled as host C++: the table against the entries it is made from, and every
 vertex that the fast expression claims against mc_vertex, bit for bit, whichever
 way the approximate reciprocal is off, with vertices drawn near the whole numbers

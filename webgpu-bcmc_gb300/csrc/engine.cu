@@ -369,9 +369,8 @@ __global__ void __launch_bounds__(16 * kTileBlocks, kBmcThreadsPerSm / (16 * kTi
 {
     constexpr int kThreads = 16 * kTileBlocks, kWarps = kThreads / 32;
     extern __shared__ __align__(16) unsigned char s_dyn[];
-    McShared<kThreads>& sm = *reinterpret_cast<McShared<kThreads>*>(s_dyn);
+    McShared<kThreads, false>& sm = *reinterpret_cast<McShared<kThreads, false>*>(s_dyn);
     __shared__ uint32_t s_warp[kWarps + 1];
-    __shared__ uint32_t s_ntri[32];  // the triangle counts, ready before the rest of the tables
     __shared__ uint32_t s_stop, s_with, s_pv, s_pb, s_cta_v, s_cta_b;
 
     EngState* st = a.st;
@@ -389,46 +388,64 @@ __global__ void __launch_bounds__(16 * kTileBlocks, kBmcThreadsPerSm / (16 * kTi
     // ranks 0 .. worked - 1 own entries; the others only help with the emit
     const uint32_t worked = div_up(A, range);
     mc_shared_begin(sm);
-    if (t < 32) s_ntri[t] = c_mc.rows.ntri[t];
     if (t == 0) s_cta_v = s_cta_b = s_pv = s_pb = 0;
-    const McLane geo = mc_lane(a.cache);
-    McWarpMem& mem = sm.warp[warp];
-    __syncthreads();
+    const McLane geo = mc_lane(a.cache, sm.warp[warp].slot);
+    McWarpMem<false>& mem = sm.warp[warp];
 
-    // lane 8j + o: neighbour o of the block of entry e (of lane 8j)
-    const auto lookup = [&](bool valid, uint32_t e, uint32_t& id, uint32_t& qi, float& iso, uint32_t& slot,
-                            uint32_t& has) {
-        id = valid ? __ldg(a.ent_id + e) : 0u;
-        qi = valid ? __ldg(a.ent_q + e) : 0u;
-        const EngQuery* Q = a.queries + qi;
-        iso = __ldg(&Q->iso);
+    // an entry: its block, its query, and the query's isovalue
+    struct Entry {
+        uint32_t id, qi;
+    };
+    struct Look {
+        McLook l;
+        uint32_t qi;
+        float iso;
+    };
+    const auto load = [&](bool valid, uint32_t e) {
+        return valid ? Entry{__ldg(a.ent_id + e), __ldg(a.ent_q + e)} : Entry{0u, 0u};
+    };
+    const auto look = [&](bool valid, const Entry& e) {
+        const EngQuery* Q = a.queries + e.qi;
         const EngVolDev& V = a.vols[__ldg(&Q->vol)];
         const uint32_t* bits = a.bitmap + __ldg(&Q->bit0);
-        mc_lookup(valid, id, V.grid, V.item_slots, slots,
-                  [&](uint32_t nid) { return (__ldg(bits + (nid >> 5)) >> (nid & 31u) & 1u) != 0u; }, &st->error, 62u,
-                  63u, slot, has);
+        return Look{mc_look(valid, e.id, V.grid, V.item_slots,
+                            [&](uint32_t nid) { return __ldg(bits + (nid >> 5)) >> (nid & 31u) & 1u; }),
+                    e.qi, __ldg(&Q->iso)};
+    };
+    const auto look_end = [&](const Look& l) {
+        uint32_t has;
+        mc_look_end(l.l, sm.tab, slots, &st->error, 62u, mem.slot, has);
+        return has;
     };
 
-    // ---- count pass
+    // ---- count pass: entries two rounds ahead, lookups one round ahead
     {
-        const uint32_t batch = min(kMcBlocks, max(range / kWarps, 1u));
+        const uint32_t batch = min(kMcBlocks, max(range / kWarps, 1u)), step = kWarps * batch;
+        uint32_t base = start + warp * batch;
+        const auto mine = [&](uint32_t at) { return jb < batch && at + jb < end; };
+        Look next = look(mine(base), load(mine(base), base + jb));
+        Entry e2 = load(mine(base + step), base + step + jb);
         uint32_t wv = 0, wb = 0;
         uint32_t cur = 0xffffffffu, cur_v = 0;  // the query being added up (one atomic per warp and run of a query)
-        for (uint32_t base = start + warp * batch; base < end; base += kWarps * batch) {
-            const uint32_t n = min(batch, end - base);
-            uint32_t id, qi, slot, has, mine = 0;
-            float iso;
-            lookup(jb < n, base + jb, id, qi, iso, slot, has);
+        async_wait<1>();
+        __syncthreads();
+        for (; base < end; base += step) {
+            const uint32_t n = min(batch, end - base), qi = next.qi;
+            const float iso = next.iso;
+            const uint32_t has = look_end(next);
+            uint32_t total = 0;
             float f[kMcBlocks][4];
-            mc_voxels(geo, slot, n, f);
+            mc_voxels(geo, n, f);
+            next = look(mine(base + step), e2);
+            e2 = load(mine(base + 2u * step), base + 2u * step + jb);
 #pragma unroll
             for (uint32_t j = 0; j < kMcBlocks; ++j)
                 if (j < n) {
                     uint32_t c0, c1;
-                    if (!mc_cases(geo, f[j], __shfl_sync(kFull, iso, 8u * j), __shfl_sync(kFull, has, 8u * j), c0, c1))
+                    if (!mc_cases<true>(geo, f[j], __shfl_sync(kFull, iso, 8u * j), __shfl_sync(kFull, has, 8u * j), c0, c1))
                         continue;
-                    const uint32_t v = 3u * __reduce_add_sync(kFull, mc_tri_count(s_ntri, c0) + mc_tri_count(s_ntri, c1));
-                    if (lane == j) mine = v;
+                    const uint32_t v = 3u * __reduce_add_sync(kFull, (uint32_t)sm.tab.count.n[c0] + sm.tab.count.n[c1]);
+                    if (lane == j) total = v;
                     wv += v;
                     wb += v != 0u ? 1u : 0u;
                     const uint32_t qj = __shfl_sync(kFull, qi, 8u * j);
@@ -439,7 +456,7 @@ __global__ void __launch_bounds__(16 * kTileBlocks, kBmcThreadsPerSm / (16 * kTi
                     }
                     cur_v += v;
                 }
-            if (lane < n) a.block_counts[base + lane] = mine;
+            if (lane < n) a.block_counts[base + lane] = total;
         }
         if (lane == 0 && wb) {
             if (cur_v) atomicAdd(a.q_nverts + cur, cur_v);
@@ -451,7 +468,7 @@ __global__ void __launch_bounds__(16 * kTileBlocks, kBmcThreadsPerSm / (16 * kTi
     if (rank < worked)
         cta_prefix_sums<kThreads>(a.status_v, a.status_b, rank, s_cta_v, s_cta_b, epoch, &st->error, 61u, 64u, &s_pv,
                                   &s_pb);
-    mc_tables_wait();
+    async_wait<0>();
     __syncthreads();
     // 32-bit prefix: a sequence over 2^32 vertices wraps here; k_bfinish
     // detects it from the 64-bit per-query totals and the host splits
@@ -493,16 +510,26 @@ __global__ void __launch_bounds__(16 * kTileBlocks, kBmcThreadsPerSm / (16 * kTi
     }
     __syncthreads();
     if (s_stop) return;
-    // emit: runs of `per` list entries, warp by warp over the whole grid
+    // emit: runs of `per` list entries, warp by warp over the whole grid; a
+    // run's list entries are read two runs ahead, its neighbours one run ahead
     const uint32_t W = s_with;
-    const uint32_t per = min(kMcBlocks, div_up(W, G * kWarps));
-    for (uint32_t first = (rank * kWarps + warp) * per; first < W; first += G * kWarps * per) {
-        const uint32_t n = min(per, W - first);
-        uint32_t id, qi, slot, has;
-        float iso;
-        lookup(jb < n, jb < n ? __ldcg(a.wv_list + first + jb) : 0u, id, qi, iso, slot, has);
-        McSink<false> sink{a.verts + vbase + __ldcg(a.wv_off + first)};
-        mc_emit(geo, sm.tab, mem, n, id, slot, has, iso, sink);
+    const uint32_t per = min(kMcBlocks, div_up(W, G * kWarps)), step = G * kWarps * per;
+    const auto mine = [&](uint32_t at) { return jb < per && at + jb < W; };
+    const auto load_entry = [&](uint32_t at) { return mine(at) ? __ldcg(a.wv_list + at + jb) : 0u; };
+    uint32_t at = (rank * kWarps + warp) * per;
+    if (at >= W) return;
+    Look next = look(mine(at), load(mine(at), load_entry(at)));
+    uint32_t entry = load_entry(at + step), off = __ldcg(a.wv_off + at);
+    for (; at < W; at += step) {
+        const uint32_t n = min(per, W - at), id = next.l.id, at1 = at + step;
+        const float iso = next.iso;
+        const uint32_t has = look_end(next);
+        mc_grids(geo, mem, n);
+        McSink<false> sink{a.verts + vbase + off};
+        const Entry e1 = load(mine(at1), entry);
+        entry = load_entry(at1 + step);
+        off = at1 < W ? __ldcg(a.wv_off + at1) : 0u;
+        mc_emit<false, false>(geo, sm.tab, mem, n, id, has, iso, sink, [&] { next = look(mine(at1), e1); });
     }
 }
 
@@ -693,7 +720,7 @@ template <int kB>
 int bmc_resident()
 {
     static const int n = [] {
-        constexpr size_t smem = sizeof(McShared<16 * kB>);
+        constexpr size_t smem = sizeof(McShared<16 * kB, false>);
         allow_smem(k_bmc<kB>, smem);
         int r = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_bmc<kB>, 16 * kB, smem) != cudaSuccess || r < 1) r = 1;
@@ -954,7 +981,7 @@ void eng_enqueue_front(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
 template <int kB>
 void bmc_launch(cudaLaunchConfig_t cfg, const BatchArgs& a)
 {
-    cfg.dynamicSmemBytes = sizeof(McShared<16 * kB>);
+    cfg.dynamicSmemBytes = sizeof(McShared<16 * kB, false>);
     allow_smem(k_bmc<kB>, cfg.dynamicSmemBytes);
     BCMC_CUDA(cudaLaunchKernelEx(&cfg, k_bmc<kB>, a));
 }

@@ -647,9 +647,8 @@ template <bool kHost>
 __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McArgs a)
 {
     extern __shared__ __align__(16) unsigned char s_dyn[];
-    McShared<kMcThreads>& sm = *reinterpret_cast<McShared<kMcThreads>*>(s_dyn);
+    McShared<kMcThreads, kHost>& sm = *reinterpret_cast<McShared<kMcThreads, kHost>*>(s_dyn);
     __shared__ uint32_t s_warp[kMcWarps + 1];
-    __shared__ uint32_t s_ntri[32];  // the triangle counts, ready before the rest of the tables
     __shared__ uint32_t s_cnt[kMcOwnRange], s_idx[kMcOwnRange], s_off[kMcOwnRange];  // short ranges
     __shared__ uint32_t s_stop, s_with, s_pv, s_pb, s_cta_v, s_cta_b;
 
@@ -668,38 +667,51 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     // ranks 0 .. worked - 1 own blocks; the others only help with the emit
     const uint32_t worked = div_up(A, range);
     mc_shared_begin(sm);
-    if (t < 32) s_ntri[t] = c_mc.rows.ntri[t];
     if (t == 0) s_cta_v = s_cta_b = s_pv = s_pb = 0;
-    const McLane geo = mc_lane(a.cache);
-    McWarpMem& mem = sm.warp[warp];
-    const auto active = [&](uint32_t nid) { return __ldg(a.active + nid) != 0u; };
-    __syncthreads();
+    const McLane geo = mc_lane(a.cache, sm.warp[warp].slot);
+    McWarpMem<kHost>& mem = sm.warp[warp];
+    const auto look = [&](bool valid, uint32_t id) {
+        return mc_look(valid, id, a.grid, a.item_slots, [&](uint32_t nid) { return __ldg(a.active + nid); });
+    };
+    const auto look_end = [&](const McLook& l) {
+        uint32_t has;
+        mc_look_end(l, sm.tab, slots, &q->error, 51u, mem.slot, has);
+        return has;
+    };
 
-    // ---- count pass
+    // ---- count pass: ids two rounds ahead, lookups one round ahead
     {
-        const uint32_t batch = min(kMcBlocks, range / kMcWarps);
+        const uint32_t batch = min(kMcBlocks, range / kMcWarps), step = kMcWarps * batch;
+        uint32_t base = start + warp * batch;
+        // the last batch of a range may be short; jb < batch keeps a lane to its batch
+        const auto mine = [&](uint32_t at) { return jb < batch && at + jb < end; };
+        const auto load_id = [&](uint32_t at) { return mine(at) ? __ldg(a.active_ids + at + jb) : 0u; };
+        McLook next = look(mine(base), load_id(base));
+        uint32_t id2 = load_id(base + step);
         uint32_t wv = 0, wb = 0;
-        for (uint32_t base = start + warp * batch; base < end; base += kMcWarps * batch) {
+        async_wait<1>();
+        __syncthreads();
+        for (; base < end; base += step) {
             const uint32_t n = min(batch, end - base);
-            const bool valid = jb < n;
-            const uint32_t id = valid ? __ldg(a.active_ids + base + jb) : 0u;
-            uint32_t slot, has, mine = 0;
-            mc_lookup(valid, id, a.grid, a.item_slots, slots, active, &q->error, 51u, 52u, slot, has);
+            const uint32_t has = look_end(next);
+            uint32_t total = 0;
             float f[kMcBlocks][4];
-            mc_voxels(geo, slot, n, f);
+            mc_voxels(geo, n, f);
+            next = look(mine(base + step), id2);
+            id2 = load_id(base + 2u * step);
 #pragma unroll
             for (uint32_t j = 0; j < kMcBlocks; ++j)
                 if (j < n) {
                     uint32_t c0, c1;
-                    if (!mc_cases(geo, f[j], iso, __shfl_sync(kFull, has, 8u * j), c0, c1)) continue;
-                    const uint32_t v = 3u * __reduce_add_sync(kFull, mc_tri_count(s_ntri, c0) + mc_tri_count(s_ntri, c1));
-                    if (lane == j) mine = v;
+                    if (!mc_cases<true>(geo, f[j], iso, __shfl_sync(kFull, has, 8u * j), c0, c1)) continue;
+                    const uint32_t v = 3u * __reduce_add_sync(kFull, (uint32_t)sm.tab.count.n[c0] + sm.tab.count.n[c1]);
+                    if (lane == j) total = v;
                     wv += v;
                     wb += v != 0u ? 1u : 0u;
                 }
             if (lane < n) {
-                a.block_counts[base + lane] = mine;
-                if (range <= kMcOwnRange) s_cnt[base - start + lane] = mine;
+                a.block_counts[base + lane] = total;
+                if (range <= kMcOwnRange) s_cnt[base - start + lane] = total;
             }
         }
         if (lane == 0 && wb) {
@@ -711,7 +723,7 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     if (rank < worked)
         cta_prefix_sums<kMcThreads>(a.status_v, a.status_b, rank, s_cta_v, s_cta_b, epoch, &q->error, 40u, 41u, &s_pv,
                                     &s_pb);
-    mc_tables_wait();
+    async_wait<0>();
     __syncthreads();
     uint32_t pv = s_pv, pb = s_pb;
     if (rank == worked - 1 && t == 0) {
@@ -720,15 +732,6 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     }
     const bool fits = (uint64_t)pv + s_cta_v <= cap;
     if (!fits && t == 0) atomicOr(&q->vert_overflow, 1u);
-
-    // a run of n list entries: lane 8j's active block `idx`, the first vertex at `off`
-    const auto emit = [&](const uint32_t idx, const uint32_t n, McSink<kHost>& sink) {
-        const bool valid = jb < n;
-        const uint32_t id = valid ? __ldg(a.active_ids + idx) : 0u;
-        uint32_t slot, has;
-        mc_lookup(valid, id, a.grid, a.item_slots, slots, active, &q->error, 51u, 52u, slot, has);
-        mc_emit(geo, sm.tab, mem, n, id, slot, has, iso, sink);
-    };
 
     if (range <= kMcOwnRange) {
         if (!fits) return;
@@ -754,8 +757,12 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
         const uint32_t first = warp * per;
         if (first < W) {
             const uint32_t n = min(per, W - first);
+            const bool valid = jb < n;
+            const uint32_t id = valid ? __ldg(a.active_ids + s_idx[first + jb]) : 0u;
+            const uint32_t has = look_end(look(valid, id));
+            mc_grids(geo, mem, n);
             McSink<kHost> sink{a.verts + s_off[first]};
-            emit(jb < n ? s_idx[first + jb] : 0u, n, sink);
+            mc_emit<kHost, true>(geo, sm.tab, mem, n, id, has, iso, sink, [] {});
             sink.finish(mem.out);
         }
         return;
@@ -794,19 +801,41 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     }
     __syncthreads();
     if (s_stop) return;
-    // emit: runs of `per` entries; into host memory a warp takes four runs one
-    // after the other, which leaves fewer windows of 32 vertices partly filled
+    // emit: runs of `per` entries, one from each warp's turn over the grid; into
+    // host memory a turn is four runs that follow each other, which leaves fewer
+    // windows of 32 vertices partly filled.  A run's list entries are read two
+    // runs ahead, its block ids and neighbours one run ahead.
     const uint32_t W = s_with;
     const uint32_t per = min(kMcBlocks, div_up(W, G * kMcWarps));
     constexpr uint32_t kRuns = kHost ? 4u : 1u;
-    for (uint32_t first = (rank * kMcWarps + warp) * per * kRuns; first < W; first += G * kMcWarps * per * kRuns) {
-        McSink<kHost> sink{a.verts + __ldcg(a.vert_offsets + first)};
-        for (uint32_t e = first; e < min(W, first + per * kRuns); e += per) {
-            const uint32_t n = min(per, W - e);
-            emit(jb < n ? __ldcg(a.with_verts + e + jb) : 0u, n, sink);
+    const uint32_t turn = per * kRuns, skip = (G * kMcWarps - 1u) * turn;
+    const auto after = [&](uint32_t at, uint32_t run) { return at + per + (run == kRuns - 1u ? skip : 0u); };
+    const auto mine = [&](uint32_t at) { return jb < per && at + jb < W; };
+    const auto load_entry = [&](uint32_t at) { return mine(at) ? __ldcg(a.with_verts + at + jb) : 0u; };
+    const auto load_id = [&](uint32_t at, uint32_t entry) { return mine(at) ? __ldg(a.active_ids + entry) : 0u; };
+    uint32_t at = (rank * kMcWarps + warp) * turn, run = 0;
+    if (at >= W) return;
+    McLook next = look(mine(at), load_id(at, load_entry(at)));
+    uint32_t entry = load_entry(after(at, 0u));
+    McSink<kHost> sink{a.verts + __ldcg(a.vert_offsets + at)};
+    for (;;) {
+        const uint32_t n = min(per, W - at), id = next.id;
+        const uint32_t has = look_end(next);
+        mc_grids(geo, mem, n);
+        const uint32_t at1 = after(at, run), run1 = run == kRuns - 1u ? 0u : run + 1u;
+        const uint32_t id1 = load_id(at1, entry);
+        entry = load_entry(after(at1, run1));
+        const uint32_t off1 = run1 == 0u && at1 < W ? __ldcg(a.vert_offsets + at1) : 0u;
+        mc_emit<kHost, true>(geo, sm.tab, mem, n, id, has, iso, sink, [&] { next = look(mine(at1), id1); });
+        at = at1;
+        run = run1;
+        if (at >= W) break;
+        if (run == 0u) {
+            sink.finish(mem.out);
+            sink.start(a.verts + off1);
         }
-        sink.finish(mem.out);
     }
+    sink.finish(mem.out);
 }
 
 // ---------------------------------------------------------------------------
@@ -871,19 +900,19 @@ void decode_new_launch(bcmc_ctx* ctx, const QueryState* q, const DecodeArgs& a, 
 
 static void mc_allow_smem()
 {
-    allow_smem(k_mc<false>, sizeof(McShared<kMcThreads>));
-    allow_smem(k_mc<true>, sizeof(McShared<kMcThreads>));
+    allow_smem(k_mc<false>, sizeof(McShared<kMcThreads, false>));
+    allow_smem(k_mc<true>, sizeof(McShared<kMcThreads, true>));
 }
 
 // CTAs of k_mc resident per SM: the bound of its cooperative grid
 static uint32_t mc_per_sm()
 {
     static const uint32_t n = [] {
-        constexpr size_t smem = sizeof(McShared<kMcThreads>);
+        constexpr size_t sa = sizeof(McShared<kMcThreads, false>), sb = sizeof(McShared<kMcThreads, true>);
         int a = 0, b = 0;
         mc_allow_smem();
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_mc<false>, kMcThreads, smem) != cudaSuccess) a = 1;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_mc<true>, kMcThreads, smem) != cudaSuccess) b = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, k_mc<false>, kMcThreads, sa) != cudaSuccess) a = 1;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_mc<true>, kMcThreads, sb) != cudaSuccess) b = 1;
         const int m = std::min(std::min(a, b), kMcPerSm);
         return (uint32_t)(m > 0 ? m : 1);
     }();
@@ -897,7 +926,7 @@ void mc_launch(bcmc_ctx* ctx, QueryState* q, const McArgs& a, uint32_t max_activ
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(mc_grid(ctx, max_active));
     cfg.blockDim = dim3(kMcThreads);
-    cfg.dynamicSmemBytes = sizeof(McShared<kMcThreads>);
+    cfg.dynamicSmemBytes = a.host_verts ? sizeof(McShared<kMcThreads, true>) : sizeof(McShared<kMcThreads, false>);
     cfg.stream = s;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeCooperative;
