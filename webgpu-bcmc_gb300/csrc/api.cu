@@ -380,6 +380,7 @@ struct bcmc_vol {
     uint64_t nwords = 0;
     size_t compressed_bytes = 0;
     float* ranges = nullptr;
+    void* flag_words = nullptr;  // k_query_flags' words (flag_bytes)
     uint32_t* active = nullptr;
     uint32_t* active_ids = nullptr;
     uint32_t* with_verts = nullptr;
@@ -428,6 +429,7 @@ static void vol_free(bcmc_vol* v)
     cudaStreamSynchronize(ctx->stream);
     dev_free(ctx, v->words, v->nwords * 8);
     dev_free(ctx, v->ranges, (size_t)v->total * 8);
+    dev_free(ctx, v->flag_words, flag_bytes(v->total));
     dev_free(ctx, v->active, (size_t)v->total * 4);
     dev_free(ctx, v->active_ids, (size_t)v->total * 4);
     dev_free(ctx, v->with_verts, (size_t)v->total * 4);
@@ -505,6 +507,7 @@ static bcmc_status vol_create_common(bcmc_ctx* ctx, const void* src, bool src_de
             BCMC_CUDA(cudaMemsetAsync(v->words, 0, v->nwords * 8, s));
             BCMC_CUDA(cudaMemcpyAsync(v->words, src, len, src_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
             v->ranges = (float*)dev_alloc(ctx, (size_t)total * 8);
+            v->flag_words = dev_alloc(ctx, flag_bytes(total));
             v->active = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
             v->active_ids = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
             v->with_verts = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
@@ -642,8 +645,8 @@ static void vol_enqueue_query(bcmc_vol* v, cudaStream_t s, float iso, int from_s
     bcmc_lru* c = v->lru;
     const uint3 nb = make_uint3(v->nb[0], v->nb[1], v->nb[2]);
     const BlockGrid grid = make_block_grid(nb);
-    ActiveArgs aa{reinterpret_cast<const float2*>(v->ranges), nb, grid, nullptr, v->active, c->item_slots,
-                  v->total, v->active_ids, c->new_ids, c->st_active_a, c->st_active_n};
+    ActiveArgs aa{grid,          nullptr,    v->active,      c->item_slots,  v->total,
+                  v->active_ids, c->new_ids, c->st_active_a, c->st_active_n};
     McArgs ma{v->active, v->active_ids, c->item_slots, reinterpret_cast<const float*>(c->cache), nb, grid,
               v->with_verts, v->vert_offsets, v->block_counts, out, c->st_mc_v, c->st_mc_b, out != v->verts ? 1u : 0u};
     SlotArgs sa{v->active,  c->slot_age, c->slot_avail, c->slot_item, c->avail_ids, c->avail_keys, c->st_slots, 1u, 1u,
@@ -652,8 +655,9 @@ static void vol_enqueue_query(bcmc_vol* v, cudaStream_t s, float iso, int from_s
                   c->item_slots, v->words, v->max_bits, reinterpret_cast<float*>(c->cache), v->stage, v->stage_blocks};
     DecodeArgs da{c->new_ids, v->words, v->max_bits, v->stage, v->stage_blocks};
     if (events) BCMC_CUDA(cudaEventRecordWithFlags(v->ev[0], s, cudaEventRecordExternal));
-    query_begin_launch(c->q, iso, 0, c->capacity, v->vert_capacity, s, from_state ? v->h_in : nullptr);
-    active_launch(ctx, c->q, aa, s);
+    query_flags_launch(ctx, c->q, iso, c->capacity, v->vert_capacity, v->ranges, grid, v->total, v->flag_words, s,
+                       from_state ? v->h_in : nullptr);
+    active_words_launch(ctx, c->q, aa, v->flag_words, s);
     if (events) BCMC_CUDA(cudaEventRecordWithFlags(v->ev[1], s, cudaEventRecordExternal));
     // branch: the new blocks' decode into the staging buffer needs only the
     // active test's new ids, so it overlaps the slot selection below
@@ -956,7 +960,7 @@ bcmc_status bcmc_memory_report(bcmc_vol* v, bcmc_memory* m)
     m->cachedItemSlots = (uint64_t)c->aligned_total * 4;
     m->slotData = (uint64_t)c->capacity * 12;
     m->scratch = (uint64_t)c->capacity * 4 * 6 + c->status_words * 8 + (uint64_t)c->total * 4 + sizeof(QueryState) +
-                 (uint64_t)v->stage_blocks * 256u;
+                 (uint64_t)v->stage_blocks * 256u + flag_bytes(v->total);
     m->deviceTotal = m->compressedData + m->vertexBuffer + m->blockActive + m->blockRanges + m->activeBlockIDs +
                      m->blocksWithVertices + m->blockVertexOffsets + m->cache + m->cachedItemSlots + m->slotData +
                      m->scratch;
@@ -1022,8 +1026,8 @@ bcmc_status bcmc_lru_update(bcmc_lru* c, const uint32_t* d_item_needed, uint32_t
         cudaStream_t s = ctx->stream;
         for (int attempt = 0;; ++attempt) {
             lru_begin(c, s, 0.0f, 0, 0);
-            ActiveArgs aa{nullptr, make_uint3(0, 0, 0), make_block_grid(make_uint3(1, 1, 1)), d_item_needed, nullptr,
-                          c->item_slots, c->total, nullptr, c->new_ids, c->st_active_a, c->st_active_n};
+            ActiveArgs aa{make_block_grid(make_uint3(1, 1, 1)), d_item_needed, nullptr,        c->item_slots,
+                          c->total, nullptr, c->new_ids, c->st_active_a, c->st_active_n};
             active_launch(ctx, c->q, aa, s);
             lru_enqueue_update(c, s, d_item_needed, nullptr, 0);
             lru_read_state(c, s);
@@ -1270,10 +1274,12 @@ bcmc_status bcmc_block_active(bcmc_ctx* ctx, const float* d_ranges, const uint32
         const uint3 nb = make_uint3(div_up(dims[0], 4), div_up(dims[1], 4), div_up(dims[2], 4));
         const uint64_t total = (uint64_t)nb.x * nb.y * nb.z;
         ensure_status(ctx, 2 * (active_tiles((uint32_t)total) + 1));
-        query_begin_launch(ctx->d_prim, iso, 0, 0, 0, s);
-        ActiveArgs aa{reinterpret_cast<const float2*>(d_ranges), nb, make_block_grid(nb), nullptr, d_active, nullptr,
-                      (uint32_t)total, nullptr, nullptr, ctx->d_status, ctx->d_status + active_tiles((uint32_t)total) + 1};
-        active_launch(ctx, ctx->d_prim, aa, s);
+        ensure_scratch(ctx, flag_bytes(total) / 4u);
+        const BlockGrid grid = make_block_grid(nb);
+        ActiveArgs aa{grid,    nullptr, d_active,      nullptr, (uint32_t)total,
+                      nullptr, nullptr, ctx->d_status, ctx->d_status + active_tiles((uint32_t)total) + 1};
+        query_flags_launch(ctx, ctx->d_prim, iso, 0, 0, d_ranges, grid, (uint32_t)total, ctx->d_scratch, s);
+        active_words_launch(ctx, ctx->d_prim, aa, ctx->d_scratch, s);
         return BCMC_OK;
     });
 }

@@ -53,7 +53,6 @@ struct QueryState {
     // dynamic tile counters (zeroed by the init kernel)
     uint32_t tiles_active;
     uint32_t tiles_slots;
-    uint32_t tiles_mc;
     uint32_t tiles_sort[4];
     uint32_t tiles_sort_hist;
     // radix sort plan (sort_plan, run by the last CTA of k_sort_hist or of
@@ -69,9 +68,8 @@ struct QueryState {
     // test hook (bcmc_debug_drop_tile): 0, or t + 1 when tile t of the active
     // test and of the primitive scans must publish no look-back status
     uint32_t debug_drop_tile;
-    // k_mc's grid barrier (CTAs arrived) and its emit tiles' counter
+    // k_mc's grid barrier (CTAs arrived)
     uint32_t mc_arrived;
-    uint32_t tiles_emit;
     uint32_t sort_arrived;  // k_sort's grid barriers between digit passes
     // the last age sort's plan was the one-pass one (k_slots then accumulates the
     // age bins alone); kept across queries, zero when the state is created
@@ -290,6 +288,46 @@ __device__ __forceinline__ uint32_t cta_exclusive_scan(uint32_t v, uint32_t* war
     *total = warp_sums[kWarps];
     __syncthreads();
     return r;
+}
+
+// The sum over the CTAs before `rank` of the two counts each published in its
+// status words (aggregates of this epoch), to *sum_a and *sum_b in shared
+// memory, zero before (`drop`: this CTA publishes nothing, the test hook's case).
+// Every thread takes a share of the predecessors, so all
+// are read in one round trip; the wait is for the slowest of them.
+template <int kThreads>
+__device__ __forceinline__ void cta_prefix_sums(uint64_t* status_a, uint64_t* status_b, uint32_t rank, uint32_t a,
+                                                uint32_t b, uint32_t epoch, uint32_t* err, uint32_t site_a,
+                                                uint32_t site_b, uint32_t* sum_a, uint32_t* sum_b, bool drop = false)
+{
+    if (threadIdx.x == 0 && !drop) {
+        lb_store(status_a + rank, lb_pack(epoch, kFlagAggregate, a));
+        lb_store(status_b + rank, lb_pack(epoch, kFlagAggregate, b));
+    }
+    uint32_t sa = 0, sb = 0;
+    for (uint32_t p = threadIdx.x; p < rank; p += kThreads) {
+        uint64_t va, vb;
+        uint32_t spins = 0;
+        for (;;) {
+            va = lb_load(status_a + p);
+            vb = lb_load(status_b + p);
+            const bool ra = (uint32_t)(va >> 34) == epoch, rb = (uint32_t)(vb >> 34) == epoch;
+            if (ra && rb) break;
+            if (++spins > kSpinLimit) {
+                atomicCAS(err, 0u, ra ? site_b : site_a);
+                break;
+            }
+            if (spins > 8) __nanosleep(100);
+        }
+        sa += (uint32_t)va;
+        sb += (uint32_t)vb;
+    }
+    sa = __reduce_add_sync(0xffffffffu, sa);
+    sb = __reduce_add_sync(0xffffffffu, sb);
+    if ((threadIdx.x & 31u) == 0u) {
+        if (sa) atomicAdd(sum_a, sa);
+        if (sb) atomicAdd(sum_b, sb);
+    }
 }
 
 // The radix sort's pass plan, made by the last of the CTAs that accumulated

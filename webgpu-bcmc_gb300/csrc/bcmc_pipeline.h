@@ -6,11 +6,20 @@
 
 namespace bcmc {
 
+// k_query_flags: every block's range tested against the isovalue, in words of
+// 32 consecutive blocks
+struct FlagArgs {
+    const float2* ranges;
+    BlockGrid grid;  // id -> (x, y, z) without integer division
+    uint32_t total;  // blocks
+    uint32_t wpw;    // words a warp takes at a time
+    uint4* near;     // per word: A, B and A & B ORed with the x neighbours', and A
+    uint32_t* hi;    // per word: B
+};
+
 struct ActiveArgs {
-    const float2* ranges;     // set: test ranges against the isovalue (MC path)
-    uint3 nb;                 // blocks per axis
-    BlockGrid grid;           // id -> (x, y, z) without integer division
-    const uint32_t* item_needed;  // set instead of ranges: standalone LRU update
+    BlockGrid grid;
+    const uint32_t* item_needed;  // standalone LRU update: the items needed (k_active)
     uint32_t* active_out;     // per-block active flags (MC path)
     const int32_t* item_slots;  // cachedItemSlots
     uint32_t total;           // blocks / items
@@ -18,6 +27,10 @@ struct ActiveArgs {
     uint32_t* new_ids;        // compacted ids that need caching
     uint64_t* status_a;
     uint64_t* status_n;
+    // MC path: k_query_flags' words, and room for each word's active and needed bits
+    const uint4* near = nullptr;
+    const uint32_t* hi = nullptr;
+    uint2* words = nullptr;
 };
 
 struct SlotArgs {
@@ -89,7 +102,15 @@ struct McArgs {
 };
 
 void query_begin_launch(QueryState* q, float iso, int mc_only, uint32_t capacity, uint32_t vert_capacity,
-                        cudaStream_t s, const QueryInputs* in = nullptr);
+                        cudaStream_t s);
+// Bytes of the word buffers of a volume of `total` blocks.
+size_t flag_bytes(uint64_t total);
+// Starts a query and makes its words; `in` set: the inputs come from there.
+void query_flags_launch(bcmc_ctx* ctx, QueryState* q, float iso, uint32_t capacity, uint32_t vert_capacity,
+                        const float* ranges, const BlockGrid& grid, uint32_t total, void* words, cudaStream_t s,
+                        const QueryInputs* in = nullptr);
+// The active test on the words.
+void active_words_launch(bcmc_ctx* ctx, QueryState* q, ActiveArgs a, void* words, cudaStream_t s);
 void query_end_launch(const QueryState* q, QueryState* host, cudaStream_t s);
 void active_launch(bcmc_ctx* ctx, QueryState* q, const ActiveArgs& a, cudaStream_t s);
 void slots_launch(bcmc_ctx* ctx, QueryState* q, const SlotArgs& a, uint32_t max_slots, cudaStream_t s);

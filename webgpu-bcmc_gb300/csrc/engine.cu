@@ -79,10 +79,9 @@ struct EngState {
     uint32_t nq, ntiles, entry_capacity, use_epoch;
     unsigned long long vert_capacity, vert_base;
     // device-side
-    uint32_t epoch, tiles_active, tiles_mc, num_entries;
+    uint32_t epoch, tiles_active, num_entries, with_verts;  // with_verts: entries with vertices
     uint32_t num_decode, pool_exhausted, entry_overflow, vert_overflow;
     uint32_t error, mc_arrived;  // mc_arrived: k_bmc's grid barrier
-    uint32_t tiles_emit, with_verts;  // k_bmc's emit tiles claimed, entries with vertices
     unsigned long long num_verts;  // this sequence's vertices (64-bit, from the per-query totals)
 };
 
@@ -171,7 +170,7 @@ __global__ void k_bbegin(EngState* st, uint32_t* q_nverts, uint32_t* q_nactive, 
 {
     if (threadIdx.x == 0) {
         st->epoch += 1;
-        st->tiles_active = st->tiles_mc = st->mc_arrived = st->tiles_emit = st->with_verts = 0;
+        st->tiles_active = st->mc_arrived = st->with_verts = 0;
         st->num_entries = st->num_decode = 0;
         st->pool_exhausted = st->entry_overflow = st->vert_overflow = 0;
         st->error = 0;

@@ -375,43 +375,4 @@ __device__ __forceinline__ void mc_emit(const McLane& m, const McTables& tab, Mc
     __syncwarp();  // the next grids and lists overwrite these
 }
 
-// The sum over the CTAs before `rank` of the two counts each published in its
-// status words (aggregates of this epoch), to *sum_a and *sum_b in shared
-// memory, zero before.  Every thread takes a share of the predecessors, so all
-// are read in one round trip; the wait is for the slowest of them.
-template <int kThreads>
-__device__ __forceinline__ void cta_prefix_sums(uint64_t* status_a, uint64_t* status_b, uint32_t rank, uint32_t a,
-                                                uint32_t b, uint32_t epoch, uint32_t* err, uint32_t site_a,
-                                                uint32_t site_b, uint32_t* sum_a, uint32_t* sum_b)
-{
-    if (threadIdx.x == 0) {
-        lb_store(status_a + rank, lb_pack(epoch, kFlagAggregate, a));
-        lb_store(status_b + rank, lb_pack(epoch, kFlagAggregate, b));
-    }
-    uint32_t sa = 0, sb = 0;
-    for (uint32_t p = threadIdx.x; p < rank; p += kThreads) {
-        uint64_t va, vb;
-        uint32_t spins = 0;
-        for (;;) {
-            va = lb_load(status_a + p);
-            vb = lb_load(status_b + p);
-            const bool ra = (uint32_t)(va >> 34) == epoch, rb = (uint32_t)(vb >> 34) == epoch;
-            if (ra && rb) break;
-            if (++spins > kSpinLimit) {
-                atomicCAS(err, 0u, ra ? site_b : site_a);
-                break;
-            }
-            if (spins > 8) __nanosleep(100);
-        }
-        sa += (uint32_t)va;
-        sb += (uint32_t)vb;
-    }
-    sa = __reduce_add_sync(kFull, sa);
-    sb = __reduce_add_sync(kFull, sb);
-    if ((threadIdx.x & 31u) == 0u) {
-        if (sa) atomicAdd(sum_a, sa);
-        if (sb) atomicAdd(sum_b, sb);
-    }
-}
-
 }  // namespace bcmc

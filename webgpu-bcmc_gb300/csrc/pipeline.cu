@@ -36,30 +36,23 @@
 
 namespace bcmc {
 
-// Starts a query: inputs come from the arguments, or, when `in` is set, from
-// the host's pinned copy, read directly (a query graph reuses the pointer and
-// needs no copy node for its inputs).
-__global__ void k_query_begin(QueryState* q, float iso, int mc_only, uint32_t capacity, uint32_t vert_capacity,
-                              const QueryInputs* in)
+// Starts a query's state: counters cleared, a new look-back epoch.  All threads
+// of one CTA call it.
+__device__ __forceinline__ void query_begin(QueryState* q, float iso, bool mc_only, uint32_t capacity,
+                                            uint32_t vert_capacity, uint32_t drop_tile)
 {
     const int t = threadIdx.x;
-    if (in) {
-        iso = __ldcv(&in->isovalue);
-        mc_only = (int)__ldcv(&in->mc_only);
-        capacity = __ldcv(&in->capacity);
-        vert_capacity = __ldcv(&in->vert_capacity);
-    }
     if (t == 0) {
         q->epoch += 1;
         q->capacity = capacity;
         q->vert_capacity = vert_capacity;
-        q->tiles_mc = q->mc_arrived = q->tiles_emit = 0;
+        q->mc_arrived = 0;
         q->error = 0;
         q->vert_overflow = 0;
         q->num_with_verts = 0;
         q->num_verts = 0;
         if (!mc_only) {
-            q->debug_drop_tile = in ? __ldcv(&in->debug_drop_tile) : 0u;
+            q->debug_drop_tile = drop_tile;
             q->isovalue = iso;
             q->tiles_active = q->tiles_slots = q->tiles_sort_hist = 0;
             for (int i = 0; i < 4; ++i) q->tiles_sort[i] = 0;
@@ -75,6 +68,112 @@ __global__ void k_query_begin(QueryState* q, float iso, int mc_only, uint32_t ca
     }
     if (!mc_only)
         for (int i = t; i < 1536; i += blockDim.x) (&q->sort_hist[0][0])[i] = 0;  // and sort_hist16
+}
+
+__global__ void k_query_begin(QueryState* q, float iso, int mc_only, uint32_t capacity, uint32_t vert_capacity)
+{
+    query_begin(q, iso, mc_only != 0, capacity, vert_capacity, 0u);
+}
+
+// ---------------------------------------------------------------------------
+// k_query_flags: starts a query, and tests every block's range against the
+// isovalue: bit A of a block is iso >= lo, bit B iso <= hi.  The bits go out in
+// words of 32 consecutive blocks, together with A, B and A & B ORed with those
+// of the x neighbours (first step of the active test's 3x3x3 neighbourhood).
+//
+// Every range is read once, 8 bytes to a lane, and a ballot makes the words; a
+// warp takes `wpw` of them, and its lanes then do the x neighbours of a word
+// each.  k_active, which follows, works on these words: 0.6 bytes a block
+// where the ranges are 8.  Before, its tiles read the ranges of all three
+// z-layers around them and tested 27 flag bytes a block, a tile at a time per
+// CTA with a look-back between tiles: 565 us of the 1024 x 1024 x 1080 volume's
+// query, for ranges that take 21 us to read.
+// The inputs come from the arguments, or, when `in` is set, from the host's
+// pinned copy, read directly (a query graph needs no copy node for them).
+// ---------------------------------------------------------------------------
+constexpr int kFlagThreads = 256;
+constexpr uint32_t kFlagBatch = 8;  // ranges in flight per lane
+
+__global__ void __launch_bounds__(kFlagThreads) k_query_flags(QueryState* q, float iso, uint32_t capacity,
+                                                             uint32_t vert_capacity, const QueryInputs* in, FlagArgs a)
+{
+    const uint32_t lane = threadIdx.x & 31u, total = a.total, nx = a.grid.nb.x, wpw = a.wpw;
+    const uint32_t nwords = div_up(total, 32u);
+    const uint32_t step = gridDim.x * (kFlagThreads / 32) * wpw;
+    uint32_t w0 = (blockIdx.x * (kFlagThreads / 32) + (threadIdx.x >> 5)) * wpw;
+    const auto load = [&](int64_t b) {
+        return b >= 0 && b < (int64_t)total ? __ldg(a.ranges + b) : make_float2(NAN, NAN);  // NaN: no flags
+    };
+    // ranges of a batch of words (none past the warp's last)
+    const auto load_batch = [&](uint32_t w, uint32_t i, float2 r[kFlagBatch]) {
+#pragma unroll
+        for (uint32_t u = 0; u < kFlagBatch; ++u)
+            r[u] = i + u < wpw ? load((int64_t)w * 32 + 32 * (i + u) + lane) : make_float2(NAN, NAN);
+    };
+    // of the blocks before the warp's first word and after its last
+    const auto load_ends = [&](uint32_t w) {
+        const int64_t b0 = (int64_t)w * 32;
+        return lane == 0 ? load(b0 - 1) : lane == wpw - 1u ? load(b0 + 32 * wpw) : make_float2(NAN, NAN);
+    };
+    float2 r[kFlagBatch], e;
+    load_batch(w0, 0, r);  // on their way while the isovalue is
+    e = load_ends(w0);
+    if (in) {  // one read of host memory per CTA
+        __shared__ float s_iso;
+        if (threadIdx.x == 0) s_iso = __ldcv(&in->isovalue);
+        __syncthreads();
+        iso = s_iso;
+    }
+    if (blockIdx.x == 0) {
+        uint32_t drop = 0;
+        if (in) {
+            capacity = __ldcv(&in->capacity);
+            vert_capacity = __ldcv(&in->vert_capacity);
+            drop = __ldcv(&in->debug_drop_tile);
+        }
+        query_begin(q, iso, false, capacity, vert_capacity, drop);
+    }
+    for (; w0 < nwords; w0 += step) {
+        uint32_t A = 0, B = 0;
+        for (uint32_t i = 0; i < wpw; i += kFlagBatch) {
+            if (i) load_batch(w0, i, r);
+#pragma unroll
+            for (uint32_t u = 0; u < kFlagBatch; ++u) {
+                const uint32_t wa = __ballot_sync(0xffffffffu, iso >= r[u].x),
+                               wb = __ballot_sync(0xffffffffu, iso <= r[u].y);
+                if (lane == i + u) {
+                    A = wa;
+                    B = wb;
+                }
+            }
+        }
+        // the word's blocks at x = 0 and x = nx - 1, which have no neighbour there
+        const uint32_t first = (w0 + lane) * 32u, x0 = first - fdiv(first, a.grid.dx) * nx;
+        uint32_t no_left = 0, no_right = 0;
+        for (uint32_t p = x0 ? nx - x0 : 0u; p < 32u; p += nx) no_left |= 1u << p;
+        for (uint32_t p = nx - 1u - x0; p < 32u; p += nx) no_right |= 1u << p;
+        uint32_t pa = __shfl_up_sync(0xffffffffu, A, 1) >> 31, pb = __shfl_up_sync(0xffffffffu, B, 1) >> 31;
+        uint32_t na = __shfl_down_sync(0xffffffffu, A, 1) & 1u, nb = __shfl_down_sync(0xffffffffu, B, 1) & 1u;
+        if (lane == 0) {
+            pa = iso >= e.x;
+            pb = iso <= e.y;
+        }
+        if (lane == wpw - 1u) {
+            na = iso >= e.x;
+            nb = iso <= e.y;
+        }
+        const auto spread = [&](uint32_t v, uint32_t prev, uint32_t next) {
+            return v | (((v << 1) | prev) & ~no_left) | (((v >> 1) | (next << 31)) & ~no_right);
+        };
+        if (lane < wpw && w0 + lane < nwords) {
+            a.near[w0 + lane] = make_uint4(spread(A, pa, na), spread(B, pb, nb), spread(A & B, pa & pb, na & nb), A);
+            a.hi[w0 + lane] = B;
+        }
+        if (w0 + step < nwords) {
+            load_batch(w0 + step, 0, r);
+            e = load_ends(w0 + step);
+        }
+    }
 }
 
 // Ends a query graph: the query state the host reads (the fields before the
@@ -135,140 +234,158 @@ __device__ __forceinline__ void active_finish(QueryState* q, uint32_t A, uint32_
     }
 }
 
-// k_active over the block ranges (the MC path), 4 consecutive blocks per
-// thread, 1024 threads per tile.  The tile's ranges and all their 3x3x3 neighbours are
-// staged once in shared memory as 2-bit flags (bit 0: iso >= lo, bit 1:
-// iso <= hi): for each z-offset dz in {-1, 0, 1}, the window of block ids
-// [B0 + dz*NX*NY - NX - 1, B0 + 2048 + dz*NX*NY + NX + 1) around the tile's
-// blocks [B0, B0 + 2048) (stage_len = 2048 + 2*NX + 2 entries each).
-// Neighbour (dx, dy, dz) of local block l sits at
-// (dz+1)*stage_len + l + (dy+1)*NX + dx + 1.  Staging turns 27 dependent
-// global loads per block into one round of independent loads per tile.
-// 2048-block tiles (128 CTAs on the 256^3 volume) measured 1.5 us faster per
-// query than 4096-block ones (64 CTAs), which kept the look-back to one
-// window there but left most SMs idle.
-constexpr int kActRThreads = 512;
-constexpr int kActRItems = 4;                          // consecutive blocks per thread
-constexpr int kActRTile = kActRThreads * kActRItems;  // blocks per tile
-constexpr int kActRStage = 5;  // staged ranges per thread and window in one round (5 * 512 >= 2048 + 2*NX + 2 for NX <= 255)
+// k_active_words: the active test of the MC path (compute_block_active.comp:24-61)
+// on k_query_flags' words, with the compaction of the active ids and of the ids
+// that no slot holds.  With A = iso >= lo and B = iso <= hi of a block, the
+// reference's test over a block's 26 neighbours is (see block_is_active)
+//   active = (A && anyB) || (B && anyA) || any(A_n && B_n),
+// any over the 3x3x3 neighbourhood.  The words hold the ORs along x, so a lane
+// ORs the nine (y, z) neighbour rows of its word, each two words and a funnel
+// shift, with masks for the blocks that have no such row.
+// A CTA owns one contiguous range of words: it tests them, keeping the results
+// in shared memory, publishes its two totals, adds up those of the CTAs before
+// it in one round trip (cooperative launch: all are resident), and writes its
+// ids.  The last CTA with words decides the cache growth.
+constexpr int kWordThreads = 256;
+constexpr int kWordPerSm = 5;
+constexpr uint32_t kWordRange = 2048;  // words whose results fit in shared memory; longer ranges keep them in global memory
 
-__global__ void __launch_bounds__(kActRThreads, 1) k_active_ranges(QueryState* q, ActiveArgs a, uint32_t stage_len)
+__global__ void __launch_bounds__(kWordThreads, kWordPerSm) k_active_words(QueryState* q, ActiveArgs a, uint32_t wpw,
+                                                                          uint32_t range)
 {
-    __shared__ uint32_t s_warp[kActRThreads / 32 + 1];
-    __shared__ uint32_t s_tile, s_pa, s_pn;
-    extern __shared__ uint8_t s_bits[];  // 3 * stage_len flag bytes
-    const uint32_t total = a.total;
-    const uint32_t ntiles = div_up(total, kActRTile);
+    __shared__ uint2 s_words[kWordRange];
+    __shared__ uint32_t s_warp[kWordThreads / 32 + 1];
+    __shared__ uint32_t s_at[kWordThreads];
+    __shared__ uint32_t s_sum_a, s_sum_n, s_pa, s_pn;
+    constexpr uint32_t kWarps = kWordThreads / 32;
+    const uint32_t total = a.total, nwords = div_up(total, 32u), rank = blockIdx.x;
+    const uint32_t first = rank * range, end = min(nwords, first + range);
+    if (first >= nwords) return;
     const uint32_t epoch = q->epoch;
-    const float iso = q->isovalue;
     const uint3 nb = a.grid.nb;
-    const uint32_t nx = nb.x, nxy = nb.x * nb.y;
-    const uint32_t t = threadIdx.x;
-    for (;;) {
-        if (t == 0) s_tile = atomicAdd(&q->tiles_active, 1u);
-        __syncthreads();
-        const uint32_t tile = s_tile;
-        if (tile >= ntiles) break;
-        // all of a thread's loads first (up to kActRStage per window, in
-        // flight together), then the flags
-        for (uint32_t i0 = 0; i0 < stage_len; i0 += kActRStage * kActRThreads) {
-            float2 r[3][kActRStage];
-#pragma unroll
-            for (int dz = 0; dz < 3; ++dz) {
-                const int64_t start = (int64_t)tile * kActRTile + (int64_t)(dz - 1) * nxy - nx - 1;
-#pragma unroll
-                for (int k = 0; k < kActRStage; ++k) {
-                    const uint32_t i = i0 + k * kActRThreads + t;
-                    const int64_t id = start + i;
-                    r[dz][k] = (i < stage_len && id >= 0 && id < (int64_t)total) ? __ldg(a.ranges + id)
-                                                                                 : make_float2(NAN, NAN);
+    const int32_t nx = (int32_t)nb.x;
+    const int64_t nxy = (int64_t)nb.x * nb.y;
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, below = (1u << lane) - 1u;
+    uint2* words = range <= kWordRange ? s_words : a.words + first;  // active and needed bits
+    if (t == 0) s_sum_a = s_sum_n = s_pa = s_pn = 0;
+    __syncthreads();
+    uint32_t na = 0, nn = 0;  // the lane's words' counts
+    for (uint32_t w0 = first + warp * wpw; w0 < end; w0 += kWarps * wpw) {
+        const uint32_t w = w0 + lane, b0 = 32u * w;
+        uint32_t act = 0;
+        if (lane < wpw && w < end) {
+            // the blocks with a row before and after them in y and in z
+            uint32_t ym = 0, yp = 0, zm = 0, zp = 0;
+            uint3 c = block_coords(b0, a.grid);
+            for (uint32_t p = 0; p < 32u;) {  // the pieces of rows in the word
+                const uint32_t len = min(nb.x - c.x, 32u - p);
+                const uint32_t m = (0xffffffffu >> (32u - len)) << p;
+                ym |= c.y > 0u ? m : 0u;
+                yp |= c.y + 1u < nb.y ? m : 0u;
+                zm |= c.z > 0u ? m : 0u;
+                zp |= c.z + 1u < nb.z ? m : 0u;
+                p += len;
+                c.x = 0;
+                if (++c.y == nb.y) {
+                    c.y = 0;
+                    ++c.z;
                 }
             }
+            uint32_t any_a = 0, any_b = 0, any_c = 0;
 #pragma unroll
-            for (int dz = 0; dz < 3; ++dz)
+            for (int dz = -1; dz < 2; ++dz)
 #pragma unroll
-                for (int k = 0; k < kActRStage; ++k) {
-                    const uint32_t i = i0 + k * kActRThreads + t;
-                    if (i < stage_len) {
-                        uint32_t ra, rb;
-                        range_bits(r[dz][k], iso, ra, rb);  // NaN (outside the volume): no flags
-                        s_bits[(uint32_t)dz * stage_len + i] = (uint8_t)(ra | (rb << 1));
+                for (int dy = -1; dy < 2; ++dy) {
+                    const uint32_t m = (dz < 0 ? zm : dz > 0 ? zp : 0xffffffffu) & (dy < 0 ? ym : dy > 0 ? yp : 0xffffffffu);
+                    // the row's first block; a word out of the volume holds no block that the masks leave
+                    const int64_t s = (int64_t)b0 + dz * nxy + dy * nx;
+                    const int64_t k = s >> 5;
+                    const uint32_t sh = (uint32_t)s & 31u;
+                    const uint4 lo = __ldg(a.near + min(max(k, (int64_t)0), (int64_t)nwords - 1)),
+                                hi = __ldg(a.near + min(max(k + 1, (int64_t)0), (int64_t)nwords - 1));
+                    any_a |= __funnelshift_r(lo.x, hi.x, sh) & m;
+                    any_b |= __funnelshift_r(lo.y, hi.y, sh) & m;
+                    any_c |= __funnelshift_r(lo.z, hi.z, sh) & m;
+                }
+            act = (a.near[w].w & any_b) | (a.hi[w] & any_a) | any_c;
+            if (total - b0 < 32u) act &= (1u << (total - b0)) - 1u;
+        }
+        // the flags out, and which active blocks no slot holds: four words at a
+        // time, four blocks to a lane
+        uint32_t need = 0;
+        const uint32_t n = min(wpw, end - w0);
+#pragma unroll 2
+        for (uint32_t i = 0; i < n; i += 4u) {
+            const uint32_t on = __shfl_sync(0xffffffffu, act, i + (lane >> 3)) >> (4u * (lane & 7u)) & 15u;
+            const uint32_t b = 32u * (w0 + i) + 4u * lane;
+            uint32_t no_slot = 0;
+            if (i + (lane >> 3) < n) {
+                if (b + 4u <= total) {
+                    *reinterpret_cast<uint4*>(a.active_out + b) =
+                        make_uint4(on & 1u, on >> 1 & 1u, on >> 2 & 1u, on >> 3);
+                    if (on && a.item_slots) {
+                        const int4 s4 = __ldg(reinterpret_cast<const int4*>(a.item_slots + b));
+                        no_slot = on & ((s4.x < 0 ? 1u : 0u) | (s4.y < 0 ? 2u : 0u) | (s4.z < 0 ? 4u : 0u) |
+                                        (s4.w < 0 ? 8u : 0u));
+                    }
+                } else {
+                    for (uint32_t k = 0; b + k < total; ++k) {
+                        a.active_out[b + k] = on >> k & 1u;
+                        if ((on >> k & 1u) && a.item_slots && a.item_slots[b + k] < 0) no_slot |= 1u << k;
                     }
                 }
-        }
-        __syncthreads();
-        const uint32_t l0 = kActRItems * t, b0 = tile * kActRTile + l0;
-        uint32_t act = 0, need = 0;  // bit j = block b0 + j
-#pragma unroll
-        for (int j = 0; j < kActRItems; ++j) {
-            const uint32_t b = b0 + j, l = l0 + j;
-            if (b >= total) break;
-            const uint3 c = block_coords(b, a.grid);
-            // valid neighbour offsets per axis: bit (d + 1) for d in {-1, 0, 1}
-            const uint32_t mx = (c.x > 0 ? 1u : 0u) | 2u | (c.x + 1 < nb.x ? 4u : 0u);
-            const uint32_t my = (c.y > 0 ? 1u : 0u) | 2u | (c.y + 1 < nb.y ? 4u : 0u);
-            const uint32_t mz = (c.z > 0 ? 1u : 0u) | 2u | (c.z + 1 < nb.z ? 4u : 0u);
-            const uint32_t self = s_bits[stage_len + l + nx + 1];
-            uint32_t orv = 0, anyc = 0;
-#pragma unroll
-            for (int dz = 0; dz < 3; ++dz)
-#pragma unroll
-                for (int dy = 0; dy < 3; ++dy) {
-                    if (!((mz >> dz) & (my >> dy) & 1u)) continue;
-                    const uint8_t* row = s_bits + (uint32_t)dz * stage_len + l + (uint32_t)dy * nx;
-#pragma unroll
-                    for (int dx = 0; dx < 3; ++dx) {
-                        const uint32_t v = (mx >> dx) & 1u ? (uint32_t)row[dx] : 0u;
-                        orv |= v;
-                        anyc |= (v + 1u) >> 2;  // 1 when both flags are set
-                    }
-                }
-            // compute_block_active.comp:24-61 (see block_is_active)
-            act |= (((self & (orv >> 1)) | ((self >> 1) & orv) | anyc) & 1u) << j;
-        }
-        if (kActRItems == 4 && b0 + kActRItems <= total) {
-            *reinterpret_cast<uint4*>(a.active_out + b0) =
-                make_uint4(act & 1u, (act >> 1) & 1u, (act >> 2) & 1u, (act >> 3) & 1u);
-            if (act && a.item_slots) {
-                const int4 s4 = __ldg(reinterpret_cast<const int4*>(a.item_slots + b0));
-                need = ((s4.x < 0 ? 1u : 0u) | (s4.y < 0 ? 2u : 0u) | (s4.z < 0 ? 4u : 0u) | (s4.w < 0 ? 8u : 0u)) & act;
             }
-        } else {
-            for (uint32_t j = 0; j < (uint32_t)kActRItems && b0 + j < total; ++j) {
-                a.active_out[b0 + j] = (act >> j) & 1u;
-                if ((act >> j & 1u) && a.item_slots && a.item_slots[b0 + j] < 0) need |= 1u << j;
-            }
+            uint32_t word = no_slot << (4u * (lane & 7u));
+            word |= __shfl_xor_sync(0xffffffffu, word, 1);
+            word |= __shfl_xor_sync(0xffffffffu, word, 2);
+            word |= __shfl_xor_sync(0xffffffffu, word, 4);
+            word = __shfl_sync(0xffffffffu, word, 8u * (lane - i));  // lanes i .. i + 3: their word
+            if (lane - i < 4u) need = word;
         }
+        if (lane < n) {
+            words[w - first] = make_uint2(act, need);
+            na += __popc(act);
+            nn += __popc(need);
+        }
+    }
+    na = __reduce_add_sync(0xffffffffu, na);
+    nn = __reduce_add_sync(0xffffffffu, nn);
+    if (lane == 0 && na) {
+        atomicAdd(&s_sum_a, na);
+        if (nn) atomicAdd(&s_sum_n, nn);
+    }
+    __syncthreads();
+    cta_prefix_sums<kWordThreads>(a.status_a, a.status_n, rank, s_sum_a, s_sum_n, epoch, &q->error, 30u, 31u, &s_pa,
+                                  &s_pn, lb_dropped(q, rank));
+    __syncthreads();
+    uint32_t pa = s_pa, pn = s_pn;
+    if (end == nwords && t == 0) active_finish(q, pa + s_sum_a, pn + s_sum_n, total);
+    if (!a.active_ids) return;
+    for (uint32_t c0 = 0; c0 < end - first; c0 += kWordThreads) {
+        const uint32_t i = c0 + t;
+        const uint2 mine = i < end - first ? words[i] : make_uint2(0u, 0u);
         uint32_t tot;
-        const uint32_t excl =
-            cta_exclusive_scan<kActRThreads>((uint32_t)__popc(act) | ((uint32_t)__popc(need) << 16), s_warp, &tot);
-        if (t < 32) {
-            const uint32_t p =
-                lb_dropped(q, tile) ? 0u : warp_lookback(a.status_a, tile, tot & 0xffffu, epoch, &q->error, 30u);
-            if (t == 0) s_pa = p;
-        } else if (t < 64) {
-            const uint32_t p =
-                lb_dropped(q, tile) ? 0u : warp_lookback(a.status_n, tile, tot >> 16, epoch, &q->error, 31u);
-            if (t == 32) s_pn = p;
+        const uint32_t ex = cta_exclusive_scan<kWordThreads>((uint32_t)__popc(mine.x) | ((uint32_t)__popc(mine.y) << 16),
+                                                             s_warp, &tot);
+        s_at[t] = ex;
+        __syncthreads();
+        // a word at a time, so that the ids go out together
+        const uint32_t n = min((uint32_t)kWordThreads, end - first - c0);
+        for (uint32_t k = warp; k < n; k += kWarps) {
+            const uint2 wd = words[c0 + k];
+            if (!wd.x) continue;
+            const uint32_t at = s_at[k], b = 32u * (first + c0 + k) + lane;
+            if (wd.x >> lane & 1u) a.active_ids[pa + (at & 0xffffu) + __popc(wd.x & below)] = b;
+            if (wd.y >> lane & 1u) a.new_ids[pn + (at >> 16) + __popc(wd.y & below)] = b;
         }
         __syncthreads();
-        uint32_t pa = s_pa + (excl & 0xffffu), pn = s_pn + (excl >> 16);
-#pragma unroll
-        for (int j = 0; j < kActRItems; ++j) {
-            if (act >> j & 1u) {
-                if (a.active_ids) a.active_ids[pa] = b0 + j;
-                ++pa;
-            }
-            if (need >> j & 1u) {
-                if (a.new_ids) a.new_ids[pn] = b0 + j;
-                ++pn;
-            }
-        }
-        if (tile == ntiles - 1 && t == 0) active_finish(q, s_pa + (tot & 0xffffu), s_pn + (tot >> 16), total);
-        __syncthreads();
+        pa += tot & 0xffffu;
+        pn += tot >> 16;
     }
 }
 
+// k_active: the standalone LRU update's side of the same: the items that are
+// needed, and of those the ones no slot holds, compacted.
 __global__ void __launch_bounds__(kActThreads) k_active(QueryState* q, ActiveArgs a)
 {
     __shared__ uint32_t s_warp[kActThreads / 32 + 1];
@@ -276,33 +393,18 @@ __global__ void __launch_bounds__(kActThreads) k_active(QueryState* q, ActiveArg
     const uint32_t total = a.total;
     const uint32_t ntiles = div_up(total, kActiveTile);
     const uint32_t epoch = q->epoch;
-    const float iso = q->isovalue;
     for (;;) {
         if (threadIdx.x == 0) s_tile = atomicAdd(&q->tiles_active, 1u);
         __syncthreads();
         const uint32_t tile = s_tile;
         if (tile >= ntiles) break;
-        // thread -> 4 consecutive blocks (thread-blocked order = block order)
+        // thread -> 4 consecutive items (thread-blocked order = item order)
         const uint32_t b0 = tile * kActiveTile + kActiveItems * threadIdx.x;
-        uint32_t act = 0, need = 0;  // bit i = block b0 + i
+        uint32_t act = 0, need = 0;  // bit i = item b0 + i
         if (b0 < total) {
             const uint32_t n = min(4u, total - b0);
-            if (a.ranges) {
-                const uint3 c = block_coords(b0, a.grid);
-                if (n == 4 && c.x + 3 < a.grid.nb.x) {
-                    act = row4_active(a.ranges, a.grid, c, b0, iso);
-                } else {
-                    for (uint32_t i = 0; i < n; ++i) act |= block_is_active(a.ranges, a.grid, b0 + i, iso) << i;
-                }
-                if (n == 4)
-                    *reinterpret_cast<uint4*>(a.active_out + b0) =
-                        make_uint4(act & 1u, (act >> 1) & 1u, (act >> 2) & 1u, (act >> 3) & 1u);
-                else
-                    for (uint32_t i = 0; i < n; ++i) a.active_out[b0 + i] = (act >> i) & 1u;
-            } else {
-                for (uint32_t i = 0; i < n; ++i) act |= (a.item_needed[b0 + i] != 0u ? 1u : 0u) << i;
-            }
-            if (a.item_slots && act) {
+            for (uint32_t i = 0; i < n; ++i) act |= (a.item_needed[b0 + i] != 0u ? 1u : 0u) << i;
+            if (act) {
                 if (n == 4) {
                     const int4 s4 = __ldg(reinterpret_cast<const int4*>(a.item_slots + b0));
                     need = (s4.x < 0 ? 1u : 0u) | (s4.y < 0 ? 2u : 0u) | (s4.z < 0 ? 4u : 0u) | (s4.w < 0 ? 8u : 0u);
@@ -325,18 +427,10 @@ __global__ void __launch_bounds__(kActThreads) k_active(QueryState* q, ActiveArg
             if (threadIdx.x == 32) s_pn = p;
         }
         __syncthreads();
-        uint32_t pa = s_pa + (excl & 0xffffu), pn = s_pn + (excl >> 16);
+        uint32_t pn = s_pn + (excl >> 16);
 #pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-            if (act >> i & 1u) {
-                if (a.active_ids) a.active_ids[pa] = b0 + i;
-                ++pa;
-            }
-            if (need >> i & 1u) {
-                if (a.new_ids) a.new_ids[pn] = b0 + i;
-                ++pn;
-            }
-        }
+        for (uint32_t i = 0; i < 4; ++i)
+            if (need >> i & 1u) a.new_ids[pn++] = b0 + i;
         if (tile == ntiles - 1 && threadIdx.x == 0) active_finish(q, s_pa + (tot & 0xffffu), s_pn + (tot >> 16), total);
         __syncthreads();
     }
@@ -771,16 +865,18 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     if (fits)
         for (uint32_t b0 = start; b0 < end; b0 += kMcThreads) {
             const uint32_t i = b0 + t;
-            const uint32_t c = i < end ? a.block_counts[i] : 0u;  // <= 64 cells x 15 vertices
+            const uint32_t c = i < end ? a.block_counts[i] : 0u;
+            // <= 512 blocks x 64 cells x 15 vertices < 2^20, and the blocks above them
+            static_assert(kMcThreads * 64 * 15 < 1 << 20 && kMcThreads < 1 << 12, "fields of the scan");
             uint32_t tot;
-            const uint32_t ex = cta_exclusive_scan<kMcThreads>(c | (c ? 1u << 18 : 0u), s_warp, &tot);
+            const uint32_t ex = cta_exclusive_scan<kMcThreads>(c | (c ? 1u << 20 : 0u), s_warp, &tot);
             if (c) {
-                const uint32_t r = pb + (ex >> 18);
+                const uint32_t r = pb + (ex >> 20);
                 a.with_verts[r] = i;
-                a.vert_offsets[r] = pv + (ex & 0x3ffffu);
+                a.vert_offsets[r] = pv + (ex & 0xfffffu);
             }
-            pv += tot & 0x3ffffu;
-            pb += tot >> 18;
+            pv += tot & 0xfffffu;
+            pb += tot >> 20;
         }
     // grid barrier (the launch is cooperative: every CTA is resident)
     __syncthreads();
@@ -848,25 +944,72 @@ static int pgrid(bcmc_ctx* ctx, uint32_t tiles, uint32_t per_sm)
 }
 
 void query_begin_launch(QueryState* q, float iso, int mc_only, uint32_t capacity, uint32_t vert_capacity,
-                        cudaStream_t s, const QueryInputs* in)
+                        cudaStream_t s)
 {
-    k_query_begin<<<1, 256, 0, s>>>(q, iso, mc_only, capacity, vert_capacity, in);
+    k_query_begin<<<1, 256, 0, s>>>(q, iso, mc_only, capacity, vert_capacity);
     count_launches(1);
     BCMC_CUDA(cudaGetLastError());
 }
 
+size_t flag_bytes(uint64_t total) { return (size_t)((total + 31u) / 32u) * (sizeof(uint4) + sizeof(uint2) + 4u) + 16u; }
+
+// CTAs of k_active_words resident per SM: the bound of its cooperative grid
+static uint32_t word_per_sm()
+{
+    static const uint32_t n = [] {
+        int r = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, k_active_words, kWordThreads, 0) != cudaSuccess || r < 1) r = 1;
+        return (uint32_t)std::min(r, kWordPerSm);
+    }();
+    return n;
+}
+
+// Words a warp takes: enough warps for every SM first (4 words each keeps the
+// 64^3 volume's 128 words on 32 warps), then longer runs, up to a word to a lane.
+static uint32_t words_per_warp(const bcmc_ctx* ctx, uint32_t nwords, uint32_t warps_per_sm)
+{
+    const uint32_t w = div_up(nwords, (uint32_t)ctx->num_sms * warps_per_sm);
+    return w <= 4u ? 4u : (w >= 32u ? 32u : w);
+}
+
+void query_flags_launch(bcmc_ctx* ctx, QueryState* q, float iso, uint32_t capacity, uint32_t vert_capacity,
+                        const float* ranges, const BlockGrid& grid, uint32_t total, void* words, cudaStream_t s,
+                        const QueryInputs* in)
+{
+    const uint32_t nwords = div_up(total, 32u), wpw = words_per_warp(ctx, nwords, 32u);
+    uint4* near = static_cast<uint4*>(words);
+    const FlagArgs f{reinterpret_cast<const float2*>(ranges), grid, total, wpw, near,
+                     reinterpret_cast<uint32_t*>(near + nwords)};
+    k_query_flags<<<pgrid(ctx, div_up(nwords, wpw * (kFlagThreads / 32)), 8), kFlagThreads, 0, s>>>(
+        q, iso, capacity, vert_capacity, in, f);
+    count_launches(1);
+    BCMC_CUDA(cudaGetLastError());
+}
+
+void active_words_launch(bcmc_ctx* ctx, QueryState* q, ActiveArgs a, void* words, cudaStream_t s)
+{
+    const uint32_t nwords = div_up(a.total, 32u), wpw = words_per_warp(ctx, nwords, kWordPerSm * (kWordThreads / 32));
+    a.near = static_cast<const uint4*>(words);
+    a.hi = reinterpret_cast<const uint32_t*>(a.near + nwords);
+    a.words = reinterpret_cast<uint2*>(static_cast<uint4*>(words) + nwords + div_up(nwords, 4u));
+    // a range per resident CTA, of whole rounds of its warps
+    const uint32_t round = wpw * (kWordThreads / 32);
+    const uint32_t range = div_up(div_up(nwords, round), (uint32_t)ctx->num_sms * word_per_sm()) * round;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(div_up(nwords, range));
+    cfg.blockDim = dim3(kWordThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    BCMC_CUDA(cudaLaunchKernelEx(&cfg, k_active_words, q, a, wpw, range));
+    count_launches(1);
+}
+
 void active_launch(bcmc_ctx* ctx, QueryState* q, const ActiveArgs& a, cudaStream_t s)
 {
-    // the staged kernel within the 48 KB of dynamic shared memory a launch
-    // gets without opting in: 3 windows of kActRTile + 2*NX + 2 bytes
-    const uint32_t stage_len = kActRTile + 2u * a.grid.nb.x + 2u;
-    if (a.ranges && 3u * stage_len <= 48u * 1024u) {
-        k_active_ranges<<<pgrid(ctx, div_up(a.total, kActRTile), 2), kActRThreads, 3u * stage_len, s>>>(q, a,
-                                                                                                        stage_len);
-        count_launches(1);
-        BCMC_CUDA(cudaGetLastError());
-        return;
-    }
     k_active<<<pgrid(ctx, div_up(a.total, kActiveTile), 8), kActThreads, 0, s>>>(q, a);
     count_launches(1);
     BCMC_CUDA(cudaGetLastError());
