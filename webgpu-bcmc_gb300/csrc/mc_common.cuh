@@ -42,19 +42,22 @@ static __device__ const __align__(16) McTables c_mc = {mc_detail::make_tri_count
 // for the few vertices that take the exact expression: read where it lies
 static __device__ const __align__(16) mc_detail::CornerPack c_corner_pack = mc_detail::make_corner_pack();
 
-// shared memory of one warp's emit (`out`: only for stores to host memory)
+// shared memory of one warp's emit (`out`: only for stores to host memory).  Kept
+// small: what shared memory leaves of an SM's 256 KB is its L1 cache, which
+// neighbouring blocks' ghost layers are read through.
 template <bool kHost>
 struct McWarpMem {
-    float vol[kMcBlocks][128];   // the blocks' 5^3 grids
-    // cells with triangles, in order: x is where vertex 0 of the run would be in
+    // cells and triangles listed at a time (one block has up to 64 and 320)
+    static constexpr uint32_t kCells = 128, kTris = 512;
+    float vol[kMcBlocks][128];  // the blocks' 5^3 grids
+    // cells with triangles, in order: x is where vertex 0 of the list would be in
     // the cell's row of the case table (in bytes, from the table's start), y the
     // cell's position (x << 20 | y << 10 | z) and from bit 23 its corner 0 in vol
-    uint2 list[kMcBlocks * 64];
-    uint8_t flag[kMcBlocks * 320];  // 1 where a triangle is its cell's first; zero between emits
-    uint32_t slot[32];              // the lookups' slots, lane 8j + o
+    uint2 list[kCells];
+    uint8_t flag[kTris];  // 1 where a triangle is its cell's first; zero between emits
+    uint32_t slot[32];    // the lookups' slots, lane 8j + o
     uint2 out[kHost ? 64 : 2];
 };
-
 static_assert(sizeof(McWarpMem<false>) % 16 == 0 && sizeof(McWarpMem<true>) % 16 == 0, "16-byte aligned in an array");
 
 template <int kThreads, bool kHost>
@@ -247,9 +250,9 @@ struct McSink {
             flush(stage, false);
         }
     }
-    __device__ __forceinline__ void next_window()
+    __device__ __forceinline__ void next_window(uint32_t n)
     {
-        if constexpr (!kHost) at += 96;
+        if constexpr (!kHost) at += n;
     }
     __device__ __forceinline__ void flush(uint2* stage, bool all)
     {
@@ -294,36 +297,41 @@ __device__ __forceinline__ void mc_grids(const McLane& m, Mem& s, uint32_t n)
 
 // The vertices of blocks 0 .. n - 1 (mc_grids done; ids, isovalues and `has` in
 // lane 8j) to the sink, in block, cell and table order.  The cells with
-// triangles are listed first, with a flag at each one's first triangle.  Then,
-// 32 triangles at a time, a ballot of the flags tells a lane which cell its
-// vertex is of: the last that starts at or before the vertex's triangle.  A
-// lane takes one vertex at a time, so that the stores are contiguous, and works
-// its position out from the cell's coordinates: what binds this loop is the
-// shared-memory pipe, and a triangle to a lane with its vertices staged through
-// shared memory, and a table of the fixed axes' positions, took over twice the
-// accesses.  `ahead` is called once the cells are listed, to start loads for
-// what comes next.
+// triangles are listed first, with a flag at each one's first triangle, as many
+// blocks' as the list holds (in most cases all).  Then, 32 triangles at a time,
+// a ballot of the flags tells a lane which cell its vertex is of: the last that
+// starts at or before the vertex's triangle.  A lane takes one vertex at a time,
+// so that the stores are contiguous, and works its position out from the cell's
+// coordinates: what binds this loop besides the issue slots is the shared-memory
+// pipe, and a triangle to a lane with its vertices staged through shared memory,
+// and a table of the fixed axes' positions, took over twice the accesses.
+// `ahead` is called once, when the grids are there, to start loads for what
+// comes next.
 template <bool kHost, bool kOneIso, typename Ahead>
 __device__ __forceinline__ void mc_emit(const McLane& m, const McTables& tab, McWarpMem<kHost>& s, uint32_t n,
                                         uint32_t id, uint32_t has, float iso, McSink<kHost>& sink, Ahead ahead)
 {
     const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-    uint32_t tris = 0, cells = 0;
     async_wait<0>();
     __syncwarp();
-#pragma unroll
-    for (uint32_t j = 0; j < kMcBlocks; ++j)
-        if (j < n) {
+    ahead();
+    uint32_t b = 0;
+    do {
+        uint32_t tris = 0, cells = 0;
+#pragma unroll 1
+        for (; b < n; ++b) {
             float f[4];
 #pragma unroll
-            for (uint32_t r = 0; r < 4; ++r) f[r] = s.vol[j][lane + 32u * r];
+            for (uint32_t r = 0; r < 4; ++r) f[r] = s.vol[b][lane + 32u * r];
             uint32_t c0, c1;
-            mc_cases<false>(m, f, kOneIso ? iso : __shfl_sync(kFull, iso, 8u * j), __shfl_sync(kFull, has, 8u * j), c0, c1);
+            mc_cases<false>(m, f, kOneIso ? iso : __shfl_sync(kFull, iso, 8u * b), __shfl_sync(kFull, has, 8u * b), c0, c1);
             const uint32_t t0 = tab.count.n[c0], t1 = tab.count.n[c1];
             const uint32_t inc = mc_scan(t0 | (t1 << 16));
-            const uint32_t tot = __shfl_sync(kFull, inc, 31);
+            const uint32_t tot = __shfl_sync(kFull, inc, 31), sum = (tot & 0xffffu) + (tot >> 16);
             const uint32_t e0 = __ballot_sync(kFull, t0 != 0u), e1 = __ballot_sync(kFull, t1 != 0u);
-            const uint32_t where = m.cell | (j << 30);  // cell lane + 32 lies two layers up
+            const uint32_t n0 = __popc(e0), n01 = n0 + __popc(e1);
+            if (cells + n01 > s.kCells || tris + sum > s.kTris) break;
+            const uint32_t where = m.cell | (b << 30);  // cell lane + 32 lies two layers up
             if (t0) {
                 const uint32_t first = tris + (inc & 0xffffu) - t0;
                 s.list[cells + __popc(e0 & below)] = make_uint2(60u * c0 - 12u * first, where);
@@ -331,48 +339,40 @@ __device__ __forceinline__ void mc_emit(const McLane& m, const McTables& tab, Mc
             }
             if (t1) {
                 const uint32_t first = tris + (tot & 0xffffu) + (inc >> 16) - t1;
-                s.list[cells + __popc(e0) + __popc(e1 & below)] =
+                s.list[cells + n0 + __popc(e1 & below)] =
                     make_uint2(60u * c1 - 12u * first, where + 2u + (50u << 23));
                 s.flag[first] = 1;
             }
-            tris += (tot & 0xffffu) + (tot >> 16);
-            cells += __popc(e0) + __popc(e1);
+            tris += sum;
+            cells += n01;
         }
-    ahead();
-    __syncwarp();
-    uint32_t before = 0;  // cells that start before the window of 32 triangles
-    for (uint32_t w = 0; w < tris; w += 32u) {
-        const uint32_t starts = __ballot_sync(kFull, s.flag[w + lane] != 0);
-        s.flag[w + lane] = 0;
-        const auto vertex = [&](uint32_t k, uint32_t n) {  // n vertices from 32k on
-            const uint32_t i = lane + 32u * k;  // of the window's vertices
-            const uint2 e = s.list[before + __popc(starts & m.upto[k]) - 1u];
-            const uint32_t j = e.y >> 30;
-            const uint32_t bid = __shfl_sync(kFull, id, 8u * j);
-            const float biso = kOneIso ? iso : __shfl_sync(kFull, iso, 8u * j);
-            uint2 v = make_uint2(0u, bid);
-            if (lane < n) {
+        __syncwarp();
+        uint32_t before = 0;  // cells that start before the window of 32 triangles
+#pragma unroll 1
+        for (uint32_t w = 0; w < tris; w += 32u) {
+            const uint32_t starts = __ballot_sync(kFull, s.flag[w + lane] != 0);
+            s.flag[w + lane] = 0;
+            const uint32_t nv = 3u * min(tris - w, 32u);
+#pragma unroll
+            for (uint32_t k = 0; k < 3; ++k) {
+                if (k && 32u * k >= nv) break;
+                const uint32_t i = lane + 32u * k;  // of the window's vertices; past the last: worked on, not kept
+                const uint2 e = s.list[before + __popc(starts & m.upto[k]) - 1u];
+                const uint32_t j = e.y >> 30;
+                const uint32_t bid = __shfl_sync(kFull, id, 8u * j);
+                const float biso = kOneIso ? iso : __shfl_sync(kFull, iso, 8u * j);
                 const uint32_t word = *reinterpret_cast<const uint32_t*>(
-                    reinterpret_cast<const char*>(&tab.rows) + (int32_t)(e.x + 4u * (3u * w + i)));
+                    reinterpret_cast<const char*>(&tab.rows) + (int32_t)(e.x + 4u * (3u * w + min(i, nv - 1u))));
                 bool again;
-                v.x = mc_vertex_fast(word, &s.vol[0][0] + (e.y >> 23), e.y & (3u * kAxisOnes), biso, &again);
-                if (again) v.x = mc_vertex_exact(word, s.vol[j], e.y, &c_corner_pack.p[0][0], biso);
+                uint32_t v = mc_vertex_fast(word, &s.vol[0][0] + (e.y >> 23), e.y & (3u * kAxisOnes), biso, &again);
+                if (again && i < nv) v = mc_vertex_exact(word, s.vol[j], e.y, &c_corner_pack.p[0][0], biso);
+                sink.put(s.out, k, nv - 32u * k, make_uint2(v, bid));
             }
-            sink.put(s.out, k, n, v);
-        };
-        if (tris - w >= 32u) {
-#pragma unroll
-            for (uint32_t k = 0; k < 3; ++k) vertex(k, 32u);
-        } else {
-            const uint32_t n = 3u * (tris - w);
-#pragma unroll
-            for (uint32_t k = 0; k < 3; ++k)
-                if (32u * k < n) vertex(k, n - 32u * k);
+            sink.next_window(nv);
+            before += __popc(starts);
         }
-        sink.next_window();
-        before += __popc(starts);
-    }
-    __syncwarp();  // the next grids and lists overwrite these
+        __syncwarp();  // the next grids and lists overwrite these
+    } while (b < n);
 }
 
 }  // namespace bcmc
