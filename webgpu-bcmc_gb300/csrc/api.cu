@@ -1259,7 +1259,6 @@ bcmc_status bcmc_zfp_encode(bcmc_ctx* ctx, const float* d_field, const uint32_t 
     if (!ctx || !d_field || !dims || !d_words || rate == 0 || rate > 32) return BCMC_E_ARG;
     return guarded(ctx, [&]() -> bcmc_status {
         cudaStream_t s = pick(ctx, stream);
-        BCMC_CUDA(cudaMemsetAsync(d_words, 0, bcmc_zfp_stream_words(dims, rate) * 8, s));
         zfp_encode_launch(ctx, d_field, dims, 64u * rate, d_words, s);
         return BCMC_OK;
     });

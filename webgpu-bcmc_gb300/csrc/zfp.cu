@@ -111,42 +111,76 @@ __global__ void __launch_bounds__(kDecThreads, kDecPerSm) k_decode_volume(const 
     }
 }
 
-// Encoder: gathers the block (zfp's padding of partial blocks) and codes it.
-__device__ __forceinline__ void pad_row(float* p, uint32_t n, uint32_t s)
-{
-    switch (n) {
-    case 0: p[0] = 0.0f; [[fallthrough]];
-    case 1: p[1 * s] = p[0]; [[fallthrough]];
-    case 2: p[2 * s] = p[1 * s]; [[fallthrough]];
-    case 3: p[3 * s] = p[0]; [[fallthrough]];
-    default: break;
-    }
-}
+// Encoder: a thread gathers its block (zfp's padding of partial blocks), codes
+// it into its row of shared memory (zfp_encode_row), and the warp's 32 blocks,
+// whole 64-bit words each, go out with coalesced stores.  Bound by instructions
+// (the transform, two to four plane transposes and some forty coding steps a
+// block at rate 4): 256^3 at rate 4 took 378 us with a bit-by-bit writer.
+constexpr int kEncThreads = 128;
+constexpr int kEncPerSm = 4;
+constexpr uint32_t kEncPlaneWords = 17;  // 16 used; odd, so that the threads' rows start on different banks
 
-__global__ void __launch_bounds__(128) k_encode(const float* __restrict__ field, uint3 dims, uint3 nb,
-                                                uint32_t max_bits, unsigned long long* words)
+__host__ __device__ __forceinline__ uint32_t enc_row_words(uint32_t rate) { return 2u * rate + 3u; }
+
+// a partial block's coordinate i on an axis with n voxels: the voxel padding
+// copies (n < 4: 0 past one voxel; the last, then the first past two; the first past three)
+__device__ __forceinline__ uint32_t pad_coord(uint32_t i, uint32_t n) { return i < n ? i : (n == 2u && i == 2u ? 1u : 0u); }
+
+__global__ void __launch_bounds__(kEncThreads, kEncPerSm) k_encode(const float* __restrict__ field, uint3 dims, BlockGrid grid,
+                                                                   uint32_t rate, uint64_t nblocks, bool rows16,
+                                                                   uint64_t* __restrict__ words)
 {
-    const uint64_t nblocks = (uint64_t)nb.x * nb.y * nb.z;
-    for (uint64_t b = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; b < nblocks;
-         b += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t x0 = 4u * (uint32_t)(b % nb.x), y0 = 4u * (uint32_t)((b / nb.x) % nb.y),
-                       z0 = 4u * (uint32_t)(b / ((uint64_t)nb.x * nb.y));
-        const uint32_t nx = min(dims.x - x0, 4u), ny = min(dims.y - y0, 4u), nz = min(dims.z - z0, 4u);
-        float blk[64];
-        for (uint32_t z = 0; z < nz; ++z) {
-            for (uint32_t y = 0; y < ny; ++y) {
-                const float* row = field + (uint64_t)x0 + (uint64_t)dims.x * ((uint64_t)(y0 + y) + (uint64_t)dims.y * (z0 + z));
-                for (uint32_t x = 0; x < nx; ++x) blk[16 * z + 4 * y + x] = row[x];
-                pad_row(blk + 16 * z + 4 * y, nx, 1);
+    uint32_t* s_rows = stage_words();
+    const uint32_t stride = enc_row_words(rate);
+    uint32_t* row = s_rows + threadIdx.x * stride;
+    uint32_t* pl = s_rows + kEncThreads * stride + threadIdx.x * kEncPlaneWords;
+    const uint32_t lane = threadIdx.x & 31u;
+    if (blockIdx.x == 0 && threadIdx.x == 0) words[nblocks * rate] = 0u;  // the stream's padding word
+    for (uint64_t w0 = (uint64_t)blockIdx.x * kEncThreads + (threadIdx.x & ~31u); w0 < nblocks;
+         w0 += (uint64_t)gridDim.x * kEncThreads) {
+        const uint32_t n = (uint32_t)(nblocks - w0 < 32u ? nblocks - w0 : 32u);  // the warp's blocks
+        if (lane < n) {
+            const uint3 c = block_coords((uint32_t)(w0 + lane), grid);
+            const uint32_t x0 = 4u * c.x, y0 = 4u * c.y, z0 = 4u * c.z;
+            const float* src = field + (uint64_t)x0 + (uint64_t)dims.x * ((uint64_t)y0 + (uint64_t)dims.y * z0);
+            const uint64_t sy = dims.x, sz = (uint64_t)dims.x * dims.y;
+            const bool whole = x0 + 4u <= dims.x && y0 + 4u <= dims.y && z0 + 4u <= dims.z;
+            float f[64];
+            if (whole && rows16) {
+#pragma unroll
+                for (int r = 0; r < 16; ++r) {
+                    const float4 v = __ldg(reinterpret_cast<const float4*>(src + (r & 3) * sy + (r >> 2) * sz));
+                    f[4 * r] = v.x;
+                    f[4 * r + 1] = v.y;
+                    f[4 * r + 2] = v.z;
+                    f[4 * r + 3] = v.w;
+                }
+            } else {
+                const uint32_t nx = min(dims.x - x0, 4u), ny = min(dims.y - y0, 4u), nz = min(dims.z - z0, 4u);
+#pragma unroll
+                for (int i = 0; i < 64; ++i)
+                    f[i] = __ldg(src + pad_coord(i & 3, nx) + pad_coord((i >> 2) & 3, ny) * sy + pad_coord(i >> 4, nz) * sz);
             }
-            for (uint32_t x = 0; x < 4; ++x) pad_row(blk + 16 * z + x, ny, 4);
+            for (uint32_t i = 0; i < stride; ++i) row[i] = 0u;
+            zfp_encode_row(f, 64u * rate, row, pl);
         }
-        for (uint32_t y = 0; y < 4; ++y)
-            for (uint32_t x = 0; x < 4; ++x) pad_row(blk + 4 * y + x, nz, 16);
-        BitWriter bw;
-        bw.init(words, b * max_bits);
-        zfp_encode_block(blk, max_bits, bw);
-        bw.finish();
+        __syncwarp();
+        // word i of the warp's run: block i / rate, word i % rate
+        uint32_t k = lane / rate, j = lane - k * rate;
+        const uint32_t dk = 32u / rate, dj = 32u - dk * rate;
+        uint64_t* out = words + w0 * rate;
+        const uint32_t* rows = row - lane * stride;
+        for (uint32_t i = lane; i < n * rate; i += 32u) {
+            const uint32_t* r = rows + k * stride + 2u * j;
+            out[i] = (uint64_t)r[0] | ((uint64_t)r[1] << 32);
+            k += dk;
+            j += dj;
+            if (j >= rate) {
+                j -= rate;
+                ++k;
+            }
+        }
+        __syncwarp();
     }
 }
 
@@ -216,8 +250,12 @@ void zfp_encode_launch(bcmc_ctx* ctx, const float* field, const uint32_t dims[3]
     const uint3 d = make_uint3(dims[0], dims[1], dims[2]);
     const uint3 nb = make_uint3(div_up(dims[0], 4), div_up(dims[1], 4), div_up(dims[2], 4));
     const uint64_t n = (uint64_t)nb.x * nb.y * nb.z;
-    k_encode<<<grid_for(ctx, n, 128, 16), 128, 0, s>>>(field, d, nb, max_bits,
-                                                       reinterpret_cast<unsigned long long*>(words));
+    const uint32_t rate = max_bits / 64u;
+    const size_t smem = (size_t)kEncThreads * (enc_row_words(rate) + kEncPlaneWords) * 4u;
+    // 16-byte loads of a block's rows: whole rows on 16-byte boundaries
+    const bool rows16 = dims[0] % 4u == 0 && reinterpret_cast<uintptr_t>(field) % 16u == 0;
+    allow_smem(k_encode, smem);
+    k_encode<<<grid_all(n, kEncThreads), kEncThreads, smem, s>>>(field, d, make_block_grid(nb), rate, n, rows16, words);
     count_launches(1);
     BCMC_CUDA(cudaGetLastError());
 }

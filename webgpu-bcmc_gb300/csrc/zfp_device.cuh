@@ -127,6 +127,15 @@ __device__ __forceinline__ uint32_t zfp_shr(uint32_t x, uint32_t s)
 #endif
 }
 
+__device__ __forceinline__ uint32_t zfp_clz(uint32_t x)
+{
+#ifdef __CUDA_ARCH__
+    return (uint32_t)__clz((int)x);
+#else
+    return x ? (uint32_t)__builtin_clz(x) : 32u;
+#endif
+}
+
 // decode_ints' bit planes (zfp_decompress.comp:265-294) as masks.  `w`: the
 // block's words (LSB first), readable for two words past the block; `pos`:
 // the first bit after the header.  Plane r (bit 31 - r of the coefficients)
@@ -192,20 +201,10 @@ __device__ __forceinline__ void zfp_dswap(uint32_t& a, uint32_t& b, uint32_t s, 
     a ^= t << s;
 }
 
-// Rows of stored planes 8c .. 8c + 7 (row j = stored plane 8c + 7 - j, zero
-// past `np`), transposed: byte g of row k is then coefficient 8g + k's bits
-// of those planes, the first at bit 7.
-__device__ __forceinline__ void zfp_chunk(const uint32_t* pl, uint32_t c, uint32_t np, uint32_t* L, uint32_t* H)
+// The 8x8 bit matrices of the eight byte columns of 8 rows (L: columns 0-3, H:
+// 4-7), transposed at once by three delta-swap stages.
+__device__ __forceinline__ void zfp_transpose(uint32_t* L, uint32_t* H)
 {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const uint4 v = reinterpret_cast<const uint4*>(pl + 16u * c)[q];
-        const uint32_t p0 = 8u * c + 2u * (uint32_t)q;
-        L[7 - 2 * q] = p0 < np ? v.x : 0u;
-        H[7 - 2 * q] = p0 < np ? v.y : 0u;
-        L[6 - 2 * q] = p0 + 1u < np ? v.z : 0u;
-        H[6 - 2 * q] = p0 + 1u < np ? v.w : 0u;
-    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         zfp_dswap(L[j], L[j + 4], 4, 0x0F0F0F0Fu);
@@ -222,6 +221,23 @@ __device__ __forceinline__ void zfp_chunk(const uint32_t* pl, uint32_t c, uint32
         zfp_dswap(L[j], L[j + 1], 1, 0x55555555u);
         zfp_dswap(H[j], H[j + 1], 1, 0x55555555u);
     }
+}
+
+// Rows of stored planes 8c .. 8c + 7 (row j = stored plane 8c + 7 - j, zero
+// past `np`), transposed: byte g of row k is then coefficient 8g + k's bits
+// of those planes, the first at bit 7.
+__device__ __forceinline__ void zfp_chunk(const uint32_t* pl, uint32_t c, uint32_t np, uint32_t* L, uint32_t* H)
+{
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const uint4 v = reinterpret_cast<const uint4*>(pl + 16u * c)[q];
+        const uint32_t p0 = 8u * c + 2u * (uint32_t)q;
+        L[7 - 2 * q] = p0 < np ? v.x : 0u;
+        H[7 - 2 * q] = p0 < np ? v.y : 0u;
+        L[6 - 2 * q] = p0 + 1u < np ? v.z : 0u;
+        H[6 - 2 * q] = p0 + 1u < np ? v.w : 0u;
+    }
+    zfp_transpose(L, H);
 }
 
 // Coefficients (stream order) from the stored planes r0 .. planes - 1: chunk
@@ -375,65 +391,27 @@ __device__ __forceinline__ void zfp_fwd_lift(int32_t& x, int32_t& y, int32_t& z,
     w += y >> 1; y -= w >> 1;
 }
 
-struct BitWriter {
-    unsigned long long* words;
-    uint64_t pos;  // absolute bit position of buf's bit 0
-    uint64_t buf;
-    uint32_t n;    // bits in buf
-
-    __device__ __forceinline__ void init(unsigned long long* w, uint64_t bit_offset)
-    {
-        words = w;
-        pos = bit_offset & ~63ull;
-        n = (uint32_t)(bit_offset & 63u);
-        buf = 0;
-    }
-    __device__ __forceinline__ void flush_word()
-    {
-        if (buf) atomicOr(words + (pos >> 6), (unsigned long long)buf);
-        pos += 64;
-        buf = 0;
-        n = 0;
-    }
-    __device__ __forceinline__ uint32_t put_bit(uint32_t b)
-    {
-        buf |= (uint64_t)(b & 1u) << n;
-        if (++n == 64) flush_word();
-        return b & 1u;
-    }
-    // writes the low k (<= 64) bits of v; returns v >> k
-    __device__ __forceinline__ uint64_t put_bits(uint64_t v, uint32_t k)
-    {
-        for (uint32_t i = 0; i < k; ++i) put_bit((uint32_t)(v >> i) & 1u);
-        return k >= 64 ? 0ull : v >> k;
-    }
-    __device__ __forceinline__ void finish()
-    {
-        if (n) {
-            if (buf) atomicOr(words + (pos >> 6), (unsigned long long)buf);
-            buf = 0;
-            n = 0;
-        }
-    }
-};
-
-__device__ __forceinline__ void zfp_encode_block(const float* f, uint32_t max_bits, BitWriter& bw)
+// The block's coefficients in stream order, negabinary, from its 64 values; *ep
+// is the biased common exponent.  False for a block coded as zero.
+__device__ __forceinline__ bool zfp_forward(const float* f, uint32_t* u, uint32_t* ep)
 {
     float amax = 0.0f;
 #pragma unroll
     for (int i = 0; i < 64; ++i) amax = fmaxf(amax, fabsf(f[i]));
     int emax = -127;
     if (amax > 0.0f) frexpf(amax, &emax);
-    const uint32_t e = (uint32_t)(emax + 127);
-    if (e == 0) {
-        bw.put_bit(0);
-        return;
-    }
-    bw.put_bit(1);
-    bw.put_bits(e, 8);
+    *ep = (uint32_t)(emax + 127);
+    if (*ep == 0u) return false;
+    const int sh = 30 - emax;
     int32_t v[64];
+    if (sh <= 127) {  // 2^sh is a float: the product rounds as ldexpf does
+        const float w = __int_as_float((sh + 127) << 23);
 #pragma unroll
-    for (int i = 0; i < 64; ++i) v[i] = (int32_t)ldexpf(f[i], 30 - emax);
+        for (int i = 0; i < 64; ++i) v[i] = (int32_t)__fmul_rn(f[i], w);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 64; ++i) v[i] = (int32_t)ldexpf(f[i], sh);
+    }
 #pragma unroll
     for (int i = 0; i < 16; ++i) zfp_fwd_lift(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);  // x
 #pragma unroll
@@ -445,23 +423,142 @@ __device__ __forceinline__ void zfp_encode_block(const float* f, uint32_t max_bi
         }
 #pragma unroll
     for (int i = 0; i < 16; ++i) zfp_fwd_lift(v[i], v[i + 16], v[i + 32], v[i + 48]);  // z
-    uint32_t un[64], u[64];
+    uint32_t un[64];
 #pragma unroll
     for (int i = 0; i < 64; ++i) un[i] = ((uint32_t)v[i] + 0xaaaaaaaau) ^ 0xaaaaaaaau;
     BCMC_ZFP_SCATTER(u, un)
-    uint32_t bits = max_bits - 9u;
-    uint32_t n = 0;
-    for (int k = 31; k >= 0 && bits != 0; --k) {
-        uint64_t x = 0;
+    return true;
+}
+
+// Planes 8c .. 8c + 7 of the coefficients (plane 0: bit 31) as masks, coefficient
+// i at bit i: plane p of the chunk goes to pl[2p] (0..31) and pl[2p + 1].  The
+// rows of bytes are transposed by the decoder's three delta-swap stages.
+__device__ __forceinline__ void zfp_planes(const uint32_t* u, uint32_t c, uint32_t* pl)
+{
+    uint32_t L[8], H[8];
+    const uint32_t sel = (3u - c) | ((7u - c) << 4);
 #pragma unroll
-        for (int i = 0; i < 64; ++i) x |= (uint64_t)((u[i] >> k) & 1u) << i;
-        const uint32_t m = n < bits ? n : bits;
-        bits -= m;
-        x = bw.put_bits(x, m);
-        for (; n < 64u && bits != 0 && (bits--, bw.put_bit(x != 0ull)); x >>= 1, n++)
-            for (; n < 63u && bits != 0 && (bits--, !bw.put_bit((uint32_t)(x & 1ull))); x >>= 1, n++)
-                ;
+    for (int k = 0; k < 8; ++k) {
+        L[k] = __byte_perm(__byte_perm(u[k], u[8 + k], sel), __byte_perm(u[16 + k], u[24 + k], sel), 0x5410u);
+        H[k] = __byte_perm(__byte_perm(u[32 + k], u[40 + k], sel), __byte_perm(u[48 + k], u[56 + k], sel), 0x5410u);
     }
+    zfp_transpose(L, H);
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+        pl[2 * p] = L[7 - p];
+        pl[2 * p + 1] = H[7 - p];
+    }
+}
+
+// Bits appended to a row of 32-bit words: the word being filled is kept in a
+// register, and an append (up to 64 bits, the ones above its length zero) stores
+// the three words it can reach without reading any.
+struct RowWriter {
+    uint32_t* row;
+    uint32_t pos, cur;
+
+    __device__ __forceinline__ void put(uint32_t lo, uint32_t hi, uint32_t len)
+    {
+        const uint32_t i = pos >> 5, sh = pos & 31u;
+        const uint32_t t0 = cur | (lo << sh), t1 = __funnelshift_l(lo, hi, sh), t2 = __funnelshift_l(hi, 0u, sh);
+        row[i] = t0;
+        row[i + 1] = t1;
+        row[i + 2] = t2;
+        pos += len;
+        const uint32_t d = (pos >> 5) - i;
+        cur = d == 0u ? t0 : (d == 1u ? t1 : t2);
+    }
+};
+
+// One block into its row of zeroed words (max_bits / 32, and two more that the
+// last append may touch).  `pl`: 16 words of scratch.
+//
+// encode_ints of the published method, in the decoder's steps: a step is either
+// a group test that finds a coefficient (a 1, the zeros before it, and its 1
+// unless the bits or the 63 coefficients before it run out first) or the end of
+// the plane with the next plane's raw bits, both computed by selects, so that a
+// warp's lanes stay together although their blocks take different numbers of
+// steps.  A bit at a time into a 64-bit buffer, with the planes picked bit by
+// bit out of 64 coefficients, took nine times as long (256^3 at rate 4: 378 us).
+__device__ __forceinline__ void zfp_encode_row(const float* f, uint32_t max_bits, uint32_t* row, uint32_t* pl)
+{
+    uint32_t u[64], e;
+    if (!zfp_forward(f, u, &e)) return;  // a single 0 bit
+    uint32_t any = 0;
+#pragma unroll
+    for (int i = 0; i < 64; ++i) any |= u[i];
+    RowWriter out{row, 9u, 1u | ((e & 255u) << 1)};
+    row[0] = out.cur;
+    uint32_t bits = max_bits - 9u;
+    // the leading empty planes, a 0 each
+    const uint32_t r0 = zfp_clz(any);
+    if (r0 >= bits || r0 == 32u) return;
+    bits -= r0;
+    out.pos += r0;
+    if (out.pos >= 32u) out.cur = 0u;
+#pragma unroll
+    for (int i = 0; i < 64; ++i) u[i] <<= r0;
+    uint32_t n = 0;
+    for (uint32_t c = 0; 8u * c < 32u - r0; ++c) {
+        zfp_planes(u, c, pl);
+        const uint32_t np = min(32u - r0 - 8u * c, 8u);  // planes of the chunk
+        // the first plane's raw bits
+        uint32_t p = 0, o = 0;
+        uint32_t xlo, xhi;
+        {
+            const uint32_t lo = pl[0], hi = pl[1], m = min(n, bits);
+            out.put(lo & (zfp_shl(1u, m) - 1u), hi & zfp_shr(0xffffffffu, 64u - m), m);
+            bits -= m;
+            xlo = m >= 32u ? zfp_shr(hi, m - 32u) : __funnelshift_r(lo, hi, m);
+            xhi = zfp_shr(hi, m);
+        }
+        for (;;) {
+            const bool test = n < 64u && bits != 0u;  // a group test is written
+            const bool one = test && (xlo | xhi) != 0u;
+            o = test ? 1u : 0u;
+            // a 1: t zeros before the next significant coefficient
+            const uint32_t t = xlo ? (uint32_t)__ffs(xlo) - 1u : (uint32_t)__ffs(xhi) + 31u;
+            const uint32_t lim = min(63u - n, bits - 1u);
+            const uint32_t z = min(t, lim), hit = t < lim ? 1u : 0u;
+            // a 0 (or no test): the plane ends, the next one's raw bits follow
+            const uint32_t be = bits - o, m = min(n, be);
+            if (!one && (++p == np || be == 0u)) break;
+            const uint32_t plo = pl[2 * (p & 7u)], phi = pl[2 * (p & 7u) + 1];
+            const uint32_t rlo = plo & (zfp_shl(1u, m) - 1u), rhi = phi & zfp_shr(0xffffffffu, 64u - m);
+            const uint32_t vlo = one ? 1u | (hit ? zfp_shl(1u, z + 1u) : 0u) : rlo << o;
+            const uint32_t vhi = one ? (hit ? zfp_shl(1u, z - 31u) : 0u) : __funnelshift_l(rlo, rhi, o);
+            const uint32_t len = one ? 1u + z + hit : o + m;
+            out.put(vlo, vhi, len);
+            bits -= len;
+            n = one ? n + z + 1u : n;
+            const uint32_t slo = one ? xlo : plo, shi = one ? xhi : phi, s = one ? z + 1u : m;
+            xlo = s >= 32u ? zfp_shr(shi, s - 32u) : __funnelshift_r(slo, shi, s);
+            xhi = zfp_shr(shi, s);
+        }
+        out.put(0u, 0u, o);  // the 0 that ended the chunk's last plane
+        bits -= o;
+        if (bits == 0u) return;
+    }
+}
+
+// The same to its place in a stream of 64-bit words, a block at a time.
+struct BitWriter {
+    unsigned long long* words;
+    uint64_t first;  // the block's first word
+
+    __device__ __forceinline__ void init(unsigned long long* w, uint64_t bit_offset)
+    {
+        words = w;
+        first = bit_offset >> 6;
+    }
+    __device__ __forceinline__ void finish() {}
+};
+__device__ __forceinline__ void zfp_encode_block(const float* f, uint32_t max_bits, BitWriter& bw)
+{
+    uint32_t row[kZfpMaxBitsLimit / 32 + 2] = {}, pl[16];
+    zfp_encode_row(f, max_bits, row, pl);
+    for (uint32_t i = 0; i < max_bits / 64u; ++i)
+        bw.words[bw.first + i] = (unsigned long long)row[2 * i] | ((unsigned long long)row[2 * i + 1] << 32);
 }
 
 }  // namespace bcmc
