@@ -471,15 +471,16 @@ struct RowWriter {
 };
 
 // One block into its row of zeroed words (max_bits / 32, and two more that the
-// last append may touch).  `pl`: 16 words of scratch.
+// last append may touch).  `pl`: 32 words of scratch.
 //
 // encode_ints of the published method, in the decoder's steps: a step is either
 // a group test that finds a coefficient (a 1, the zeros before it, and its 1
 // unless the bits or the 63 coefficients before it run out first) or the end of
 // the plane with the next plane's raw bits, both computed by selects, so that a
 // warp's lanes stay together although their blocks take different numbers of
-// steps.  A bit at a time into a 64-bit buffer, with the planes picked bit by
-// bit out of 64 coefficients, took nine times as long (256^3 at rate 4: 378 us).
+// steps; they wait for each other at every sixteenth plane (eighth: 57 us at
+// 256^3 and rate 4, sixteenth: 49 us).  A bit at a time into a 64-bit buffer,
+// with the planes picked bit by bit out of 64 coefficients, took 378 us.
 __device__ __forceinline__ void zfp_encode_row(const float* f, uint32_t max_bits, uint32_t* row, uint32_t* pl)
 {
     uint32_t u[64], e;
@@ -499,9 +500,10 @@ __device__ __forceinline__ void zfp_encode_row(const float* f, uint32_t max_bits
 #pragma unroll
     for (int i = 0; i < 64; ++i) u[i] <<= r0;
     uint32_t n = 0;
-    for (uint32_t c = 0; 8u * c < 32u - r0; ++c) {
+    for (uint32_t c = 0; 8u * c < 32u - r0; c += 2) {
         zfp_planes(u, c, pl);
-        const uint32_t np = min(32u - r0 - 8u * c, 8u);  // planes of the chunk
+        zfp_planes(u, c + 1, pl + 16);
+        const uint32_t np = min(32u - r0 - 8u * c, 16u);  // planes of the chunk
         // the first plane's raw bits
         uint32_t p = 0, o = 0;
         uint32_t xlo, xhi;
@@ -523,7 +525,7 @@ __device__ __forceinline__ void zfp_encode_row(const float* f, uint32_t max_bits
             // a 0 (or no test): the plane ends, the next one's raw bits follow
             const uint32_t be = bits - o, m = min(n, be);
             if (!one && (++p == np || be == 0u)) break;
-            const uint32_t plo = pl[2 * (p & 7u)], phi = pl[2 * (p & 7u) + 1];
+            const uint32_t plo = pl[2 * (p & 15u)], phi = pl[2 * (p & 15u) + 1];
             const uint32_t rlo = plo & (zfp_shl(1u, m) - 1u), rhi = phi & zfp_shr(0xffffffffu, 64u - m);
             const uint32_t vlo = one ? 1u | (hit ? zfp_shl(1u, z + 1u) : 0u) : rlo << o;
             const uint32_t vhi = one ? (hit ? zfp_shl(1u, z - 31u) : 0u) : __funnelshift_l(rlo, rhi, o);
@@ -555,7 +557,7 @@ struct BitWriter {
 };
 __device__ __forceinline__ void zfp_encode_block(const float* f, uint32_t max_bits, BitWriter& bw)
 {
-    uint32_t row[kZfpMaxBitsLimit / 32 + 2] = {}, pl[16];
+    uint32_t row[kZfpMaxBitsLimit / 32 + 2] = {}, pl[32];
     zfp_encode_row(f, max_bits, row, pl);
     for (uint32_t i = 0; i < max_bits / 64u; ++i)
         bw.words[bw.first + i] = (unsigned long long)row[2 * i] | ((unsigned long long)row[2 * i + 1] << 32);
