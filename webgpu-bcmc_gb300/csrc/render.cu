@@ -3,46 +3,51 @@
 // shading of shaders/mc_isosurface.vert/.frag, as CUDA kernels instead of a
 // graphics pipeline (no window, swapchain or graphics API).
 //
-//   vertex stage  unpack_launch (unpack.cu): world and clip positions, plus
-//                 the fog entry distance of mc_isosurface.vert:35-49
-//   k_raster      one thread per triangle: clip -> NDC -> pixels (WebGPU
-//                 conventions: y up in NDC, depth in [0, 1]), edge functions
-//                 with a top-left rule at pixel centres, depth "less" against a
-//                 buffer cleared to 1.0 -- each covered pixel takes the 64-bit
-//                 atomicMin of (depth bits, triangle id), so the result does not
-//                 depend on thread order
+//   k_raster      one thread per triangle: its three vertices' clip positions
+//                 (unpack.cuh) -> NDC -> pixels (WebGPU conventions: y up in
+//                 NDC, depth in [0, 1]), edge functions with a top-left rule at
+//                 pixel centres, depth "less" against a buffer cleared to 1.0 --
+//                 each covered pixel takes the 64-bit atomicMin of (depth bits,
+//                 triangle id), so the result does not depend on thread order
 //   k_resolve     one thread per pixel: the winning triangle's fragment shading
 //                 (mc_isosurface.frag:15-40: flat normal, Blinn-Phong, optional
-//                 fog), background (1, 1, 1, 1) where no triangle won
+//                 fog with mc_isosurface.vert:35-49's entry distances),
+//                 background (1, 1, 1, 1) where no triangle won
+// Positions are worked out from the packed vertices where they are needed: 24
+// bytes a triangle, and a covered pixel again, where stored world and clip
+// positions were 84 written and read back.
 // Triangles with a vertex at w <= 1e-6 (behind the eye) or more than 2^21
 // pixels off the image are not drawn: there is no clipping.  Every float
 // operation is an explicitly rounded IEEE operation (no contraction), so the
 // CPU restatement in the oracle reproduces the depth/triangle buffers bit for
 // bit.
 #include "bcmc_impl.h"
+#include "unpack.cuh"
 
 namespace bcmc {
 namespace {
 
 struct RenderArgs {
-    const float* world;  // 3 per vertex
-    const float* clip;   // 4 per vertex
-    const float* tenter; // 1 per vertex (fog), or null
+    const uint2* verts;
+    VertexStage stage;
     uint64_t ntri;
     uint32_t w, h;
     float eye[3];
+    float half[3];  // the volume's box is [-half, half]
     int fog;
     unsigned long long* keys;  // per pixel
     float* rgba;               // 4 per pixel
     float* depth;              // 1 per pixel, or null
     uint32_t* triangle;        // 1 per pixel, or null
     uint32_t* big;             // triangles left to k_raster_big
-    unsigned int* nbig;
+    unsigned int* nbig;        // their number less one
 };
 
-// a triangle whose pixel box holds more than this many pixels is rasterised by
-// a whole CTA (k_raster_big) instead of one thread
+// a triangle whose pixel box holds more than this many pixels, or is wider or
+// higher than kBigSide, is rasterised by a whole CTA (k_raster_big) instead of
+// one thread: below it the edge functions fit 32 bits
 constexpr long long kBigBox = 256;
+constexpr int kBigSide = 64;
 
 // Screen positions are snapped to 1/256 pixel (the sub-pixel precision
 // WebGPU's rasterisers use) and the edge functions are evaluated in 64-bit
@@ -68,6 +73,21 @@ __device__ __forceinline__ long long edge_fn(int ax, int ay, int bx, int by, int
 // an edge belongs to the triangle when the edge is a top edge (horizontal,
 // running in +x) or a left edge (running in -y)
 __device__ __forceinline__ bool top_left(int ax, int ay, int bx, int by) { return (ay == by && bx > ax) || (by < ay); }
+
+// the world and clip positions of triangle t's vertices
+__device__ __forceinline__ void load_triangle(const RenderArgs& a, uint64_t t, float world[9], float clip[12])
+{
+    uint2 v[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[k] = __ldg(a.verts + 3 * t + k);
+    uint3 b = block_coords(v[0].y, a.stage.grid);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (k && v[k].y != v[k - 1].y) b = block_coords(v[k].y, a.stage.grid);  // a mesh's triangles lie in one block
+        vertex_world(a.stage, v[k].x, b, world + 3 * k);
+        vertex_clip(a.stage, world + 3 * k, clip + 4 * k);
+    }
+}
 
 // false when the triangle is not drawn: a vertex at w <= 1e-6, a vertex
 // beyond the guard band (or not finite), or zero area
@@ -110,45 +130,105 @@ __device__ __forceinline__ void edges_at(const Tri& t, int px, int py, long long
     e[2] = edge_fn(t.x[0], t.y[0], t.x[1], t.y[1], cx, cy);
 }
 
-// coverage and depth test of one pixel centre: the 64-bit atomicMin of
-// (depth bits, triangle index) keeps the nearest fragment, the earlier
-// triangle on ties (depth >= 0, so its bits order as the values do)
-__device__ __forceinline__ void shade_sample(const RenderArgs& a, const Tri& t, uint32_t ti, int px, int py)
+// depth test of a covered pixel with edge values e: the 64-bit atomicMin of
+// (depth bits, triangle index) keeps the nearest fragment, the earlier triangle
+// on ties (depth >= 0, so its bits order as the values do)
+__device__ __forceinline__ void put_fragment(const RenderArgs& a, const float e[3], const float tz[3], float area,
+                                             float inv_area, uint32_t ti, int px, int py)
 {
-    long long e[3];
-    edges_at(t, px, py, e);
-    const bool in0 = e[0] > 0 || (e[0] == 0 && top_left(t.x[1], t.y[1], t.x[2], t.y[2]));
-    const bool in1 = e[1] > 0 || (e[1] == 0 && top_left(t.x[2], t.y[2], t.x[0], t.y[0]));
-    const bool in2 = e[2] > 0 || (e[2] == 0 && top_left(t.x[0], t.y[0], t.x[1], t.y[1]));
-    if (!(in0 && in1 && in2)) return;
-    // depth: NDC z interpolated linearly in screen space
-    const float z = __fdiv_rn(__fadd_rn(__fadd_rn(__fmul_rn(__ll2float_rn(e[0]), t.z[0]),
-                                                  __fmul_rn(__ll2float_rn(e[1]), t.z[1])),
-                                        __fmul_rn(__ll2float_rn(e[2]), t.z[2])),
-                              __ll2float_rn(t.area));
+    // depth: NDC z interpolated linearly in screen space (the area is at least 1)
+    const float num = __fadd_rn(__fadd_rn(__fmul_rn(e[0], tz[0]), __fmul_rn(e[1], tz[1])), __fmul_rn(e[2], tz[2]));
+    const float z = num > 1e-20f && num < 1e30f ? exact_div(num, area, inv_area) : __fdiv_rn(num, area);
     if (!(z >= 0.0f && z < 1.0f)) return;  // outside the depth range, or not less than the clear value
     const unsigned long long key = ((unsigned long long)__float_as_uint(z) << 32) | ti;
     atomicMin(a.keys + (uint64_t)py * a.w + px, key);
 }
 
+// pixels whose centre (256 p + 128) lies in the triangle's box, clamped to the
+// image: x0 > x1 or y0 > y1 when there are none
+__device__ __forceinline__ int4 pixel_box(const RenderArgs& a, const Tri& t)
+{
+    const int xmin = min(t.x[0], min(t.x[1], t.x[2])), xmax = max(t.x[0], max(t.x[1], t.x[2]));
+    const int ymin = min(t.y[0], min(t.y[1], t.y[2])), ymax = max(t.y[0], max(t.y[1], t.y[2]));
+    return make_int4(max(0, floor_div256(xmin - 128 + 255)), max(0, floor_div256(ymin - 128 + 255)),
+                     min((int)a.w - 1, floor_div256(xmax - 128)), min((int)a.h - 1, floor_div256(ymax - 128)));
+}
+
+// One thread per triangle.  A small triangle's edge functions are exact in 32
+// bits (corners within 2^15 of each other and of the box's pixel centres), each
+// less the top-left rule's one, so that a pixel is covered when no value is
+// negative: its box is gone through once with an add per edge and pixel, four
+// pixels of a row at a time, and only the covered ones then take the depth test -- the
+// lanes of a warp differ less in covered pixels than in boxes.  With 64-bit
+// products per pixel and the depth test inside the loop this took 203 us on
+// 1.27 M triangles at 1080p.
 __global__ void __launch_bounds__(256) k_raster(RenderArgs a)
 {
     for (uint64_t ti = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; ti < a.ntri;
          ti += (uint64_t)gridDim.x * blockDim.x) {
+        float world[9], clip[12];
+        load_triangle(a, ti, world, clip);
         Tri t;
-        if (!tri_setup(a.clip + 12 * ti, a.w, a.h, t)) continue;
-        const int xmin = min(t.x[0], min(t.x[1], t.x[2])), xmax = max(t.x[0], max(t.x[1], t.x[2]));
-        const int ymin = min(t.y[0], min(t.y[1], t.y[2])), ymax = max(t.y[0], max(t.y[1], t.y[2]));
-        // pixels whose centre (256 p + 128) lies in the box, clamped to the image
-        const int x0 = max(0, floor_div256(xmin - 128 + 255)), x1 = min((int)a.w - 1, floor_div256(xmax - 128));
-        const int y0 = max(0, floor_div256(ymin - 128 + 255)), y1 = min((int)a.h - 1, floor_div256(ymax - 128));
-        if (x0 > x1 || y0 > y1) continue;
-        if ((long long)(x1 - x0 + 1) * (y1 - y0 + 1) > kBigBox) {
-            a.big[atomicAdd(a.nbig, 1u)] = (uint32_t)ti;
+        if (!tri_setup(clip, a.w, a.h, t)) continue;
+        const int4 box = pixel_box(a, t);
+        if (box.x > box.z || box.y > box.w) continue;
+        const int bw = box.z - box.x + 1, bh = box.w - box.y + 1;
+        if ((long long)bw * bh > kBigBox || max(max(t.x[0], t.x[1]), t.x[2]) - min(min(t.x[0], t.x[1]), t.x[2]) > 256 * kBigSide ||
+            max(max(t.y[0], t.y[1]), t.y[2]) - min(min(t.y[0], t.y[1]), t.y[2]) > 256 * kBigSide) {
+            a.big[atomicAdd(a.nbig, 1u) + 1u] = (uint32_t)ti;
             continue;
         }
-        for (int py = y0; py <= y1; ++py)
-            for (int px = x0; px <= x1; ++px) shade_sample(a, t, (uint32_t)ti, px, py);
+        // edge k runs from corner k + 1 to corner k + 2; its value at the first
+        // pixel's centre, its steps to the right and down, and whether a centre
+        // on it is outside
+        const int cx = box.x * 256 + 128, cy = box.y * 256 + 128;
+        int at0[3], right[3], down[3], out[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int p = (k + 1) % 3, q = (k + 2) % 3;
+            const int dx = t.x[q] - t.x[p], dy = t.y[q] - t.y[p];
+            out[k] = top_left(t.x[p], t.y[p], t.x[q], t.y[q]) ? 0 : 1;
+            at0[k] = dx * (cy - t.y[p]) - dy * (cx - t.x[p]);
+            right[k] = -256 * dy;
+            down[k] = 256 * dx;
+        }
+        const float area = __ll2float_rn(t.area), inv_area = __frcp_rn(area);
+        // the box in groups of four pixels of a row, eight groups to a mask
+        const uint32_t per_row = (uint32_t)(bw + 3) >> 2, groups = per_row * (uint32_t)bh;
+        const uint32_t inv = (65535u + per_row) / per_row;  // g / per_row = g * inv >> 16 for g < 1024
+        const uint32_t last = (1u << (bw - 4 * ((int)per_row - 1))) - 1u;  // pixels of a row's last group
+        uint32_t gx = 0;
+        int row[3] = {at0[0] - out[0], at0[1] - out[1], at0[2] - out[2]}, e[3] = {row[0], row[1], row[2]};
+        for (uint32_t first = 0; first < groups; first += 8u) {
+            uint32_t covered = 0;
+            const uint32_t n = min(8u, groups - first);
+            for (uint32_t i = 0; i < n; ++i) {
+                uint32_t four = 0;
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    four |= ((e[0] | e[1] | e[2]) >= 0 ? 1u : 0u) << x;
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) e[k] += right[k];
+                }
+                const bool end = ++gx == per_row;
+                covered |= (four & (end ? last : 15u)) << (4u * i);
+                if (end) {
+                    gx = 0;
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) e[k] = row[k] += down[k];
+                }
+            }
+            while (covered) {
+                const uint32_t i = (uint32_t)__ffs(covered) - 1u, g = first + (i >> 2);
+                covered &= covered - 1u;
+                const uint32_t r = g * inv >> 16;
+                const int py = (int)r, px = (int)(4u * (g - r * per_row) + (i & 3u));
+                float f[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) f[k] = __int2float_rn(at0[k] + px * right[k] + py * down[k]);
+                put_fragment(a, f, t.z, area, inv_area, (uint32_t)ti, box.x + px, box.y + py);
+            }
+        }
     }
 }
 
@@ -156,18 +236,27 @@ __global__ void __launch_bounds__(256) k_raster(RenderArgs a)
 // the pixel box
 __global__ void __launch_bounds__(256) k_raster_big(RenderArgs a)
 {
-    const unsigned int nbig = *a.nbig;
+    const unsigned int nbig = *a.nbig + 1u;
     for (unsigned int b = blockIdx.x; b < nbig; b += gridDim.x) {
         const uint32_t ti = a.big[b];
+        float world[9], clip[12];
+        load_triangle(a, ti, world, clip);
         Tri t;
-        tri_setup(a.clip + 12 * (uint64_t)ti, a.w, a.h, t);
-        const int xmin = min(t.x[0], min(t.x[1], t.x[2])), xmax = max(t.x[0], max(t.x[1], t.x[2]));
-        const int ymin = min(t.y[0], min(t.y[1], t.y[2])), ymax = max(t.y[0], max(t.y[1], t.y[2]));
-        const int x0 = max(0, floor_div256(xmin - 128 + 255)), x1 = min((int)a.w - 1, floor_div256(xmax - 128));
-        const int y0 = max(0, floor_div256(ymin - 128 + 255)), y1 = min((int)a.h - 1, floor_div256(ymax - 128));
-        const long long bw = x1 - x0 + 1, npix = bw * (y1 - y0 + 1);
-        for (long long p = threadIdx.x; p < npix; p += blockDim.x)
-            shade_sample(a, t, ti, x0 + (int)(p % bw), y0 + (int)(p / bw));
+        tri_setup(clip, a.w, a.h, t);
+        const int4 box = pixel_box(a, t);
+        const long long bw = box.z - box.x + 1, npix = bw * (box.w - box.y + 1);
+        const float area = __ll2float_rn(t.area), inv_area = __frcp_rn(area);
+        for (long long p = threadIdx.x; p < npix; p += blockDim.x) {
+            const int px = box.x + (int)(p % bw), py = box.y + (int)(p / bw);
+            long long e[3];
+            edges_at(t, px, py, e);
+            const bool in0 = e[0] > 0 || (e[0] == 0 && top_left(t.x[1], t.y[1], t.x[2], t.y[2]));
+            const bool in1 = e[1] > 0 || (e[1] == 0 && top_left(t.x[2], t.y[2], t.x[0], t.y[0]));
+            const bool in2 = e[2] > 0 || (e[2] == 0 && top_left(t.x[0], t.y[0], t.x[1], t.y[1]));
+            if (!(in0 && in1 && in2)) continue;
+            const float f[3] = {__ll2float_rn(e[0]), __ll2float_rn(e[1]), __ll2float_rn(e[2])};
+            put_fragment(a, f, t.z, area, inv_area, ti, px, py);
+        }
     }
 }
 
@@ -201,6 +290,22 @@ __device__ __forceinline__ float3 cross3(float3 a, float3 b)
 }
 __device__ __forceinline__ float clamp01(float x) { return gmin(gmax(x, 0.0f), 1.0f); }
 
+// mc_isosurface.vert:35-49: distance along the eye ray where it enters the
+// volume's box [-scale/2, scale/2], clamped at 0
+__device__ __forceinline__ float fog_enter(const RenderArgs& a, const float* world, float3 eye)
+{
+    const float3 d = norm3(sub3(f3(world), eye));
+    const float o[3] = {eye.x, eye.y, eye.z}, dd[3] = {d.x, d.y, d.z};
+    float tmin[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float inv = __frcp_rn(dd[k]);
+        const float ta = __fmul_rn(__fsub_rn(-a.half[k], o[k]), inv), tb = __fmul_rn(__fsub_rn(a.half[k], o[k]), inv);
+        tmin[k] = gmin(ta, tb);
+    }
+    return gmax(gmax(tmin[0], gmax(tmin[1], tmin[2])), 0.0f);
+}
+
 __global__ void __launch_bounds__(256) k_resolve(RenderArgs a)
 {
     const uint64_t npix = (uint64_t)a.w * a.h;
@@ -213,35 +318,41 @@ __global__ void __launch_bounds__(256) k_resolve(RenderArgs a)
             const uint64_t t = key & 0xffffffffull;
             tri = (uint32_t)t;
             depth = __uint_as_float((uint32_t)(key >> 32));
+            float world[9], clip[12];
+            load_triangle(a, t, world, clip);
             Tri tr;
-            tri_setup(a.clip + 12 * t, a.w, a.h, tr);  // drawn, so set up as in k_raster
+            tri_setup(clip, a.w, a.h, tr);  // drawn, so set up as in k_raster
             long long ee[3];
             edges_at(tr, (int)(i % a.w), (int)(i / a.w), ee);
-            const float e[3] = {__ll2float_rn(ee[0]), __ll2float_rn(ee[1]), __ll2float_rn(ee[2])};
-            const int* idx = tr.idx;
-            // perspective-correct weights of the varyings: (e_k / w_k) / sum
+            const float3 eye = make_float3(a.eye[0], a.eye[1], a.eye[2]);
+            // perspective-correct weights of the varyings: (e_k / w_k) / sum.  The
+            // edges come in the winding's order: corners 1 and 2 may be exchanged
+            const bool flip = tr.idx[1] == 2;
             float pw[3], psum = 0.0f;
+#pragma unroll
             for (int k = 0; k < 3; ++k) {
-                pw[k] = __fdiv_rn(e[k], a.clip[12 * t + 4 * idx[k] + 3]);
+                const float cw = k == 0 ? clip[3] : ((k == 1) != flip ? clip[7] : clip[11]);
+                pw[k] = __fdiv_rn(__ll2float_rn(ee[k]), cw);
                 psum = __fadd_rn(psum, pw[k]);
             }
             float3 wp = make_float3(0.0f, 0.0f, 0.0f);
             float te = 0.0f;
+#pragma unroll
             for (int k = 0; k < 3; ++k) {
                 const float b = __fdiv_rn(pw[k], psum);
-                const float* wk = a.world + 3 * (3 * t + idx[k]);
+                float wk[3];
+#pragma unroll
+                for (int c = 0; c < 3; ++c) wk[c] = k == 0 ? world[c] : ((k == 1) != flip ? world[3 + c] : world[6 + c]);
                 wp = make_float3(__fadd_rn(wp.x, __fmul_rn(b, wk[0])), __fadd_rn(wp.y, __fmul_rn(b, wk[1])),
                                  __fadd_rn(wp.z, __fmul_rn(b, wk[2])));
-                if (a.fog) te = __fadd_rn(te, __fmul_rn(b, a.tenter[3 * t + idx[k]]));
+                if (a.fog) te = __fadd_rn(te, __fmul_rn(b, fog_enter(a, wk, eye)));
             }
             // mc_isosurface.frag:15-40
-            const float3 eye = make_float3(a.eye[0], a.eye[1], a.eye[2]);
             float3 v = sub3(wp, eye);
             const float dist = __fsqrt_rn(dot3(v, v));
             v = scale3(norm3(v), -1.0f);
             const float3 light = v;
-            const float* w0 = a.world + 9 * t;
-            float3 n = norm3(cross3(sub3(f3(w0 + 3), f3(w0)), sub3(f3(w0 + 6), f3(w0))));
+            float3 n = norm3(cross3(sub3(f3(world + 3), f3(world)), sub3(f3(world + 6), f3(world))));
             if (dot3(n, light) < 0.0f) n = scale3(n, -1.0f);
             const float3 base = make_float3(0.3f, 0.3f, 0.9f);
             const float3 hv = norm3(make_float3(__fadd_rn(v.x, light.x), __fadd_rn(v.y, light.y), __fadd_rn(v.z, light.z)));
@@ -266,24 +377,6 @@ __global__ void __launch_bounds__(256) k_resolve(RenderArgs a)
     }
 }
 
-// mc_isosurface.vert:35-49: distance along the eye ray where it enters the
-// volume's box [-scale/2, scale/2], clamped at 0
-__global__ void __launch_bounds__(256) k_fog_enter(const float* world, uint64_t n, float3 eye, float3 half,
-                                                   float* tenter)
-{
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const float3 d = norm3(sub3(f3(world + 3 * i), eye));
-        const float o[3] = {eye.x, eye.y, eye.z}, dd[3] = {d.x, d.y, d.z}, hh[3] = {half.x, half.y, half.z};
-        float tmin[3];
-        for (int k = 0; k < 3; ++k) {
-            const float inv = __fdiv_rn(1.0f, dd[k]);
-            const float ta = __fmul_rn(__fsub_rn(-hh[k], o[k]), inv), tb = __fmul_rn(__fsub_rn(hh[k], o[k]), inv);
-            tmin[k] = gmin(ta, tb);
-        }
-        tenter[i] = gmax(gmax(tmin[0], gmax(tmin[1], tmin[2])), 0.0f);
-    }
-}
-
 int grid_of(bcmc_ctx* ctx, uint64_t n)
 {
     const uint64_t want = (n + 255) / 256, cap = (uint64_t)ctx->num_sms * 16;
@@ -295,14 +388,10 @@ int grid_of(bcmc_ctx* ctx, uint64_t n)
 void render_launch(bcmc_ctx* ctx, const uint2* verts, uint64_t n, const uint32_t dims[3], const float scale[3],
                    const bcmc_render_params& p, float* rgba, float* depth, uint32_t* triangle, cudaStream_t s)
 {
-    const uint64_t ntri = n / 3, nv = ntri * 3, npix = (uint64_t)p.width * p.height;
-    // working buffers, carved from one grow-only context allocation: world and
-    // clip positions, fog entry distances, the per-pixel keys, the list of
-    // large triangles and its counter
-    auto up = [](uint64_t b) { return (b + 255) & ~uint64_t(255); };
-    const uint64_t b_world = up(nv * 12), b_clip = up(nv * 16), b_tenter = p.fog ? up(nv * 4) : 0,
-                   b_keys = up(npix * 8), b_big = up((ntri + 1) * 4);
-    const uint64_t need = b_world + b_clip + b_tenter + b_keys + b_big;
+    const uint64_t ntri = n / 3, npix = (uint64_t)p.width * p.height;
+    // working buffers, carved from one grow-only context allocation: the
+    // per-pixel keys, the list of large triangles and its counter
+    const uint64_t b_keys = (npix * 8 + 255) & ~uint64_t(255), need = b_keys + (ntri + 1) * 4;
     if (need > ctx->render_bytes) {
         dev_free(ctx, ctx->d_render, ctx->render_bytes);
         ctx->d_render = nullptr;
@@ -310,40 +399,27 @@ void render_launch(bcmc_ctx* ctx, const uint2* verts, uint64_t n, const uint32_t
         ctx->d_render = dev_alloc(ctx, need);
         ctx->render_bytes = need;
     }
-    char* base = static_cast<char*>(ctx->d_render);
-    float* world = reinterpret_cast<float*>(base);
-    float* clip = reinterpret_cast<float*>(base + b_world);
-    float* tenter = p.fog ? reinterpret_cast<float*>(base + b_world + b_clip) : nullptr;
-    unsigned long long* keys = reinterpret_cast<unsigned long long*>(base + b_world + b_clip + b_tenter);
-    uint32_t* big = reinterpret_cast<uint32_t*>(base + b_world + b_clip + b_tenter + b_keys);
+    unsigned long long* keys = static_cast<unsigned long long*>(ctx->d_render);
+    uint32_t* big = reinterpret_cast<uint32_t*>(static_cast<char*>(ctx->d_render) + b_keys);
     try {
-        BCMC_CUDA(cudaMemsetAsync(keys, 0xff, npix * 8, s));
-        if (nv) {
-            BCMC_CUDA(cudaMemsetAsync(big + ntri, 0, 4, s));
-            unpack_launch(ctx, verts, nv, dims, scale, p.proj_view, world, clip, s);
-            if (p.fog) {
-                const float3 half = make_float3((scale ? scale[0] : 1.0f) * 0.5f, (scale ? scale[1] : 1.0f) * 0.5f,
-                                                (scale ? scale[2] : 1.0f) * 0.5f);
-                k_fog_enter<<<grid_of(ctx, nv), 256, 0, s>>>(world, nv, make_float3(p.eye_pos[0], p.eye_pos[1],
-                                                                                    p.eye_pos[2]), half, tenter);
-                count_launches(1);
-            }
-        }
+        BCMC_CUDA(cudaMemsetAsync(keys, 0xff, b_keys + 4, s));  // the keys, and the counter at -1
         RenderArgs a{};
-        a.world = world;
-        a.clip = clip;
-        a.tenter = tenter;
+        a.verts = verts;
+        a.stage = make_vertex_stage(dims, scale, p.proj_view);
         a.ntri = ntri;
         a.w = p.width;
         a.h = p.height;
-        for (int k = 0; k < 3; ++k) a.eye[k] = p.eye_pos[k];
+        for (int k = 0; k < 3; ++k) {
+            a.eye[k] = p.eye_pos[k];
+            a.half[k] = (scale ? scale[k] : 1.0f) * 0.5f;
+        }
         a.fog = p.fog ? 1 : 0;
         a.keys = keys;
         a.rgba = rgba;
         a.depth = depth;
         a.triangle = triangle;
-        a.big = big;
-        a.nbig = reinterpret_cast<unsigned int*>(big + ntri);
+        a.nbig = big;
+        a.big = big + 1;
         if (ntri) {
             k_raster<<<grid_of(ctx, ntri), 256, 0, s>>>(a);
             k_raster_big<<<ctx->num_sms * 4, 256, 0, s>>>(a);
