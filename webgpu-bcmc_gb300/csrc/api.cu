@@ -100,6 +100,7 @@ static void ctx_release(bcmc_ctx* ctx)
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     dev_free(ctx, ctx->d_prim, sizeof(QueryState));
     dev_free(ctx, ctx->d_status, ctx->status_words * 8);
+    if (ctx->d_counts) dev_free(ctx, ctx->d_counts, sort_count_bytes(ctx));
     dev_free(ctx, ctx->d_scratch, ctx->scratch_words * 4);
     dev_free(ctx, ctx->d_render, ctx->render_bytes);
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
@@ -144,6 +145,7 @@ struct bcmc_lru {
     // age bins: joint histogram and dense ranks (k_slots' one-pass sort plan)
     uint32_t* age_hist = nullptr;
     uint8_t* age_rank = nullptr;
+    uint16_t* sort_counts = nullptr;  // the sort's tile counts (sort_count_bytes)
     uint64_t* status = nullptr;
     size_t status_words = 0;
     uint64_t* st_active_a = nullptr;
@@ -288,6 +290,7 @@ static bcmc_lru* lru_new(bcmc_ctx* ctx, uint32_t initial_size, uint32_t element_
         BCMC_CUDA(cudaMallocHost(&c->h_q, sizeof(QueryState)));
         c->age_hist = (uint32_t*)dev_alloc(ctx, (size_t)kAgeBins * 4);
         c->age_rank = (uint8_t*)dev_alloc(ctx, (size_t)kAgeBins);
+        c->sort_counts = (uint16_t*)dev_alloc(ctx, sort_count_bytes(ctx));
         cudaStream_t s = ctx->stream;
         lru_clear_key16(c, s);
         BCMC_CUDA(cudaMemsetAsync(c->status, 0, c->status_words * 8, s));
@@ -306,6 +309,7 @@ static bcmc_lru* lru_new(bcmc_ctx* ctx, uint32_t initial_size, uint32_t element_
         dev_free(ctx, c->item_slots, (size_t)c->aligned_total * 4);
         dev_free(ctx, c->new_ids, (size_t)(total ? total : 1) * 4);
         dev_free(ctx, c->status, c->status_words * 8);
+        dev_free(ctx, c->sort_counts, sort_count_bytes(ctx));
         dev_free(ctx, c->q, sizeof(QueryState));
         if (c->h_q) cudaFreeHost(c->h_q);
         delete c;
@@ -326,6 +330,7 @@ static void lru_delete(bcmc_lru* c)
     dev_free(ctx, c->status, c->status_words * 8);
     dev_free(ctx, c->age_hist, (size_t)kAgeBins * 4);
     dev_free(ctx, c->age_rank, (size_t)kAgeBins);
+    dev_free(ctx, c->sort_counts, sort_count_bytes(ctx));
     dev_free(ctx, c->q, sizeof(QueryState));
     if (c->h_q) cudaFreeHost(c->h_q);
     delete c;
@@ -343,6 +348,7 @@ static SortBuffers lru_sort_buffers(bcmc_lru* c)
     b.c_vals = c->sort_cv;
     b.status = c->st_sort;
     b.age_rank = c->age_rank;
+    b.counts = c->sort_counts;
     return b;
 }
 
@@ -578,6 +584,7 @@ bcmc_status bcmc_ctx_create(const bcmc_opts* opts, bcmc_ctx** out)
         BCMC_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
         ctx->d_prim = (QueryState*)dev_alloc(ctx, sizeof(QueryState));
         BCMC_CUDA(cudaMemset(ctx->d_prim, 0, sizeof(QueryState)));
+        ctx->d_counts = (uint16_t*)dev_alloc(ctx, sort_count_bytes(ctx));
         BCMC_CUDA(cudaMallocHost(&ctx->h_pinned, 4096));
         return BCMC_OK;
     });
@@ -1175,9 +1182,11 @@ bcmc_status bcmc_sort_pairs_u32(bcmc_ctx* ctx, uint32_t* d_keys, uint32_t* d_val
         b.c_keys = ctx->d_scratch + 2 * (size_t)n;
         b.c_vals = ctx->d_scratch + 3 * (size_t)n;
         b.status = ctx->d_status;
+        b.counts = ctx->d_counts;
+        b.out_keys = d_keys;
+        b.out_vals = d_values;
         prim_begin(ctx->d_prim, s);
         sort_launch(ctx, ctx->d_prim, nullptr, n, b, reverse ? 1 : 0, s);
-        sort_writeback(ctx, ctx->d_prim, nullptr, n, b, d_keys, d_values, reverse ? 1 : 0, s);
         return BCMC_OK;
     });
 }

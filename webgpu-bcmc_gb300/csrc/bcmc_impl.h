@@ -20,6 +20,7 @@ struct bcmc_ctx {
     bcmc::QueryState* d_prim = nullptr;
     uint64_t* d_status = nullptr;  // look-back status words for primitives
     size_t status_words = 0;
+    uint16_t* d_counts = nullptr;   // the sort's tile counts (sort_count_bytes)
     uint32_t* d_scratch = nullptr;  // sort ping-pong buffers for primitives
     size_t scratch_words = 0;
     uint32_t* h_pinned = nullptr;   // small pinned host staging
@@ -91,7 +92,8 @@ constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys per tile
 // Plan + onesweep passes over n (device-resident) pairs.  Input arrays are in
 // natural order; the first pass applies the reference's tie-order permutation
 // and the key transform (~key when descending).  Result lands in buffer
-// q->sort_final (1 = b, 2 = c) as transformed keys + values.
+// q->sort_final (1 = b, 2 = c) as transformed keys + values, or in out_keys and
+// out_vals where those are set (the input's own arrays may be).
 struct SortBuffers {
     const uint32_t* in_keys;
     const uint32_t* in_vals;
@@ -102,16 +104,18 @@ struct SortBuffers {
     uint64_t* status;  // kSortTileStatus words per tile (256 per tile)
     // the LRU's age sort: dense rank of each age bin (age_bin; sort_key16 == 2)
     const uint8_t* age_rank = nullptr;
+    // set: the sorted pairs go there (keys as they came in), not to b or c
+    uint32_t* out_keys = nullptr;
+    uint32_t* out_vals = nullptr;
+    // room for the tiles' digit counts when all run at once (sort_count_bytes)
+    uint16_t* counts = nullptr;
 };
 // plan_ready: the keys' producer already made the pass plan and bucket
 // offsets in q (sort_plan), so the histogram kernel is not launched.
 void sort_launch(bcmc_ctx* ctx, QueryState* q, const uint32_t* d_n, uint32_t n_max,
                  const SortBuffers& bufs, int reverse, cudaStream_t s, int plan_ready = 0);
-// Copies the sorted pairs back to (keys, values) with the inverse key transform.
-void sort_writeback(bcmc_ctx* ctx, QueryState* q, const uint32_t* d_n, uint32_t n_max,
-                    const SortBuffers& bufs, uint32_t* keys, uint32_t* vals, int reverse,
-                    cudaStream_t s);
 size_t sort_status_words(uint32_t n_max);
+size_t sort_count_bytes(bcmc_ctx* ctx);
 int sort_grid(bcmc_ctx* ctx, uint32_t n_max);
 
 // ---- scan.cu ----------------------------------------------------------------

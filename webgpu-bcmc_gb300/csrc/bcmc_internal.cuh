@@ -337,13 +337,16 @@ __device__ __forceinline__ void cta_prefix_sums(uint64_t* status_a, uint64_t* st
 // ping-pong between the two sort buffers, the first reading the input.
 // `hist` holds the raw histograms of the first `ndig` digits; the digits
 // after them are not sorted on (their passes are skipped).
+// Called by all kThreads threads of a CTA (256 or more; the first 256 have a digit each).
+template <int kThreads>
 __device__ __forceinline__ void sort_plan(QueryState* q, uint32_t n, uint32_t* warp_sums, const uint32_t* hist,
                                           int ndig)
 {
+    const bool mine = threadIdx.x < 256u;
     uint32_t* gh = &q->sort_hist[0][0];
     uint32_t run[4], hv[4];
 #pragma unroll
-    for (int d = 0; d < 4; ++d) hv[d] = d < ndig ? __ldcg(hist + d * 256 + threadIdx.x) : 0u;  // all in flight
+    for (int d = 0; d < 4; ++d) hv[d] = d < ndig && mine ? __ldcg(hist + d * 256 + threadIdx.x) : 0u;  // all in flight
     for (int d = 0; d < 4; ++d) {
         if (d >= ndig) {
             run[d] = 0;
@@ -353,8 +356,8 @@ __device__ __forceinline__ void sort_plan(QueryState* q, uint32_t n, uint32_t* w
         const int full = __syncthreads_or(n > 0 && v == n);
         run[d] = (n > 0 && !full) ? 1u : 0u;
         uint32_t tot;
-        const uint32_t ex = cta_exclusive_scan<256>(v, warp_sums, &tot);
-        gh[d * 256 + threadIdx.x] = ex;
+        const uint32_t ex = cta_exclusive_scan<kThreads>(v, warp_sums, &tot);
+        if (mine) gh[d * 256 + threadIdx.x] = ex;
     }
     if (threadIdx.x == 0) {
         if (n > 0 && !(run[0] | run[1] | run[2] | run[3])) run[0] = 1;  // permutation still applies

@@ -619,9 +619,9 @@ __global__ void __launch_bounds__(kActThreads) k_slots(QueryState* q, SlotArgs a
         q->sort_key16 = dense ? 2u : (key16 ? 1u : 0u);
         q->sort_prev_dense = dense ? 1u : 0u;
     }
-    if (dense) sort_plan(q, q->num_avail, s_warp, rank_hist, 1);
-    else if (key16) sort_plan(q, q->num_avail, s_warp, &q->sort_hist16[0][0], 2);
-    else sort_plan(q, q->num_avail, s_warp, &q->sort_hist[0][0], 4);
+    if (dense) sort_plan<kActThreads>(q, q->num_avail, s_warp, rank_hist, 1);
+    else if (key16) sort_plan<kActThreads>(q, q->num_avail, s_warp, &q->sort_hist16[0][0], 2);
+    else sort_plan<kActThreads>(q, q->num_avail, s_warp, &q->sort_hist[0][0], 4);
 }
 
 // ---------------------------------------------------------------------------

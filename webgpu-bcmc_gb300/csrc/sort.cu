@@ -16,8 +16,8 @@
 // read, exclusive bucket offsets, and which digit passes can be skipped because
 // every key shares the digit), then one cooperative kernel that runs the onesweep
 // pass of each digit the plan keeps, grid barriers between them: tiles of 4096
-// keys are ranked with warp match/popc, each tile publishes its 256 digit
-// counts through decoupled look-back, and keys are scattered via shared memory
+// keys are ranked with warp match/popc, each tile finds its 256 digits' places
+// from the tiles' counts before it, and keys are scattered via shared memory
 // so that global writes come out in runs.
 //
 // The LRU's age sort skips the histogram kernel: k_slots, which compacts the
@@ -46,33 +46,37 @@ __device__ __forceinline__ uint32_t tie_perm(uint32_t q, uint32_t n, int reverse
     return 64u * (chunks - 2u - (qq >> 6)) + (qq & 63u);
 }
 
-__global__ void __launch_bounds__(256) k_sort_hist(QueryState* q, const uint32_t* d_n, uint32_t n_host,
+constexpr int kHistThreads = 512;
+
+__global__ void __launch_bounds__(kHistThreads) k_sort_hist(QueryState* q, const uint32_t* d_n, uint32_t n_host,
                                                    const uint32_t* __restrict__ keys, int reverse)
 {
     __shared__ uint32_t h[4 * 256];
-    __shared__ uint32_t warp_sums[9];
+    __shared__ uint32_t warp_sums[kHistThreads / 32 + 1];
     __shared__ bool is_last;
     const uint32_t n = d_n ? *d_n : n_host;
-    for (int i = threadIdx.x; i < 1024; i += 256) h[i] = 0;
+    for (int i = threadIdx.x; i < 1024; i += kHistThreads) h[i] = 0;
     __syncthreads();
-    // one shared atomic per distinct digit and warp: keys such as cache-slot
-    // ages take few distinct values, and per-key atomics on them serialise
-    for (uint32_t i0 = blockIdx.x * 256u; i0 < n; i0 += gridDim.x * 256u) {
-        const uint32_t i = i0 + threadIdx.x;
-        const bool valid = i < n;
-        uint32_t k = valid ? keys[i] : 0u;
-        if (reverse) k = ~k;
+    // plain increments: shared memory adds up a warp's increments of one counter
+    // by itself, whether the keys are spread (a match per digit and warp took
+    // 39 us on 2^20 random keys) or take few distinct values, as ages do; few
+    // CTAs, since each ends with an atomic per counter
+    const uint32_t flip = reverse ? 0xffffffffu : 0u;
+    const uint32_t step = gridDim.x * kHistThreads;
+    for (uint32_t i0 = blockIdx.x * kHistThreads + threadIdx.x; i0 < n; i0 += 8u * step) {
+        uint32_t k[8];
 #pragma unroll
-        for (int d = 0; d < 4; ++d) {
-            const uint32_t digit = valid ? (k >> (8 * d)) & 255u : 256u;
-            const uint32_t peers = __match_any_sync(0xffffffffu, digit);
-            if (valid && (threadIdx.x & 31u) == (uint32_t)__ffs(peers) - 1u)
-                atomicAdd(&h[256 * d + digit], (uint32_t)__popc(peers));
-        }
+        for (int u = 0; u < 8; ++u) k[u] = i0 + u * step < n ? __ldg(keys + i0 + u * step) : 0u;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (i0 + u * step < n) {
+#pragma unroll
+                for (int d = 0; d < 4; ++d) atomicAdd(&h[256 * d + (((k[u] ^ flip) >> (8 * d)) & 255u)], 1u);
+            }
     }
     __syncthreads();
     uint32_t* gh = &q->sort_hist[0][0];
-    for (int i = threadIdx.x; i < 1024; i += 256)
+    for (int i = threadIdx.x; i < 1024; i += kHistThreads)
         if (h[i]) atomicAdd(gh + i, h[i]);
     __threadfence();
     __syncthreads();
@@ -80,66 +84,94 @@ __global__ void __launch_bounds__(256) k_sort_hist(QueryState* q, const uint32_t
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    sort_plan(q, n, warp_sums, &q->sort_hist[0][0], 4);
+    sort_plan<kHistThreads>(q, n, warp_sums, &q->sort_hist[0][0], 4);
+}
+
+// Grid barrier of the first `ctas` CTAs of k_sort, its n-th (counted by the
+// caller): every CTA's stores before it are seen by every CTA after it.
+__device__ __forceinline__ void sort_barrier(QueryState* q, uint32_t n, uint32_t ctas)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(&q->sort_arrived, 1u);
+        uint32_t spins = 0;
+        while (*reinterpret_cast<volatile uint32_t*>(&q->sort_arrived) < n * ctas) {
+            if (++spins > kSpinLimit) {
+                atomicCAS(&q->error, 0u, 28u);
+                break;
+            }
+            if (spins > 8) __nanosleep(100);
+        }
+        __threadfence();
+    }
+    __syncthreads();
 }
 
 // All the digit passes of the plan in one cooperative launch: the passes
 // that run are separated by grid barriers (each reads what the one before it
 // scattered, so its key and value loads bypass L1), the others cost nothing.
+//
+// A tile's place for each digit is the sum of the tiles' counts before it.  Where
+// every tile has a CTA of its own (up to 304 tiles), all have their counts at the
+// same time and a look-back walks over nearly all of them, eight to a round trip;
+// there the tiles store their counts, pass a barrier, and each adds up the rows
+// before its own, 256 counts to a warp's load, in one round (kSortWave: from so
+// many tiles on the barrier and the sum are the faster; below, the walk is short).
+// More tiles are claimed in order and look back, which then mostly finds sums.
+// 2^20 random pairs: 88 us by look-back, four passes.
+//
+// b.out_keys set: the last pass scatters to there, with the key transform undone,
+// unless it is the only one (its input lies there): then the CTAs copy at the end.
+constexpr uint32_t kSortWave = 8;
+
 __global__ void __launch_bounds__(kSortThreads, 2) k_sort(QueryState* q, const uint32_t* d_n, uint32_t n_host,
                                                        SortBuffers b, int reverse)
 {
-    __shared__ uint32_t s_keys[kSortTile];
-    __shared__ uint32_t s_vals[kSortTile];
-    __shared__ uint16_t s_whist[kSortThreads / 32][256];  // per warp and digit: < 2^16
+    __shared__ __align__(16) uint32_t s_keys[kSortTile];
+    __shared__ __align__(16) uint32_t s_vals[kSortTile];
+    __shared__ __align__(16) uint16_t s_whist[kSortThreads / 32][256];  // per warp and digit: < 2^16
     __shared__ uint32_t s_start[256];
     __shared__ uint32_t s_gbase[256];
     __shared__ uint32_t s_warp_sums[kSortThreads / 32 + 1];
     __shared__ uint32_t s_tile;
 
     const uint32_t n = d_n ? *d_n : n_host;
-    uint32_t barriers = 0;  // thread 0's count of grid barriers passed
-    bool ran = false;
+    const uint32_t ntiles = div_up(n, kSortTile);
+    const bool wave = b.counts && ntiles >= kSortWave && ntiles <= gridDim.x;
+    const uint32_t ctas = wave ? ntiles : gridDim.x;
+    if (blockIdx.x >= ctas) return;
+    uint32_t barriers = 0;
+    int last = -1, ran = 0;
+    for (int pass = 0; pass < 4; ++pass)
+        if (q->sort_run[pass]) last = pass;
     for (int pass = 0; pass < 4; ++pass) {
         if (!q->sort_run[pass]) continue;
-        if (ran) {
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                __threadfence();
-                ++barriers;
-                atomicAdd(&q->sort_arrived, 1u);
-                uint32_t spins = 0;
-                while (*reinterpret_cast<volatile uint32_t*>(&q->sort_arrived) < barriers * gridDim.x) {
-                    if (++spins > kSpinLimit) {
-                        atomicCAS(&q->error, 0u, 28u);
-                        break;
-                    }
-                    if (spins > 8) __nanosleep(100);
-                }
-                __threadfence();
-            }
-            __syncthreads();
-        }
-        ran = true;
+        if (ran++) sort_barrier(q, ++barriers, ctas);
         const uint32_t src = q->sort_src[pass];
+        const bool to_out = b.out_keys && pass == last && src != 0;
         const uint32_t* __restrict__ ks = src == 0 ? b.in_keys : (src == 1 ? b.b_keys : b.c_keys);
         const uint32_t* __restrict__ vs = src == 0 ? b.in_vals : (src == 1 ? b.b_vals : b.c_vals);
-        uint32_t* __restrict__ kd = src == 1 ? b.c_keys : b.b_keys;
-        uint32_t* __restrict__ vd = src == 1 ? b.c_vals : b.b_vals;
+        uint32_t* __restrict__ kd = to_out ? b.out_keys : (src == 1 ? b.c_keys : b.b_keys);
+        uint32_t* __restrict__ vd = to_out ? b.out_vals : (src == 1 ? b.c_vals : b.b_vals);
+        const uint32_t undo = to_out && reverse ? 0xffffffffu : 0u;
         const bool gather = src == 0;
         const uint32_t kmode = q->sort_key16;  // 0: the keys, 1: 16-bit age keys, 2: their dense ranks
         const uint32_t shift = 8u * (uint32_t)pass;
         const uint32_t epoch = q->epoch * 4u + (uint32_t)pass;
-        const uint32_t ntiles = div_up(n, kSortTile);
         const uint32_t* bucket = q->sort_hist[pass];
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const uint32_t lt_mask = (1u << lane) - 1u;
 
         for (;;) {
-            if (threadIdx.x == 0) s_tile = atomicAdd(&q->tiles_sort[pass], 1u);
-            for (int i = threadIdx.x; i < (kSortThreads / 32) * 256; i += kSortThreads) (&s_whist[0][0])[i] = 0;
+            if (!wave && threadIdx.x == 0) s_tile = atomicAdd(&q->tiles_sort[pass], 1u);
+            reinterpret_cast<uint4*>(&s_whist[0][0])[threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                reinterpret_cast<uint4*>(s_vals)[threadIdx.x + i * kSortThreads] = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();
-            const uint32_t tile = s_tile;
+            uint32_t* mask = s_vals + warp * 256;  // lanes by digit; s_vals is used for values only later
+            const uint32_t tile = wave ? blockIdx.x : s_tile;
             if (tile >= ntiles) break;
 
             uint32_t key[kSortItems], val[kSortItems], rank[kSortItems];
@@ -165,11 +197,26 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(QueryState* q, const u
 #pragma unroll
             for (int j = 0; j < kSortItems; ++j) {
                 const uint32_t qi = base + 32u * j + lane;
-                const uint32_t digit = qi < n ? (key[j] >> shift) & 255u : 256u;
-                const uint32_t peers = __match_any_sync(0xffffffffu, digit);
-                const uint32_t cnt = digit < 256u ? s_whist[warp][digit] : 0u;
+                const uint32_t digit = (key[j] >> shift) & 255u;
+                // the lanes with the same digit.  Spread digits: each lane sets its
+                // bit in the digit's mask, and the first of them clears it again
+                // (a match took 82 us on 2^20 random pairs, a ballot per bit 68,
+                // this 61).  Ages have few values, which a match finds at once and
+                // whose masks the lanes would queue for
+                uint32_t peers;
+                if (kmode == 0u) {
+                    if (qi < n) atomicOr(&mask[digit], 1u << lane);
+                    __syncwarp();
+                    peers = qi < n ? mask[digit] : 0u;
+                } else {
+                    peers = __match_any_sync(0xffffffffu, qi < n ? digit : 256u);
+                }
+                const uint32_t cnt = qi < n ? s_whist[warp][digit] : 0u;
                 __syncwarp();
-                if (digit < 256u && lane == __ffs(peers) - 1) s_whist[warp][digit] = (uint16_t)(cnt + __popc(peers));
+                if (qi < n && lane == __ffs(peers) - 1) {
+                    s_whist[warp][digit] = (uint16_t)(cnt + __popc(peers));
+                    mask[digit] = 0u;
+                }
                 __syncwarp();
                 rank[j] = cnt + __popc(peers & lt_mask);
             }
@@ -184,10 +231,37 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(QueryState* q, const u
                     s_whist[w][t] = (uint16_t)run;
                     run += c;
                 }
+                if (wave) b.counts[tile * 256u + t] = (uint16_t)run;
             }
             uint32_t tile_total;
             const uint32_t start = cta_exclusive_scan<kSortThreads>(run, s_warp_sums, &tile_total);
-            if (t < 256) {
+            if (wave) {
+                sort_barrier(q, ++barriers, ctas);
+                // rows of counts before this tile's, every sixteenth to a warp
+                static_assert(kSortThreads == 512 && kSortTile == 4096, "16 warps: 8 KB of counts, 16 KB of masks or sums");
+                uint32_t sum[8] = {};
+#pragma unroll 4
+                for (uint32_t k = (uint32_t)warp; k < tile; k += kSortThreads / 32) {
+                    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(b.counts + k * 256u) + lane);
+                    const uint32_t c[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        sum[2 * i] += c[i] & 0xffffu;
+                        sum[2 * i + 1] += c[i] >> 16;
+                    }
+                }
+                uint4* part = reinterpret_cast<uint4*>(s_keys + warp * 256 + lane * 8);
+                part[0] = make_uint4(sum[0], sum[1], sum[2], sum[3]);
+                part[1] = make_uint4(sum[4], sum[5], sum[6], sum[7]);
+                __syncthreads();
+                if (t < 256) {
+                    uint32_t excl = 0;
+#pragma unroll
+                    for (int w = 0; w < kSortThreads / 32; ++w) excl += s_keys[w * 256 + t];
+                    s_start[t] = start;
+                    s_gbase[t] = bucket[t] + excl - start;
+                }
+            } else if (t < 256) {
                 s_start[t] = start;
                 const uint32_t excl = lookback_exclusive_w8(b.status + t, tile, run, epoch, &q->error, 20u + pass, 256u);
                 s_gbase[t] = bucket[t] + excl - start;
@@ -208,27 +282,22 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(QueryState* q, const u
             for (uint32_t i = threadIdx.x; i < count; i += kSortThreads) {
                 const uint32_t k = s_keys[i];
                 const uint32_t pos = s_gbase[(k >> shift) & 255u] + i;
-                if (pos < n) {  // always true unless a look-back wait timed out
-                    kd[pos] = k;
+                if (pos < n) {  // always true unless a wait timed out
+                    kd[pos] = k ^ undo;
                     vd[pos] = s_vals[i];
                 }
             }
             __syncthreads();
+            if (wave) break;
         }
     }
-}
-
-__global__ void k_sort_writeback(QueryState* q, const uint32_t* d_n, uint32_t n_host, SortBuffers b,
-                                 uint32_t* keys, uint32_t* vals, int reverse)
-{
-    const uint32_t n = d_n ? *d_n : n_host;
-    const uint32_t f = q->sort_final;
-    const uint32_t* ks = f == 1 ? b.b_keys : b.c_keys;
-    const uint32_t* vs = f == 1 ? b.b_vals : b.c_vals;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t k = ks[i];
-        keys[i] = reverse ? ~k : k;
-        vals[i] = vs[i];
+    if (b.out_keys && ran == 1) {  // one pass: in b
+        sort_barrier(q, ++barriers, ctas);
+        for (uint32_t i = blockIdx.x * kSortThreads + threadIdx.x; i < n; i += ctas * kSortThreads) {
+            const uint32_t k = __ldcg(b.b_keys + i);
+            b.out_keys[i] = reverse ? ~k : k;
+            b.out_vals[i] = __ldcg(b.b_vals + i);
+        }
     }
 }
 
@@ -245,6 +314,8 @@ static uint32_t sort_per_sm()
     return n;
 }
 
+size_t sort_count_bytes(bcmc_ctx* ctx) { return (size_t)ctx->num_sms * sort_per_sm() * 256u * 2u; }
+
 int sort_grid(bcmc_ctx* ctx, uint32_t n_max)
 {
     const uint32_t tiles = div_up(n_max ? n_max : 1, kSortTile);
@@ -256,8 +327,8 @@ void sort_launch(bcmc_ctx* ctx, QueryState* q, const uint32_t* d_n, uint32_t n_m
                  const SortBuffers& bufs, int reverse, cudaStream_t s, int plan_ready)
 {
     if (!plan_ready) {
-        const int hist_grid = (int)min(div_up(n_max ? n_max : 1, 256u * 8u), (uint32_t)ctx->num_sms * 4u);
-        k_sort_hist<<<hist_grid, 256, 0, s>>>(q, d_n, n_max, bufs.in_keys, reverse);
+        const int hist_grid = (int)min(div_up(n_max ? n_max : 1, (uint32_t)kHistThreads * 8u), (uint32_t)ctx->num_sms);
+        k_sort_hist<<<hist_grid, kHistThreads, 0, s>>>(q, d_n, n_max, bufs.in_keys, reverse);
         count_launches(1);
     }
     // cooperative: the grid barriers between digit passes need every CTA resident
@@ -273,16 +344,6 @@ void sort_launch(bcmc_ctx* ctx, QueryState* q, const uint32_t* d_n, uint32_t n_m
     cfg.numAttrs = 1;
     BCMC_CUDA(cudaLaunchKernelEx(&cfg, k_sort, q, d_n, n_max, bufs, reverse));
     count_launches(1);
-}
-
-void sort_writeback(bcmc_ctx* ctx, QueryState* q, const uint32_t* d_n, uint32_t n_max,
-                    const SortBuffers& bufs, uint32_t* keys, uint32_t* vals, int reverse,
-                    cudaStream_t s)
-{
-    const int grid = (int)min(div_up(n_max ? n_max : 1, 256u), (uint32_t)ctx->num_sms * 8u);
-    k_sort_writeback<<<grid, 256, 0, s>>>(q, d_n, n_max, bufs, keys, vals, reverse);
-    count_launches(1);
-    BCMC_CUDA(cudaGetLastError());
 }
 
 }  // namespace bcmc
