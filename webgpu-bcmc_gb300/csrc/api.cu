@@ -1099,7 +1099,7 @@ bcmc_status bcmc_scan_exclusive_u32_async(bcmc_ctx* ctx, const uint32_t* d_in, u
         }
         ensure_status(ctx, div_up(n, kScanTile) + 1);
         prim_begin(ctx->d_prim, s);
-        scan_launch(ctx, ctx->d_prim, d_in, d_out, n, d_total, ctx->d_status, s);
+        scan_launch(ctx, ctx->d_prim, d_in, d_out, n, ScanTotals{d_total}, ctx->d_status, s);
         return BCMC_OK;
     });
 }
@@ -1110,19 +1110,19 @@ bcmc_status bcmc_scan_exclusive_u32(bcmc_ctx* ctx, uint32_t* d_data, uint32_t n,
     if (!ctx || (n && !d_data) || aligned_size < n) return BCMC_E_ARG;
     return guarded(ctx, [&]() -> bcmc_status {
         cudaStream_t s = ctx->stream;
-        uint32_t* d_tot = &ctx->d_prim->pad[0];
         if (n == 0) {
-            BCMC_CUDA(cudaMemsetAsync(d_tot, 0, 4, s));
-        } else {
-            ensure_status(ctx, div_up(n, kScanTile) + 1);
-            prim_begin(ctx->d_prim, s);
-            scan_launch(ctx, ctx->d_prim, d_data, d_data, n, d_tot, ctx->d_status, s);
+            if (aligned_size) BCMC_CUDA(cudaMemsetAsync(d_data, 0, 4, s));
+            BCMC_CUDA(cudaStreamSynchronize(s));
+            if (total) *total = 0;
+            return BCMC_OK;
         }
-        if (n < aligned_size) BCMC_CUDA(cudaMemcpyAsync(d_data + n, d_tot, 4, cudaMemcpyDeviceToDevice, s));
-        BCMC_CUDA(cudaMemcpyAsync(ctx->h_pinned, d_tot, 4, cudaMemcpyDeviceToHost, s));
-        BCMC_CUDA(cudaMemcpyAsync(ctx->h_pinned + 1, &ctx->d_prim->error, 4, cudaMemcpyDeviceToHost, s));
+        ensure_status(ctx, div_up(n, kScanTile) + 1);
+        prim_begin(ctx->d_prim, s);
+        ctx->h_pinned[0] = ctx->h_pinned[1] = 0;  // the kernel stores the total, and whether a wait timed out
+        scan_launch(ctx, ctx->d_prim, d_data, d_data, n,
+                    ScanTotals{nullptr, n < aligned_size ? d_data + n : nullptr, ctx->h_pinned}, ctx->d_status, s);
         BCMC_CUDA(cudaStreamSynchronize(s));
-        if (n && ctx->h_pinned[1]) return fail(ctx, BCMC_E_TIMEOUT, "device wait timed out");
+        if (ctx->h_pinned[1]) return fail(ctx, BCMC_E_TIMEOUT, "device wait timed out");
         if (total) *total = ctx->h_pinned[0];
         return BCMC_OK;
     });

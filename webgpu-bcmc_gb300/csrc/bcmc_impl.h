@@ -119,11 +119,17 @@ size_t sort_count_bytes(bcmc_ctx* ctx);
 int sort_grid(bcmc_ctx* ctx, uint32_t n_max);
 
 // ---- scan.cu ----------------------------------------------------------------
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = 16;
-constexpr int kScanTile = kScanThreads * kScanItems;
+constexpr int kScanTile = 4096;  // elements per status word
+// Where a scan's total goes, each nullable: device memory, the word after the
+// scanned data, page-locked host memory (whose second word is set if a wait
+// timed out).
+struct ScanTotals {
+    uint32_t* device = nullptr;
+    uint32_t* after = nullptr;
+    uint32_t* host = nullptr;
+};
 void scan_launch(bcmc_ctx* ctx, QueryState* q, const uint32_t* in, uint32_t* out, uint32_t n,
-                 uint32_t* d_total, uint64_t* status, cudaStream_t s);
+                 const ScanTotals& tot, uint64_t* status, cudaStream_t s);
 // Same kernel as scan_launch, sized from an SM count instead of a context;
 // reports a launch error by return value (throws nothing).
 cudaError_t scan_launch_sms(int num_sms, QueryState* q, const uint32_t* in, uint32_t* out, uint32_t n,

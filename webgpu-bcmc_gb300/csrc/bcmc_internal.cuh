@@ -330,6 +330,34 @@ __device__ __forceinline__ void cta_prefix_sums(uint64_t* status_a, uint64_t* st
     }
 }
 
+// The same for one count; true when this thread's wait timed out.
+template <int kThreads>
+__device__ __forceinline__ bool cta_prefix_sum(uint64_t* status, uint32_t rank, uint32_t a, uint32_t epoch, uint32_t* err,
+                                               uint32_t site, uint32_t* sum, bool drop = false)
+{
+    if (threadIdx.x == 0 && !drop) lb_store(status + rank, lb_pack(epoch, kFlagAggregate, a));
+    uint32_t sa = 0;
+    bool late = false;
+    for (uint32_t p = threadIdx.x; p < rank; p += kThreads) {
+        uint64_t v;
+        uint32_t spins = 0;
+        for (;;) {
+            v = lb_load(status + p);
+            if ((uint32_t)(v >> 34) == epoch) break;
+            if (++spins > kSpinLimit) {
+                atomicCAS(err, 0u, site);
+                late = true;
+                break;
+            }
+            if (spins > 8) __nanosleep(100);
+        }
+        sa += (uint32_t)v;
+    }
+    sa = __reduce_add_sync(0xffffffffu, sa);
+    if ((threadIdx.x & 31u) == 0u && sa) atomicAdd(sum, sa);
+    return late;
+}
+
 // The radix sort's pass plan, made by the last of the CTAs that accumulated
 // the four raw 8-bit digit histograms in q->sort_hist (256 threads, after a
 // fence): a digit pass is skipped when every one of the n keys has the same

@@ -5,8 +5,8 @@
 // add_block_sums.comp) per 512^2-element chunk with a host-side carry and a
 // mapAsync readback of the total, and StreamCompact.compactActiveIDs
 // (js/stream_compact.js:56-165, stream_compact.comp:26-32), one thread per
-// workgroup.  Here a scan is one launch: 4096-element tiles scanned with warp
-// shuffles, tiles chained by decoupled look-back.  uint32 sums wrap mod 2^32 as
+// workgroup.  Here a scan is one launch: a range of 8192-element tiles per CTA,
+// scanned with warp shuffles, the ranges joined by their published sums.  uint32 sums wrap mod 2^32 as
 // in the reference.
 #include "bcmc_impl.h"
 
@@ -40,162 +40,177 @@ void prim_begin(QueryState* q, cudaStream_t s)
     BCMC_CUDA(cudaGetLastError());
 }
 
-// Shared-memory index with one pad word per 32, so that both the striped
-// (coalesced) and the per-thread-consecutive views are free of bank conflicts.
-__device__ __forceinline__ uint32_t spad(uint32_t i) { return i + (i >> 5); }
-constexpr int kScanSmem = kScanTile + kScanTile / 32;
+// A CTA owns one contiguous range of tiles: it adds them up, publishes the sum,
+// adds up the sums of the CTAs before it in one round trip (their ranks are
+// claimed in order, so all of them run), and scans its tiles again from there --
+// out of its registers when the range is one tile, which it is up to 5 M
+// elements, else out of L2.  Tiles claimed one by one with a look-back each took
+// 25 us on 4 M elements, most of it in the chain from tile to tile.
+// Loads and stores are 16 bytes where the arrays allow it (kWide).
+constexpr int kRangeThreads = 512;
+constexpr int kRangeItems = 16;  // consecutive elements per thread
+constexpr uint32_t kRangeTile = kRangeThreads * kRangeItems;
+constexpr int kRangePerSm = 3;
+static_assert(kRangeTile % kScanTile == 0, "the status words are sized by kScanTile");
 
-// Loads a tile striped (coalesced) into shared memory, then each thread owns
-// kScanItems consecutive elements.
-template <typename Op>
-__device__ __forceinline__ void tile_scan(const uint32_t* __restrict__ in, uint32_t n, uint32_t tile,
-                                          uint32_t* s_buf, uint32_t* s_warp, Op per_item_value,
-                                          uint32_t vals[kScanItems], uint32_t* thread_excl,
-                                          uint32_t* tile_total)
+template <bool kWide>
+__device__ __forceinline__ void load_items(const uint32_t* in, uint64_t first, uint32_t n, uint32_t v[kRangeItems])
 {
-    const uint32_t base = tile * kScanTile;
+    if (kWide && first + kRangeItems <= n) {
 #pragma unroll
-    for (int j = 0; j < kScanItems; ++j) {
-        const uint32_t i = base + j * kScanThreads + threadIdx.x;
-        s_buf[spad(j * kScanThreads + threadIdx.x)] = i < n ? in[i] : 0u;
+        for (int j = 0; j < kRangeItems / 4; ++j) {
+            const uint4 x = reinterpret_cast<const uint4*>(in + first)[j];
+            v[4 * j] = x.x;
+            v[4 * j + 1] = x.y;
+            v[4 * j + 2] = x.z;
+            v[4 * j + 3] = x.w;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < kRangeItems; ++j) v[j] = first + j < n ? in[first + j] : 0u;
+    }
+}
+
+// kSelect: the input is flags, the output the indices of the nonzero ones;
+// otherwise the output is the exclusive scan.
+template <bool kSelect, bool kWide>
+__global__ void __launch_bounds__(kRangeThreads, kRangePerSm) k_scan(QueryState* q, const uint32_t* in, uint32_t* out,
+                                                                     uint32_t n, uint32_t per_cta, ScanTotals tot,
+                                                                     uint64_t* status)
+{
+    __shared__ uint32_t s_warp[kRangeThreads / 32 + 1];
+    __shared__ uint32_t s_rank, s_sum, s_prefix;
+    const uint32_t t = threadIdx.x;
+    if (t == 0) {
+        s_rank = atomicAdd(&q->tiles_active, 1u);
+        s_sum = s_prefix = 0;
     }
     __syncthreads();
-    uint32_t sum = 0;
+    const uint32_t rank = s_rank, ntiles = div_up(n, kRangeTile);
+    const uint32_t first = rank * per_cta, end = min(ntiles, first + per_cta);
+    uint32_t v[kRangeItems], sum = 0, all = 0;
+    for (uint32_t tile = first; tile < end; ++tile) {
+        load_items<kWide>(in, (uint64_t)tile * kRangeTile + t * kRangeItems, n, v);
+        sum = 0;
 #pragma unroll
-    for (int j = 0; j < kScanItems; ++j) {
-        const uint32_t v = per_item_value(s_buf[spad(threadIdx.x * kScanItems + j)]);
-        vals[j] = v;
-        sum += v;
+        for (int j = 0; j < kRangeItems; ++j) sum += kSelect ? (v[j] != 0u ? 1u : 0u) : v[j];
+        all += sum;
     }
+    all = __reduce_add_sync(0xffffffffu, all);
+    if ((t & 31u) == 0u && all) atomicAdd(&s_sum, all);
     __syncthreads();
-    *thread_excl = cta_exclusive_scan<kScanThreads>(sum, s_warp, tile_total);
-}
-
-__global__ void __launch_bounds__(kScanThreads) k_scan(QueryState* q, const uint32_t* __restrict__ in,
-                                                       uint32_t* out, uint32_t n, uint32_t* d_total,
-                                                       uint64_t* status)
-{
-    __shared__ uint32_t s_buf[kScanSmem];
-    __shared__ uint32_t s_warp[kScanThreads / 32 + 1];
-    __shared__ uint32_t s_tile, s_prefix;
-    const uint32_t ntiles = div_up(n, kScanTile);
-    const uint32_t epoch = q->epoch;
-    for (;;) {
-        if (threadIdx.x == 0) s_tile = atomicAdd(&q->tiles_active, 1u);
-        __syncthreads();
-        const uint32_t tile = s_tile;
-        if (tile >= ntiles) break;
-        uint32_t vals[kScanItems], excl, total;
-        tile_scan(in, n, tile, s_buf, s_warp, [](uint32_t v) { return v; }, vals, &excl, &total);
-        if (threadIdx.x < 32) {
-            const uint32_t p = lb_dropped(q, tile) ? 0u : warp_lookback(status, tile, total, epoch, &q->error, 1u);
-            if (threadIdx.x == 0) {
-                s_prefix = p;
-                if (tile == ntiles - 1 && d_total) *d_total = p + total;
+    const bool late = cta_prefix_sum<kRangeThreads>(status, rank, s_sum, q->epoch, &q->error, kSelect ? 2u : 1u,
+                                                    &s_prefix, lb_dropped(q, rank));
+    if (late && tot.host) tot.host[1] = 1u;
+    __syncthreads();
+    uint32_t run = s_prefix;
+    if (end == ntiles && t == 0) {
+        const uint32_t total = run + s_sum;
+        if (tot.device) *tot.device = total;
+        if (tot.after) *tot.after = total;
+        if (tot.host) tot.host[0] = total;
+    }
+    for (uint32_t tile = first; tile < end; ++tile) {
+        const uint64_t at = (uint64_t)tile * kRangeTile + t * kRangeItems;
+        if (end - first > 1u) {
+            load_items<kWide>(in, at, n, v);
+            sum = 0;
+#pragma unroll
+            for (int j = 0; j < kRangeItems; ++j) sum += kSelect ? (v[j] != 0u ? 1u : 0u) : v[j];
+        }
+        uint32_t total;
+        uint32_t pos = run + cta_exclusive_scan<kRangeThreads>(sum, s_warp, &total);
+        run += total;
+        if (kSelect) {
+#pragma unroll
+            for (int j = 0; j < kRangeItems; ++j)
+                if (v[j] != 0u) {
+                    if (pos < n) out[pos] = (uint32_t)at + j;  // pos < n unless a wait timed out
+                    ++pos;
+                }
+        } else if (kWide && at + kRangeItems <= n) {
+#pragma unroll
+            for (int j = 0; j < kRangeItems / 4; ++j) {
+                uint4 x;
+                x.x = pos;
+                x.y = x.x + v[4 * j];
+                x.z = x.y + v[4 * j + 1];
+                x.w = x.z + v[4 * j + 2];
+                pos = x.w + v[4 * j + 3];
+                reinterpret_cast<uint4*>(out + at)[j] = x;
             }
-        }
-        __syncthreads();
-        uint32_t run = s_prefix + excl;
+        } else {
 #pragma unroll
-        for (int j = 0; j < kScanItems; ++j) {
-            s_buf[spad(threadIdx.x * kScanItems + j)] = run;
-            run += vals[j];
+            for (int j = 0; j < kRangeItems; ++j)
+                if (at + j < n) {
+                    out[at + j] = pos;
+                    pos += v[j];
+                }
         }
-        __syncthreads();
-        const uint32_t base = tile * kScanTile;
-#pragma unroll
-        for (int j = 0; j < kScanItems; ++j) {
-            const uint32_t i = base + j * kScanThreads + threadIdx.x;
-            if (i < n) out[i] = s_buf[spad(j * kScanThreads + threadIdx.x)];
-        }
-        __syncthreads();
     }
 }
 
-// Fused scan + compaction: out[k] = index of the k-th nonzero flag.
-__global__ void __launch_bounds__(kScanThreads) k_select(QueryState* q, const uint32_t* __restrict__ flags,
-                                                         uint32_t* out, uint32_t n, uint32_t* d_count,
-                                                         uint64_t* status)
+// Four elements a thread where the arrays allow 16-byte loads (16 -> 7 us on 4 M).
+__global__ void __launch_bounds__(256) k_compact(uint32_t n, const uint32_t* __restrict__ flags,
+                                                 const uint32_t* __restrict__ offsets, uint32_t* out, bool wide)
 {
-    __shared__ uint32_t s_buf[kScanSmem];
-    __shared__ uint32_t s_warp[kScanThreads / 32 + 1];
-    __shared__ uint32_t s_tile, s_prefix;
-    const uint32_t ntiles = div_up(n, kScanTile);
-    const uint32_t epoch = q->epoch;
-    for (;;) {
-        if (threadIdx.x == 0) s_tile = atomicAdd(&q->tiles_active, 1u);
-        __syncthreads();
-        const uint32_t tile = s_tile;
-        if (tile >= ntiles) break;
-        uint32_t vals[kScanItems], excl, total;
-        tile_scan(flags, n, tile, s_buf, s_warp, [](uint32_t v) { return v != 0u ? 1u : 0u; }, vals, &excl,
-                  &total);
-        if (threadIdx.x < 32) {
-            const uint32_t p = lb_dropped(q, tile) ? 0u : warp_lookback(status, tile, total, epoch, &q->error, 2u);
-            if (threadIdx.x == 0) {
-                s_prefix = p;
-                if (tile == ntiles - 1 && d_count) *d_count = p + total;
-            }
-        }
-        __syncthreads();
-        uint32_t pos = s_prefix + excl;
-        const uint32_t first = tile * kScanTile + threadIdx.x * kScanItems;
-#pragma unroll
-        for (int j = 0; j < kScanItems; ++j)
-            if (vals[j]) {
-                if (pos < n) out[pos] = first + j;  // pos < n unless a look-back wait timed out
-                ++pos;
-            }
-        __syncthreads();
+    const uint32_t step = gridDim.x * blockDim.x, t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t fours = wide ? n / 4u : 0u;
+    for (uint32_t i = t; i < fours; i += step) {
+        const uint4 f = __ldg(reinterpret_cast<const uint4*>(flags) + i);
+        if (!(f.x | f.y | f.z | f.w)) continue;
+        const uint4 o = __ldg(reinterpret_cast<const uint4*>(offsets) + i);
+        if (f.x) out[o.x] = 4u * i;
+        if (f.y) out[o.y] = 4u * i + 1u;
+        if (f.z) out[o.z] = 4u * i + 2u;
+        if (f.w) out[o.w] = 4u * i + 3u;
     }
-}
-
-__global__ void k_compact(uint32_t n, const uint32_t* __restrict__ flags, const uint32_t* __restrict__ offsets,
-                          uint32_t* out)
-{
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    for (uint32_t i = 4u * fours + t; i < n; i += step)
         if (flags[i] != 0u) out[offsets[i]] = i;
 }
 
-static int persistent_grid(bcmc_ctx* ctx, uint32_t tiles, uint32_t per_sm)
+static bool aligned16(const void* a, const void* b)
 {
-    const uint32_t r = (uint32_t)ctx->num_sms * per_sm;
-    return (int)(tiles < r ? (tiles ? tiles : 1) : r);
+    return (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) % 16u == 0;
+}
+
+template <bool kSelect>
+static cudaError_t launch_ranges(int num_sms, QueryState* q, const uint32_t* in, uint32_t* out, uint32_t n,
+                                 const ScanTotals& tot, uint64_t* status, cudaStream_t s)
+{
+    const uint32_t tiles = div_up(n, kRangeTile), most = (uint32_t)num_sms * kRangePerSm;
+    const uint32_t per_cta = div_up(tiles, most), grid = div_up(tiles, per_cta);
+    // (a select's output is written element by element: its alignment is not asked for)
+    if (aligned16(in, kSelect ? in : out)) k_scan<kSelect, true><<<grid, kRangeThreads, 0, s>>>(q, in, out, n, per_cta, tot, status);
+    else k_scan<kSelect, false><<<grid, kRangeThreads, 0, s>>>(q, in, out, n, per_cta, tot, status);
+    count_launches(1);
+    return cudaGetLastError();
 }
 
 void scan_launch(bcmc_ctx* ctx, QueryState* q, const uint32_t* in, uint32_t* out, uint32_t n,
-                 uint32_t* d_total, uint64_t* status, cudaStream_t s)
+                 const ScanTotals& tot, uint64_t* status, cudaStream_t s)
 {
-    k_scan<<<persistent_grid(ctx, div_up(n, kScanTile), 4), kScanThreads, 0, s>>>(q, in, out, n, d_total, status);
-    count_launches(1);
-    BCMC_CUDA(cudaGetLastError());
+    BCMC_CUDA(launch_ranges<false>(ctx->num_sms, q, in, out, n, tot, status, s));
 }
 
 cudaError_t scan_launch_sms(int num_sms, QueryState* q, const uint32_t* in, uint32_t* out, uint32_t n,
                             uint32_t* d_total, uint64_t* status, cudaStream_t s)
 {
-    const uint32_t tiles = div_up(n, kScanTile), r = (uint32_t)num_sms * 4u;
-    const int grid = (int)(tiles < r ? (tiles ? tiles : 1) : r);
-    k_scan<<<grid, kScanThreads, 0, s>>>(q, in, out, n, d_total, status);
-    count_launches(1);
-    return cudaGetLastError();
+    return launch_ranges<false>(num_sms, q, in, out, n, ScanTotals{d_total}, status, s);
 }
 
 void select_launch(bcmc_ctx* ctx, QueryState* q, const uint32_t* flags, uint32_t* out, uint32_t n,
                    uint32_t* d_count, uint64_t* status, cudaStream_t s)
 {
-    k_select<<<persistent_grid(ctx, div_up(n, kScanTile), 4), kScanThreads, 0, s>>>(q, flags, out, n, d_count,
-                                                                                     status);
-    count_launches(1);
-    BCMC_CUDA(cudaGetLastError());
+    BCMC_CUDA(launch_ranges<true>(ctx->num_sms, q, flags, out, n, ScanTotals{d_count}, status, s));
 }
 
 void compact_launch(bcmc_ctx* ctx, uint32_t n, const uint32_t* flags, const uint32_t* offsets, uint32_t* out,
                     cudaStream_t s)
 {
     if (n == 0) return;
-    const int grid = (int)min(div_up(n, 256u), (uint32_t)ctx->num_sms * 16u);
-    k_compact<<<grid, 256, 0, s>>>(n, flags, offsets, out);
+    const int grid = (int)min(div_up(n, 1024u), (uint32_t)ctx->num_sms * 8u);
+    k_compact<<<grid, 256, 0, s>>>(n, flags, offsets, out, aligned16(flags, offsets));
     count_launches(1);
     BCMC_CUDA(cudaGetLastError());
 }
