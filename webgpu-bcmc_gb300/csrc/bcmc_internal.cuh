@@ -290,6 +290,28 @@ __device__ __forceinline__ uint32_t cta_exclusive_scan(uint32_t v, uint32_t* war
     return r;
 }
 
+// Grid barrier of a cooperative launch (every CTA resident): `arrived` counts the
+// CTAs, `target` is what it reaches when all have come this far.  Every CTA's
+// stores before it are seen by every CTA after it.
+__device__ __forceinline__ void grid_barrier(uint32_t* arrived, uint32_t target, uint32_t* err, uint32_t site)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(arrived, 1u);
+        uint32_t spins = 0;
+        while (*reinterpret_cast<volatile uint32_t*>(arrived) < target) {
+            if (++spins > kSpinLimit) {
+                atomicCAS(err, 0u, site);
+                break;
+            }
+            if (spins > 8) __nanosleep(100);
+        }
+        __threadfence();
+    }
+    __syncthreads();
+}
+
 // The sum over the CTAs before `rank` of the two counts each published in its
 // status words (aggregates of this epoch), to *sum_a and *sum_b in shared
 // memory, zero before (`drop`: this CTA publishes nothing, the test hook's case).

@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(16 * kTileBlocks, kBmcThreadsPerSm / (16 * kTi
     extern __shared__ __align__(16) unsigned char s_dyn[];
     McShared<kThreads, false>& sm = *reinterpret_cast<McShared<kThreads, false>*>(s_dyn);
     __shared__ uint32_t s_warp[kWarps + 1];
-    __shared__ uint32_t s_stop, s_with, s_pv, s_pb, s_cta_v, s_cta_b;
+    __shared__ uint32_t s_pv, s_pb, s_cta_v, s_cta_b;
 
     EngState* st = a.st;
     const uint32_t A = min(st->num_entries, st->entry_capacity);
@@ -490,28 +490,11 @@ __global__ void __launch_bounds__(16 * kTileBlocks, kBmcThreadsPerSm / (16 * kTi
             pv += v;
             pb += w;
         }
-    // grid barrier (the launch is cooperative: every CTA is resident)
-    __syncthreads();
-    if (t == 0) {
-        __threadfence();
-        atomicAdd(&st->mc_arrived, 1u);
-        uint32_t spins = 0;
-        while (*reinterpret_cast<volatile uint32_t*>(&st->mc_arrived) < G) {
-            if (++spins > kSpinLimit) {
-                atomicCAS(&st->error, 0u, 65u);
-                break;
-            }
-            if (spins > 8) __nanosleep(100);
-        }
-        __threadfence();
-        s_stop = *reinterpret_cast<volatile uint32_t*>(&st->error) | *reinterpret_cast<volatile uint32_t*>(&st->vert_overflow);
-        s_with = *reinterpret_cast<volatile uint32_t*>(&st->with_verts);
-    }
-    __syncthreads();
-    if (s_stop) return;
+    grid_barrier(&st->mc_arrived, G, &st->error, 65u);
+    if (__ldcg(&st->error) | __ldcg(&st->vert_overflow)) return;
     // emit: runs of `per` list entries, warp by warp over the whole grid; a
     // run's list entries are read two runs ahead, its neighbours one run ahead
-    const uint32_t W = s_with;
+    const uint32_t W = __ldcg(&st->with_verts);
     const uint32_t per = min(kMcBlocks, div_up(W, G * kWarps)), step = G * kWarps * per;
     const auto mine = [&](uint32_t at) { return jb < per && at + jb < W; };
     const auto load_entry = [&](uint32_t at) { return mine(at) ? __ldcg(a.wv_list + at + jb) : 0u; };

@@ -201,10 +201,6 @@ void query_end_launch(const QueryState* q, QueryState* host, cudaStream_t s)
 constexpr int kActThreads = 256;
 constexpr int kActiveItems = 4;
 constexpr int kActiveTile = kActThreads * kActiveItems;  // blocks per k_active tile
-constexpr int kSlotItems = 2;
-constexpr int kSlotTile = kActThreads * kSlotItems;  // slots per k_slots tile
-
-__device__ __forceinline__ uint32_t spad8(uint32_t i) { return i + (i >> 5); }
 
 // The last tile of the active test: totals, and the cache growth decision.
 __device__ __forceinline__ void active_finish(QueryState* q, uint32_t A, uint32_t N, uint32_t total)
@@ -439,17 +435,25 @@ __global__ void __launch_bounds__(kActThreads) k_active(QueryState* q, ActiveArg
 // ---------------------------------------------------------------------------
 // k_slots: age + mark + init of new slots, fused with the compaction of the
 // available slots (ascending slot id) and their ages.
+//
+// A CTA owns one contiguous range of slots, four to a thread at a time: ages and
+// marks them, then, when new items need slots, joins its count of available ones
+// to those of the CTAs before it (ranks are claimed in order, so all of them
+// run) and writes their ids and ages.  512-slot tiles claimed one by one, each
+// waiting for its claim, its items and their flags in turn, took 80 us on the
+// 1024 x 1024 x 1080 volume's 2.6 M slots.
 // ---------------------------------------------------------------------------
+constexpr uint32_t kSlotChunk = 4u * kActThreads;
+
 __global__ void __launch_bounds__(kActThreads) k_slots(QueryState* q, SlotArgs a)
 {
-    __shared__ uint8_t s_flags[kSlotTile + kSlotTile / 32];
     __shared__ uint32_t s_warp[kActThreads / 32 + 1];
-    __shared__ uint32_t s_tile, s_prefix;
+    __shared__ uint32_t s_rank, s_sum, s_prefix;
     __shared__ uint32_t s_hist[6][256];  // ~age digits 0-3, then the 16-bit keys' digits 0-1
     __shared__ uint32_t s_bins[kAgeBins];  // age bins (age_bin)
     __shared__ bool s_last;
     if ((a.skip_when_inactive && q->num_active == 0) || q->grow_needed) return;
-    const uint32_t old = q->old_cache_size, nsz = q->new_cache_size;
+    const uint32_t old = q->old_cache_size, nsz = q->new_cache_size;  // multiples of 32
     const bool compact = q->num_new > 0;
     const bool hist = compact && a.plan != 0u;
     // the six digit histograms of the sort keys are needed unless the plan is
@@ -464,85 +468,77 @@ __global__ void __launch_bounds__(kActThreads) k_slots(QueryState* q, SlotArgs a
             for (int i = threadIdx.x; i < 1536; i += kActThreads) (&s_hist[0][0])[i] = 0;
         for (int i = threadIdx.x; i < (int)kAgeBins; i += kActThreads) s_bins[i] = 0;
     }
-    const uint32_t ntiles = div_up(nsz, kSlotTile);
-    const uint32_t epoch = q->epoch;
-    for (;;) {
-        if (threadIdx.x == 0) s_tile = atomicAdd(&q->tiles_slots, 1u);
-        __syncthreads();
-        const uint32_t tile = s_tile;
-        if (tile >= ntiles) break;
-        const uint32_t base = tile * kSlotTile;
+    if (threadIdx.x == 0) {
+        s_rank = atomicAdd(&q->tiles_slots, 1u);
+        s_sum = s_prefix = 0;
+    }
+    __syncthreads();
+    const uint32_t range = align_up(div_up(nsz, gridDim.x), kSlotChunk);
+    const uint32_t first = min((uint64_t)nsz, (uint64_t)s_rank * range), end = min((uint64_t)nsz, (uint64_t)first + range);
+    uint32_t count = 0;
+    for (uint32_t base = first; base < end; base += kSlotChunk) {
+        const uint32_t s = base + 4u * threadIdx.x;
+        uint32_t age[4] = {100000u, 100000u, 100000u, 100000u}, av[4] = {1u, 1u, 1u, 1u};
+        if (s < old) {
+            const int4 i4 = *reinterpret_cast<const int4*>(a.slot_item + s);
+            const uint4 a4 = *reinterpret_cast<const uint4*>(a.slot_age + s);
+            const int32_t it[4] = {i4.x, i4.y, i4.z, i4.w};
+            const uint32_t was[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
-        for (int j = 0; j < kSlotItems; ++j) {
-            const uint32_t local = j * kActThreads + threadIdx.x;
-            const uint32_t s = base + local;
-            uint32_t av = 0;
-            if (s < old) {
-                const int32_t it = a.slot_item[s];
-                const bool keep = it >= 0 && a.needed[it] != 0u;
-                const uint32_t age = keep ? 0u : a.slot_age[s] + 1u;
-                av = keep ? 0u : 1u;
-                a.slot_age[s] = age;
-                a.slot_avail[s] = av;
-            } else if (s < nsz) {  // lru_cache_init.comp:27-29
-                a.slot_age[s] = 100000u;
-                a.slot_avail[s] = 1u;
-                a.slot_item[s] = -1;
-                av = 1u;
-            }
-            s_flags[spad8(local)] = (uint8_t)av;
+            for (int j = 0; j < 4; ++j) av[j] = it[j] >= 0 && a.needed[it[j]] != 0u ? 0u : 1u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) age[j] = av[j] ? was[j] + 1u : 0u;
+        } else if (s < end) {  // lru_cache_init.comp:27-29
+            *reinterpret_cast<int4*>(a.slot_item + s) = make_int4(-1, -1, -1, -1);
         }
-        if (compact) {
-            __syncthreads();
-            uint32_t cnt = 0;
-            uint8_t fl[kSlotItems];
+        if (s >= end) continue;
+        *reinterpret_cast<uint4*>(a.slot_age + s) = make_uint4(age[0], age[1], age[2], age[3]);
+        *reinterpret_cast<uint4*>(a.slot_avail + s) = make_uint4(av[0], av[1], av[2], av[3]);
+        count += av[0] + av[1] + av[2] + av[3];
+        if (!hist) continue;
+        // plain increments: shared memory adds up a warp's increments of one
+        // counter by itself, and ages take few distinct values
 #pragma unroll
-            for (int j = 0; j < kSlotItems; ++j) {
-                fl[j] = s_flags[spad8(threadIdx.x * kSlotItems + j)];
-                cnt += fl[j];
+        for (int j = 0; j < 4; ++j)
+            if (av[j]) {
+                const uint32_t k = ~age[j], k16 = ~age_key16(age[j]), bin = age_bin(age[j]);
+                if (!age_has_key16(age[j])) wide = 1;
+                if (bin == kAgeBins) binless = 1;
+                else atomicAdd(&s_bins[bin], 1u);
+                if (digits) {
+#pragma unroll
+                    for (int d = 0; d < 6; ++d) atomicAdd(&s_hist[d][((d < 4 ? k : k16) >> (8 * (d & 3))) & 255u], 1u);
+                }
+            }
+    }
+    if (compact) {
+        count = __reduce_add_sync(0xffffffffu, count);
+        if (lane == 0 && count) atomicAdd(&s_sum, count);
+        __syncthreads();
+        cta_prefix_sum<kActThreads>(a.status, s_rank, s_sum, q->epoch, &q->error, 32u, &s_prefix);
+        __syncthreads();
+        uint32_t run = s_prefix;
+        for (uint32_t base = first; base < end; base += kSlotChunk) {
+            const uint32_t s = base + 4u * threadIdx.x;
+            uint4 av = make_uint4(0u, 0u, 0u, 0u), age = av;
+            if (s < end) {
+                av = *reinterpret_cast<const uint4*>(a.slot_avail + s);
+                age = *reinterpret_cast<const uint4*>(a.slot_age + s);
             }
             uint32_t tot;
-            const uint32_t excl = cta_exclusive_scan<kActThreads>(cnt, s_warp, &tot);
-            if (threadIdx.x < 32) {
-                const uint32_t p = warp_lookback(a.status, tile, tot, epoch, &q->error, 32u);
-                if (threadIdx.x == 0) s_prefix = p;
-            }
-            __syncthreads();
-            uint32_t p = s_prefix + excl;
-            const uint32_t first = base + threadIdx.x * kSlotItems;
+            uint32_t p = run + cta_exclusive_scan<kActThreads>(av.x + av.y + av.z + av.w, s_warp, &tot);
+            const uint32_t on[4] = {av.x, av.y, av.z, av.w}, ages[4] = {age.x, age.y, age.z, age.w};
 #pragma unroll
-            for (int j = 0; j < kSlotItems; ++j) {
-                uint32_t age = 0;
-                if (fl[j]) {
-                    const uint32_t s = first + j;
-                    age = a.slot_age[s];
-                    a.avail_ids[p] = s;
-                    a.avail_keys[p] = age;
+            for (uint32_t j = 0; j < 4; ++j)
+                if (on[j]) {
+                    a.avail_ids[p] = s + j;
+                    a.avail_keys[p] = ages[j];
                     ++p;
                 }
-                if (hist) {  // one shared atomic per distinct digit and warp
-                    const uint32_t k = ~age, k16 = ~age_key16(age);
-                    const bool has16 = fl[j] && age_has_key16(age);
-                    if (fl[j] && !has16) wide = 1;
-                    // the joint histogram of the age bins (one shared atomic per distinct bin and warp)
-                    const uint32_t bin = fl[j] ? age_bin(age) : kAgeBins + 1u;
-                    if (bin == kAgeBins) binless = 1;
-                    const uint32_t bp = __match_any_sync(0xffffffffu, bin);
-                    if (bin < kAgeBins && lane == (uint32_t)__ffs(bp) - 1u) atomicAdd(&s_bins[bin], (uint32_t)__popc(bp));
-                    if (digits) {
-#pragma unroll
-                        for (int d = 0; d < 6; ++d) {
-                            const uint32_t digit = fl[j] ? ((d < 4 ? k : k16) >> (8 * (d & 3))) & 255u : 256u;
-                            const uint32_t peers = __match_any_sync(0xffffffffu, digit);
-                            if (fl[j] && lane == (uint32_t)__ffs(peers) - 1u)
-                                atomicAdd(&s_hist[d][digit], (uint32_t)__popc(peers));
-                        }
-                    }
-                }
-            }
+            run += tot;
         }
-        __syncthreads();
     }
+    __syncthreads();
     if (!hist) return;
     // this CTA's histograms into q->sort_hist; the last CTA to finish makes
     // the sort's pass plan (what k_sort_hist's last CTA does)
@@ -717,24 +713,29 @@ constexpr int kMcPerSm = 2;  // resident CTAs per SM (the grid: one launch, all 
 // Ranges of at most this many blocks per CTA (small queries) are emitted by
 // their own CTA; longer ones go through a grid barrier and an even share-out.
 constexpr uint32_t kMcOwnRange = kMcWarps * kMcBlocks;
+// Ranges longer than this are counted by all CTAs together, which costs a barrier.
+constexpr uint32_t kMcSharedRange = 1024;
 
 // Marching cubes over the active blocks, one cooperative launch (every CTA
-// resident), all of its block work done by single warps (mc_common.cuh).  Each
-// CTA owns one contiguous range of active blocks:
-//   count pass: the warps take up to four blocks at a time, look their
-//     neighbours up, load their grids and count the triangles of their cells
-//     from the corner masks; block totals are kept;
-//   the CTA publishes its totals and adds up those of the CTAs before it: its
-//     vertex offset and its place in the blocks-with-vertices list;
+// resident), all of its block work done by single warps (mc_common.cuh):
+//   count pass: the blocks in batches of four to a warp: look the neighbours up,
+//     load the grids and count the triangles of the cells from the corner masks;
+//     block totals are kept.  Each CTA counts its own range of the blocks, or,
+//     when the ranges are long, its share of batches from the whole grid, with a
+//     barrier after it: a batch's cost depends on whether the surface passes
+//     through it (512^3: 878 -> 867 us, 1024 x 1024 x 1080: 636 -> 612 us, but
+//     256^3: 59 -> 63 us, where the barrier costs more than the balance saves);
+//   each CTA publishes its range's totals and adds up those of the CTAs before
+//     it: its vertex offset and its place in the blocks-with-vertices list;
 //   it writes its entries of that list and their vertex offsets, then a grid
 //     barrier;
-//   emit: the list in runs of up to four consecutive entries, warp by warp
-//     over the whole grid -- vertex counts differ between ranges by up to 7x,
-//     so the emit work is shared out by list entry, not by range.  Entries that
-//     follow each other in the list have their vertices one after the other,
-//     so a run needs only its first entry's offset.
-// Short ranges (small queries) skip the barrier: each CTA emits its own
-// entries.
+//   emit: the list in runs of up to four consecutive entries, warp by warp over
+//     the whole grid.  Entries that follow each other in the list have their
+//     vertices one after the other, so a run needs only its first entry's offset.
+// Few blocks (at most kMcOwnRange a CTA): a warp keeps the grids of the up to
+// four blocks it counted and emits them itself, once its place is known; the
+// barrier and the second load would take longer than the balance saves (64^3:
+// 16.6 -> 13.9 us against own entries shared out in the CTA and loaded again).
 // Output order = the reference's: active-block order, cell order, table order.
 // kHost: the vertices go to page-locked host memory (a.host_verts).
 template <bool kHost>
@@ -743,8 +744,8 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     extern __shared__ __align__(16) unsigned char s_dyn[];
     McShared<kMcThreads, kHost>& sm = *reinterpret_cast<McShared<kMcThreads, kHost>*>(s_dyn);
     __shared__ uint32_t s_warp[kMcWarps + 1];
-    __shared__ uint32_t s_cnt[kMcOwnRange], s_idx[kMcOwnRange], s_off[kMcOwnRange];  // short ranges
-    __shared__ uint32_t s_stop, s_with, s_pv, s_pb, s_cta_v, s_cta_b;
+    __shared__ uint32_t s_cnt[kMcOwnRange];  // few blocks: the counts of the CTA's
+    __shared__ uint32_t s_pv, s_pb, s_cta_v, s_cta_b;
 
     const uint32_t A = q->num_active;
     if (A == 0 || q->grow_needed) return;
@@ -754,11 +755,11 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     const uint32_t slots = q->cache_size;
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, jb = lane >> 3;
     const uint32_t G = gridDim.x, rank = blockIdx.x;
-    // whole batches for every warp: 8, 16, 24 or 32 blocks, or a multiple of a batch
     const uint32_t share = div_up(A, G);
-    const uint32_t range = align_up(share, share <= kMcOwnRange ? (uint32_t)kMcWarps : kMcBlocks);
+    const bool own = share <= kMcOwnRange, together = share > kMcSharedRange;
+    const uint32_t range = own ? align_up(share, (uint32_t)kMcWarps) : share;
     const uint32_t start = min(A, rank * range), end = min(A, start + range);
-    // ranks 0 .. worked - 1 own blocks; the others only help with the emit
+    // ranks 0 .. worked - 1 have blocks in their range
     const uint32_t worked = div_up(A, range);
     mc_shared_begin(sm);
     if (t == 0) s_cta_v = s_cta_b = s_pv = s_pb = 0;
@@ -774,25 +775,37 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     };
 
     // ---- count pass: ids two rounds ahead, lookups one round ahead
+    uint32_t own_n = 0, own_id = 0, own_has = 0;  // few blocks: the warp's batch
+    const uint32_t batch = own ? range / kMcWarps : kMcBlocks;
     {
-        const uint32_t batch = min(kMcBlocks, range / kMcWarps), step = kMcWarps * batch;
-        uint32_t base = start + warp * batch;
-        // the last batch of a range may be short; jb < batch keeps a lane to its batch
-        const auto mine = [&](uint32_t at) { return jb < batch && at + jb < end; };
+        const uint32_t stop = together ? A : end, step = (together ? G : 1u) * kMcWarps * batch;
+        uint32_t base = together ? (rank * kMcWarps + warp) * batch : start + warp * batch;
+        const auto mine = [&](uint32_t at) { return jb < batch && at + jb < stop; };
         const auto load_id = [&](uint32_t at) { return mine(at) ? __ldg(a.active_ids + at + jb) : 0u; };
         McLook next = look(mine(base), load_id(base));
         uint32_t id2 = load_id(base + step);
         uint32_t wv = 0, wb = 0;
         async_wait<1>();
         __syncthreads();
-        for (; base < end; base += step) {
-            const uint32_t n = min(batch, end - base);
+        for (; base < stop; base += step) {
+            const uint32_t n = min(batch, stop - base), id = next.id;
             const uint32_t has = look_end(next);
             uint32_t total = 0;
             float f[kMcBlocks][4];
             mc_voxels(geo, n, f);
             next = look(mine(base + step), id2);
             id2 = load_id(base + 2u * step);
+            if (own) {
+                own_n = n;
+                own_id = id;
+                own_has = has;
+#pragma unroll
+                for (uint32_t j = 0; j < kMcBlocks; ++j)
+                    if (j < n) {
+#pragma unroll
+                        for (uint32_t r = 0; r < 4; ++r) mem.vol[j][lane + 32u * r] = f[j][r];
+                    }
+            }
 #pragma unroll
             for (uint32_t j = 0; j < kMcBlocks; ++j)
                 if (j < n) {
@@ -805,12 +818,27 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
                 }
             if (lane < n) {
                 a.block_counts[base + lane] = total;
-                if (range <= kMcOwnRange) s_cnt[base - start + lane] = total;
+                if (own) s_cnt[base - start + lane] = total;
             }
         }
-        if (lane == 0 && wb) {
+        if (!together && lane == 0 && wb) {
             atomicAdd(&s_cta_v, wv);
             atomicAdd(&s_cta_b, wb);
+        }
+    }
+    if (together) {
+        grid_barrier(&q->mc_arrived, G, &q->error, 42u);
+        uint32_t v = 0, b = 0;
+        for (uint32_t i = start + t; i < end; i += kMcThreads) {
+            const uint32_t c = __ldcg(a.block_counts + i);
+            v += c;
+            b += c ? 1u : 0u;
+        }
+        v = __reduce_add_sync(kFull, v);
+        b = __reduce_add_sync(kFull, b);
+        if (lane == 0 && b) {
+            atomicAdd(&s_cta_v, v);
+            atomicAdd(&s_cta_b, b);
         }
     }
     __syncthreads();
@@ -827,45 +855,34 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     const bool fits = (uint64_t)pv + s_cta_v <= cap;
     if (!fits && t == 0) atomicOr(&q->vert_overflow, 1u);
 
-    if (range <= kMcOwnRange) {
-        if (!fits) return;
-        // the range's blocks with vertices, by one warp
-        if (warp == 0)
-            for (uint32_t i0 = 0; start + i0 < end; i0 += 32u) {
-                const uint32_t i = start + i0 + lane;
-                const uint32_t c = i < end ? s_cnt[i0 + lane] : 0u;
-                const uint32_t inc = warp_inclusive_scan(c);
-                const uint32_t some = __ballot_sync(kFull, c != 0u);
-                const uint32_t r = pb + __popc(some & ((1u << lane) - 1u));
-                if (c) {
-                    s_idx[r - s_pb] = i;
-                    s_off[r - s_pb] = pv + inc - c;
-                    a.with_verts[r] = i;
-                    a.vert_offsets[r] = pv + inc - c;
-                }
-                pv += __shfl_sync(kFull, inc, 31);
-                pb += __popc(some);
-            }
-        __syncthreads();
-        const uint32_t W = s_cta_b, per = div_up(W, (uint32_t)kMcWarps);
-        const uint32_t first = warp * per;
-        if (first < W) {
-            const uint32_t n = min(per, W - first);
-            const bool valid = jb < n;
-            const uint32_t id = valid ? __ldg(a.active_ids + s_idx[first + jb]) : 0u;
-            const uint32_t has = look_end(look(valid, id));
-            mc_grids(geo, mem, n);
-            McSink<kHost> sink{a.verts + s_off[first]};
-            mc_emit<kHost, true>(geo, sm.tab, mem, n, id, has, iso, sink, [] {});
-            sink.finish(mem.out);
+    if (own) {
+        if (!fits || own_n == 0) return;
+        // the CTA's blocks before the warp's: their vertices, and those that have any
+        const uint32_t first = warp * batch, done = first < 32u ? first : 32u;
+        static_assert(kMcOwnRange <= 64, "two counts to a lane");
+        const uint32_t c0 = lane < done ? s_cnt[lane] : 0u, c1 = 32u + lane < first ? s_cnt[32u + lane] : 0u;
+        pv += __reduce_add_sync(kFull, c0 + c1);
+        pb += __popc(__ballot_sync(kFull, c0 != 0u)) + __popc(__ballot_sync(kFull, c1 != 0u));
+        // the warp's own
+        const uint32_t c = lane < own_n ? s_cnt[first + lane] : 0u;
+        const uint32_t off = pv + mc_scan(c) - c;
+        const uint32_t some = __ballot_sync(kFull, c != 0u);
+        if (c) {
+            const uint32_t r = pb + __popc(some & ((1u << lane) - 1u));
+            a.with_verts[r] = start + first + lane;
+            a.vert_offsets[r] = off;
         }
+        if (!some) return;
+        McSink<kHost> sink{a.verts + pv};
+        mc_emit<kHost, true>(geo, sm.tab, mem, own_n, own_id, own_has, iso, sink, [] {});
+        sink.finish(mem.out);
         return;
     }
     // the range's blocks with vertices: their list entries and vertex offsets
     if (fits)
         for (uint32_t b0 = start; b0 < end; b0 += kMcThreads) {
             const uint32_t i = b0 + t;
-            const uint32_t c = i < end ? a.block_counts[i] : 0u;
+            const uint32_t c = i < end ? __ldcg(a.block_counts + i) : 0u;
             // <= 512 blocks x 64 cells x 15 vertices < 2^20, and the blocks above them
             static_assert(kMcThreads * 64 * 15 < 1 << 20 && kMcThreads < 1 << 12, "fields of the scan");
             uint32_t tot;
@@ -878,30 +895,13 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
             pv += tot & 0xfffffu;
             pb += tot >> 20;
         }
-    // grid barrier (the launch is cooperative: every CTA is resident)
-    __syncthreads();
-    if (t == 0) {
-        __threadfence();
-        atomicAdd(&q->mc_arrived, 1u);
-        uint32_t spins = 0;
-        while (*reinterpret_cast<volatile uint32_t*>(&q->mc_arrived) < G) {
-            if (++spins > kSpinLimit) {
-                atomicCAS(&q->error, 0u, 42u);
-                break;
-            }
-            if (spins > 8) __nanosleep(100);
-        }
-        __threadfence();
-        s_stop = *reinterpret_cast<volatile uint32_t*>(&q->error) | *reinterpret_cast<volatile uint32_t*>(&q->vert_overflow);
-        s_with = *reinterpret_cast<volatile uint32_t*>(&q->num_with_verts);
-    }
-    __syncthreads();
-    if (s_stop) return;
+    grid_barrier(&q->mc_arrived, together ? 2u * G : G, &q->error, 42u);
+    if (__ldcg(&q->error) | __ldcg(&q->vert_overflow)) return;
     // emit: runs of `per` entries, one from each warp's turn over the grid; into
     // host memory a turn is four runs that follow each other, which leaves fewer
     // windows of 32 vertices partly filled.  A run's list entries are read two
     // runs ahead, its block ids and neighbours one run ahead.
-    const uint32_t W = s_with;
+    const uint32_t W = __ldcg(&q->num_with_verts);
     const uint32_t per = min(kMcBlocks, div_up(W, G * kMcWarps));
     constexpr uint32_t kRuns = kHost ? 4u : 1u;
     const uint32_t turn = per * kRuns, skip = (G * kMcWarps - 1u) * turn;
@@ -964,12 +964,13 @@ static uint32_t word_per_sm()
     return n;
 }
 
-// Words a warp takes: enough warps for every SM first (4 words each keeps the
-// 64^3 volume's 128 words on 32 warps), then longer runs, up to a word to a lane.
+// Words a warp takes, a multiple of 4 up to a word to a lane: enough for
+// `warps_per_sm` warps on every SM first, then longer runs (4 words each keep
+// the 64^3 volume's 128 words on 32 warps).
 static uint32_t words_per_warp(const bcmc_ctx* ctx, uint32_t nwords, uint32_t warps_per_sm)
 {
-    const uint32_t w = div_up(nwords, (uint32_t)ctx->num_sms * warps_per_sm);
-    return w <= 4u ? 4u : (w >= 32u ? 32u : w);
+    const uint32_t w = align_up(div_up(nwords, (uint32_t)ctx->num_sms * warps_per_sm), 4u);
+    return w >= 32u ? 32u : w;
 }
 
 void query_flags_launch(bcmc_ctx* ctx, QueryState* q, float iso, uint32_t capacity, uint32_t vert_capacity,
@@ -988,11 +989,12 @@ void query_flags_launch(bcmc_ctx* ctx, QueryState* q, float iso, uint32_t capaci
 
 void active_words_launch(bcmc_ctx* ctx, QueryState* q, ActiveArgs a, void* words, cudaStream_t s)
 {
-    const uint32_t nwords = div_up(a.total, 32u), wpw = words_per_warp(ctx, nwords, kWordPerSm * (kWordThreads / 32));
+    const uint32_t nwords = div_up(a.total, 32u), wpw = words_per_warp(ctx, nwords, kWordThreads / 32);
     a.near = static_cast<const uint4*>(words);
     a.hi = reinterpret_cast<const uint32_t*>(a.near + nwords);
     a.words = reinterpret_cast<uint2*>(static_cast<uint4*>(words) + nwords + div_up(nwords, 4u));
-    // a range per resident CTA, of whole rounds of its warps
+    // a CTA an SM first: the CTAs wait for each other's counts (256^3: 128 of them
+    // 1.3 us faster than 256); then a range of whole rounds per resident CTA
     const uint32_t round = wpw * (kWordThreads / 32);
     const uint32_t range = div_up(div_up(nwords, round), (uint32_t)ctx->num_sms * word_per_sm()) * round;
     cudaLaunchConfig_t cfg{};
@@ -1017,7 +1019,7 @@ void active_launch(bcmc_ctx* ctx, QueryState* q, const ActiveArgs& a, cudaStream
 
 void slots_launch(bcmc_ctx* ctx, QueryState* q, const SlotArgs& a, uint32_t max_slots, cudaStream_t s)
 {
-    k_slots<<<pgrid(ctx, div_up(max_slots, kSlotTile), 8), kActThreads, 0, s>>>(q, a);
+    k_slots<<<pgrid(ctx, div_up(max_slots, kSlotChunk), 4), kActThreads, 0, s>>>(q, a);
     count_launches(1);
     BCMC_CUDA(cudaGetLastError());
 }
@@ -1082,7 +1084,7 @@ void mc_launch(bcmc_ctx* ctx, QueryState* q, const McArgs& a, uint32_t max_activ
 }
 
 uint32_t active_tiles(uint32_t total) { return div_up(total, kActiveTile); }
-uint32_t slot_tiles(uint32_t slots) { return div_up(slots, kSlotTile); }
+uint32_t slot_tiles(uint32_t slots) { return div_up(slots, kSlotChunk); }
 // one CTA per range of active blocks, every CTA resident; at least a block to a warp
 uint32_t mc_grid(bcmc_ctx* ctx, uint32_t max_active)
 {

@@ -87,27 +87,6 @@ __global__ void __launch_bounds__(kHistThreads) k_sort_hist(QueryState* q, const
     sort_plan<kHistThreads>(q, n, warp_sums, &q->sort_hist[0][0], 4);
 }
 
-// Grid barrier of the first `ctas` CTAs of k_sort, its n-th (counted by the
-// caller): every CTA's stores before it are seen by every CTA after it.
-__device__ __forceinline__ void sort_barrier(QueryState* q, uint32_t n, uint32_t ctas)
-{
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(&q->sort_arrived, 1u);
-        uint32_t spins = 0;
-        while (*reinterpret_cast<volatile uint32_t*>(&q->sort_arrived) < n * ctas) {
-            if (++spins > kSpinLimit) {
-                atomicCAS(&q->error, 0u, 28u);
-                break;
-            }
-            if (spins > 8) __nanosleep(100);
-        }
-        __threadfence();
-    }
-    __syncthreads();
-}
-
 // All the digit passes of the plan in one cooperative launch: the passes
 // that run are separated by grid barriers (each reads what the one before it
 // scattered, so its key and value loads bypass L1), the others cost nothing.
@@ -147,7 +126,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(QueryState* q, const u
         if (q->sort_run[pass]) last = pass;
     for (int pass = 0; pass < 4; ++pass) {
         if (!q->sort_run[pass]) continue;
-        if (ran++) sort_barrier(q, ++barriers, ctas);
+        if (ran++) grid_barrier(&q->sort_arrived, ++barriers * ctas, &q->error, 28u);
         const uint32_t src = q->sort_src[pass];
         const bool to_out = b.out_keys && pass == last && src != 0;
         const uint32_t* __restrict__ ks = src == 0 ? b.in_keys : (src == 1 ? b.b_keys : b.c_keys);
@@ -236,7 +215,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(QueryState* q, const u
             uint32_t tile_total;
             const uint32_t start = cta_exclusive_scan<kSortThreads>(run, s_warp_sums, &tile_total);
             if (wave) {
-                sort_barrier(q, ++barriers, ctas);
+                grid_barrier(&q->sort_arrived, ++barriers * ctas, &q->error, 28u);
                 // rows of counts before this tile's, every sixteenth to a warp
                 static_assert(kSortThreads == 512 && kSortTile == 4096, "16 warps: 8 KB of counts, 16 KB of masks or sums");
                 uint32_t sum[8] = {};
@@ -292,7 +271,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(QueryState* q, const u
         }
     }
     if (b.out_keys && ran == 1) {  // one pass: in b
-        sort_barrier(q, ++barriers, ctas);
+        grid_barrier(&q->sort_arrived, ++barriers * ctas, &q->error, 28u);
         for (uint32_t i = blockIdx.x * kSortThreads + threadIdx.x; i < n; i += ctas * kSortThreads) {
             const uint32_t k = __ldcg(b.b_keys + i);
             b.out_keys[i] = reverse ? ~k : k;
