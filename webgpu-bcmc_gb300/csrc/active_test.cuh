@@ -1,87 +1,71 @@
-// active_test.cuh -- the active-block test of compute_block_active.comp,
-// shared by the per-query pipeline (pipeline.cu) and the batched engine
+// active_test.cuh -- the active-block test of compute_block_active.comp in words
+// of 32 blocks, for the per-query pipeline (pipeline.cu) and the batched engine
 // (engine.cu).
+//
+// compute_block_active.comp:24-61 tests, for each of the 26 neighbours n, iso in
+// [min(lo_b, lo_n), max(hi_b, hi_n)].  With A = (iso >= lo), B = (iso <= hi) that
+// is (A_b || A_n) && (B_b || B_n), so over all neighbours (and b itself, which
+// adds nothing new):
+//   active = (A_b && anyB) || (B_b && anyA) || any(A_n && B_n)
+// -- the same booleans.  The bits of A, B and A && B are ORed along x (spread),
+// then over the nine (y, z) rows of a word's blocks, those that the volume has
+// (word_rows).
 #pragma once
 
 #include "bcmc_internal.cuh"
 
 namespace bcmc {
 
-// compute_block_active.comp:24-61.  The reference tests, for each of the 26
-// neighbours n, iso in [min(lo_b, lo_n), max(hi_b, hi_n)].  With A = (iso >=
-// lo), B = (iso <= hi) that is (A_b || A_n) && (B_b || B_n), so over all
-// neighbours (and b itself, which adds nothing new):
-//   active = (A_b && anyB) || (B_b && anyA) || any(A_n && B_n)
-// -- the same booleans, evaluated without branches or early exits.
-__device__ __forceinline__ uint32_t block_is_active(const float2* __restrict__ ranges, const BlockGrid& g,
-                                                    uint32_t b, float iso)
-{
-    const uint3 nb = g.nb;
-    const float2 r = __ldg(ranges + b);
-    const bool A = iso >= r.x, B = iso <= r.y;
-    const uint3 c = block_coords(b, g);
-    const int bx = (int)c.x, by = (int)c.y, bz = (int)c.z;
-    bool anyA = false, anyB = false, anyC = false;
-#pragma unroll
-    for (int k = -1; k < 2; ++k)
-#pragma unroll
-        for (int j = -1; j < 2; ++j)
-#pragma unroll
-            for (int i = -1; i < 2; ++i) {
-                const int cx = bx + i, cy = by + j, cz = bz + k;
-                if (cx < 0 || cy < 0 || cz < 0 || cx >= (int)nb.x || cy >= (int)nb.y || cz >= (int)nb.z) continue;
-                const float2 n = __ldg(ranges + ((uint32_t)cx + nb.x * ((uint32_t)cy + nb.y * (uint32_t)cz)));
-                const bool an = iso >= n.x, bn = iso <= n.y;
-                anyA |= an;
-                anyB |= bn;
-                anyC |= an && bn;
-            }
-    return ((A && anyB) || (B && anyA) || anyC) ? 1u : 0u;
-}
+// Of the 32 blocks from b0 on: those with a row before and after them in y and in z.
+struct WordRows {
+    uint32_t ym, yp, zm, zp;
 
-__device__ __forceinline__ void range_bits(const float2 r, float iso, uint32_t& a, uint32_t& b)
-{
-    a = iso >= r.x ? 1u : 0u;
-    b = iso <= r.y ? 1u : 0u;
-}
+    __device__ __forceinline__ uint32_t mask(int dy, int dz) const
+    {
+        return (dz < 0 ? zm : dz > 0 ? zp : 0xffffffffu) & (dy < 0 ? ym : dy > 0 ? yp : 0xffffffffu);
+    }
+};
 
-// Active flags of the 4 consecutive blocks b0..b0+3 of one x-row: the 9
-// neighbour rows (y-1..y+1, z-1..z+1) are read once for the 4 blocks (6 ranges
-// per row), 13.5 loads per block instead of 27.
-__device__ __forceinline__ uint32_t row4_active(const float2* __restrict__ ranges, const BlockGrid& g, uint3 c,
-                                                uint32_t b0, float iso)
+__device__ __forceinline__ WordRows word_rows(uint32_t b0, const BlockGrid& g)
 {
-    const uint3 nb = g.nb;
-    uint32_t anyA = 0, anyB = 0, anyC = 0, selfA = 0, selfB = 0;  // bit i = block b0+i
-#pragma unroll
-    for (int dz = -1; dz < 2; ++dz)
-#pragma unroll
-        for (int dy = -1; dy < 2; ++dy) {
-            const int yy = (int)c.y + dy, zz = (int)c.z + dz;
-            if (yy < 0 || zz < 0 || yy >= (int)nb.y || zz >= (int)nb.z) continue;
-            const int64_t shift = (int64_t)dy * nb.x + (int64_t)dz * nb.x * nb.y;
-            const float2* row = ranges + (int64_t)b0 + shift;  // position x0 of the neighbour row
-            uint32_t A = 0, B = 0;  // bit p = position x0 - 1 + p, p = 0..5
-#pragma unroll
-            for (int p = 0; p < 6; ++p) {
-                const int xx = (int)c.x - 1 + p;
-                if (xx < 0 || xx >= (int)nb.x) continue;
-                uint32_t a, b;
-                range_bits(__ldg(row + (p - 1)), iso, a, b);
-                A |= a << p;
-                B |= b << p;
-            }
-            const uint32_t C = A & B;
-            // window of block i covers positions i..i+2
-            anyA |= (A | (A >> 1) | (A >> 2)) & 15u;
-            anyB |= (B | (B >> 1) | (B >> 2)) & 15u;
-            anyC |= (C | (C >> 1) | (C >> 2)) & 15u;
-            if (dy == 0 && dz == 0) {
-                selfA = (A >> 1) & 15u;
-                selfB = (B >> 1) & 15u;
-            }
+    WordRows r{0u, 0u, 0u, 0u};
+    uint3 c = block_coords(b0, g);
+    for (uint32_t p = 0; p < 32u;) {  // the pieces of rows in the word
+        const uint32_t len = min(g.nb.x - c.x, 32u - p);
+        const uint32_t m = (0xffffffffu >> (32u - len)) << p;
+        r.ym |= c.y > 0u ? m : 0u;
+        r.yp |= c.y + 1u < g.nb.y ? m : 0u;
+        r.zm |= c.z > 0u ? m : 0u;
+        r.zp |= c.z + 1u < g.nb.z ? m : 0u;
+        p += len;
+        c.x = 0;
+        if (++c.y == g.nb.y) {
+            c.y = 0;
+            ++c.z;
         }
-    return ((selfA & anyB) | (selfB & anyA) | anyC) & 15u;
+    }
+    return r;
+}
+
+// Of the 32 blocks from b0 on: those at x = 0 and at x = nx - 1, which have no neighbour there.
+struct WordEnds {
+    uint32_t no_left, no_right;
+
+    // The word's bits ORed with those of the blocks before and after each along x;
+    // the last bit of `prev` and the first of `next` are those beside the word.
+    __device__ __forceinline__ uint32_t spread(uint32_t v, uint32_t prev, uint32_t next) const
+    {
+        return v | (__funnelshift_l(prev, v, 1) & ~no_left) | (__funnelshift_r(v, next, 1) & ~no_right);
+    }
+};
+
+__device__ __forceinline__ WordEnds word_ends(uint32_t b0, const BlockGrid& g)
+{
+    const uint32_t nx = g.nb.x, x0 = b0 - fdiv(b0, g.dx) * nx;
+    WordEnds e{0u, 0u};
+    for (uint32_t p = x0 ? nx - x0 : 0u; p < 32u; p += nx) e.no_left |= 1u << p;
+    for (uint32_t p = nx - 1u - x0; p < 32u; p += nx) e.no_right |= 1u << p;
+    return e;
 }
 
 }  // namespace bcmc

@@ -2,21 +2,21 @@
 // one shared pool of decoded-block slots (bcmc_engine_* in include/bcmc.h).
 //
 // A launch sequence answers up to max_batch (volume, isovalue) queries:
-//   k_bbegin   new look-back epoch, counters cleared
+//   k_bbegin   new epoch of the status words, counters cleared
 //   k_bactive  every query's active test over its volume's blocks, as one
-//              stream of 1024-block tiles (query-major).  A tile whose
-//              extended value range (its blocks and their 26 neighbours, from
-//              volume load) excludes the isovalue is skipped whole.  Active
-//              flags go to a per-query bitmap; active (query, block) entries
-//              are compacted in query-major, block-ascending order by one
-//              decoupled look-back over all tiles; blocks no slot holds are
-//              claimed (one claim per block across the batch) and given a
-//              slot from the pool's free list
+//              stream of 1024-block tiles (query-major), in words of 32 blocks.
+//              A tile whose extended value range (its blocks and their 26
+//              neighbours, from volume load) excludes the isovalue is skipped
+//              whole.  Active bits go to a per-query bitmap, counts to the tiles
+//   k_bentries active (query, block) entries in query-major, block-ascending
+//              order from the tiles' counts; blocks no slot holds are claimed
+//              (one claim per block across the batch) and given a slot from
+//              the pool's free list
 //   k_bdecode  ZFP decode of every claimed block into its slot
 //   k_bmc      marching cubes over all entries: the per-query kernel's
-//              range-per-CTA count pass, one look-back per CTA, the list of
-//              entries with vertices, a grid barrier (cooperative launch) and
-//              emit tiles claimed by whichever CTA is free;
+//              range-per-CTA count pass, one round trip for the counts of the
+//              CTAs before, the list of entries with vertices, a grid barrier
+//              (cooperative launch) and the emit shared out over the grid;
 //              per-block isovalue, volume and neighbour flags come from the
 //              entry's query; every query's vertices come out contiguous and
 //              in the plain path's order
@@ -79,7 +79,7 @@ struct EngState {
     uint32_t nq, ntiles, entry_capacity, use_epoch;
     unsigned long long vert_capacity, vert_base;
     // device-side
-    uint32_t epoch, tiles_active, num_entries, with_verts;  // with_verts: entries with vertices
+    uint32_t epoch, num_entries, with_verts;  // with_verts: entries with vertices
     uint32_t num_decode, pool_exhausted, entry_overflow, vert_overflow;
     uint32_t error, mc_arrived;  // mc_arrived: k_bmc's grid barrier
     unsigned long long num_verts;  // this sequence's vertices (64-bit, from the per-query totals)
@@ -116,9 +116,9 @@ struct BatchArgs {
     uint32_t* dec_block;
     uint32_t* dec_slot;
     uint2* verts;
-    uint64_t* status_a;  // look-back over active tiles
-    uint64_t* status_v;  // look-back over MC CTAs (vertices)
-    uint64_t* status_b;  // look-back over MC CTAs (entries with vertices)
+    uint32_t* tile_counts;  // active blocks of each tile, then of each group of tiles (k_bactive)
+    uint64_t* status_v;  // counts of the MC CTAs (vertices)
+    uint64_t* status_b;  // counts of the MC CTAs (entries with vertices)
 };
 
 // ---------------------------------------------------------------------------
@@ -170,7 +170,7 @@ __global__ void k_bbegin(EngState* st, uint32_t* q_nverts, uint32_t* q_nactive, 
 {
     if (threadIdx.x == 0) {
         st->epoch += 1;
-        st->tiles_active = st->mc_arrived = st->with_verts = 0;
+        st->mc_arrived = st->with_verts = 0;
         st->num_entries = st->num_decode = 0;
         st->pool_exhausted = st->entry_overflow = st->vert_overflow = 0;
         st->error = 0;
@@ -180,116 +180,272 @@ __global__ void k_bbegin(EngState* st, uint32_t* q_nverts, uint32_t* q_nactive, 
 }
 
 // ---------------------------------------------------------------------------
-// k_bactive
+// k_bactive: the active test of every query over its volume's blocks, a bit per
+// block, and the counts of the tiles and of groups of eight tiles.
+//
+// The tests of a batch read each block's range over and over: what bounds the
+// kernel is the instructions and loads per block.  A warp takes a tile of 1024
+// blocks.  The neighbours of its blocks lie in three runs of ids, one per z:
+// the tile moved by a plane, a row and a block longer at either end.  A lane
+// reads a block's range once for a run and two ballots make it two bits of a
+// word; the words are ORed along x, and a lane ORs the nine (y, z) rows of its
+// word of the tile, each two words and a funnel shift (the test in bit words is
+// k_active_words', pipeline.cu).  That is 3.4 ranges read per block at 64 blocks
+// a row.  Rows longer than kRunRow blocks would make the runs mostly ends: each
+// of the nine rows is then a run of its own, 9.1 ranges per block.
+// 32 queries over 64^3-block volumes (8.4 M block tests): 23 us, and
+// 15 us in k_bentries; 105 us as one kernel that read six ranges of each of the
+// nine rows for four blocks and ordered the entries by a look-back over tiles.
 // ---------------------------------------------------------------------------
+constexpr uint32_t kGroup = kEngThreads / 32;  // tiles of a CTA's turn, a warp each
+constexpr uint32_t kRunRow = 256;
+constexpr uint32_t kRunWords = (kEngTile + 2 * kRunRow + 2) / 32 + 2;  // 1538 bits that start anywhere in a word
+constexpr uint32_t kRunBatch = 10;  // ranges in flight per lane
+
+// The query that tile `tile` of the batch's stream belongs to: the last with
+// tile0 <= tile (a warp's lanes look at 32 at a time).
 __device__ __forceinline__ uint32_t find_query(const EngQuery* __restrict__ qs, uint32_t nq, uint32_t tile)
 {
-    uint32_t lo = 0, hi = nq;  // last q with tile0 <= tile
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(&qs[mid].tile0) <= tile) lo = mid;
-        else hi = mid;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t n = 0;
+    for (uint32_t q = 0; q < nq; q += 32u) {
+        const uint32_t in = __popc(__ballot_sync(0xffffffffu, q + lane < nq && __ldg(&qs[min(q + lane, nq - 1u)].tile0) <= tile));
+        n += in;
+        if (in < 32u) break;
     }
-    return lo;
+    return n - 1u;
 }
 
-// Claims block b of volume v for this batch and gives it a slot from the free
-// list; when the pool has no free slot the claim is released and the batch
-// flagged (the host evicts and re-runs).
-__device__ __forceinline__ void claim_block(const BatchArgs& a, uint32_t v, int32_t* item_slots, uint32_t b,
-                                            uint32_t use_epoch)
-{
-    if (atomicCAS(item_slots + b, -1, -2) != -1) return;  // cached meanwhile, or claimed by another query
-    EngPool* pool = a.pool;
-    const uint32_t idx = atomicAdd(&pool->head, 1u);
-    const uint32_t tail = *(volatile uint32_t*)&pool->tail;
-    if ((int32_t)(idx - tail) >= 0) {  // no free slot: release the claim
-        atomicExch(item_slots + b, -1);
-        atomicOr(&a.st->pool_exhausted, 1u);
-        return;
-    }
-    const uint32_t slot = a.free_list[idx % pool->capacity];
-    a.last_use[slot] = use_epoch;
-    const uint32_t d = atomicAdd(&a.st->num_decode, 1u);
-    a.dec_vol[d] = v;
-    a.dec_block[d] = b;
-    a.dec_slot[d] = slot;
-}
+// Counts of the batch's tiles, then of its groups of tiles.
+__device__ __forceinline__ uint32_t* group_counts(const BatchArgs& a, uint32_t ntiles) { return a.tile_counts + ntiles; }
 
-__global__ void __launch_bounds__(kEngThreads) k_bactive(BatchArgs a)
+struct RunWords {
+    uint2 bits[kRunWords];  // iso >= lo, iso <= hi of the run's blocks
+    uint32_t near[3][kRunWords + 1];  // those and their AND, of a block or a neighbour along x
+};
+
+// Active bits of the 32 blocks of the lane's word of the tile that starts at b0.
+__device__ __forceinline__ uint32_t tile_active(const EngVolDev& V, uint32_t b0, float iso, RunWords& run)
 {
-    __shared__ uint32_t s_warp[kEngThreads / 32 + 1];
-    __shared__ uint32_t s_tile, s_q, s_p;
-    EngState* st = a.st;
-    const uint32_t ntiles = st->ntiles, nq = st->nq, epoch = st->epoch, cap = st->entry_capacity;
-    const uint32_t use_epoch = st->use_epoch;
-    for (;;) {
-        if (threadIdx.x == 0) {
-            const uint32_t tile = atomicAdd(&st->tiles_active, 1u);
-            s_tile = tile;
-            s_q = tile < ntiles ? find_query(a.queries, nq, tile) : 0u;
-        }
-        __syncthreads();
-        const uint32_t tile = s_tile;
-        if (tile >= ntiles) break;
-        const uint32_t qi = s_q;
-        const EngQuery Q = a.queries[qi];
-        const EngVolDev& V = a.vols[Q.vol];
-        const uint32_t lt = tile - Q.tile0;
-        const uint32_t total = V.total;
-        const float iso = Q.iso;
-        const uint32_t b0 = lt * kEngTile + 4u * threadIdx.x;
-        uint32_t act = 0;
-        const float2 ext = __ldg(V.tile_ext + lt);
-        if (iso >= ext.x && iso <= ext.y && b0 < total) {
-            const uint32_t n = min(4u, total - b0);
-            const uint3 c = block_coords(b0, V.grid);
-            if (n == 4 && c.x + 3 < V.grid.nb.x) {
-                act = row4_active(V.ranges, V.grid, c, b0, iso);
-            } else {
-                for (uint32_t i = 0; i < n; ++i) act |= block_is_active(V.ranges, V.grid, b0 + i, iso) << i;
-            }
-            // cache lookup: mark use, claim what no slot holds
-            for (uint32_t i = 0; i < 4; ++i) {
-                if (!(act >> i & 1u)) continue;
-                const int32_t s = *(volatile int32_t*)(V.item_slots + b0 + i);
-                if (s >= 0) a.last_use[s] = use_epoch;
-                else if (s == -1) claim_block(a, Q.vol, V.item_slots, b0 + i, use_epoch);
-            }
-        }
-        // active bitmap: 8 threads (32 blocks) per word
-        uint32_t word = act << (4u * (threadIdx.x & 7u));
-        word |= __shfl_xor_sync(0xffffffffu, word, 1);
-        word |= __shfl_xor_sync(0xffffffffu, word, 2);
-        word |= __shfl_xor_sync(0xffffffffu, word, 4);
-        if ((threadIdx.x & 7u) == 0) a.bitmap[Q.bit0 + lt * (kEngTile / 32) + (threadIdx.x >> 3)] = word;
-        // compaction of (block, query) entries over the whole tile stream
-        uint32_t tot;
-        const uint32_t excl = cta_exclusive_scan<kEngThreads>((uint32_t)__popc(act), s_warp, &tot);
-        if (threadIdx.x < 32) {
-            const uint32_t p = warp_lookback(a.status_a, tile, tot, epoch, &st->error, 60u);
-            if (threadIdx.x == 0) {
-                s_p = p;
-                if (tot) atomicAdd(a.q_nactive + qi, tot);
-                if (tile == ntiles - 1) {
-                    st->num_entries = p + tot;
-                    if (p + tot > cap) st->entry_overflow = 1;
-                }
-            }
-        }
-        __syncthreads();
-        uint32_t pos = s_p + excl;
+    const uint32_t lane = threadIdx.x & 31u, total = V.total, nwords = div_up(total, 32u);
+    const uint3 nb = V.grid.nb;
+    const int64_t nx = nb.x, nxy = (int64_t)nb.x * nb.y;
+    const float2* ranges = V.ranges;
+    const uint32_t mine = b0 + 32u * lane;
+    const WordRows in_volume = word_rows(min(mine, total - 1u), V.grid);
+    const int rows = nb.x <= kRunRow ? 3 : 1;  // rows in a run
+    uint32_t any_a = 0, any_b = 0, any_c = 0, self_a = 0, self_b = 0;
+    for (int dz = -1; dz < 2; ++dz)
+        for (int dy0 = -1; dy0 < 2; dy0 += rows) {
+            // its words: the run's blocks and one more at either end
+            const int64_t lo = (int64_t)b0 + dz * nxy + dy0 * nx - 1,
+                          hi = (int64_t)b0 + dz * nxy + (dy0 + rows - 1) * nx + kEngTile;
+            const int64_t k0 = lo >> 5;
+            const uint32_t n = (uint32_t)((hi >> 5) - k0) + 1u;
+            const int64_t r0 = k0 * 32 + lane;
+            for (uint32_t w = 0; w < n; w += kRunBatch) {
+                float2 r[kRunBatch];
 #pragma unroll
-        for (uint32_t i = 0; i < 4; ++i) {
-            if (act >> i & 1u) {
-                if (pos < cap) {
-                    a.ent_id[pos] = b0 + i;
-                    a.ent_q[pos] = qi;
+                for (uint32_t u = 0; u < kRunBatch; ++u) {
+                    const int64_t b = r0 + 32 * (w + u);
+                    r[u] = w + u < n && b >= 0 && b < (int64_t)total ? __ldg(ranges + b) : make_float2(NAN, NAN);  // NaN: no bits
                 }
-                ++pos;
+                uint2 ab = make_uint2(0u, 0u);
+#pragma unroll
+                for (uint32_t u = 0; u < kRunBatch; ++u) {
+                    const uint32_t wa = __ballot_sync(0xffffffffu, iso >= r[u].x),
+                                   wb = __ballot_sync(0xffffffffu, iso <= r[u].y);
+                    if (lane == u) ab = make_uint2(wa, wb);
+                }
+                if (lane < kRunBatch && w + lane < n) run.bits[w + lane] = ab;
             }
+            __syncwarp();
+            for (uint32_t i = lane; i < n; i += 32u) {
+                const int64_t k = k0 + i;
+                const uint2 v = run.bits[i];
+                const uint2 p = i ? run.bits[i - 1u] : make_uint2(0u, 0u),
+                            q = i + 1u < n ? run.bits[i + 1u] : make_uint2(0u, 0u);
+                const WordEnds ends = word_ends((uint32_t)min(max(k, (int64_t)0), (int64_t)nwords - 1) * 32u, V.grid);
+                run.near[0][i] = ends.spread(v.x, p.x, q.x);
+                run.near[1][i] = ends.spread(v.y, p.y, q.y);
+                run.near[2][i] = ends.spread(v.x & v.y, p.x & p.y, q.x & q.y);
+            }
+            __syncwarp();
+            for (int dy = dy0; dy < dy0 + rows; ++dy) {
+                const uint32_t m = in_volume.mask(dy, dz);
+                const int64_t s = (int64_t)mine + dz * nxy + dy * nx;
+                const uint32_t k = (uint32_t)((s >> 5) - k0), sh = (uint32_t)s & 31u;
+                any_a |= __funnelshift_r(run.near[0][k], run.near[0][k + 1u], sh) & m;
+                any_b |= __funnelshift_r(run.near[1][k], run.near[1][k + 1u], sh) & m;
+                any_c |= __funnelshift_r(run.near[2][k], run.near[2][k + 1u], sh) & m;
+                if (dz == 0 && dy == 0) {
+                    self_a = run.bits[k].x;
+                    self_b = run.bits[k].y;
+                }
+            }
+            __syncwarp();
         }
+    const uint32_t act = (self_a & any_b) | (self_b & any_a) | any_c;
+    return mine >= total ? 0u : total - mine < 32u ? act & ((1u << (total - mine)) - 1u) : act;
+}
+
+__global__ void __launch_bounds__(kEngThreads, 4) k_bactive(BatchArgs a)
+{
+    __shared__ RunWords s_run[kGroup];
+    __shared__ uint32_t s_count[2][kGroup];
+    const uint32_t ntiles = a.st->ntiles, nq = a.st->nq, ngroups = div_up(ntiles, kGroup);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t turn = 0;
+    for (uint32_t g = blockIdx.x; g < ngroups; g += gridDim.x, turn ^= 1u) {
+        const uint32_t tile = g * kGroup + warp;
+        uint32_t count = 0;
+        if (tile < ntiles) {
+            const EngQuery Q = a.queries[find_query(a.queries, nq, tile)];
+            const EngVolDev& V = a.vols[Q.vol];
+            const uint32_t lt = tile - Q.tile0;
+            const float2 ext = __ldg(V.tile_ext + lt);
+            const uint32_t act = Q.iso >= ext.x && Q.iso <= ext.y ? tile_active(V, lt * kEngTile, Q.iso, s_run[warp]) : 0u;
+            a.bitmap[Q.bit0 + lt * (kEngTile / 32) + lane] = act;
+            count = __reduce_add_sync(0xffffffffu, __popc(act));
+            if (lane == 0) a.tile_counts[tile] = count;
+        }
+        if (lane == 0) s_count[turn][warp] = count;
         __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t sum = 0;
+            for (uint32_t w = 0; w < kGroup; ++w) sum += s_count[turn][w];
+            group_counts(a, ntiles)[g] = sum;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// k_bentries: the active (block, query) entries in the order of the tile
+// stream, and the claims of the blocks that no slot holds
+//
+// A CTA owns a contiguous range of groups of tiles.  Every count is known, so
+// it adds up those of the groups before its range and waits for nobody; a warp
+// takes a tile of a group, whose words' bits say where each entry goes.
+// ---------------------------------------------------------------------------
+// Claims for this batch those of a warp's blocks b[0 .. kN) that no slot held
+// (`open`, bit j for b[j]), and gives them slots from the free list; when the
+// pool has no free slot the claims are released and the batch flagged (the host
+// evicts and re-runs).  A claim is a chain of four round trips, so a warp takes
+// the slots and the decode list's places of all its claims at once
+// (k_bentries of a
+// first batch, all of whose blocks are new: 130 -> 57 us; of one with a few: 48 -> 29 us).
+template <int kN>
+__device__ __forceinline__ void claim_blocks(const BatchArgs& a, uint32_t v, int32_t* item_slots, const uint32_t b[kN],
+                                             uint32_t open, uint32_t use_epoch)
+{
+    const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    uint32_t won = 0, n = 0, at[kN];
+#pragma unroll
+    for (int j = 0; j < kN; ++j)  // not: cached meanwhile, or claimed by another query
+        if (open >> j & 1u) won |= (atomicCAS(item_slots + b[j], -1, -2) == -1 ? 1u : 0u) << j;
+#pragma unroll
+    for (int j = 0; j < kN; ++j) {
+        const uint32_t m = __ballot_sync(0xffffffffu, won >> j & 1u);
+        at[j] = n + __popc(m & below);
+        n += __popc(m);
+    }
+    if (!n) return;
+    EngPool* pool = a.pool;
+    uint32_t head = 0, tail = 0, d = 0;
+    if (lane == 0) {
+        tail = *(volatile uint32_t*)&pool->tail;
+        head = atomicAdd(&pool->head, n);
+    }
+    head = __shfl_sync(0xffffffffu, head, 0);
+    tail = __shfl_sync(0xffffffffu, tail, 0);
+    const int32_t free_slots = (int32_t)(tail - head);
+    const uint32_t got = free_slots <= 0 ? 0u : min(n, (uint32_t)free_slots);
+    uint32_t slot[kN];
+#pragma unroll
+    for (int j = 0; j < kN; ++j)
+        slot[j] = (won >> j & 1u) && at[j] < got ? __ldg(a.free_list + (head + at[j]) % pool->capacity) : 0u;
+    if (lane == 0) {
+        if (got) d = atomicAdd(&a.st->num_decode, got);
+        if (got < n) atomicOr(&a.st->pool_exhausted, 1u);
+    }
+    d = __shfl_sync(0xffffffffu, d, 0);
+#pragma unroll
+    for (int j = 0; j < kN; ++j) {
+        if (!(won >> j & 1u)) continue;
+        if (at[j] < got) {
+            a.last_use[slot[j]] = use_epoch;
+            a.dec_vol[d + at[j]] = v;
+            a.dec_block[d + at[j]] = b[j];
+            a.dec_slot[d + at[j]] = slot[j];
+        } else {
+            atomicExch(item_slots + b[j], -1);  // no free slot: release the claim
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kEngThreads) k_bentries(BatchArgs a)
+{
+    __shared__ uint32_t s_sum;
+    EngState* st = a.st;
+    const uint32_t ntiles = st->ntiles, nq = st->nq, cap = st->entry_capacity, use_epoch = st->use_epoch;
+    const uint32_t ngroups = div_up(ntiles, kGroup), per = div_up(ngroups, gridDim.x);
+    const uint32_t first = blockIdx.x * per, end = min(ngroups, first + per);
+    if (first >= ngroups) return;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
+    const uint32_t* groups = group_counts(a, ntiles);
+    if (threadIdx.x == 0) s_sum = 0;
+    __syncthreads();
+    uint32_t sum = 0;
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < first; i += kEngThreads) sum += __ldg(groups + i);
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0 && sum) atomicAdd(&s_sum, sum);
+    __syncthreads();
+    uint32_t base = s_sum;
+    for (uint32_t g = first; g < end; ++g) {
+        const uint32_t t0 = g * kGroup, tile = t0 + warp;
+        const uint32_t n = lane < kGroup && t0 + lane < ntiles ? __ldg(a.tile_counts + t0 + lane) : 0u;
+        const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? n : 0u);
+        const uint32_t count = __shfl_sync(0xffffffffu, n, warp);
+        uint32_t at = base + before;
+        base += __reduce_add_sync(0xffffffffu, n);
+        if (!count) continue;
+        const uint32_t qi = find_query(a.queries, nq, tile);
+        const EngQuery Q = a.queries[qi];
+        int32_t* item_slots = a.vols[Q.vol].item_slots;
+        const uint32_t lt = tile - Q.tile0;
+        const uint32_t word = __ldg(a.bitmap + Q.bit0 + lt * (kEngTile / 32) + lane);
+        if (lane == 0) atomicAdd(a.q_nactive + qi, count);
+        // kN words at a time, their blocks' slots read together
+        constexpr int kN = 4;
+        for (uint32_t i = 0; i < 32u; i += kN) {
+            uint32_t w[kN], b[kN], open = 0;
+            int32_t s[kN];
+#pragma unroll
+            for (int j = 0; j < kN; ++j) {
+                w[j] = __shfl_sync(0xffffffffu, word, i + j);
+                b[j] = lt * kEngTile + 32u * (i + j) + lane;
+                s[j] = w[j] >> lane & 1u ? *(volatile int32_t*)(item_slots + b[j]) : -2;
+            }
+#pragma unroll
+            for (int j = 0; j < kN; ++j) {
+                if (w[j] >> lane & 1u) {
+                    const uint32_t pos = at + __popc(w[j] & below);
+                    if (pos < cap) {
+                        a.ent_id[pos] = b[j];
+                        a.ent_q[pos] = qi;
+                    }
+                    if (s[j] >= 0) a.last_use[s[j]] = use_epoch;
+                    open |= (s[j] == -1 ? 1u : 0u) << j;
+                }
+                at += __popc(w[j]);
+            }
+            if (__any_sync(0xffffffffu, open)) claim_blocks<kN>(a, Q.vol, item_slots, b, open, use_epoch);
+        }
+    }
+    if (end == ngroups && threadIdx.x == 0) {
+        st->num_entries = base;
+        if (base > cap) st->entry_overflow = 1;
     }
 }
 
@@ -613,7 +769,7 @@ struct EngVolume {
 // Launch parameters the autotuner chooses per batch-size bucket (the kernels'
 // tile shapes are compile-time; these are the runtime knobs).
 struct EngConfig {
-    int act_per_sm = 8;      // k_bactive CTAs per SM
+    int act_per_sm = 8;      // k_bactive and k_bentries CTAs per SM
     int dec_threads = 128;   // k_bdecode threads per CTA (64, 128, 256)
     int dec_per_sm = 16;     // k_bdecode CTAs per SM
     int mc_per_sm = kBmcPerSm;  // k_bmc CTAs per SM of the 16-block tile (<= its residency, 6); scaled
@@ -753,7 +909,7 @@ BatchArgs eng_args(bcmc_engine* e)
     a.dec_block = e->dec_block;
     a.dec_slot = e->dec_slot;
     a.verts = e->L->verts;
-    a.status_a = e->L->status;
+    a.tile_counts = reinterpret_cast<uint32_t*>(e->L->status);  // two words to a tile: the groups fit as well
     a.status_v = e->L->status + e->L->status_a_words;
     a.status_b = a.status_v + eng_grid_mc_max(e) + 1;
     return a;
@@ -942,6 +1098,7 @@ void eng_enqueue_front(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
     BCMC_CUDA(cudaEventRecordWithFlags(e->L->ev0, s, cudaEventRecordExternal));
     k_bbegin<<<1, 1024, 0, s>>>(e->L->d_st, e->L->q_nverts, e->L->q_nactive, bucket);
     k_bactive<<<eng_grid_act(e), kEngThreads, 0, s>>>(a);
+    k_bentries<<<eng_grid_act(e), kEngThreads, 0, s>>>(a);
     const uint32_t r = e->max_rate;
     if (e->cfg.dec_threads == 64) {
         const size_t smem = zfp_stage_smem(64, r);
@@ -956,7 +1113,7 @@ void eng_enqueue_front(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
         allow_smem(k_bdecode<128>, smem);
         k_bdecode<128><<<eng_grid_dec(e), 128, smem, s>>>(a, r);
     }
-    count_launches(3);
+    count_launches(4);
     BCMC_CUDA(cudaGetLastError());
 }
 

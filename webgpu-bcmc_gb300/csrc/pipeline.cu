@@ -97,7 +97,7 @@ constexpr uint32_t kFlagBatch = 8;  // ranges in flight per lane
 __global__ void __launch_bounds__(kFlagThreads) k_query_flags(QueryState* q, float iso, uint32_t capacity,
                                                              uint32_t vert_capacity, const QueryInputs* in, FlagArgs a)
 {
-    const uint32_t lane = threadIdx.x & 31u, total = a.total, nx = a.grid.nb.x, wpw = a.wpw;
+    const uint32_t lane = threadIdx.x & 31u, total = a.total, wpw = a.wpw;
     const uint32_t nwords = div_up(total, 32u);
     const uint32_t step = gridDim.x * (kFlagThreads / 32) * wpw;
     uint32_t w0 = (blockIdx.x * (kFlagThreads / 32) + (threadIdx.x >> 5)) * wpw;
@@ -147,26 +147,20 @@ __global__ void __launch_bounds__(kFlagThreads) k_query_flags(QueryState* q, flo
                 }
             }
         }
-        // the word's blocks at x = 0 and x = nx - 1, which have no neighbour there
-        const uint32_t first = (w0 + lane) * 32u, x0 = first - fdiv(first, a.grid.dx) * nx;
-        uint32_t no_left = 0, no_right = 0;
-        for (uint32_t p = x0 ? nx - x0 : 0u; p < 32u; p += nx) no_left |= 1u << p;
-        for (uint32_t p = nx - 1u - x0; p < 32u; p += nx) no_right |= 1u << p;
-        uint32_t pa = __shfl_up_sync(0xffffffffu, A, 1) >> 31, pb = __shfl_up_sync(0xffffffffu, B, 1) >> 31;
-        uint32_t na = __shfl_down_sync(0xffffffffu, A, 1) & 1u, nb = __shfl_down_sync(0xffffffffu, B, 1) & 1u;
+        const WordEnds ends = word_ends((w0 + lane) * 32u, a.grid);
+        uint32_t pa = __shfl_up_sync(0xffffffffu, A, 1), pb = __shfl_up_sync(0xffffffffu, B, 1);
+        uint32_t na = __shfl_down_sync(0xffffffffu, A, 1), nb = __shfl_down_sync(0xffffffffu, B, 1);
         if (lane == 0) {
-            pa = iso >= e.x;
-            pb = iso <= e.y;
+            pa = iso >= e.x ? 1u << 31 : 0u;
+            pb = iso <= e.y ? 1u << 31 : 0u;
         }
         if (lane == wpw - 1u) {
             na = iso >= e.x;
             nb = iso <= e.y;
         }
-        const auto spread = [&](uint32_t v, uint32_t prev, uint32_t next) {
-            return v | (((v << 1) | prev) & ~no_left) | (((v >> 1) | (next << 31)) & ~no_right);
-        };
         if (lane < wpw && w0 + lane < nwords) {
-            a.near[w0 + lane] = make_uint4(spread(A, pa, na), spread(B, pb, nb), spread(A & B, pa & pb, na & nb), A);
+            a.near[w0 + lane] = make_uint4(ends.spread(A, pa, na), ends.spread(B, pb, nb),
+                                           ends.spread(A & B, pa & pb, na & nb), A);
             a.hi[w0 + lane] = B;
         }
         if (w0 + step < nwords) {
@@ -233,7 +227,7 @@ __device__ __forceinline__ void active_finish(QueryState* q, uint32_t A, uint32_
 // k_active_words: the active test of the MC path (compute_block_active.comp:24-61)
 // on k_query_flags' words, with the compaction of the active ids and of the ids
 // that no slot holds.  With A = iso >= lo and B = iso <= hi of a block, the
-// reference's test over a block's 26 neighbours is (see block_is_active)
+// reference's test over a block's 26 neighbours is (see active_test.cuh)
 //   active = (A && anyB) || (B && anyA) || any(A_n && B_n),
 // any over the 3x3x3 neighbourhood.  The words hold the ORs along x, so a lane
 // ORs the nine (y, z) neighbour rows of its word, each two words and a funnel
@@ -270,29 +264,13 @@ __global__ void __launch_bounds__(kWordThreads, kWordPerSm) k_active_words(Query
         const uint32_t w = w0 + lane, b0 = 32u * w;
         uint32_t act = 0;
         if (lane < wpw && w < end) {
-            // the blocks with a row before and after them in y and in z
-            uint32_t ym = 0, yp = 0, zm = 0, zp = 0;
-            uint3 c = block_coords(b0, a.grid);
-            for (uint32_t p = 0; p < 32u;) {  // the pieces of rows in the word
-                const uint32_t len = min(nb.x - c.x, 32u - p);
-                const uint32_t m = (0xffffffffu >> (32u - len)) << p;
-                ym |= c.y > 0u ? m : 0u;
-                yp |= c.y + 1u < nb.y ? m : 0u;
-                zm |= c.z > 0u ? m : 0u;
-                zp |= c.z + 1u < nb.z ? m : 0u;
-                p += len;
-                c.x = 0;
-                if (++c.y == nb.y) {
-                    c.y = 0;
-                    ++c.z;
-                }
-            }
+            const WordRows in_volume = word_rows(b0, a.grid);
             uint32_t any_a = 0, any_b = 0, any_c = 0;
 #pragma unroll
             for (int dz = -1; dz < 2; ++dz)
 #pragma unroll
                 for (int dy = -1; dy < 2; ++dy) {
-                    const uint32_t m = (dz < 0 ? zm : dz > 0 ? zp : 0xffffffffu) & (dy < 0 ? ym : dy > 0 ? yp : 0xffffffffu);
+                    const uint32_t m = in_volume.mask(dy, dz);
                     // the row's first block; a word out of the volume holds no block that the masks leave
                     const int64_t s = (int64_t)b0 + dz * nxy + dy * nx;
                     const int64_t k = s >> 5;
