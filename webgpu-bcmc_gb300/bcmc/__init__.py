@@ -60,7 +60,7 @@ class DeviceArray:
         """Zero-copy torch view; unsigned words appear as int32/int64 (same bits)."""
         t = _torch()
         signed = {"<u4": "<i4", "<u8": "<i8"}.get(self.typestr, self.typestr)
-        if int(np.prod(self.shape)) == 0:
+        if 0 in self.shape:
             dt = {"<i4": t.int32, "<f4": t.float32, "<i8": t.int64}[signed]
             return t.zeros(self.shape, dtype=dt, device="cuda")
         return t.as_tensor(DeviceArray(self.ptr, self.shape, signed, self), device="cuda")
