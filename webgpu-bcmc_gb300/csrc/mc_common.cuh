@@ -33,12 +33,13 @@ constexpr uint32_t kMcBlocks = 4;  // blocks a warp works on at a time
 struct McTables {
     mc_detail::TriCounts count;
     mc_detail::GhostAxes ghost;
-    mc_detail::CaseRows rows;
+    mc_detail::TriRows rows;
+    mc_detail::CellRecs cells;
 };
 constexpr uint32_t kMcFirstTables = (sizeof(mc_detail::TriCounts) + sizeof(mc_detail::GhostAxes)) / 16;
 static_assert(sizeof(McTables) % 16 == 0 && offsetof(McTables, rows) == 16 * kMcFirstTables, "16-byte pieces");
 static __device__ const __align__(16) McTables c_mc = {mc_detail::make_tri_counts(), mc_detail::make_ghost_axes(),
-                                                       mc_detail::make_case_rows()};
+                                                       mc_detail::make_tri_rows(), mc_detail::make_cell_recs()};
 // for the few vertices that take the exact expression: read where it lies
 static __device__ const __align__(16) mc_detail::CornerPack c_corner_pack = mc_detail::make_corner_pack();
 
@@ -50,9 +51,10 @@ struct McWarpMem {
     // cells and triangles listed at a time (one block has up to 64 and 320)
     static constexpr uint32_t kCells = 128, kTris = 512;
     float vol[kMcBlocks][128];  // the blocks' 5^3 grids
-    // cells with triangles, in order: x is where vertex 0 of the list would be in
-    // the cell's row of the case table (in bytes, from the table's start), y the
-    // cell's position (x << 20 | y << 10 | z) and from bit 23 its corner 0 in vol
+    // cells with triangles, in order: x is, from bit 16, where triangle 0 of the list
+    // would be in the cell's row of the case table, and below where the cell is in
+    // the cells' table; y its corner 0 in vol, and from bit 30 the block (all but
+    // the last in bytes from the table's or array's start)
     uint2 list[kCells];
     uint8_t flag[kTris];  // 1 where a triangle is its cell's first; zero between emits
     uint32_t slot[32];    // the lookups' slots, lane 8j + o
@@ -107,8 +109,9 @@ struct McLane {
     const uint32_t* where[4];  // the slot of its neighbour of block 0, in the warp's memory
     uint32_t g;           // corner 0 of cell `lane` in the grid; cell lane + 32's is at g + 50
     uint32_t need;        // axes on which cell `lane` needs the ghost layer, and from bit 3 cell lane + 32
-    uint32_t cell;        // cell `lane` as the emit lists it: x << 20 | y << 10 | z | g << 23
-    uint32_t upto[3];     // of 32 triangles, those up to that of vertex lane + 32k
+    // the emit's turn of 32 triangles into 96 vertices in order (mc_emit)
+    uint32_t from, turn;  // the lane whose first vertex comes here, and which of the three it then is
+    uint32_t tri[3];      // the lanes whose triangles vertices lane, 32 + lane and 64 + lane are of
 };
 __device__ __forceinline__ McLane mc_lane(const float* cache, const uint32_t* slots)
 {
@@ -126,9 +129,10 @@ __device__ __forceinline__ McLane mc_lane(const float* cache, const uint32_t* sl
     m.g = x + 5u * (y + 5u * z);
     const uint32_t xy = (x == 3u ? 1u : 0u) | (y == 3u ? 2u : 0u);
     m.need = xy | ((xy | (z == 1u ? 4u : 0u)) << 3);
-    m.cell = (x << 20) | (y << 10) | z | (m.g << 23);
+    m.from = (11u * lane) & 31u;
+    m.turn = (3u * m.from) >> 5;
 #pragma unroll
-    for (uint32_t k = 0; k < 3; ++k) m.upto[k] = 0xffffffffu >> (31u - (lane + 32u * k) / 3u);
+    for (uint32_t k = 0; k < 3; ++k) m.tri[k] = (lane + 32u * k) / 3u;
     return m;
 }
 
@@ -237,13 +241,14 @@ struct McSink {
 
     __device__ __forceinline__ explicit McSink(uint2* first) { start(first); }
     __device__ __forceinline__ void start(uint2* first) { at = first + (kHost ? 0u : threadIdx.x & 31u); }
-    // vertices 32k + lane of a window of up to 96, n of them still to come
-    __device__ __forceinline__ void put(uint2* stage, uint32_t k, uint32_t n, uint2 v)
+    // vertices 32k + lane of a window's nv (up to 96)
+    __device__ __forceinline__ void put(uint2* stage, uint32_t k, uint32_t nv, uint2 v)
     {
         const uint32_t lane = threadIdx.x & 31u;
         if constexpr (!kHost) {
-            if (lane < n) at[32u * k] = v;
+            if (lane + 32u * k < nv) at[32u * k] = v;
         } else {
+            const uint32_t n = nv - min(nv, 32u * k);
             if (lane < n) stage[held + lane] = v;
             __syncwarp();
             held += min(n, 32u);
@@ -299,12 +304,17 @@ __device__ __forceinline__ void mc_grids(const McLane& m, Mem& s, uint32_t n)
 // lane 8j) to the sink, in block, cell and table order.  The cells with
 // triangles are listed first, with a flag at each one's first triangle, as many
 // blocks' as the list holds (in most cases all).  Then, 32 triangles at a time,
-// a ballot of the flags tells a lane which cell its vertex is of: the last that
-// starts at or before the vertex's triangle.  A lane takes one vertex at a time,
-// so that the stores are contiguous, and works its position out from the cell's
-// coordinates: what binds this loop besides the issue slots is the shared-memory
-// pipe, and a triangle to a lane with its vertices staged through shared memory,
-// and a table of the fixed axes' positions, took over twice the accesses.
+// a ballot of the flags tells a lane which cell its triangle is of: the last that
+// starts at or before it.  What is the cell's is so looked up once for three
+// vertices; for stores that are contiguous the 96 then change lanes: vertex
+// 3 s + r of lane s's triangle belongs in lane (3 s + r) mod 32, for one r a
+// different lane for each s, so three shuffles move them, and a lane's three
+// arrive turned by 0, 1 or 2 places, which is the same in every window.
+// Issue slots (75 % taken) and the shared-memory pipe (79 %) bind this loop alike:
+// with a vertex to a lane the kernel took 868 us of the 512^3 volume's query (165 M
+// vertices, 812 M warp instructions), now 789 us (720 M).  A shuffle takes two
+// turns of that pipe; still, staging the 96 in shared memory instead, and a table
+// of the edges' or fixed axes' positions, took over twice the accesses.
 // `ahead` is called once, when the grids are there, to start loads for what
 // comes next.
 template <bool kHost, bool kOneIso, typename Ahead>
@@ -312,6 +322,7 @@ __device__ __forceinline__ void mc_emit(const McLane& m, const McTables& tab, Mc
                                         uint32_t id, uint32_t has, float iso, McSink<kHost>& sink, Ahead ahead)
 {
     const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    const char *rows = reinterpret_cast<const char*>(&tab.rows), *cell_recs = reinterpret_cast<const char*>(&tab.cells);
     async_wait<0>();
     __syncwarp();
     ahead();
@@ -331,16 +342,16 @@ __device__ __forceinline__ void mc_emit(const McLane& m, const McTables& tab, Mc
             const uint32_t e0 = __ballot_sync(kFull, t0 != 0u), e1 = __ballot_sync(kFull, t1 != 0u);
             const uint32_t n0 = __popc(e0), n01 = n0 + __popc(e1);
             if (cells + n01 > s.kCells || tris + sum > s.kTris) break;
-            const uint32_t where = m.cell | (b << 30);  // cell lane + 32 lies two layers up
+            const uint32_t where = 4u * m.g + 512u * b + (b << 30);  // cell lane + 32 lies two layers up
             if (t0) {
                 const uint32_t first = tris + (inc & 0xffffu) - t0;
-                s.list[cells + __popc(e0 & below)] = make_uint2(60u * c0 - 12u * first, where);
+                s.list[cells + __popc(e0 & below)] = make_uint2(((80u * c0 - 16u * first) << 16) + 8u * lane, where);
                 s.flag[first] = 1;
             }
             if (t1) {
                 const uint32_t first = tris + (tot & 0xffffu) + (inc >> 16) - t1;
                 s.list[cells + n0 + __popc(e1 & below)] =
-                    make_uint2(60u * c1 - 12u * first, where + 2u + (50u << 23));
+                    make_uint2(((80u * c1 - 16u * first) << 16) + 8u * lane + 256u, where + 200u);
                 s.flag[first] = 1;
             }
             tris += sum;
@@ -352,22 +363,40 @@ __device__ __forceinline__ void mc_emit(const McLane& m, const McTables& tab, Mc
         for (uint32_t w = 0; w < tris; w += 32u) {
             const uint32_t starts = __ballot_sync(kFull, s.flag[w + lane] != 0);
             s.flag[w + lane] = 0;
-            const uint32_t nv = 3u * min(tris - w, 32u);
-#pragma unroll
-            for (uint32_t k = 0; k < 3; ++k) {
-                if (k && 32u * k >= nv) break;
-                const uint32_t i = lane + 32u * k;  // of the window's vertices; past the last: worked on, not kept
-                const uint2 e = s.list[before + __popc(starts & m.upto[k]) - 1u];
-                const uint32_t j = e.y >> 30;
-                const uint32_t bid = __shfl_sync(kFull, id, 8u * j);
-                const float biso = kOneIso ? iso : __shfl_sync(kFull, iso, 8u * j);
-                const uint32_t word = *reinterpret_cast<const uint32_t*>(
-                    reinterpret_cast<const char*>(&tab.rows) + (int32_t)(e.x + 4u * (3u * w + min(i, nv - 1u))));
-                bool again;
-                uint32_t v = mc_vertex_fast(word, &s.vol[0][0] + (e.y >> 23), e.y & (3u * kAxisOnes), biso, &again);
-                if (again && i < nv) v = mc_vertex_exact(word, s.vol[j], e.y, &c_corner_pack.p[0][0], biso);
-                sink.put(s.out, k, nv - 32u * k, make_uint2(v, bid));
+            const uint32_t nt = min(tris - w, 32u), nv = 3u * nt;
+            const uint2 e = s.list[before + __popc(starts & (2u * below + 1u)) - 1u];
+            const uint32_t block = e.y >> 27;  // the lane that has the block's values: 8j
+            const uint32_t bid = __shfl_sync(kFull, id, block);
+            const float biso = kOneIso ? iso : __shfl_sync(kFull, iso, block);
+            // lanes past the last triangle work on that, which is not kept
+            const uint4 row = *reinterpret_cast<const uint4*>(rows + ((int32_t)e.x >> 16) +
+                                                              (int32_t)(16u * (w + min(lane, nt - 1u))));
+            const uint2 rec2 = *reinterpret_cast<const uint2*>(cell_recs + (e.x & 0xffffu));
+            const mc_detail::CellRec rec{rec2.x, rec2.y};
+            const float* vol = reinterpret_cast<const float*>(reinterpret_cast<const char*>(&s.vol[0][0]) + (e.y & 0x7ffu));
+            bool a0, a1, a2;
+            uint32_t v0 = mc_vertex_fast(row.x, vol, rec, biso, &a0), v1 = mc_vertex_fast(row.y, vol, rec, biso, &a1),
+                     v2 = mc_vertex_fast(row.z, vol, rec, biso, &a2);
+            if ((a0 || a1 || a2) && lane < nt) {
+                const uint32_t c = (e.x & 0xffffu) >> 3, cell = ((c & 3u) << 20) | (((c >> 2) & 3u) << 10) | (c >> 4);
+                uint32_t redo = (a0 ? 1u : 0u) | (a1 ? 2u : 0u) | (a2 ? 4u : 0u);
+#pragma unroll 1
+                for (; redo; redo &= redo - 1u) {
+                    const uint32_t v = mc_vertex_exact(redo & 1u ? row.x : redo & 2u ? row.y : row.z, s.vol[block >> 3], cell,
+                                                       &c_corner_pack.p[0][0], biso);
+                    if (redo & 1u) v0 = v;
+                    else if (redo & 2u) v1 = v;
+                    else v2 = v;
+                }
             }
+            __syncwarp();
+            v0 = __shfl_sync(kFull, v0, m.from);
+            v1 = __shfl_sync(kFull, v1, m.from - 11u);
+            v2 = __shfl_sync(kFull, v2, m.from - 22u);
+            const bool one = m.turn == 1u, two = m.turn == 2u;
+            sink.put(s.out, 0u, nv, make_uint2(one ? v1 : two ? v2 : v0, __shfl_sync(kFull, bid, m.tri[0])));
+            sink.put(s.out, 1u, nv, make_uint2(one ? v0 : two ? v1 : v2, __shfl_sync(kFull, bid, m.tri[1])));
+            sink.put(s.out, 2u, nv, make_uint2(one ? v2 : two ? v0 : v1, __shfl_sync(kFull, bid, m.tri[2])));
             sink.next_window(nv);
             before += __popc(starts);
         }
