@@ -23,11 +23,6 @@ namespace bcmc {
 
 constexpr uint32_t kZfpMaxBitsLimit = 64u * 32u;  // rate <= 32 bits/value
 
-__device__ __forceinline__ int32_t zfp_uint2int(uint32_t x)
-{
-    return (int32_t)((x ^ 0xaaaaaaaau) - 0xaaaaaaaau);
-}
-
 // inverse_lift (zfp_decompress.comp:296-332).  WGSL integer arithmetic wraps,
 // and streams that are not encoder output (or corrupt ones) do overflow here,
 // so adds, subtracts and left shifts run in uint32 (C++ signed overflow would
@@ -101,7 +96,7 @@ __device__ __forceinline__ float zfp_inv_weight(int32_t emax)
 // Deposit (zfp_planes_deposit): the plane masks go to a per-thread row of
 // shared memory; each 8-plane chunk is read back as 8 rows of 64 bits and all
 // eight 8x8 byte columns are transposed at once by three delta-swap stages,
-// after which byte g of row k is coefficient 8g + k's bits of those planes.
+// after which byte g of row k is coefficient 8g + k's digits in those planes.
 // ---------------------------------------------------------------------------
 
 // PTX shifts clamp the count: a shift by 32 or more gives 0 (the host
@@ -124,6 +119,29 @@ __device__ __forceinline__ uint32_t zfp_shr(uint32_t x, uint32_t s)
     return r;
 #else
     return s >= 32u ? 0u : x >> s;
+#endif
+}
+
+// the low m bits, all from 32 on
+__device__ __forceinline__ uint32_t zfp_low(uint32_t m)
+{
+#ifdef __CUDA_ARCH__
+    uint32_t r;
+    asm("bmsk.clamp.b32 %0, 0, %1;" : "=r"(r) : "r"(m));
+    return r;
+#else
+    return m >= 32u ? 0xffffffffu : (1u << m) - 1u;
+#endif
+}
+// the zeros below the lowest 1, all ones (a large number) for 0
+__device__ __forceinline__ uint32_t zfp_ctz(uint32_t x)
+{
+#ifdef __CUDA_ARCH__
+    uint32_t r;
+    asm("bfind.shiftamt.u32 %0, %1;" : "=r"(r) : "r"(__brev(x)));
+    return r;
+#else
+    return x ? (uint32_t)__builtin_ctz(x) : 0xffffffffu;
 #endif
 }
 
@@ -167,21 +185,20 @@ __device__ __forceinline__ uint32_t zfp_parse_planes(const uint32_t* w, uint32_t
         const uint32_t b0 = __funnelshift_r(a0, a1, 1), b1 = a1 >> 1;  // window bits 1..63
         const bool gtr = n < 64u && bits != 0u;  // a group test is read
         const bool one = gtr && (a0 & 1u);
-        // a 1: t zeros before the next one (63: none within the window)
-        const uint32_t t = b0 ? (uint32_t)__ffs(b0) - 1u : (b1 ? (uint32_t)__ffs(b1) + 31u : 63u);
+        // a 1: t zeros before the next one (all ones: none within the window)
+        const uint32_t t = min(zfp_ctz(b0), zfp_ctz(b1) | 32u);
         const uint32_t lim = min(63u - n, bits - 1u);
         const uint32_t z = min(t, lim), hit = t < lim ? 1u : 0u;
         const uint32_t nt = n + z;  // the coefficient that becomes significant
         // a 0 (or no read): the plane ends; the next plane's raw bits follow
         const uint32_t o = gtr ? 1u : 0u, be = bits - o, m = min(n, be);
         if (!one) {
-            pl[2 * r] = xlo;
-            pl[2 * r + 1] = xhi;
+            reinterpret_cast<uint2*>(pl)[r] = make_uint2(xlo, xhi);
             ++r;
             if (r == 32u || be == 0u) break;
         }
         const uint32_t c0 = gtr ? b0 : a0, c1 = gtr ? b1 : a1;
-        const uint32_t rlo = c0 & (zfp_shl(1u, m) - 1u), rhi = c1 & zfp_shr(0xffffffffu, 64u - m);
+        const uint32_t rlo = c0 & zfp_low(m), rhi = c1 & zfp_shr(0xffffffffu, 64u - m);
         const uint32_t tlo = xlo | zfp_shl(1u, nt), thi = xhi | zfp_shl(1u, nt - 32u);
         xlo = one ? tlo : rlo;
         xhi = one ? thi : rhi;
@@ -240,36 +257,66 @@ __device__ __forceinline__ void zfp_chunk(const uint32_t* pl, uint32_t c, uint32
     zfp_transpose(L, H);
 }
 
-// Coefficients (stream order) from the stored planes r0 .. planes - 1: chunk
-// c's byte of a coefficient goes to bits 31 - r0 - 8c down to 24 - r0 - 8c.
-__device__ __forceinline__ void zfp_planes_deposit(const uint32_t* pl, uint32_t planes, uint32_t r0, uint32_t* u)
+// Coefficients (stream order) from the stored planes r0 .. planes - 1.  A plane
+// is a negabinary digit: a coefficient is the sum of +-2^p over its digits' bit
+// positions p, plus for even p, minus for odd (mod 2^32, as (u ^ 0xaaaaaaaa) -
+// 0xaaaaaaaa is).  A chunk's byte of digits, the lowest at position k, is so
+// ((byte ^ 0xaa) - 0xaa) * (-2)^k: the exclusive-or is done to four bytes at
+// once, the subtractions of all chunks are one constant, and a coefficient takes
+// a byte permute and a multiply-add a chunk -- of which the second is in the pipe
+// that has time left -- where a permute, a shift, an or, and the two steps from
+// negabinary at the end took 2.3 of the other's.
+__device__ __forceinline__ void zfp_planes_deposit(const uint32_t* pl, uint32_t planes, uint32_t r0, uint32_t* v)
 {
     const uint32_t np = planes - r0;
+    // (-2)^k of chunk c, k = 24 - r0 - 8 c; 1 where k is negative: that chunk has fewer than 8 planes
+    const auto scale_of = [&](uint32_t c) {
+        const int32_t k = 24 - (int32_t)(r0 + 8u * c);
+        const uint32_t s = k > 0 ? 1u << k : 1u;
+        return k > 0 && (k & 1) ? 0u - s : s;
+    };
+    const auto chunk = [&](uint32_t c, uint32_t* L, uint32_t* H) {
+        zfp_chunk(pl, c, np, L, H);
+        const int32_t k = 24 - (int32_t)(r0 + 8u * c);
+        if (k < 0) {  // its planes to the low end
+            const uint32_t s = (uint32_t)-k, keep = zfp_shr(0xffu, s) * 0x01010101u;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                L[j] = zfp_shr(L[j], s) & keep;
+                H[j] = zfp_shr(H[j], s) & keep;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            L[j] ^= 0xaaaaaaaau;
+            H[j] ^= 0xaaaaaaaau;
+        }
+    };
+    uint32_t scales = scale_of(0u);
+    for (uint32_t c = 1; c * 8u < np; ++c) scales += scale_of(c);
+    const uint32_t base = 0u - 0xaau * scales;
     {
         uint32_t L[8], H[8];
-        zfp_chunk(pl, 0u, np, L, H);
-        // r0 is 32 only for a block whose 32 planes are all empty: np is 0,
-        // every row is zero, and the shift (kept below 32, as C++ requires)
-        // moves nothing
-        const uint32_t s0 = r0 & 31u;
+        chunk(0u, L, H);
+        const uint32_t scale = scale_of(0u);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-                u[8 * g + k] = __byte_perm(L[k], 0u, 0x0444u | ((uint32_t)g << 12)) >> s0;
-                u[8 * (g + 4) + k] = __byte_perm(H[k], 0u, 0x0444u | ((uint32_t)g << 12)) >> s0;
+                v[8 * g + k] = __byte_perm(L[k], 0u, 0x4440u | (uint32_t)g) * scale + base;
+                v[8 * (g + 4) + k] = __byte_perm(H[k], 0u, 0x4440u | (uint32_t)g) * scale + base;
             }
     }
     for (uint32_t c = 1; c * 8u < np; ++c) {
         uint32_t L[8], H[8];
-        zfp_chunk(pl, c, np, L, H);
-        const uint32_t rs = 8u * c + r0;
+        chunk(c, L, H);
+        const uint32_t scale = scale_of(c);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-                u[8 * g + k] |= __byte_perm(L[k], 0u, 0x0444u | ((uint32_t)g << 12)) >> rs;
-                u[8 * (g + 4) + k] |= __byte_perm(H[k], 0u, 0x0444u | ((uint32_t)g << 12)) >> rs;
+                v[8 * g + k] += __byte_perm(L[k], 0u, 0x4440u | (uint32_t)g) * scale;
+                v[8 * (g + 4) + k] += __byte_perm(H[k], 0u, 0x4440u | (uint32_t)g) * scale;
             }
     }
 }
@@ -292,10 +339,7 @@ __device__ __forceinline__ void zfp_decode_staged(const uint32_t* w, uint32_t ma
     uint32_t u[64];
     zfp_planes_deposit(pl, planes, r0, u);
     int32_t v[64];
-    uint32_t un[64];
-    BCMC_ZFP_GATHER(un, u)
-#pragma unroll
-    for (int i = 0; i < 64; ++i) v[i] = zfp_uint2int(un[i]);
+    BCMC_ZFP_GATHER(v, (int32_t)u)
     zfp_inverse_transform(v);
     const float wt = zfp_inv_weight(emax);
 #pragma unroll
