@@ -13,12 +13,14 @@
 #pragma once
 
 #include "bcmc_internal.cuh"
+#include "bcmc_pipeline.h"
 
 namespace bcmc {
 
 // Of the 32 blocks from b0 on: those with a row before and after them in y and in z.
 struct WordRows {
     uint32_t ym, yp, zm, zp;
+    uint32_t sound;  // those whose coordinates are below SoundRanges'
 
     __device__ __forceinline__ uint32_t mask(int dy, int dz) const
     {
@@ -26,9 +28,9 @@ struct WordRows {
     }
 };
 
-__device__ __forceinline__ WordRows word_rows(uint32_t b0, const BlockGrid& g)
+__device__ __forceinline__ WordRows word_rows(uint32_t b0, const BlockGrid& g, const SoundRanges& sound)
 {
-    WordRows r{0u, 0u, 0u, 0u};
+    WordRows r{0u, 0u, 0u, 0u, 0u};
     uint3 c = block_coords(b0, g);
     for (uint32_t p = 0; p < 32u;) {  // the pieces of rows in the word
         const uint32_t len = min(g.nb.x - c.x, 32u - p);
@@ -37,6 +39,8 @@ __device__ __forceinline__ WordRows word_rows(uint32_t b0, const BlockGrid& g)
         r.yp |= c.y + 1u < g.nb.y ? m : 0u;
         r.zm |= c.z > 0u ? m : 0u;
         r.zp |= c.z + 1u < g.nb.z ? m : 0u;
+        const uint32_t n = c.y < sound.y && c.z < sound.z && c.x < sound.x ? min(len, sound.x - c.x) : 0u;
+        r.sound |= n ? (0xffffffffu >> (32u - n)) << p : 0u;
         p += len;
         c.x = 0;
         if (++c.y == g.nb.y) {
@@ -51,11 +55,16 @@ __device__ __forceinline__ WordRows word_rows(uint32_t b0, const BlockGrid& g)
 struct WordEnds {
     uint32_t no_left, no_right;
 
+    // The word's bits ORed with those of the block after each along x.
+    __device__ __forceinline__ uint32_t up(uint32_t v, uint32_t next) const
+    {
+        return v | (__funnelshift_r(v, next, 1) & ~no_right);
+    }
     // The word's bits ORed with those of the blocks before and after each along x;
     // the last bit of `prev` and the first of `next` are those beside the word.
     __device__ __forceinline__ uint32_t spread(uint32_t v, uint32_t prev, uint32_t next) const
     {
-        return v | (__funnelshift_l(prev, v, 1) & ~no_left) | (__funnelshift_r(v, next, 1) & ~no_right);
+        return up(v, next) | (__funnelshift_l(prev, v, 1) & ~no_left);
     }
 };
 

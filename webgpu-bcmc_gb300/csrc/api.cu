@@ -150,6 +150,7 @@ struct bcmc_lru {
     size_t status_words = 0;
     uint64_t* st_active_a = nullptr;
     uint64_t* st_active_n = nullptr;
+    uint64_t* st_active_l = nullptr;
     uint64_t* st_slots = nullptr;
     uint64_t* st_sort = nullptr;
     uint64_t* st_mc_v = nullptr;
@@ -278,11 +279,12 @@ static bcmc_lru* lru_new(bcmc_ctx* ctx, uint32_t initial_size, uint32_t element_
         lru_alloc_slots(c, c->cache_size ? c->cache_size : 32u);
         const size_t wa = active_tiles(total) + 1, ws = slot_tiles(c->aligned_total) + 1,
                      wsort = sort_status_words(c->aligned_total), wm = mc_grid(ctx, total) + 1;
-        c->status_words = 2 * wa + ws + wsort + 2 * wm;
+        c->status_words = 3 * wa + ws + wsort + 2 * wm;
         c->status = (uint64_t*)dev_alloc(ctx, c->status_words * 8);
         c->st_active_a = c->status;
         c->st_active_n = c->st_active_a + wa;
-        c->st_slots = c->st_active_n + wa;
+        c->st_active_l = c->st_active_n + wa;
+        c->st_slots = c->st_active_l + wa;
         c->st_sort = c->st_slots + ws;
         c->st_mc_v = c->st_sort + wsort;
         c->st_mc_b = c->st_mc_v + wm;
@@ -389,6 +391,7 @@ struct bcmc_vol {
     void* flag_words = nullptr;  // k_query_flags' words (flag_bytes)
     uint32_t* active = nullptr;
     uint32_t* active_ids = nullptr;
+    uint32_t *live_ids = nullptr, *live_at = nullptr;  // the active blocks that can have vertices
     uint32_t* with_verts = nullptr;
     uint32_t* vert_offsets = nullptr;
     uint32_t* block_counts = nullptr;
@@ -438,6 +441,8 @@ static void vol_free(bcmc_vol* v)
     dev_free(ctx, v->flag_words, flag_bytes(v->total));
     dev_free(ctx, v->active, (size_t)v->total * 4);
     dev_free(ctx, v->active_ids, (size_t)v->total * 4);
+    dev_free(ctx, v->live_ids, (size_t)v->total * 4);
+    dev_free(ctx, v->live_at, (size_t)v->total * 4);
     dev_free(ctx, v->with_verts, (size_t)v->total * 4);
     dev_free(ctx, v->vert_offsets, (size_t)v->total * 4);
     dev_free(ctx, v->block_counts, (size_t)v->total * 4);
@@ -516,6 +521,8 @@ static bcmc_status vol_create_common(bcmc_ctx* ctx, const void* src, bool src_de
             v->flag_words = dev_alloc(ctx, flag_bytes(total));
             v->active = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
             v->active_ids = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
+            v->live_ids = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
+            v->live_at = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
             v->with_verts = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
             v->vert_offsets = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
             v->block_counts = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
@@ -654,7 +661,11 @@ static void vol_enqueue_query(bcmc_vol* v, cudaStream_t s, float iso, int from_s
     const BlockGrid grid = make_block_grid(nb);
     ActiveArgs aa{grid,          nullptr,    v->active,      c->item_slots,  v->total,
                   v->active_ids, c->new_ids, c->st_active_a, c->st_active_n};
-    McArgs ma{v->active, v->active_ids, c->item_slots, reinterpret_cast<const float*>(c->cache), nb, grid,
+    aa.live_ids = v->live_ids;
+    aa.live_at = v->live_at;
+    aa.status_l = c->st_active_l;
+    aa.sound = sound_ranges(v->dims, grid, zfp_ranged_blocks(ctx, v->dims));
+    McArgs ma{v->active, v->active_ids, v->live_ids, v->live_at, c->item_slots, reinterpret_cast<const float*>(c->cache), nb, grid,
               v->with_verts, v->vert_offsets, v->block_counts, out, c->st_mc_v, c->st_mc_b, out != v->verts ? 1u : 0u};
     SlotArgs sa{v->active,  c->slot_age, c->slot_avail, c->slot_item, c->avail_ids, c->avail_keys, c->st_slots, 1u, 1u,
                 c->age_hist, c->age_rank};
@@ -760,7 +771,7 @@ static bcmc_status vol_query(bcmc_vol* v, float iso, bcmc_perf* perf, uint32_t* 
             break;
         }
         const uint3 nb = make_uint3(v->nb[0], v->nb[1], v->nb[2]);
-        McArgs ma{v->active, v->active_ids, c->item_slots, reinterpret_cast<const float*>(c->cache), nb,
+        McArgs ma{v->active, v->active_ids, v->live_ids, v->live_at, c->item_slots, reinterpret_cast<const float*>(c->cache), nb,
                   make_block_grid(nb), v->with_verts, v->vert_offsets, v->block_counts, v->verts, c->st_mc_v,
                   c->st_mc_b};
         QueryState& h = *c->h_q;

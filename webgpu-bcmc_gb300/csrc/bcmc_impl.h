@@ -142,6 +142,8 @@ void compact_launch(bcmc_ctx* ctx, uint32_t n, const uint32_t* flags, const uint
 void prim_begin(QueryState* q, cudaStream_t s);
 
 // ---- zfp.cu -----------------------------------------------------------------
+// how many blocks zfp_ranges_launch gives their range; the others get (0, 0)
+uint64_t zfp_ranged_blocks(const bcmc_ctx* ctx, const uint32_t dims[3]);
 void zfp_ranges_launch(bcmc_ctx* ctx, const uint64_t* words, const uint32_t dims[3],
                        uint32_t max_bits, float* ranges, cudaStream_t s);
 void zfp_decode_blocks_launch(bcmc_ctx* ctx, const uint64_t* words, uint32_t max_bits,

@@ -37,6 +37,7 @@ struct QueryState {
     uint32_t vert_capacity;  // entries of the vertex buffer
     // active-block pass
     uint32_t num_active;
+    uint32_t num_live;       // of those, the blocks that marching cubes looks at
     uint32_t num_new;
     uint32_t old_cache_size;
     uint32_t new_cache_size;
@@ -312,43 +313,50 @@ __device__ __forceinline__ void grid_barrier(uint32_t* arrived, uint32_t target,
     __syncthreads();
 }
 
-// The sum over the CTAs before `rank` of the two counts each published in its
-// status words (aggregates of this epoch), to *sum_a and *sum_b in shared
-// memory, zero before (`drop`: this CTA publishes nothing, the test hook's case).
-// Every thread takes a share of the predecessors, so all
+// A count that every CTA publishes in its status word of `status`: this CTA's, the
+// code of a wait that gives up, and where the sum goes (shared memory, zero before).
+struct CtaCount {
+    uint64_t* status;
+    uint32_t count, site;
+    uint32_t* sum;
+};
+
+// The sums over the CTAs before `rank` of kN counts that each published in its
+// status words (aggregates of this epoch; `drop`: this CTA publishes nothing, the
+// test hook's case).  Every thread takes a share of the predecessors, so all
 // are read in one round trip; the wait is for the slowest of them.
-template <int kThreads>
-__device__ __forceinline__ void cta_prefix_sums(uint64_t* status_a, uint64_t* status_b, uint32_t rank, uint32_t a,
-                                                uint32_t b, uint32_t epoch, uint32_t* err, uint32_t site_a,
-                                                uint32_t site_b, uint32_t* sum_a, uint32_t* sum_b, bool drop = false)
+template <int kThreads, int kN>
+__device__ __forceinline__ void cta_prefix_sums(const CtaCount (&c)[kN], uint32_t rank, uint32_t epoch, uint32_t* err,
+                                                bool drop = false)
 {
     if (threadIdx.x == 0 && !drop) {
-        lb_store(status_a + rank, lb_pack(epoch, kFlagAggregate, a));
-        lb_store(status_b + rank, lb_pack(epoch, kFlagAggregate, b));
+#pragma unroll
+        for (int i = 0; i < kN; ++i) lb_store(c[i].status + rank, lb_pack(epoch, kFlagAggregate, c[i].count));
     }
-    uint32_t sa = 0, sb = 0;
+    uint32_t sum[kN] = {};
     for (uint32_t p = threadIdx.x; p < rank; p += kThreads) {
-        uint64_t va, vb;
+        uint64_t v[kN];
         uint32_t spins = 0;
         for (;;) {
-            va = lb_load(status_a + p);
-            vb = lb_load(status_b + p);
-            const bool ra = (uint32_t)(va >> 34) == epoch, rb = (uint32_t)(vb >> 34) == epoch;
-            if (ra && rb) break;
+            uint32_t late = 0;  // the site of a count that is not there yet
+#pragma unroll
+            for (int i = 0; i < kN; ++i) v[i] = lb_load(c[i].status + p);
+#pragma unroll
+            for (int i = kN - 1; i >= 0; --i) late = (uint32_t)(v[i] >> 34) == epoch ? late : c[i].site;
+            if (!late) break;
             if (++spins > kSpinLimit) {
-                atomicCAS(err, 0u, ra ? site_b : site_a);
+                atomicCAS(err, 0u, late);
                 break;
             }
             if (spins > 8) __nanosleep(100);
         }
-        sa += (uint32_t)va;
-        sb += (uint32_t)vb;
+#pragma unroll
+        for (int i = 0; i < kN; ++i) sum[i] += (uint32_t)v[i];
     }
-    sa = __reduce_add_sync(0xffffffffu, sa);
-    sb = __reduce_add_sync(0xffffffffu, sb);
-    if ((threadIdx.x & 31u) == 0u) {
-        if (sa) atomicAdd(sum_a, sa);
-        if (sb) atomicAdd(sum_b, sb);
+#pragma unroll
+    for (int i = 0; i < kN; ++i) {
+        sum[i] = __reduce_add_sync(0xffffffffu, sum[i]);
+        if ((threadIdx.x & 31u) == 0u && sum[i]) atomicAdd(c[i].sum, sum[i]);
     }
 }
 

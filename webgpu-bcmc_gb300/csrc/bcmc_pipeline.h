@@ -14,8 +14,16 @@ struct FlagArgs {
     uint32_t total;  // blocks
     uint32_t wpw;    // words a warp takes at a time
     uint4* near;     // per word: A, B and A & B ORed with the x neighbours', and A
-    uint32_t* hi;    // per word: B
+    uint4* up;       // per word: A and B ORed with the next block's along x, and B
 };
+
+// Of which blocks the range, and the ranges of the neighbours on the + sides, hold
+// all voxels: those below these coordinates and this id.
+struct SoundRanges {
+    uint32_t x, y, z, id;
+};
+// dims in voxels; `ranged`: how many blocks have their range (zfp_ranged_blocks)
+SoundRanges sound_ranges(const uint32_t dims[3], const BlockGrid& grid, uint64_t ranged);
 
 struct ActiveArgs {
     BlockGrid grid;
@@ -29,8 +37,15 @@ struct ActiveArgs {
     uint64_t* status_n;
     // MC path: k_query_flags' words, and room for each word's active and needed bits
     const uint4* near = nullptr;
-    const uint32_t* hi = nullptr;
+    const uint4* up = nullptr;
     uint2* words = nullptr;
+    // MC path: the active blocks that can have vertices, their ids and their places
+    // among the active ids, and the blocks for which the ranges can tell
+    uint32_t* live_ids = nullptr;
+    uint32_t* live_at = nullptr;
+    uint64_t* status_l = nullptr;
+    uint32_t* live_words = nullptr;
+    SoundRanges sound{};
 };
 
 struct SlotArgs {
@@ -86,13 +101,15 @@ struct DecodeArgs {
 struct McArgs {
     const uint32_t* active;
     const uint32_t* active_ids;
+    const uint32_t* live_ids;  // the blocks to look at (ActiveArgs)
+    const uint32_t* live_at;
     const int32_t* item_slots;
     const float* cache;
     uint3 nb;
     BlockGrid grid;
     uint32_t* with_verts;
     uint32_t* vert_offsets;
-    uint32_t* block_counts;  // vertices of each active block (count pass -> list entries)
+    uint32_t* block_counts;  // vertices of each block looked at (count pass -> list entries)
     uint2* verts;
     uint64_t* status_v;
     uint64_t* status_b;

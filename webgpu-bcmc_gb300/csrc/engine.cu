@@ -232,7 +232,7 @@ __device__ __forceinline__ uint32_t tile_active(const EngVolDev& V, uint32_t b0,
     const int64_t nx = nb.x, nxy = (int64_t)nb.x * nb.y;
     const float2* ranges = V.ranges;
     const uint32_t mine = b0 + 32u * lane;
-    const WordRows in_volume = word_rows(min(mine, total - 1u), V.grid);
+    const WordRows in_volume = word_rows(min(mine, total - 1u), V.grid, SoundRanges{});
     const int rows = nb.x <= kRunRow ? 3 : 1;  // rows in a run
     uint32_t any_a = 0, any_b = 0, any_c = 0, self_a = 0, self_b = 0;
     for (int dz = -1; dz < 2; ++dz)
@@ -621,8 +621,8 @@ __global__ void __launch_bounds__(16 * kTileBlocks, kBmcThreadsPerSm / (16 * kTi
     }
     __syncthreads();
     if (rank < worked)
-        cta_prefix_sums<kThreads>(a.status_v, a.status_b, rank, s_cta_v, s_cta_b, epoch, &st->error, 61u, 64u, &s_pv,
-                                  &s_pb);
+        cta_prefix_sums<kThreads>({{a.status_v, s_cta_v, 61u, &s_pv}, {a.status_b, s_cta_b, 64u, &s_pb}}, rank, epoch,
+                                  &st->error);
     async_wait<0>();
     __syncthreads();
     // 32-bit prefix: a sequence over 2^32 vertices wraps here; k_bfinish

@@ -57,7 +57,7 @@ __device__ __forceinline__ void query_begin(QueryState* q, float iso, bool mc_on
             q->tiles_active = q->tiles_slots = q->tiles_sort_hist = 0;
             for (int i = 0; i < 4; ++i) q->tiles_sort[i] = 0;
             q->sort_arrived = 0;
-            q->num_active = q->num_new = q->num_avail = 0;
+            q->num_active = q->num_live = q->num_new = q->num_avail = 0;
             q->grow_needed = 0;
             // the sort plan of zero keys (k_slots replaces it when it sorts)
             for (int i = 0; i < 4; ++i) q->sort_run[i] = q->sort_src[i] = 0;
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kFlagThreads) k_query_flags(QueryState* q, flo
         if (lane < wpw && w0 + lane < nwords) {
             a.near[w0 + lane] = make_uint4(ends.spread(A, pa, na), ends.spread(B, pb, nb),
                                            ends.spread(A & B, pa & pb, na & nb), A);
-            a.hi[w0 + lane] = B;
+            a.up[w0 + lane] = make_uint4(ends.up(A, na), ends.up(B, nb), B, 0u);
         }
         if (w0 + step < nwords) {
             load_batch(w0 + step, 0, r);
@@ -232,8 +232,16 @@ __device__ __forceinline__ void active_finish(QueryState* q, uint32_t A, uint32_
 // any over the 3x3x3 neighbourhood.  The words hold the ORs along x, so a lane
 // ORs the nine (y, z) neighbour rows of its word, each two words and a funnel
 // shift, with masks for the blocks that have no such row.
+// A block is active for neighbours on all sides, but its cells reach into those
+// on the + sides only: where the isovalue lies outside the ranges of the block and
+// of these seven (up_a, up_b), all its voxels and ghost voxels are on one side of
+// it, and it cannot have vertices.  k_mc looks at the others, the live ones, alone:
+// an and of two words here saves it 125 voxel loads and their tests a block (1024 x
+// 1024 x 1080, a quarter of whose active blocks have vertices: MC 586 -> 529 us
+// for 10 us more here; 512^3 789 -> 771 us for 2).  Blocks whose ranges do not hold
+// all their voxels (SoundRanges) are live when they are active.
 // A CTA owns one contiguous range of words: it tests them, keeping the results
-// in shared memory, publishes its two totals, adds up those of the CTAs before
+// in shared memory, publishes its totals, adds up those of the CTAs before
 // it in one round trip (cooperative launch: all are resident), and writes its
 // ids.  The last CTA with words decides the cache growth.
 constexpr int kWordThreads = 256;
@@ -244,9 +252,10 @@ __global__ void __launch_bounds__(kWordThreads, kWordPerSm) k_active_words(Query
                                                                           uint32_t range)
 {
     __shared__ uint2 s_words[kWordRange];
+    __shared__ uint32_t s_live[kWordRange];
     __shared__ uint32_t s_warp[kWordThreads / 32 + 1];
-    __shared__ uint32_t s_at[kWordThreads];
-    __shared__ uint32_t s_sum_a, s_sum_n, s_pa, s_pn;
+    __shared__ uint2 s_at[kWordThreads];
+    __shared__ uint32_t s_sum_a, s_sum_n, s_sum_l, s_pa, s_pn, s_pl;
     constexpr uint32_t kWarps = kWordThreads / 32;
     const uint32_t total = a.total, nwords = div_up(total, 32u), rank = blockIdx.x;
     const uint32_t first = rank * range, end = min(nwords, first + range);
@@ -257,15 +266,16 @@ __global__ void __launch_bounds__(kWordThreads, kWordPerSm) k_active_words(Query
     const int64_t nxy = (int64_t)nb.x * nb.y;
     const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, below = (1u << lane) - 1u;
     uint2* words = range <= kWordRange ? s_words : a.words + first;  // active and needed bits
-    if (t == 0) s_sum_a = s_sum_n = s_pa = s_pn = 0;
+    uint32_t* live_words = range <= kWordRange ? s_live : a.live_words + first;
+    if (t == 0) s_sum_a = s_sum_n = s_sum_l = s_pa = s_pn = s_pl = 0;
     __syncthreads();
-    uint32_t na = 0, nn = 0;  // the lane's words' counts
+    uint32_t na = 0, nn = 0, nl = 0;  // the lane's words' counts
     for (uint32_t w0 = first + warp * wpw; w0 < end; w0 += kWarps * wpw) {
         const uint32_t w = w0 + lane, b0 = 32u * w;
-        uint32_t act = 0;
+        uint32_t act = 0, live = 0;
         if (lane < wpw && w < end) {
-            const WordRows in_volume = word_rows(b0, a.grid);
-            uint32_t any_a = 0, any_b = 0, any_c = 0;
+            const WordRows in_volume = word_rows(b0, a.grid, a.sound);
+            uint32_t any_a = 0, any_b = 0, any_c = 0, up_a = 0, up_b = 0, self_a = 0, self_b = 0;
 #pragma unroll
             for (int dz = -1; dz < 2; ++dz)
 #pragma unroll
@@ -275,14 +285,25 @@ __global__ void __launch_bounds__(kWordThreads, kWordPerSm) k_active_words(Query
                     const int64_t s = (int64_t)b0 + dz * nxy + dy * nx;
                     const int64_t k = s >> 5;
                     const uint32_t sh = (uint32_t)s & 31u;
-                    const uint4 lo = __ldg(a.near + min(max(k, (int64_t)0), (int64_t)nwords - 1)),
-                                hi = __ldg(a.near + min(max(k + 1, (int64_t)0), (int64_t)nwords - 1));
+                    const int64_t k0 = min(max(k, (int64_t)0), (int64_t)nwords - 1),
+                                  k1 = min(max(k + 1, (int64_t)0), (int64_t)nwords - 1);
+                    const uint4 lo = __ldg(a.near + k0), hi = __ldg(a.near + k1);
                     any_a |= __funnelshift_r(lo.x, hi.x, sh) & m;
                     any_b |= __funnelshift_r(lo.y, hi.y, sh) & m;
                     any_c |= __funnelshift_r(lo.z, hi.z, sh) & m;
+                    if (dz >= 0 && dy >= 0) {
+                        const uint4 l = __ldg(a.up + k0), h = __ldg(a.up + k1);
+                        up_a |= __funnelshift_r(l.x, h.x, sh) & m;
+                        up_b |= __funnelshift_r(l.y, h.y, sh) & m;
+                        if (dz == 0 && dy == 0) self_b = l.z;
+                    }
+                    if (dz == 0 && dy == 0) self_a = lo.w;
                 }
-            act = (a.near[w].w & any_b) | (a.hi[w] & any_a) | any_c;
+            act = (self_a & any_b) | (self_b & any_a) | any_c;
             if (total - b0 < 32u) act &= (1u << (total - b0)) - 1u;
+            uint32_t sound = b0 < a.sound.id ? in_volume.sound : 0u;
+            if (a.sound.id - b0 < 32u) sound &= (1u << (a.sound.id - b0)) - 1u;
+            live = act & ((up_a & up_b) | ~sound);
         }
         // the flags out, and which active blocks no slot holds: four words at a
         // time, four blocks to a lane
@@ -318,43 +339,65 @@ __global__ void __launch_bounds__(kWordThreads, kWordPerSm) k_active_words(Query
         }
         if (lane < n) {
             words[w - first] = make_uint2(act, need);
+            live_words[w - first] = live;
+            nl += __popc(live);
             na += __popc(act);
             nn += __popc(need);
         }
     }
     na = __reduce_add_sync(0xffffffffu, na);
     nn = __reduce_add_sync(0xffffffffu, nn);
+    nl = __reduce_add_sync(0xffffffffu, nl);
     if (lane == 0 && na) {
         atomicAdd(&s_sum_a, na);
         if (nn) atomicAdd(&s_sum_n, nn);
+        if (nl) atomicAdd(&s_sum_l, nl);
     }
     __syncthreads();
-    cta_prefix_sums<kWordThreads>(a.status_a, a.status_n, rank, s_sum_a, s_sum_n, epoch, &q->error, 30u, 31u, &s_pa,
-                                  &s_pn, lb_dropped(q, rank));
+    if (a.active_ids)
+        cta_prefix_sums<kWordThreads>({{a.status_a, s_sum_a, 30u, &s_pa}, {a.status_n, s_sum_n, 31u, &s_pn}, {a.status_l, s_sum_l, 33u, &s_pl}},
+                                      rank, epoch, &q->error, lb_dropped(q, rank));
+    else
+        cta_prefix_sums<kWordThreads>({{a.status_a, s_sum_a, 30u, &s_pa}, {a.status_n, s_sum_n, 31u, &s_pn}}, rank, epoch,
+                                      &q->error, lb_dropped(q, rank));
     __syncthreads();
-    uint32_t pa = s_pa, pn = s_pn;
-    if (end == nwords && t == 0) active_finish(q, pa + s_sum_a, pn + s_sum_n, total);
+    uint32_t pa = s_pa, pn = s_pn, pl = s_pl;
+    if (end == nwords && t == 0) {
+        active_finish(q, pa + s_sum_a, pn + s_sum_n, total);
+        q->num_live = pl + s_sum_l;
+    }
     if (!a.active_ids) return;
     for (uint32_t c0 = 0; c0 < end - first; c0 += kWordThreads) {
         const uint32_t i = c0 + t;
         const uint2 mine = i < end - first ? words[i] : make_uint2(0u, 0u);
-        uint32_t tot;
-        const uint32_t ex = cta_exclusive_scan<kWordThreads>((uint32_t)__popc(mine.x) | ((uint32_t)__popc(mine.y) << 16),
+        const uint32_t mine_live = i < end - first ? live_words[i] : 0u;
+        uint32_t tot, tot_n = 0, ex_n = 0;
+        const uint32_t ex = cta_exclusive_scan<kWordThreads>((uint32_t)__popc(mine.x) | ((uint32_t)__popc(mine_live) << 16),
                                                              s_warp, &tot);
-        s_at[t] = ex;
+        if (s_sum_n) ex_n = cta_exclusive_scan<kWordThreads>((uint32_t)__popc(mine.y), s_warp, &tot_n);
+        s_at[t] = make_uint2(ex, ex_n);
         __syncthreads();
         // a word at a time, so that the ids go out together
         const uint32_t n = min((uint32_t)kWordThreads, end - first - c0);
         for (uint32_t k = warp; k < n; k += kWarps) {
             const uint2 wd = words[c0 + k];
             if (!wd.x) continue;
-            const uint32_t at = s_at[k], b = 32u * (first + c0 + k) + lane;
-            if (wd.x >> lane & 1u) a.active_ids[pa + (at & 0xffffu) + __popc(wd.x & below)] = b;
-            if (wd.y >> lane & 1u) a.new_ids[pn + (at >> 16) + __popc(wd.y & below)] = b;
+            const uint32_t wl = live_words[c0 + k];
+            const uint2 at = s_at[k];
+            const uint32_t b = 32u * (first + c0 + k) + lane;
+            const uint32_t place = pa + (at.x & 0xffffu) + __popc(wd.x & below);
+            if (wd.x >> lane & 1u) a.active_ids[place] = b;
+            if (wd.y >> lane & 1u) a.new_ids[pn + at.y + __popc(wd.y & below)] = b;
+            if (wl >> lane & 1u) {
+                const uint32_t l = pl + (at.x >> 16) + __popc(wl & below);
+                a.live_ids[l] = b;
+                a.live_at[l] = place;
+            }
         }
         __syncthreads();
         pa += tot & 0xffffu;
-        pn += tot >> 16;
+        pl += tot >> 16;
+        pn += tot_n;
     }
 }
 
@@ -696,7 +739,7 @@ constexpr uint32_t kMcSharedRange = 1024;
 
 // Marching cubes over the active blocks, one cooperative launch (every CTA
 // resident), all of its block work done by single warps (mc_common.cuh):
-//   count pass: the blocks in batches of four to a warp: look the neighbours up,
+//   count pass: the live blocks in batches of four to a warp: look the neighbours up,
 //     load the grids and count the triangles of the cells from the corner masks;
 //     block totals are kept.  Each CTA counts its own range of the blocks, or,
 //     when the ranges are long, its share of batches from the whole grid, with a
@@ -725,7 +768,7 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     __shared__ uint32_t s_cnt[kMcOwnRange];  // few blocks: the counts of the CTA's
     __shared__ uint32_t s_pv, s_pb, s_cta_v, s_cta_b;
 
-    const uint32_t A = q->num_active;
+    const uint32_t A = q->num_live;
     if (A == 0 || q->grow_needed) return;
     const uint32_t epoch = q->epoch;
     const float iso = q->isovalue;
@@ -753,13 +796,13 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     };
 
     // ---- count pass: ids two rounds ahead, lookups one round ahead
-    uint32_t own_n = 0, own_id = 0, own_has = 0;  // few blocks: the warp's batch
+    uint32_t own_n = 0, own_id = 0, own_has = 0, own_at = 0;  // few blocks: the warp's batch
     const uint32_t batch = own ? range / kMcWarps : kMcBlocks;
     {
         const uint32_t stop = together ? A : end, step = (together ? G : 1u) * kMcWarps * batch;
         uint32_t base = together ? (rank * kMcWarps + warp) * batch : start + warp * batch;
         const auto mine = [&](uint32_t at) { return jb < batch && at + jb < stop; };
-        const auto load_id = [&](uint32_t at) { return mine(at) ? __ldg(a.active_ids + at + jb) : 0u; };
+        const auto load_id = [&](uint32_t at) { return mine(at) ? __ldg(a.live_ids + at + jb) : 0u; };
         McLook next = look(mine(base), load_id(base));
         uint32_t id2 = load_id(base + step);
         uint32_t wv = 0, wb = 0;
@@ -777,6 +820,7 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
                 own_n = n;
                 own_id = id;
                 own_has = has;
+                if (lane < n) own_at = __ldg(a.live_at + base + lane);
 #pragma unroll
                 for (uint32_t j = 0; j < kMcBlocks; ++j)
                     if (j < n) {
@@ -821,8 +865,8 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     }
     __syncthreads();
     if (rank < worked)
-        cta_prefix_sums<kMcThreads>(a.status_v, a.status_b, rank, s_cta_v, s_cta_b, epoch, &q->error, 40u, 41u, &s_pv,
-                                    &s_pb);
+        cta_prefix_sums<kMcThreads>({{a.status_v, s_cta_v, 40u, &s_pv}, {a.status_b, s_cta_b, 41u, &s_pb}}, rank, epoch,
+                                    &q->error);
     async_wait<0>();
     __syncthreads();
     uint32_t pv = s_pv, pb = s_pb;
@@ -847,7 +891,7 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
         const uint32_t some = __ballot_sync(kFull, c != 0u);
         if (c) {
             const uint32_t r = pb + __popc(some & ((1u << lane) - 1u));
-            a.with_verts[r] = start + first + lane;
+            a.with_verts[r] = own_at;
             a.vert_offsets[r] = off;
         }
         if (!some) return;
@@ -860,14 +904,14 @@ __global__ void __launch_bounds__(kMcThreads, kMcPerSm) k_mc(QueryState* q, McAr
     if (fits)
         for (uint32_t b0 = start; b0 < end; b0 += kMcThreads) {
             const uint32_t i = b0 + t;
-            const uint32_t c = i < end ? __ldcg(a.block_counts + i) : 0u;
+            const uint32_t c = i < end ? __ldcg(a.block_counts + i) : 0u, at = i < end ? __ldg(a.live_at + i) : 0u;
             // <= 512 blocks x 64 cells x 15 vertices < 2^20, and the blocks above them
             static_assert(kMcThreads * 64 * 15 < 1 << 20 && kMcThreads < 1 << 12, "fields of the scan");
             uint32_t tot;
             const uint32_t ex = cta_exclusive_scan<kMcThreads>(c | (c ? 1u << 20 : 0u), s_warp, &tot);
             if (c) {
                 const uint32_t r = pb + (ex >> 20);
-                a.with_verts[r] = i;
+                a.with_verts[r] = at;
                 a.vert_offsets[r] = pv + (ex & 0xfffffu);
             }
             pv += tot & 0xfffffu;
@@ -929,7 +973,17 @@ void query_begin_launch(QueryState* q, float iso, int mc_only, uint32_t capacity
     BCMC_CUDA(cudaGetLastError());
 }
 
-size_t flag_bytes(uint64_t total) { return (size_t)((total + 31u) / 32u) * (sizeof(uint4) + sizeof(uint2) + 4u) + 16u; }
+size_t flag_bytes(uint64_t total) { return (size_t)((total + 31u) / 32u) * (2u * sizeof(uint4) + sizeof(uint2) + 4u); }
+
+SoundRanges sound_ranges(const uint32_t dims[3], const BlockGrid& grid, uint64_t ranged)
+{
+    // the last block on an axis that is not a multiple of 4 has voxels past the
+    // volume, which its range leaves out and its grid does not
+    const auto axis = [](uint32_t n, uint32_t blocks) { return n % 4u == 0u ? blocks : blocks > 2u ? blocks - 2u : 0u; };
+    const uint64_t total = (uint64_t)grid.nb.x * grid.nb.y * grid.nb.z, reach = (uint64_t)grid.nb.x * grid.nb.y + grid.nb.x + 1u;
+    return {axis(dims[0], grid.nb.x), axis(dims[1], grid.nb.y), axis(dims[2], grid.nb.z),
+            (uint32_t)(ranged >= total ? total : ranged > reach ? ranged - reach : 0u)};
+}
 
 // CTAs of k_active_words resident per SM: the bound of its cooperative grid
 static uint32_t word_per_sm()
@@ -958,7 +1012,7 @@ void query_flags_launch(bcmc_ctx* ctx, QueryState* q, float iso, uint32_t capaci
     const uint32_t nwords = div_up(total, 32u), wpw = words_per_warp(ctx, nwords, 32u);
     uint4* near = static_cast<uint4*>(words);
     const FlagArgs f{reinterpret_cast<const float2*>(ranges), grid, total, wpw, near,
-                     reinterpret_cast<uint32_t*>(near + nwords)};
+                     near + nwords};
     k_query_flags<<<pgrid(ctx, div_up(nwords, wpw * (kFlagThreads / 32)), 8), kFlagThreads, 0, s>>>(
         q, iso, capacity, vert_capacity, in, f);
     count_launches(1);
@@ -969,8 +1023,9 @@ void active_words_launch(bcmc_ctx* ctx, QueryState* q, ActiveArgs a, void* words
 {
     const uint32_t nwords = div_up(a.total, 32u), wpw = words_per_warp(ctx, nwords, kWordThreads / 32);
     a.near = static_cast<const uint4*>(words);
-    a.hi = reinterpret_cast<const uint32_t*>(a.near + nwords);
-    a.words = reinterpret_cast<uint2*>(static_cast<uint4*>(words) + nwords + div_up(nwords, 4u));
+    a.up = a.near + nwords;
+    a.words = reinterpret_cast<uint2*>(static_cast<uint4*>(words) + 2u * (size_t)nwords);
+    a.live_words = reinterpret_cast<uint32_t*>(a.words + nwords);
     // a CTA an SM first: the CTAs wait for each other's counts (256^3: 128 of them
     // 1.3 us faster than 256); then a range of whole rounds per resident CTA
     const uint32_t round = wpw * (kWordThreads / 32);

@@ -198,18 +198,24 @@ static int grid_all(uint64_t n, int threads)
     return (int)(want == 0 ? 1 : (want < 0x7fffffffull ? want : 0x7fffffffull));
 }
 
+// zfp_compute_block_range.comp:22 counts (padded x * padded y) / 64 * padded z
+// blocks in u32, which truncates when nb.x * nb.y is not a multiple of 4;
+// the blocks past that count keep the zero of the new range buffer
+// (compressed_marching_cubes.js:526-529).  BCMC_FLAG_FULL_RANGES ranges all.
+uint64_t zfp_ranged_blocks(const bcmc_ctx* ctx, const uint32_t dims[3])
+{
+    const uint32_t nx = div_up(dims[0], 4), ny = div_up(dims[1], 4), nz = div_up(dims[2], 4);
+    const uint64_t n = (uint64_t)nx * ny * nz;
+    const uint32_t ref_count = (4u * nx * 4u * ny) / 64u * (4u * nz);
+    return (ctx->opts.flags & BCMC_FLAG_FULL_RANGES) ? n : (ref_count < n ? ref_count : n);
+}
+
 void zfp_ranges_launch(bcmc_ctx* ctx, const uint64_t* words, const uint32_t dims[3], uint32_t max_bits,
                        float* ranges, cudaStream_t s)
 {
     const uint3 d = make_uint3(dims[0], dims[1], dims[2]);
     const uint3 nb = make_uint3(div_up(dims[0], 4), div_up(dims[1], 4), div_up(dims[2], 4));
-    const uint64_t n = (uint64_t)nb.x * nb.y * nb.z;
-    // zfp_compute_block_range.comp:22 counts (padded x * padded y) / 64 * padded z
-    // blocks in u32, which truncates when nb.x * nb.y is not a multiple of 4;
-    // the blocks past that count keep the zero of the new range buffer
-    // (compressed_marching_cubes.js:526-529).  BCMC_FLAG_FULL_RANGES ranges all.
-    const uint32_t ref_count = (4u * nb.x * 4u * nb.y) / 64u * (4u * nb.z);
-    const uint64_t ranged = (ctx->opts.flags & BCMC_FLAG_FULL_RANGES) ? n : (ref_count < n ? ref_count : n);
+    const uint64_t n = (uint64_t)nb.x * nb.y * nb.z, ranged = zfp_ranged_blocks(ctx, dims);
     const uint32_t rate = max_bits / 64u;
     const size_t smem = zfp_stage_smem(kDecThreads, rate);
     allow_smem(k_block_ranges, smem);
