@@ -8,8 +8,9 @@
 //              A tile whose extended value range (its blocks and their 26
 //              neighbours, from volume load) excludes the isovalue is skipped
 //              whole.  Active bits go to a per-query bitmap, counts to the tiles
-//   k_bentries active (query, block) entries in query-major, block-ascending
-//              order from the tiles' counts; blocks no slot holds are claimed
+//   k_bentries (query, block) entries of the active blocks that can have vertices
+//              in query-major, block-ascending order from the tiles' counts;
+//              active blocks no slot holds are claimed
 //              (one claim per block across the batch) and given a slot from
 //              the pool's free list
 //   k_bdecode  ZFP decode of every claimed block into its slot
@@ -57,6 +58,7 @@ struct EngVolDev {
     BlockGrid grid;
     uint32_t total;
     uint32_t max_bits;
+    SoundRanges sound;
 };
 
 struct EngQuery {
@@ -104,7 +106,8 @@ struct BatchArgs {
     uint32_t* owner_vol;
     uint32_t* owner_block;
     float* cache;
-    uint32_t* bitmap;
+    uint32_t* bitmap;  // a bit per block of every query: active
+    uint32_t* live;    // the same: and can have vertices (k_active_words, pipeline.cu)
     uint32_t* ent_id;
     uint32_t* ent_q;
     uint32_t* block_counts;
@@ -116,7 +119,7 @@ struct BatchArgs {
     uint32_t* dec_block;
     uint32_t* dec_slot;
     uint2* verts;
-    uint32_t* tile_counts;  // active blocks of each tile, then of each group of tiles (k_bactive)
+    uint32_t* tile_counts;  // live and (from bit 16) active blocks of each tile, then live of each group of tiles
     uint64_t* status_v;  // counts of the MC CTAs (vertices)
     uint64_t* status_b;  // counts of the MC CTAs (entries with vertices)
 };
@@ -181,7 +184,7 @@ __global__ void k_bbegin(EngState* st, uint32_t* q_nverts, uint32_t* q_nactive, 
 
 // ---------------------------------------------------------------------------
 // k_bactive: the active test of every query over its volume's blocks, a bit per
-// block, and the counts of the tiles and of groups of eight tiles.
+// block, which of those can have vertices, another, and the counts of the tiles and of groups of eight tiles.
 //
 // The tests of a batch read each block's range over and over: what bounds the
 // kernel is the instructions and loads per block.  A warp takes a tile of 1024
@@ -222,19 +225,20 @@ __device__ __forceinline__ uint32_t* group_counts(const BatchArgs& a, uint32_t n
 struct RunWords {
     uint2 bits[kRunWords];  // iso >= lo, iso <= hi of the run's blocks
     uint32_t near[3][kRunWords + 1];  // those and their AND, of a block or a neighbour along x
+    uint2 up[kRunWords + 1];          // those, of a block or the next along x
 };
 
-// Active bits of the 32 blocks of the lane's word of the tile that starts at b0.
-__device__ __forceinline__ uint32_t tile_active(const EngVolDev& V, uint32_t b0, float iso, RunWords& run)
+// Active and live bits of the 32 blocks of the lane's word of the tile that starts at b0.
+__device__ __forceinline__ uint2 tile_active(const EngVolDev& V, uint32_t b0, float iso, RunWords& run)
 {
     const uint32_t lane = threadIdx.x & 31u, total = V.total, nwords = div_up(total, 32u);
     const uint3 nb = V.grid.nb;
     const int64_t nx = nb.x, nxy = (int64_t)nb.x * nb.y;
     const float2* ranges = V.ranges;
     const uint32_t mine = b0 + 32u * lane;
-    const WordRows in_volume = word_rows(min(mine, total - 1u), V.grid, SoundRanges{});
+    const WordRows in_volume = word_rows(min(mine, total - 1u), V.grid, V.sound);
     const int rows = nb.x <= kRunRow ? 3 : 1;  // rows in a run
-    uint32_t any_a = 0, any_b = 0, any_c = 0, self_a = 0, self_b = 0;
+    uint32_t any_a = 0, any_b = 0, any_c = 0, self_a = 0, self_b = 0, up_a = 0, up_b = 0;
     for (int dz = -1; dz < 2; ++dz)
         for (int dy0 = -1; dy0 < 2; dy0 += rows) {
             // its words: the run's blocks and one more at either end
@@ -269,6 +273,7 @@ __device__ __forceinline__ uint32_t tile_active(const EngVolDev& V, uint32_t b0,
                 run.near[0][i] = ends.spread(v.x, p.x, q.x);
                 run.near[1][i] = ends.spread(v.y, p.y, q.y);
                 run.near[2][i] = ends.spread(v.x & v.y, p.x & p.y, q.x & q.y);
+                run.up[i] = make_uint2(ends.up(v.x, q.x), ends.up(v.y, q.y));
             }
             __syncwarp();
             for (int dy = dy0; dy < dy0 + rows; ++dy) {
@@ -278,6 +283,11 @@ __device__ __forceinline__ uint32_t tile_active(const EngVolDev& V, uint32_t b0,
                 any_a |= __funnelshift_r(run.near[0][k], run.near[0][k + 1u], sh) & m;
                 any_b |= __funnelshift_r(run.near[1][k], run.near[1][k + 1u], sh) & m;
                 any_c |= __funnelshift_r(run.near[2][k], run.near[2][k + 1u], sh) & m;
+                if (dz >= 0 && dy >= 0) {
+                    const uint2 l = run.up[k], h = run.up[k + 1u];
+                    up_a |= __funnelshift_r(l.x, h.x, sh) & m;
+                    up_b |= __funnelshift_r(l.y, h.y, sh) & m;
+                }
                 if (dz == 0 && dy == 0) {
                     self_a = run.bits[k].x;
                     self_b = run.bits[k].y;
@@ -285,11 +295,14 @@ __device__ __forceinline__ uint32_t tile_active(const EngVolDev& V, uint32_t b0,
             }
             __syncwarp();
         }
-    const uint32_t act = (self_a & any_b) | (self_b & any_a) | any_c;
-    return mine >= total ? 0u : total - mine < 32u ? act & ((1u << (total - mine)) - 1u) : act;
+    uint32_t act = mine >= total ? 0u : (self_a & any_b) | (self_b & any_a) | any_c;
+    if (total - mine < 32u) act &= (1u << (total - mine)) - 1u;
+    uint32_t sound = mine < V.sound.id ? in_volume.sound : 0u;
+    if (V.sound.id - mine < 32u) sound &= (1u << (V.sound.id - mine)) - 1u;
+    return make_uint2(act, act & ((up_a & up_b) | ~sound));
 }
 
-__global__ void __launch_bounds__(kEngThreads, 4) k_bactive(BatchArgs a)
+__global__ void __launch_bounds__(kEngThreads, 3) k_bactive(BatchArgs a)
 {
     __shared__ RunWords s_run[kGroup];
     __shared__ uint32_t s_count[2][kGroup];
@@ -304,12 +317,13 @@ __global__ void __launch_bounds__(kEngThreads, 4) k_bactive(BatchArgs a)
             const EngVolDev& V = a.vols[Q.vol];
             const uint32_t lt = tile - Q.tile0;
             const float2 ext = __ldg(V.tile_ext + lt);
-            const uint32_t act = Q.iso >= ext.x && Q.iso <= ext.y ? tile_active(V, lt * kEngTile, Q.iso, s_run[warp]) : 0u;
-            a.bitmap[Q.bit0 + lt * (kEngTile / 32) + lane] = act;
-            count = __reduce_add_sync(0xffffffffu, __popc(act));
+            const uint2 w = Q.iso >= ext.x && Q.iso <= ext.y ? tile_active(V, lt * kEngTile, Q.iso, s_run[warp]) : make_uint2(0u, 0u);
+            a.bitmap[Q.bit0 + lt * (kEngTile / 32) + lane] = w.x;
+            a.live[Q.bit0 + lt * (kEngTile / 32) + lane] = w.y;
+            count = __reduce_add_sync(0xffffffffu, __popc(w.y) + ((uint32_t)__popc(w.x) << 16));
             if (lane == 0) a.tile_counts[tile] = count;
         }
-        if (lane == 0) s_count[turn][warp] = count;
+        if (lane == 0) s_count[turn][warp] = count & 0xffffu;
         __syncthreads();
         if (threadIdx.x == 0) {
             uint32_t sum = 0;
@@ -320,8 +334,8 @@ __global__ void __launch_bounds__(kEngThreads, 4) k_bactive(BatchArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// k_bentries: the active (block, query) entries in the order of the tile
-// stream, and the claims of the blocks that no slot holds
+// k_bentries: the live (block, query) entries in the order of the tile stream,
+// and the claims of the active blocks that no slot holds
 //
 // A CTA owns a contiguous range of groups of tiles.  Every count is known, so
 // it adds up those of the groups before its range and waits for nobody; a warp
@@ -404,9 +418,9 @@ __global__ void __launch_bounds__(kEngThreads) k_bentries(BatchArgs a)
     uint32_t base = s_sum;
     for (uint32_t g = first; g < end; ++g) {
         const uint32_t t0 = g * kGroup, tile = t0 + warp;
-        const uint32_t n = lane < kGroup && t0 + lane < ntiles ? __ldg(a.tile_counts + t0 + lane) : 0u;
+        const uint32_t n2 = lane < kGroup && t0 + lane < ntiles ? __ldg(a.tile_counts + t0 + lane) : 0u, n = n2 & 0xffffu;
         const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? n : 0u);
-        const uint32_t count = __shfl_sync(0xffffffffu, n, warp);
+        const uint32_t count = __shfl_sync(0xffffffffu, n2, warp) >> 16;  // active
         uint32_t at = base + before;
         base += __reduce_add_sync(0xffffffffu, n);
         if (!count) continue;
@@ -415,6 +429,7 @@ __global__ void __launch_bounds__(kEngThreads) k_bentries(BatchArgs a)
         int32_t* item_slots = a.vols[Q.vol].item_slots;
         const uint32_t lt = tile - Q.tile0;
         const uint32_t word = __ldg(a.bitmap + Q.bit0 + lt * (kEngTile / 32) + lane);
+        const uint32_t live = __ldg(a.live + Q.bit0 + lt * (kEngTile / 32) + lane);
         if (lane == 0) atomicAdd(a.q_nactive + qi, count);
         // kN words at a time, their blocks' slots read together
         constexpr int kN = 4;
@@ -429,16 +444,17 @@ __global__ void __launch_bounds__(kEngThreads) k_bentries(BatchArgs a)
             }
 #pragma unroll
             for (int j = 0; j < kN; ++j) {
+                const uint32_t l = __shfl_sync(0xffffffffu, live, i + j);
                 if (w[j] >> lane & 1u) {
-                    const uint32_t pos = at + __popc(w[j] & below);
-                    if (pos < cap) {
+                    const uint32_t pos = at + __popc(l & below);
+                    if ((l >> lane & 1u) && pos < cap) {
                         a.ent_id[pos] = b[j];
                         a.ent_q[pos] = qi;
                     }
                     if (s[j] >= 0) a.last_use[s[j]] = use_epoch;
                     open |= (s[j] == -1 ? 1u : 0u) << j;
                 }
-                at += __popc(w[j]);
+                at += __popc(l);
             }
             if (__any_sync(0xffffffffu, open)) claim_blocks<kN>(a, Q.vol, item_slots, b, open, use_epoch);
         }
@@ -790,7 +806,7 @@ struct EngLane {
     EngState* h_st = nullptr;  // pinned
     uint32_t *q_nactive = nullptr, *q_nverts = nullptr;
     uint32_t* bitmap = nullptr;
-    uint64_t bitmap_words = 0;
+    uint64_t bitmap_words = 0;  // of the active bits, and as many of the live ones after them
     uint32_t *ent_id = nullptr, *ent_q = nullptr, *block_counts = nullptr, *wv_list = nullptr, *wv_off = nullptr;
     uint32_t entry_cap = 0;
     uint2* verts = nullptr;
@@ -898,6 +914,7 @@ BatchArgs eng_args(bcmc_engine* e)
     a.owner_block = e->owner_block;
     a.cache = e->cache;
     a.bitmap = e->L->bitmap;
+    a.live = e->L->bitmap + e->L->bitmap_words;
     a.ent_id = e->L->ent_id;
     a.ent_q = e->L->ent_q;
     a.block_counts = e->L->block_counts;
@@ -950,7 +967,8 @@ void eng_upload_vols(bcmc_engine* e)
     std::vector<EngVolDev> h(n);
     for (uint32_t i = 0; i < n; ++i) {
         const EngVolume& v = e->vols[i];
-        h[i] = EngVolDev{v.words, v.ranges, v.tile_ext, v.item_slots, v.grid, v.total, 64u * v.rate};
+        h[i] = EngVolDev{v.words, v.ranges, v.tile_ext, v.item_slots, v.grid, v.total, 64u * v.rate,
+                         sound_ranges(v.dims, v.grid, zfp_ranged_blocks(e->ctx, v.dims))};
     }
     BCMC_CUDA(cudaMemcpyAsync(e->d_vols, h.data(), n * sizeof(EngVolDev), cudaMemcpyHostToDevice, e->stream));
     BCMC_CUDA(cudaStreamSynchronize(e->stream));
@@ -989,7 +1007,7 @@ void eng_ensure_batch(bcmc_engine* e, uint64_t bitmap_words, uint32_t entries)
     if (bitmap_words > e->L->bitmap_words) {
         BCMC_CUDA(cudaStreamSynchronize(e->stream));
         const uint64_t n = std::max<uint64_t>(bitmap_words + bitmap_words / 2, 1u << 16);
-        eng_realloc(e, e->L->bitmap, e->L->bitmap_words, n);
+        eng_realloc(e, e->L->bitmap, 2 * e->L->bitmap_words, 2 * n);
         e->L->bitmap_words = n;
         ++e->L->generation;
     }
@@ -1069,7 +1087,7 @@ void eng_lane_free(bcmc_engine* e, EngLane& l)
     dev_free(ctx, l.d_st, sizeof(EngState));
     dev_free(ctx, l.q_nactive, e->max_batch * 4);
     dev_free(ctx, l.q_nverts, e->max_batch * 4);
-    dev_free(ctx, l.bitmap, l.bitmap_words * 4);
+    dev_free(ctx, l.bitmap, 2 * l.bitmap_words * 4);
     dev_free(ctx, l.ent_id, (size_t)l.entry_cap * 4);
     dev_free(ctx, l.ent_q, (size_t)l.entry_cap * 4);
     dev_free(ctx, l.block_counts, (size_t)l.entry_cap * 4);
