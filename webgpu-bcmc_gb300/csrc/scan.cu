@@ -43,32 +43,44 @@ void prim_begin(QueryState* q, cudaStream_t s)
 // A CTA owns one contiguous range of tiles: it adds them up, publishes the sum,
 // adds up the sums of the CTAs before it in one round trip (their ranks are
 // claimed in order, so all of them run), and scans its tiles again from there --
-// out of its registers when the range is one tile, which it is up to 5 M
-// elements, else out of L2.  Tiles claimed one by one with a look-back each took
+// out of its registers when the range is one tile, which it is up to 3.7 M
+// elements, else out of L2 (tiles of up to 12288, one to a CTA up to 5.6 M, were no
+// faster on 4 M).  Tiles claimed one by one with a look-back each took
 // 25 us on 4 M elements, most of it in the chain from tile to tile.
-// Loads and stores are 16 bytes where the arrays allow it (kWide).
+// A warp has 512 consecutive elements of a tile, in four groups of four to a lane,
+// so that its loads and stores are contiguous, 16 bytes a lane where the arrays
+// allow it (kWide): sixteen elements to a thread take one scan instead of four,
+// but 16-byte pieces of 64 (18.8 -> 15.1 us on 4 M elements).
 constexpr int kRangeThreads = 512;
-constexpr int kRangeItems = 16;  // consecutive elements per thread
-constexpr uint32_t kRangeTile = kRangeThreads * kRangeItems;
+constexpr uint32_t kRangeGroups = 4;
+constexpr uint32_t kRangeTile = kRangeThreads * 4u * kRangeGroups;
 constexpr int kRangePerSm = 3;
 static_assert(kRangeTile % kScanTile == 0, "the status words are sized by kScanTile");
 
+// The lane's elements of the warp's 512 from `first` on.
 template <bool kWide>
-__device__ __forceinline__ void load_items(const uint32_t* in, uint64_t first, uint32_t n, uint32_t v[kRangeItems])
+__device__ __forceinline__ void load_items(const uint32_t* in, uint64_t first, uint32_t n, uint4 v[kRangeGroups])
 {
-    if (kWide && first + kRangeItems <= n) {
 #pragma unroll
-        for (int j = 0; j < kRangeItems / 4; ++j) {
-            const uint4 x = reinterpret_cast<const uint4*>(in + first)[j];
-            v[4 * j] = x.x;
-            v[4 * j + 1] = x.y;
-            v[4 * j + 2] = x.z;
-            v[4 * j + 3] = x.w;
+    for (uint32_t j = 0; j < kRangeGroups; ++j) {
+        const uint64_t i = first + 128u * j + 4u * (threadIdx.x & 31u);
+        if (kWide && i + 4u <= n) {
+            v[j] = *reinterpret_cast<const uint4*>(in + i);
+        } else {
+            v[j].x = i < n ? in[i] : 0u;
+            v[j].y = i + 1u < n ? in[i + 1u] : 0u;
+            v[j].z = i + 2u < n ? in[i + 2u] : 0u;
+            v[j].w = i + 3u < n ? in[i + 3u] : 0u;
         }
-    } else {
-#pragma unroll
-        for (int j = 0; j < kRangeItems; ++j) v[j] = first + j < n ? in[first + j] : 0u;
     }
+}
+
+// What the scan adds up: the elements, or (kSelect) how many are not 0.
+template <bool kSelect>
+__device__ __forceinline__ uint4 addends(uint4 v)
+{
+    if (kSelect) return make_uint4(v.x ? 1u : 0u, v.y ? 1u : 0u, v.z ? 1u : 0u, v.w ? 1u : 0u);
+    return v;
 }
 
 // kSelect: the input is flags, the output the indices of the nonzero ones;
@@ -88,13 +100,16 @@ __global__ void __launch_bounds__(kRangeThreads, kRangePerSm) k_scan(QueryState*
     __syncthreads();
     const uint32_t rank = s_rank, ntiles = div_up(n, kRangeTile);
     const uint32_t first = rank * per_cta, end = min(ntiles, first + per_cta);
-    uint32_t v[kRangeItems], sum = 0, all = 0;
+    const uint32_t lane = t & 31u, warp = t >> 5;
+    uint4 v[kRangeGroups];
+    uint32_t all = 0;
     for (uint32_t tile = first; tile < end; ++tile) {
-        load_items<kWide>(in, (uint64_t)tile * kRangeTile + t * kRangeItems, n, v);
-        sum = 0;
+        load_items<kWide>(in, (uint64_t)tile * kRangeTile + 128u * kRangeGroups * warp, n, v);
 #pragma unroll
-        for (int j = 0; j < kRangeItems; ++j) sum += kSelect ? (v[j] != 0u ? 1u : 0u) : v[j];
-        all += sum;
+        for (uint32_t j = 0; j < kRangeGroups; ++j) {
+                const uint4 x = addends<kSelect>(v[j]);
+            all += x.x + x.y + x.z + x.w;
+        }
     }
     all = __reduce_add_sync(0xffffffffu, all);
     if ((t & 31u) == 0u && all) atomicAdd(&s_sum, all);
@@ -111,41 +126,42 @@ __global__ void __launch_bounds__(kRangeThreads, kRangePerSm) k_scan(QueryState*
         if (tot.host) tot.host[0] = total;
     }
     for (uint32_t tile = first; tile < end; ++tile) {
-        const uint64_t at = (uint64_t)tile * kRangeTile + t * kRangeItems;
-        if (end - first > 1u) {
-            load_items<kWide>(in, at, n, v);
-            sum = 0;
+        const uint64_t base = (uint64_t)tile * kRangeTile + 128u * kRangeGroups * warp;
+        if (end - first > 1u) load_items<kWide>(in, base, n, v);
+        uint32_t before[kRangeGroups], sum = 0;  // of the warp's elements
 #pragma unroll
-            for (int j = 0; j < kRangeItems; ++j) sum += kSelect ? (v[j] != 0u ? 1u : 0u) : v[j];
+        for (uint32_t j = 0; j < kRangeGroups; ++j) {
+                const uint4 x = addends<kSelect>(v[j]);
+            const uint32_t mine = x.x + x.y + x.z + x.w, inc = warp_inclusive_scan(mine);
+            before[j] = sum + inc - mine;
+            sum += __shfl_sync(0xffffffffu, inc, 31);
         }
         uint32_t total;
-        uint32_t pos = run + cta_exclusive_scan<kRangeThreads>(sum, s_warp, &total);
+        const uint32_t warps = cta_exclusive_scan<kRangeThreads>(lane == 0 ? sum : 0u, s_warp, &total);
+        const uint32_t start = run + __shfl_sync(0xffffffffu, warps, 0);
         run += total;
-        if (kSelect) {
 #pragma unroll
-            for (int j = 0; j < kRangeItems; ++j)
-                if (v[j] != 0u) {
-                    if (pos < n) out[pos] = (uint32_t)at + j;  // pos < n unless a wait timed out
-                    ++pos;
-                }
-        } else if (kWide && at + kRangeItems <= n) {
-#pragma unroll
-            for (int j = 0; j < kRangeItems / 4; ++j) {
-                uint4 x;
-                x.x = pos;
-                x.y = x.x + v[4 * j];
-                x.z = x.y + v[4 * j + 1];
-                x.w = x.z + v[4 * j + 2];
-                pos = x.w + v[4 * j + 3];
-                reinterpret_cast<uint4*>(out + at)[j] = x;
+        for (uint32_t j = 0; j < kRangeGroups; ++j) {
+                const uint64_t i = base + 128u * j + 4u * lane;
+            const uint4 x = addends<kSelect>(v[j]);
+            uint4 p;
+            p.x = start + before[j];
+            p.y = p.x + x.x;
+            p.z = p.y + x.y;
+            p.w = p.z + x.z;
+            if (kSelect) {  // positions are below n unless a wait timed out
+                if (x.x && p.x < n) out[p.x] = (uint32_t)i;
+                if (x.y && p.y < n) out[p.y] = (uint32_t)i + 1u;
+                if (x.z && p.z < n) out[p.z] = (uint32_t)i + 2u;
+                if (x.w && p.w < n) out[p.w] = (uint32_t)i + 3u;
+            } else if (kWide && i + 4u <= n) {
+                *reinterpret_cast<uint4*>(out + i) = p;
+            } else {
+                if (i < n) out[i] = p.x;
+                if (i + 1u < n) out[i + 1u] = p.y;
+                if (i + 2u < n) out[i + 2u] = p.z;
+                if (i + 3u < n) out[i + 3u] = p.w;
             }
-        } else {
-#pragma unroll
-            for (int j = 0; j < kRangeItems; ++j)
-                if (at + j < n) {
-                    out[at + j] = pos;
-                    pos += v[j];
-                }
         }
     }
 }
