@@ -72,10 +72,11 @@ struct QueryState {
     // k_mc's grid barrier (CTAs arrived)
     uint32_t mc_arrived;
     uint32_t sort_arrived;  // k_sort's grid barriers between digit passes
+    uint32_t sort_set, sort_clear;  // bits that are 1 in some key, and 0 in some (k_sort that plans by itself)
     // the last age sort's plan was the one-pass one (k_slots then accumulates the
     // age bins alone); kept across queries, zero when the state is created
     uint32_t sort_prev_dense;
-    uint32_t pad[3];
+    uint32_t pad[1];
 };
 
 // The test hook's check: this tile publishes nothing, so the tiles after it
