@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kDecThreads, kDecPerSm) k_decode_volume(const 
 // (the transform, two to four plane transposes and some forty coding steps a
 // block at rate 4): 256^3 at rate 4 took 378 us with a bit-by-bit writer.
 constexpr int kEncThreads = 128;
-constexpr int kEncPerSm = 4;
+constexpr int kEncPerSm = 5;  // 256^3 at rate 4: 4 CTAs 49.4 us, 5 47.1, 6 (spills) 50.4
 constexpr uint32_t kEncPlaneWords = 33;  // 32 used; odd, so that the threads' rows start on different banks
 
 __host__ __device__ __forceinline__ uint32_t enc_row_words(uint32_t rate) { return 2u * rate + 3u; }
