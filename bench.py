@@ -629,13 +629,13 @@ def served_bench() -> dict:
 # DRAM bytes (read + write) per launch of k_mc on this workload, from one ncu
 # capture of 16 consecutive launches (dram__bytes_read.sum + dram__bytes_write.sum,
 # mean over one 16-isovalue sweep): a profile constant, reported as such
-NCU_TRAFFIC = {"k_mc": 42.979e6}
+NCU_TRAFFIC = {"k_mc": 39.957e6}
 
 
 def algorithmic_bytes(stage: str, st: dict, rate: int, total_blocks: int) -> float:
     """Algorithmic DRAM bytes per launch of each stage's kernel."""
-    if stage == "computeVertices":  # k_mc: block data + ids/slots + vertices
-        return st["numActiveBlocks"] * (256 + 4 + 4) + st["numVertices"] * 8 + st["numBlocksWithVertices"] * 8
+    if stage == "computeVertices":  # k_mc: data, id and slot of the blocks with vertices, their list entries, vertices
+        return st["numBlocksWithVertices"] * (256 + 4 + 4 + 8) + st["numVertices"] * 8
     if stage == "decompression":  # k_decode_new + k_assign: compressed bits, the decoded
         # block staged, read back and written into its slot, ids
         return st["newDecompressed"] * (8 * rate + 3 * 256 + 8)

@@ -414,8 +414,8 @@ bcmc_status bcmc_engine_stats_get(bcmc_engine* eng, bcmc_engine_stats* out);
  * the CTAs per SM of the active test and of the MC kernel (coordinate descent
  * from the defaults), and times a decode probe over up to 2^18 blocks of the
  * largest volume for the decode kernel's threads per CTA and CTAs per SM.  The
- * MC kernel's tile (active blocks per CTA tile: 8, 16 or 32, each a compiled
- * instance of the kernel) is tuned first, then its CTAs per SM.  The chosen
+ * MC kernel's CTA size (mc_blocks_per_tile: 8, 16 or 32, 16 threads to each; a
+ * compiled instance of the kernel per size) is tuned first, then its CTAs per SM.  The chosen
  * parameters are used (and captured into that bucket's graph) from then on.
  * The engine has no sort (its pool hands out free slots instead of the LRU's
  * age order), so no radix digit width is tuned here. */

@@ -76,7 +76,6 @@ struct QueryState {
     // the last age sort's plan was the one-pass one (k_slots then accumulates the
     // age bins alone); kept across queries, zero when the state is created
     uint32_t sort_prev_dense;
-    uint32_t pad[1];
 };
 
 // The test hook's check: this tile publishes nothing, so the tiles after it

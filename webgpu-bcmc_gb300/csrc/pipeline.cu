@@ -5,13 +5,15 @@
 // The reference runs ~20 dispatches with six host readbacks per query.  Here a
 // query is a fixed sequence of launches that read every count from the
 // QueryState on the device:
-//   k_query_begin  new look-back epoch, counters cleared
-//   k_active_ranges / k_active
-//                  active test (compute_block_active.comp) for every block,
+//   k_query_flags  new epoch of the status words, counters cleared; every block's
+//                  range against the isovalue, in words of 32 blocks
+//   k_active_words active test (compute_block_active.comp) on those words,
 //                  fused with the compaction of active ids, the cache lookup
-//                  (lru_cache_mark_new_items.comp's "needs caching") and the
-//                  compaction of new item ids; the last tile decides the cache
-//                  growth (js/lru_cache.js:510-522)
+//                  (lru_cache_mark_new_items.comp's "needs caching"), the
+//                  compaction of new item ids and that of the blocks that can
+//                  have vertices; its last CTA decides the cache growth
+//                  (js/lru_cache.js:510-522).  The standalone LRU update has
+//                  k_query_begin and k_active in their place
 //   k_slots        age/mark/grow of every slot (lru_cache_age_slots.comp,
 //                  lru_cache_mark_new_items.comp, lru_cache_init.comp) fused
 //                  with the compaction of available slots and their ages, the
@@ -22,11 +24,11 @@
 //                  into a staging buffer
 //   k_assign       lru_cache_update.comp, and the staged blocks copied into
 //                  their slots
-//   k_query_end    the query state the host reads, into its pinned copy
 //   k_mc           marching cubes count + scan + emit in one cooperative launch
 //                  (compute_block_has_vertices.comp,
 //                  compute_block_voxel_num_verts.comp,
 //                  compute_block_vertices.comp)
+//   k_query_end    the query state the host reads, into its pinned copy
 #include <algorithm>
 
 #include "active_test.cuh"
@@ -36,7 +38,7 @@
 
 namespace bcmc {
 
-// Starts a query's state: counters cleared, a new look-back epoch.  All threads
+// Starts a query's state: counters cleared, a new epoch.  All threads
 // of one CTA call it.
 __device__ __forceinline__ void query_begin(QueryState* q, float iso, bool mc_only, uint32_t capacity,
                                             uint32_t vert_capacity, uint32_t drop_tile)
@@ -83,7 +85,7 @@ __global__ void k_query_begin(QueryState* q, float iso, int mc_only, uint32_t ca
 //
 // Every range is read once, 8 bytes to a lane, and a ballot makes the words; a
 // warp takes `wpw` of them, and its lanes then do the x neighbours of a word
-// each.  k_active, which follows, works on these words: 0.6 bytes a block
+// each.  k_active_words, which follows, works on these words: a byte a block
 // where the ranges are 8.  Before, its tiles read the ranges of all three
 // z-layers around them and tested 27 flag bytes a block, a tile at a time per
 // CTA with a look-back between tiles: 565 us of the 1024 x 1024 x 1080 volume's

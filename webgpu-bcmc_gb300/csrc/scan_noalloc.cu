@@ -1,7 +1,6 @@
 // scan_noalloc.cu -- exclusive scan that allocates nothing.
 //
-// Same result as bcmc_scan_exclusive_u32_async (the single-pass look-back scan
-// of scan.cu), for callers that must not allocate device memory on the call:
+// Same result as bcmc_scan_exclusive_u32_async (the scan by ranges of scan.cu), for callers that must not allocate device memory on the call:
 // a host runtime that owns every device byte through its own pool and forbids
 // cudaMalloc/cudaFree outside it, code running between a stream's enqueue and
 // its synchronisation where an allocation's implicit device synchronisation
@@ -11,11 +10,11 @@
 // BCMC_SCAN_NOALLOC_MAX_N (2^26 elements = 16,384 tiles).
 //
 // Scratch layout (one array per device, in this module's static memory):
-//   words [0, kQueryWords)          QueryState: look-back epoch, tile counter,
+//   words [0, kQueryWords)          QueryState: epoch, range counter,
 //                                   wait-timeout error word
-//   words [kQueryWords, +kStatus)   one look-back status word per 4096-element
-//                                   tile, plus one
-// Every call first runs k_noalloc_begin, which zeroes the tile counter, the
+//   words [kQueryWords, +kStatus)   one status word per 4096 elements (a CTA's
+//                                   range is longer), plus one
+// Every call first runs k_noalloc_begin, which zeroes the range counter, the
 // error word and the status words the call will use, and sets epoch 1; so no
 // state carries from one call to the next and nothing relies on the array's
 // zero initialisation at module load.
@@ -31,7 +30,7 @@
 // threads) race on it and both results are undefined.  Order them on one
 // stream, or with events.
 //
-// A look-back wait that runs out of spins (it cannot hang the GPU) marks the
+// A wait that runs out of spins (it cannot hang the GPU) marks the
 // error word in the shared scratch, which no caller can read, and the prefixes
 // after it are wrong: this entry point does not report wait timeouts.  The
 // context-based scans report them as BCMC_E_TIMEOUT.
