@@ -673,14 +673,19 @@ static void vol_enqueue_query(bcmc_vol* v, cudaStream_t s, float iso, int from_s
                   c->item_slots, v->words, v->max_bits, reinterpret_cast<float*>(c->cache), v->stage, v->stage_blocks};
     DecodeArgs da{c->new_ids, v->words, v->max_bits, v->stage, v->stage_blocks};
     if (events) BCMC_CUDA(cudaEventRecordWithFlags(v->ev[0], s, cudaEventRecordExternal));
-    query_flags_launch(ctx, c->q, iso, c->capacity, v->vert_capacity, v->ranges, grid, v->total, v->flag_words, s,
-                       from_state ? v->h_in : nullptr);
-    active_words_launch(ctx, c->q, aa, v->flag_words, s);
+    const bool front = from_state && !events && query_front_takes(v->total);
+    if (front) {
+        query_front_launch(c->q, v->h_in, v->ranges, aa, v->flag_words, sa, s);
+    } else {
+        query_flags_launch(ctx, c->q, iso, c->capacity, v->vert_capacity, v->ranges, grid, v->total, v->flag_words, s,
+                           from_state ? v->h_in : nullptr);
+        active_words_launch(ctx, c->q, aa, v->flag_words, s);
+    }
     if (events) BCMC_CUDA(cudaEventRecordWithFlags(v->ev[1], s, cudaEventRecordExternal));
     // branch: the new blocks' decode into the staging buffer needs only the
     // active test's new ids, so it overlaps the slot selection below
     BCMC_CUDA(cudaEventRecord(v->fork_ev, s));
-    slots_launch(ctx, c->q, sa, c->capacity, s);
+    if (!front) slots_launch(ctx, c->q, sa, c->capacity, s);
     BCMC_CUDA(cudaStreamWaitEvent(v->side, v->fork_ev, 0));
     decode_new_launch(ctx, c->q, da, v->side);
     BCMC_CUDA(cudaEventRecord(v->join_ev, v->side));

@@ -129,6 +129,10 @@ void query_flags_launch(bcmc_ctx* ctx, QueryState* q, float iso, uint32_t capaci
 // The active test on the words.
 void active_words_launch(bcmc_ctx* ctx, QueryState* q, ActiveArgs a, void* words, cudaStream_t s);
 void query_end_launch(const QueryState* q, QueryState* host, cudaStream_t s);
+// The flags, the active test and the slots of a volume that is small enough, in one launch.
+bool query_front_takes(uint32_t total);
+void query_front_launch(QueryState* q, const QueryInputs* in, const float* ranges, ActiveArgs a, void* words, const SlotArgs& sa,
+                        cudaStream_t s);
 void active_launch(bcmc_ctx* ctx, QueryState* q, const ActiveArgs& a, cudaStream_t s);
 void slots_launch(bcmc_ctx* ctx, QueryState* q, const SlotArgs& a, uint32_t max_slots, cudaStream_t s);
 void assign_launch(bcmc_ctx* ctx, QueryState* q, const AssignArgs& a, uint32_t max_new, cudaStream_t s);

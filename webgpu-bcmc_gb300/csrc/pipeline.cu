@@ -14,6 +14,7 @@
 //                  have vertices; its last CTA decides the cache growth
 //                  (js/lru_cache.js:510-522).  The standalone LRU update has
 //                  k_query_begin and k_active in their place
+//   (k_query_front those two and the next in one launch, for a small volume)
 //   k_slots        age/mark/grow of every slot (lru_cache_age_slots.comp,
 //                  lru_cache_mark_new_items.comp, lru_cache_init.comp) fused
 //                  with the compaction of available slots and their ages, the
@@ -96,8 +97,8 @@ __global__ void k_query_begin(QueryState* q, float iso, int mc_only, uint32_t ca
 constexpr int kFlagThreads = 256;
 constexpr uint32_t kFlagBatch = 8;  // ranges in flight per lane
 
-__global__ void __launch_bounds__(kFlagThreads) k_query_flags(QueryState* q, float iso, uint32_t capacity,
-                                                             uint32_t vert_capacity, const QueryInputs* in, FlagArgs a)
+__device__ __forceinline__ void query_flags(QueryState* q, float iso, uint32_t capacity, uint32_t vert_capacity,
+                                            const QueryInputs* in, const FlagArgs& a)
 {
     const uint32_t lane = threadIdx.x & 31u, total = a.total, wpw = a.wpw;
     const uint32_t nwords = div_up(total, 32u);
@@ -170,6 +171,12 @@ __global__ void __launch_bounds__(kFlagThreads) k_query_flags(QueryState* q, flo
             e = load_ends(w0 + step);
         }
     }
+}
+
+__global__ void __launch_bounds__(kFlagThreads) k_query_flags(QueryState* q, float iso, uint32_t capacity,
+                                                             uint32_t vert_capacity, const QueryInputs* in, FlagArgs a)
+{
+    query_flags(q, iso, capacity, vert_capacity, in, a);
 }
 
 // Ends a query graph: the query state the host reads (the fields before the
@@ -250,8 +257,9 @@ constexpr int kWordThreads = 256;
 constexpr int kWordPerSm = 5;
 constexpr uint32_t kWordRange = 2048;  // words whose results fit in shared memory; longer ranges keep them in global memory
 
-__global__ void __launch_bounds__(kWordThreads, kWordPerSm) k_active_words(QueryState* q, ActiveArgs a, uint32_t wpw,
-                                                                          uint32_t range)
+// kSameLaunch: other CTAs of this launch wrote the words, which are read from L2.
+template <bool kSameLaunch>
+__device__ __forceinline__ void active_words(QueryState* q, const ActiveArgs& a, uint32_t wpw, uint32_t range)
 {
     __shared__ uint2 s_words[kWordRange];
     __shared__ uint32_t s_live[kWordRange];
@@ -262,6 +270,7 @@ __global__ void __launch_bounds__(kWordThreads, kWordPerSm) k_active_words(Query
     const uint32_t total = a.total, nwords = div_up(total, 32u), rank = blockIdx.x;
     const uint32_t first = rank * range, end = min(nwords, first + range);
     if (first >= nwords) return;
+    const auto word = [](const uint4* p) { return kSameLaunch ? __ldcg(p) : __ldg(p); };
     const uint32_t epoch = q->epoch;
     const uint3 nb = a.grid.nb;
     const int32_t nx = (int32_t)nb.x;
@@ -289,12 +298,12 @@ __global__ void __launch_bounds__(kWordThreads, kWordPerSm) k_active_words(Query
                     const uint32_t sh = (uint32_t)s & 31u;
                     const int64_t k0 = min(max(k, (int64_t)0), (int64_t)nwords - 1),
                                   k1 = min(max(k + 1, (int64_t)0), (int64_t)nwords - 1);
-                    const uint4 lo = __ldg(a.near + k0), hi = __ldg(a.near + k1);
+                    const uint4 lo = word(a.near + k0), hi = word(a.near + k1);
                     any_a |= __funnelshift_r(lo.x, hi.x, sh) & m;
                     any_b |= __funnelshift_r(lo.y, hi.y, sh) & m;
                     any_c |= __funnelshift_r(lo.z, hi.z, sh) & m;
                     if (dz >= 0 && dy >= 0) {
-                        const uint4 l = __ldg(a.up + k0), h = __ldg(a.up + k1);
+                        const uint4 l = word(a.up + k0), h = word(a.up + k1);
                         up_a |= __funnelshift_r(l.x, h.x, sh) & m;
                         up_b |= __funnelshift_r(l.y, h.y, sh) & m;
                         if (dz == 0 && dy == 0) self_b = l.z;
@@ -403,6 +412,12 @@ __global__ void __launch_bounds__(kWordThreads, kWordPerSm) k_active_words(Query
     }
 }
 
+__global__ void __launch_bounds__(kWordThreads, kWordPerSm) k_active_words(QueryState* q, ActiveArgs a, uint32_t wpw,
+                                                                          uint32_t range)
+{
+    active_words<false>(q, a, wpw, range);
+}
+
 // k_active: the standalone LRU update's side of the same: the items that are
 // needed, and of those the ones no slot holds, compacted.
 __global__ void __launch_bounds__(kActThreads) k_active(QueryState* q, ActiveArgs a)
@@ -468,7 +483,7 @@ __global__ void __launch_bounds__(kActThreads) k_active(QueryState* q, ActiveArg
 // ---------------------------------------------------------------------------
 constexpr uint32_t kSlotChunk = 4u * kActThreads;
 
-__global__ void __launch_bounds__(kActThreads) k_slots(QueryState* q, SlotArgs a)
+__device__ __forceinline__ void update_slots(QueryState* q, const SlotArgs& a)
 {
     __shared__ uint32_t s_warp[kActThreads / 32 + 1];
     __shared__ uint32_t s_rank, s_sum, s_prefix;
@@ -641,6 +656,39 @@ __global__ void __launch_bounds__(kActThreads) k_slots(QueryState* q, SlotArgs a
     if (dense) sort_plan<kActThreads>(q, q->num_avail, s_warp, rank_hist, 1);
     else if (key16) sort_plan<kActThreads>(q, q->num_avail, s_warp, &q->sort_hist16[0][0], 2);
     else sort_plan<kActThreads>(q, q->num_avail, s_warp, &q->sort_hist[0][0], 4);
+}
+
+__global__ void __launch_bounds__(kActThreads) k_slots(QueryState* q, SlotArgs a) { update_slots(q, a); }
+
+// ---------------------------------------------------------------------------
+// k_query_front: k_query_flags, k_active_words and k_slots of a small volume in one
+// launch, one cluster of CTAs, with the cluster's barrier where the kernels end.
+// A query of a small volume is a chain of launches that each take longer to start
+// and to drain than to run; beyond kFrontBlocks the sixteen SMs' throughput costs
+// more than two launches.  Whole queries, all cached and with 5 % of the blocks
+// cached: 4096 blocks 37.0 -> 35.5 and 35.4 -> 33.2 us, 13,824 41.0 -> 39.9 and 41.4 ->
+// 40.3, 21,952 41.6 -> 39.7 and 50.6 -> 49.1, 32,768 42.0 -> 43.0 and 44.5 -> 44.4
+// (clusters of eight: as good at 4096, 0.5 us slower than the kernels at 13,824).
+// With a perf tracker the three run as kernels, whose times it reports.
+// ---------------------------------------------------------------------------
+constexpr int kFrontCtas = 16;  // the largest cluster, which a kernel has to ask for
+constexpr uint32_t kFrontBlocks = 24576;
+static_assert(kFlagThreads == kWordThreads && kFlagThreads == kActThreads, "one CTA does the work of all three");
+
+__device__ __forceinline__ void cluster_barrier()
+{
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(kFrontCtas, 1, 1) __launch_bounds__(kActThreads)
+    k_query_front(QueryState* q, const QueryInputs* in, FlagArgs f, ActiveArgs a, uint32_t wpw, uint32_t range, SlotArgs sa)
+{
+    query_flags(q, 0.0f, 0u, 0u, in, f);
+    cluster_barrier();
+    active_words<true>(q, a, wpw, range);
+    cluster_barrier();
+    update_slots(q, sa);
 }
 
 // ---------------------------------------------------------------------------
@@ -1021,13 +1069,19 @@ void query_flags_launch(bcmc_ctx* ctx, QueryState* q, float iso, uint32_t capaci
     BCMC_CUDA(cudaGetLastError());
 }
 
-void active_words_launch(bcmc_ctx* ctx, QueryState* q, ActiveArgs a, void* words, cudaStream_t s)
+// Where the words of a query lie in their buffer (flag_bytes).
+static void word_buffers(ActiveArgs& a, void* words, uint32_t nwords)
 {
-    const uint32_t nwords = div_up(a.total, 32u), wpw = words_per_warp(ctx, nwords, kWordThreads / 32);
     a.near = static_cast<const uint4*>(words);
     a.up = a.near + nwords;
     a.words = reinterpret_cast<uint2*>(static_cast<uint4*>(words) + 2u * (size_t)nwords);
     a.live_words = reinterpret_cast<uint32_t*>(a.words + nwords);
+}
+
+void active_words_launch(bcmc_ctx* ctx, QueryState* q, ActiveArgs a, void* words, cudaStream_t s)
+{
+    const uint32_t nwords = div_up(a.total, 32u), wpw = words_per_warp(ctx, nwords, kWordThreads / 32);
+    word_buffers(a, words, nwords);
     // a CTA an SM first: the CTAs wait for each other's counts (256^3: 128 of them
     // 1.3 us faster than 256); then a range of whole rounds per resident CTA
     const uint32_t round = wpw * (kWordThreads / 32);
@@ -1043,6 +1097,45 @@ void active_words_launch(bcmc_ctx* ctx, QueryState* q, ActiveArgs a, void* words
     cfg.numAttrs = 1;
     BCMC_CUDA(cudaLaunchKernelEx(&cfg, k_active_words, q, a, wpw, range));
     count_launches(1);
+}
+
+// Whether the device has room for the cluster (a slice of one may not).
+static bool front_fits()
+{
+    static const bool fits = [] {
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = kFrontCtas;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kFrontCtas);
+        cfg.blockDim = dim3(kActThreads);
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        const bool ok = cudaFuncSetAttribute(k_query_front, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&n, k_query_front, &cfg) == cudaSuccess && n > 0;
+        if (!ok) cudaGetLastError();
+        return ok;
+    }();
+    return fits;
+}
+
+bool query_front_takes(uint32_t total) { return total <= kFrontBlocks && front_fits(); }
+
+void query_front_launch(QueryState* q, const QueryInputs* in, const float* ranges, ActiveArgs a, void* words, const SlotArgs& sa,
+                        cudaStream_t s)
+{
+    constexpr uint32_t kWarps = kWordThreads / 32;
+    const uint32_t nwords = div_up(a.total, 32u), wpw = std::min(align_up(div_up(nwords, kFrontCtas * kWarps), 4u), 32u);
+    const uint32_t range = div_up(div_up(nwords, wpw * kWarps), kFrontCtas) * wpw * kWarps;
+    uint4* near = static_cast<uint4*>(words);
+    const FlagArgs f{reinterpret_cast<const float2*>(ranges), a.grid, a.total, wpw, near, near + nwords};
+    word_buffers(a, words, nwords);
+    BCMC_CUDA(cudaFuncSetAttribute(k_query_front, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    k_query_front<<<kFrontCtas, kActThreads, 0, s>>>(q, in, f, a, wpw, range, sa);
+    count_launches(1);
+    BCMC_CUDA(cudaGetLastError());
 }
 
 void active_launch(bcmc_ctx* ctx, QueryState* q, const ActiveArgs& a, cudaStream_t s)
