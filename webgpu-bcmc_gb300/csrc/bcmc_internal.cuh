@@ -78,6 +78,15 @@ struct QueryState {
     uint32_t sort_prev_dense;
 };
 
+// The tag of status words that several kernels share: the sort, the scans, the select
+// and the active test lay their words out differently in a context's, the two active
+// tests use the same ones of a cache.  Four tags to an operation, so that none of an
+// operation's is one that an earlier sort's passes left.
+__device__ __forceinline__ uint32_t status_tag(const QueryState* q, uint32_t pass = 0u)
+{
+    return (q->epoch * 4u + pass) & 0x3fffffffu;
+}
+
 // The test hook's check: this tile publishes nothing, so the tiles after it
 // wait on a status word that nobody sets until their bounded spin runs out.
 __device__ __forceinline__ bool lb_dropped(const QueryState* q, uint32_t tile)

@@ -271,7 +271,7 @@ __device__ __forceinline__ void active_words(QueryState* q, const ActiveArgs& a,
     const uint32_t first = rank * range, end = min(nwords, first + range);
     if (first >= nwords) return;
     const auto word = [](const uint4* p) { return kSameLaunch ? __ldcg(p) : __ldg(p); };
-    const uint32_t epoch = q->epoch;
+    const uint32_t epoch = status_tag(q);
     const uint3 nb = a.grid.nb;
     const int32_t nx = (int32_t)nb.x;
     const int64_t nxy = (int64_t)nb.x * nb.y;
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(kActThreads) k_active(QueryState* q, ActiveArg
     __shared__ uint32_t s_tile, s_pa, s_pn;
     const uint32_t total = a.total;
     const uint32_t ntiles = div_up(total, kActiveTile);
-    const uint32_t epoch = q->epoch;
+    const uint32_t epoch = status_tag(q);
     for (;;) {
         if (threadIdx.x == 0) s_tile = atomicAdd(&q->tiles_active, 1u);
         __syncthreads();

@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kRangeThreads, kRangePerSm) k_scan(QueryState*
     all = __reduce_add_sync(0xffffffffu, all);
     if ((t & 31u) == 0u && all) atomicAdd(&s_sum, all);
     __syncthreads();
-    const bool late = cta_prefix_sum<kRangeThreads>(status, rank, s_sum, q->epoch, &q->error, kSelect ? 2u : 1u,
+    const bool late = cta_prefix_sum<kRangeThreads>(status, rank, s_sum, status_tag(q), &q->error, kSelect ? 2u : 1u,
                                                     &s_prefix, lb_dropped(q, rank));
     if (late && tot.host) tot.host[1] = 1u;
     __syncthreads();

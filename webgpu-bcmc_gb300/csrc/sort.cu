@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort(QueryState* q, const u
         const bool gather = src == 0;
         const uint32_t kmode = kSelf ? 0u : q->sort_key16;  // 0: the keys, 1: 16-bit age keys, 2: their dense ranks
         const uint32_t shift = 8u * pass;
-        const uint32_t epoch = q->epoch * 4u + pass;
+        const uint32_t epoch = status_tag(q, pass);
         const uint32_t* bucket = q->sort_hist[pass];
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
         const uint32_t lt_mask = (1u << lane) - 1u;
