@@ -1,6 +1,8 @@
 """The primitives of one context share its status words, which a sort of more tiles
 than run at once leaves with the tags of its passes: the scans, selects and active
-tests that follow, at every distance, take none of them for their own."""
+tests that follow, at every distance, take none of them for their own.  (A wrong tag
+shows only when a CTA reads a word before its owner has written it: this holds the
+sequences that could go wrong to their results, it does not force that order.)"""
 import ctypes as C
 
 import numpy as np
