@@ -122,6 +122,15 @@ __device__ __forceinline__ uint32_t zfp_shr(uint32_t x, uint32_t s)
 #endif
 }
 
+// the low word of hi:lo shifted right by s, up to 32
+__device__ __forceinline__ uint32_t zfp_window(uint32_t lo, uint32_t hi, uint32_t s)
+{
+#ifdef __CUDA_ARCH__
+    return __funnelshift_rc(lo, hi, s);
+#else
+    return s >= 32u ? hi : __funnelshift_r(lo, hi, s);
+#endif
+}
 // the low m bits, all from 32 on
 __device__ __forceinline__ uint32_t zfp_low(uint32_t m)
 {
@@ -161,15 +170,14 @@ __device__ __forceinline__ uint32_t zfp_clz(uint32_t x)
 // where *r0 is the number of leading empty planes, which are not stored.
 // Returns the number of planes decoded, r0 included.
 //
-// A 64-bit window suffices: a run after a group test needs bits 1..63 (one
-// that would reach bit 64 is cut at 63 coefficients first), raw bits after a
-// group test number at most 63 (n < 64 there), and 64 raw bits are read only
-// where no group test is (n = 64).
+// A 64-bit window after the group test suffices: a run in it is cut at 63
+// coefficients first, raw bits after a group test number at most 63 (n < 64
+// there), and 64 raw bits are read only where no group test is (n = 64).
 __device__ __forceinline__ uint32_t zfp_parse_planes(const uint32_t* w, uint32_t pos, uint32_t budget, uint32_t* pl,
                                                      uint32_t* r0p)
 {
-    uint32_t bits = budget, n = 0, xlo = 0, xhi = 0, a0, a1;
-    a0 = __funnelshift_r(w[pos >> 5], w[(pos >> 5) + 1], pos & 31u);
+    uint32_t bits = budget, n = 0, xlo = 0, xhi = 0;
+    const uint32_t a0 = __funnelshift_r(w[pos >> 5], w[(pos >> 5) + 1], pos & 31u);
     const uint32_t r0 = min(a0 ? (uint32_t)__ffs(a0) - 1u : 32u, bits);
     pos += r0;
     bits -= r0;
@@ -180,24 +188,22 @@ __device__ __forceinline__ uint32_t zfp_parse_planes(const uint32_t* w, uint32_t
     for (;;) {
         const uint32_t i = pos >> 5, sh = pos & 31u;
         const uint32_t w0 = w[i], w1 = w[i + 1], w2 = w[i + 2];
-        a0 = __funnelshift_r(w0, w1, sh);
-        a1 = __funnelshift_r(w1, w2, sh);
-        const uint32_t b0 = __funnelshift_r(a0, a1, 1), b1 = a1 >> 1;  // window bits 1..63
         const bool gtr = n < 64u && bits != 0u;  // a group test is read
-        const bool one = gtr && (a0 & 1u);
+        const bool one = gtr && (w0 >> sh & 1u);
+        // the 64 bits after it (or from here, if none is)
+        const uint32_t o = gtr ? 1u : 0u, c0 = zfp_window(w0, w1, sh + o), c1 = zfp_window(w1, w2, sh + o);
         // a 1: t zeros before the next one (all ones: none within the window)
-        const uint32_t t = min(zfp_ctz(b0), zfp_ctz(b1) | 32u);
-        const uint32_t lim = min(63u - n, bits - 1u);
+        const uint32_t t = min(zfp_ctz(c0), zfp_ctz(c1) | 32u);
+        // a 0 (or no read): the plane ends; the next plane's raw bits follow
+        const uint32_t be = bits - o, m = min(n, be);
+        const uint32_t lim = min(63u - n, be);
         const uint32_t z = min(t, lim), hit = t < lim ? 1u : 0u;
         const uint32_t nt = n + z;  // the coefficient that becomes significant
-        // a 0 (or no read): the plane ends; the next plane's raw bits follow
-        const uint32_t o = gtr ? 1u : 0u, be = bits - o, m = min(n, be);
         if (!one) {
             reinterpret_cast<uint2*>(pl)[r] = make_uint2(xlo, xhi);
             ++r;
             if (r == 32u || be == 0u) break;
         }
-        const uint32_t c0 = gtr ? b0 : a0, c1 = gtr ? b1 : a1;
         const uint32_t rlo = c0 & zfp_low(m), rhi = c1 & zfp_shr(0xffffffffu, 64u - m);
         const uint32_t tlo = xlo | zfp_shl(1u, nt), thi = xhi | zfp_shl(1u, nt - 32u);
         xlo = one ? tlo : rlo;
