@@ -80,9 +80,9 @@ __device__ __forceinline__ float zfp_inv_weight(int32_t emax)
 // block per thread), then parsed there.
 //
 // Parse (zfp_parse_planes): one loop step per group-test read.  A step loads
-// a 64-bit window at the bit position (three words, two funnel shifts) and
-// computes both outcomes with selects: a 1 (the run of zeros after it found
-// with one find-first-set, clamped by the bit budget and by coefficient 63,
+// the 64-bit window after the test (three words, two funnel shifts) and
+// computes both outcomes with selects: a 1 (the run of zeros after it is the
+// window's trailing zeros, clamped by the bit budget and by coefficient 63,
 // decode_ints' two limits) or a 0, which ends the plane and takes the next
 // plane's raw bits from the same window.  Only the plane store and the loop
 // exit branch, so a warp's lanes stay converged although their blocks take
@@ -91,7 +91,9 @@ __device__ __forceinline__ float zfp_inv_weight(int32_t emax)
 // spectral field at rate 2 (about 19 steps per block) this took the full
 // decode from 0.390 ms (8-bit group-test table steps, a bit-by-bit tail near
 // the limits, branches per outcome) to 0.257 ms; the branching form of the
-// same step measured 0.333 ms.
+// same step measured 0.333 ms.  With trailing zeros and masks by one instruction
+// each, whole-plane stores, the multiply-add deposit and one window a step it
+// takes 0.226 ms (220 -> 203 M warp instructions).
 //
 // Deposit (zfp_planes_deposit): the plane masks go to a per-thread row of
 // shared memory; each 8-plane chunk is read back as 8 rows of 64 bits and all
