@@ -16,6 +16,7 @@
 #include <string>
 
 #include "bcmc_pipeline.h"
+#include "slot_ranges.cuh"
 
 using namespace bcmc;
 

@@ -139,7 +139,6 @@ void assign_launch(bcmc_ctx* ctx, QueryState* q, const AssignArgs& a, uint32_t m
 void decode_new_launch(bcmc_ctx* ctx, const QueryState* q, const DecodeArgs& a, cudaStream_t s);
 void mc_launch(bcmc_ctx* ctx, QueryState* q, const McArgs& a, uint32_t max_active, cudaStream_t s);
 uint32_t active_tiles(uint32_t total);
-uint32_t slot_tiles(uint32_t slots);
 uint32_t mc_grid(bcmc_ctx* ctx, uint32_t max_active);
 
 }  // namespace bcmc

@@ -35,6 +35,7 @@
 #include "active_test.cuh"
 #include "bcmc_pipeline.h"
 #include "mc_common.cuh"
+#include "slot_ranges.cuh"
 #include "zfp_device.cuh"
 
 namespace bcmc {
@@ -475,13 +476,13 @@ __global__ void __launch_bounds__(kActThreads) k_active(QueryState* q, ActiveArg
 // available slots (ascending slot id) and their ages.
 //
 // A CTA owns one contiguous range of slots, four to a thread at a time: ages and
-// marks them, then, when new items need slots, joins its count of available ones
-// to those of the CTAs before it (ranks are claimed in order, so all of them
-// run) and writes their ids and ages.  512-slot tiles claimed one by one, each
-// waiting for its claim, its items and their flags in turn, took 80 us on the
-// 1024 x 1024 x 1080 volume's 2.6 M slots.
+// marks them, then, when new items need slots and it has any, joins its count of
+// available ones to those of the CTAs before it (ranks are claimed in order, so
+// all of them run) and writes their ids and ages.  512-slot tiles claimed one by
+// one, each waiting for its claim, its items and their flags in turn, took 80 us
+// on the 1024 x 1024 x 1080 volume's 2.6 M slots.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kSlotChunk = 4u * kActThreads;
+static_assert(kSlotChunk == 4u * kActThreads, "four slots to a thread");
 
 __device__ __forceinline__ void update_slots(QueryState* q, const SlotArgs& a)
 {
@@ -511,8 +512,8 @@ __device__ __forceinline__ void update_slots(QueryState* q, const SlotArgs& a)
         s_sum = s_prefix = 0;
     }
     __syncthreads();
-    const uint32_t range = align_up(div_up(nsz, gridDim.x), kSlotChunk);
-    const uint32_t first = min((uint64_t)nsz, (uint64_t)s_rank * range), end = min((uint64_t)nsz, (uint64_t)first + range);
+    const SlotRange mine = slot_range(nsz, gridDim.x, s_rank);
+    const uint32_t first = mine.first, end = mine.end;
     uint32_t count = 0;
     for (uint32_t base = first; base < end; base += kSlotChunk) {
         const uint32_t s = base + 4u * threadIdx.x;
@@ -549,7 +550,7 @@ __device__ __forceinline__ void update_slots(QueryState* q, const SlotArgs& a)
                 }
             }
     }
-    if (compact) {
+    if (compact && mine.any()) {
         count = __reduce_add_sync(0xffffffffu, count);
         if (lane == 0 && count) atomicAdd(&s_sum, count);
         __syncthreads();
@@ -1212,7 +1213,6 @@ void mc_launch(bcmc_ctx* ctx, QueryState* q, const McArgs& a, uint32_t max_activ
 }
 
 uint32_t active_tiles(uint32_t total) { return div_up(total, kActiveTile); }
-uint32_t slot_tiles(uint32_t slots) { return div_up(slots, kSlotChunk); }
 // one CTA per range of active blocks, every CTA resident; at least a block to a warp
 uint32_t mc_grid(bcmc_ctx* ctx, uint32_t max_active)
 {
