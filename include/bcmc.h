@@ -265,7 +265,8 @@ bcmc_status bcmc_scan_exclusive_u32_noalloc(const uint32_t* d_in, uint32_t* d_ou
  * out[offsets[i]] = i for every i < n with flags[i] != 0. */
 bcmc_status bcmc_compact_ids(bcmc_ctx* ctx, uint32_t n, const uint32_t* d_flags,
                              const uint32_t* d_offsets, uint32_t* d_out, void* stream);
-/* Fused scan + compaction of the ids of nonzero flags (no offsets buffer). */
+/* Fused scan + compaction of the ids of nonzero flags (no offsets buffer);
+ * d_out may equal d_flags. */
 bcmc_status bcmc_select_ids(bcmc_ctx* ctx, uint32_t n, const uint32_t* d_flags, uint32_t* d_out,
                             uint32_t* d_count, void* stream);
 

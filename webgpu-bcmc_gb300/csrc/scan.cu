@@ -195,7 +195,11 @@ static cudaError_t launch_ranges(int num_sms, QueryState* q, const uint32_t* in,
                                  const ScanTotals& tot, uint64_t* status, cudaStream_t s)
 {
     const uint32_t tiles = div_up(n, kRangeTile), most = (uint32_t)num_sms * kRangePerSm;
-    const uint32_t per_cta = div_up(tiles, most), grid = div_up(tiles, per_cta);
+    // A select's ids go to places at or before their flags.  Where these are the
+    // flags' own words, a CTA must not read a tile again after others may have
+    // written: one tile to a CTA, which then keeps it in registers.
+    const bool overlap = kSelect && in < out + n && out < in + n;
+    const uint32_t per_cta = overlap ? 1u : div_up(tiles, most), grid = div_up(tiles, per_cta);
     // (a select's output is written element by element: its alignment is not asked for)
     if (aligned16(in, kSelect ? in : out)) k_scan<kSelect, true><<<grid, kRangeThreads, 0, s>>>(q, in, out, n, per_cta, tot, status);
     else k_scan<kSelect, false><<<grid, kRangeThreads, 0, s>>>(q, in, out, n, per_cta, tot, status);
