@@ -1297,13 +1297,14 @@ bcmc_status bcmc_block_active(bcmc_ctx* ctx, const float* d_ranges, const uint32
     return guarded(ctx, [&]() -> bcmc_status {
         cudaStream_t s = pick(ctx, stream);
         const uint3 nb = make_uint3(div_up(dims[0], 4), div_up(dims[1], 4), div_up(dims[2], 4));
-        const uint64_t total = (uint64_t)nb.x * nb.y * nb.z;
-        ensure_status(ctx, 2 * (active_tiles((uint32_t)total) + 1));
+        const uint32_t total = nb.x * nb.y * nb.z;
+        if (total == 0) return BCMC_OK;
+        ensure_status(ctx, 2 * (active_tiles(total) + 1));
         ensure_scratch(ctx, flag_bytes(total) / 4u);
         const BlockGrid grid = make_block_grid(nb);
-        ActiveArgs aa{grid,    nullptr, d_active,      nullptr, (uint32_t)total,
-                      nullptr, nullptr, ctx->d_status, ctx->d_status + active_tiles((uint32_t)total) + 1};
-        query_flags_launch(ctx, ctx->d_prim, iso, 0, 0, d_ranges, grid, (uint32_t)total, ctx->d_scratch, s);
+        ActiveArgs aa{grid,    nullptr, d_active,      nullptr, total,
+                      nullptr, nullptr, ctx->d_status, ctx->d_status + active_tiles(total) + 1};
+        query_flags_launch(ctx, ctx->d_prim, iso, 0, 0, d_ranges, grid, total, ctx->d_scratch, s);
         active_words_launch(ctx, ctx->d_prim, aa, ctx->d_scratch, s);
         return BCMC_OK;
     });
