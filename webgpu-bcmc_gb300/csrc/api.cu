@@ -66,6 +66,19 @@ void ensure_scratch(bcmc_ctx* ctx, size_t words)
     ctx->scratch_words = words;
 }
 
+// Not part of the scratch: a sort captured into a graph keeps the scratch's address,
+// which an active test of a larger volume would otherwise move.
+void ensure_flags(bcmc_ctx* ctx, size_t bytes)
+{
+    if (bytes <= ctx->flags_bytes) return;
+    BCMC_CUDA(cudaStreamSynchronize(ctx->stream));
+    dev_free(ctx, ctx->d_flags, ctx->flags_bytes);
+    ctx->d_flags = nullptr;
+    ctx->flags_bytes = 0;
+    ctx->d_flags = dev_alloc(ctx, bytes);
+    ctx->flags_bytes = bytes;
+}
+
 }  // namespace bcmc
 
 std::atomic<uint64_t> bcmc::g_kernel_launches{0};
@@ -103,6 +116,7 @@ static void ctx_release(bcmc_ctx* ctx)
     dev_free(ctx, ctx->d_status, ctx->status_words * 8);
     if (ctx->d_counts) dev_free(ctx, ctx->d_counts, sort_count_bytes(ctx));
     dev_free(ctx, ctx->d_scratch, ctx->scratch_words * 4);
+    dev_free(ctx, ctx->d_flags, ctx->flags_bytes);
     dev_free(ctx, ctx->d_render, ctx->render_bytes);
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
@@ -1300,12 +1314,12 @@ bcmc_status bcmc_block_active(bcmc_ctx* ctx, const float* d_ranges, const uint32
         const uint32_t total = nb.x * nb.y * nb.z;
         if (total == 0) return BCMC_OK;
         ensure_status(ctx, 2 * (active_tiles(total) + 1));
-        ensure_scratch(ctx, flag_bytes(total) / 4u);
+        ensure_flags(ctx, flag_bytes(total));
         const BlockGrid grid = make_block_grid(nb);
         ActiveArgs aa{grid,    nullptr, d_active,      nullptr, total,
                       nullptr, nullptr, ctx->d_status, ctx->d_status + active_tiles(total) + 1};
-        query_flags_launch(ctx, ctx->d_prim, iso, 0, 0, d_ranges, grid, total, ctx->d_scratch, s);
-        active_words_launch(ctx, ctx->d_prim, aa, ctx->d_scratch, s);
+        query_flags_launch(ctx, ctx->d_prim, iso, 0, 0, d_ranges, grid, total, ctx->d_flags, s);
+        active_words_launch(ctx, ctx->d_prim, aa, ctx->d_flags, s);
         return BCMC_OK;
     });
 }

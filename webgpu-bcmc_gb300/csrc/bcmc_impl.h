@@ -23,6 +23,8 @@ struct bcmc_ctx {
     uint16_t* d_counts = nullptr;   // the sort's tile counts (sort_count_bytes)
     uint32_t* d_scratch = nullptr;  // sort ping-pong buffers for primitives
     size_t scratch_words = 0;
+    void* d_flags = nullptr;        // bcmc_block_active's words (flag_bytes)
+    size_t flags_bytes = 0;
     uint32_t* h_pinned = nullptr;   // small pinned host staging
     void* d_render = nullptr;       // render pass working buffers (grow-only)
     size_t render_bytes = 0;
@@ -58,6 +60,7 @@ void* dev_alloc(bcmc_ctx* ctx, size_t bytes);
 void dev_free(bcmc_ctx* ctx, void* p, size_t bytes);
 void ensure_status(bcmc_ctx* ctx, size_t words);
 void ensure_scratch(bcmc_ctx* ctx, size_t words);
+void ensure_flags(bcmc_ctx* ctx, size_t bytes);
 
 // ---- unpack.cu ----------------------------------------------------------------
 void unpack_launch(bcmc_ctx* ctx, const uint2* verts, uint64_t n, const uint32_t dims[3], const float scale[3],
