@@ -120,8 +120,6 @@ constexpr int kEncThreads = 128;
 constexpr int kEncPerSm = 5;  // 256^3 at rate 4: 4 CTAs 49.4 us, 5 47.1, 6 (spills) 50.4
 constexpr uint32_t kEncPlaneWords = 33;  // 32 used; odd, so that the threads' rows start on different banks
 
-__host__ __device__ __forceinline__ uint32_t enc_row_words(uint32_t rate) { return 2u * rate + 3u; }
-
 // a partial block's coordinate i on an axis with n voxels: the voxel padding
 // copies (n < 4: 0 past one voxel; the last, then the first past two; the first past three)
 __device__ __forceinline__ uint32_t pad_coord(uint32_t i, uint32_t n) { return i < n ? i : (n == 2u && i == 2u ? 1u : 0u); }
@@ -131,7 +129,7 @@ __global__ void __launch_bounds__(kEncThreads, kEncPerSm) k_encode(const float* 
                                                                    uint64_t* __restrict__ words)
 {
     uint32_t* s_rows = stage_words();
-    const uint32_t stride = enc_row_words(rate);
+    const uint32_t stride = zfp_encode_row_words(rate);
     uint32_t* row = s_rows + threadIdx.x * stride;
     uint32_t* pl = s_rows + kEncThreads * stride + threadIdx.x * kEncPlaneWords;
     const uint32_t lane = threadIdx.x & 31u;
@@ -257,7 +255,7 @@ void zfp_encode_launch(bcmc_ctx* ctx, const float* field, const uint32_t dims[3]
     const uint3 nb = make_uint3(div_up(dims[0], 4), div_up(dims[1], 4), div_up(dims[2], 4));
     const uint64_t n = (uint64_t)nb.x * nb.y * nb.z;
     const uint32_t rate = max_bits / 64u;
-    const size_t smem = (size_t)kEncThreads * (enc_row_words(rate) + kEncPlaneWords) * 4u;
+    const size_t smem = (size_t)kEncThreads * (zfp_encode_row_words(rate) + kEncPlaneWords) * 4u;
     // 16-byte loads of a block's rows: whole rows on 16-byte boundaries
     const bool rows16 = dims[0] % 4u == 0 && reinterpret_cast<uintptr_t>(field) % 16u == 0;
     allow_smem(k_encode, smem);

@@ -166,7 +166,7 @@ __device__ __forceinline__ uint32_t zfp_clz(uint32_t x)
 }
 
 // decode_ints' bit planes (zfp_decompress.comp:265-294) as masks.  `w`: the
-// block's words (LSB first), readable for two words past the block; `pos`:
+// block's words (LSB first), readable for three words past the block; `pos`:
 // the first bit after the header.  Plane r (bit 31 - r of the coefficients)
 // goes to pl[2(r - r0)] (coefficients 0..31) and pl[2(r - r0) + 1] (32..63),
 // where *r0 is the number of leading empty planes, which are not stored.
@@ -330,7 +330,7 @@ __device__ __forceinline__ void zfp_planes_deposit(const uint32_t* pl, uint32_t 
 }
 
 // One block from its words `w` (2 * rate 32-bit words, 64 * rate bits; staged
-// in shared memory, or in place in global memory), readable for two words
+// in shared memory, or in place in global memory), readable for three words
 // past the block.  `pl` is the thread's plane scratch: 64 words, 16-byte
 // aligned (a row of shared memory, or a thread-local array).
 __device__ __forceinline__ void zfp_decode_staged(const uint32_t* w, uint32_t max_bits, uint32_t* pl, float* out)
@@ -522,8 +522,12 @@ struct RowWriter {
     }
 };
 
-// One block into its row of zeroed words (max_bits / 32, and two more that the
-// last append may touch).  `pl`: 32 words of scratch.
+// Words of a block's row: the block's bits, and three more that an append at its
+// end touches (RowWriter::put).
+__host__ __device__ __forceinline__ constexpr uint32_t zfp_encode_row_words(uint32_t rate) { return 2u * rate + 3u; }
+
+// One block into its row of zeroed words (zfp_encode_row_words).  `pl`: 32 words
+// of scratch.
 //
 // encode_ints of the published method, in the decoder's steps: a step is either
 // a group test that finds a coefficient (a 1, the zeros before it, and its 1
@@ -595,7 +599,8 @@ __device__ __forceinline__ void zfp_encode_row(const float* f, uint32_t max_bits
     }
 }
 
-// The same to its place in a stream of 64-bit words, a block at a time.
+// The same to its place in a stream of 64-bit words, a block at a time (k_encode
+// stores a warp's rows together; this is the form that host builds test).
 struct BitWriter {
     unsigned long long* words;
     uint64_t first;  // the block's first word
@@ -609,7 +614,7 @@ struct BitWriter {
 };
 __device__ __forceinline__ void zfp_encode_block(const float* f, uint32_t max_bits, BitWriter& bw)
 {
-    uint32_t row[kZfpMaxBitsLimit / 32 + 2] = {}, pl[32];
+    uint32_t row[zfp_encode_row_words(kZfpMaxBitsLimit / 64u)] = {}, pl[32];
     zfp_encode_row(f, max_bits, row, pl);
     for (uint32_t i = 0; i < max_bits / 64u; ++i)
         bw.words[bw.first + i] = (unsigned long long)row[2 * i] | ((unsigned long long)row[2 * i + 1] << 32);
