@@ -206,17 +206,19 @@ constexpr uint32_t kRunWords = (kEngTile + 2 * kRunRow + 2) / 32 + 2;  // 1538 b
 constexpr uint32_t kRunBatch = 10;  // ranges in flight per lane
 
 // The query that tile `tile` of the batch's stream belongs to: the last with
-// tile0 <= tile (a warp's lanes look at 32 at a time).
+// tile0 <= tile.  A warp's lanes look at 32 queries spread over those that are
+// left, which leaves a 32nd of them: three rounds for 32,768 queries.
 __device__ __forceinline__ uint32_t find_query(const EngQuery* __restrict__ qs, uint32_t nq, uint32_t tile)
 {
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t n = 0;
-    for (uint32_t q = 0; q < nq; q += 32u) {
-        const uint32_t in = __popc(__ballot_sync(0xffffffffu, q + lane < nq && __ldg(&qs[min(q + lane, nq - 1u)].tile0) <= tile));
-        n += in;
-        if (in < 32u) break;
+    uint32_t q0 = 0, left = nq;  // the query is in q0 .. q0 + left - 1
+    for (;;) {
+        const uint32_t step = div_up(left, 32u), q = lane * step;
+        const uint32_t at = __popc(__ballot_sync(0xffffffffu, q < left && __ldg(&qs[q0 + min(q, left - 1u)].tile0) <= tile)) - 1u;
+        q0 += at * step;
+        if (step == 1u) return q0;
+        left = min(step, left - at * step);
     }
-    return n - 1u;
 }
 
 // Counts of the batch's tiles, then of its groups of tiles.
