@@ -160,9 +160,9 @@ struct bcmc_lru {
     // age bins: joint histogram and dense ranks (k_slots' one-pass sort plan)
     uint32_t* age_hist = nullptr;
     uint8_t* age_rank = nullptr;
-    uint16_t* sort_counts = nullptr;  // the sort's tile counts (sort_count_bytes)
     uint64_t* status = nullptr;
-    size_t status_words = 0;
+    size_t status_words = 0;          // an even number
+    uint16_t* sort_counts = nullptr;  // the sort's tile counts, after the status words
     uint64_t* st_active_a = nullptr;
     uint64_t* st_active_n = nullptr;
     uint64_t* st_active_l = nullptr;
@@ -177,6 +177,7 @@ struct bcmc_lru {
 };
 
 static size_t slot_array_bytes(uint32_t cap) { return (size_t)cap * 4u; }
+static size_t lru_status_bytes(const bcmc_lru* c) { return c->status_words * 8u + sort_count_bytes(c->ctx); }
 
 // k_slots leaves the age histogram zero after every update; it is cleared
 // here when an update may not have finished (a wait gave up)
@@ -294,8 +295,9 @@ static bcmc_lru* lru_new(bcmc_ctx* ctx, uint32_t initial_size, uint32_t element_
         lru_alloc_slots(c, c->cache_size ? c->cache_size : 32u);
         const size_t wa = active_tiles(total) + 1, ws = slot_tiles(c->aligned_total) + 1,
                      wsort = sort_status_words(c->aligned_total), wm = mc_grid(ctx, total) + 1;
-        c->status_words = 3 * wa + ws + wsort + 2 * wm;
-        c->status = (uint64_t*)dev_alloc(ctx, c->status_words * 8);
+        c->status_words = (3 * wa + ws + wsort + 2 * wm + 1) / 2 * 2;
+        c->status = (uint64_t*)dev_alloc(ctx, lru_status_bytes(c));
+        c->sort_counts = (uint16_t*)(c->status + c->status_words);
         c->st_active_a = c->status;
         c->st_active_n = c->st_active_a + wa;
         c->st_active_l = c->st_active_n + wa;
@@ -307,7 +309,6 @@ static bcmc_lru* lru_new(bcmc_ctx* ctx, uint32_t initial_size, uint32_t element_
         BCMC_CUDA(cudaMallocHost(&c->h_q, sizeof(QueryState)));
         c->age_hist = (uint32_t*)dev_alloc(ctx, (size_t)kAgeBins * 4);
         c->age_rank = (uint8_t*)dev_alloc(ctx, (size_t)kAgeBins);
-        c->sort_counts = (uint16_t*)dev_alloc(ctx, sort_count_bytes(ctx));
         cudaStream_t s = ctx->stream;
         lru_clear_key16(c, s);
         BCMC_CUDA(cudaMemsetAsync(c->status, 0, c->status_words * 8, s));
@@ -325,8 +326,7 @@ static bcmc_lru* lru_new(bcmc_ctx* ctx, uint32_t initial_size, uint32_t element_
         if (c->capacity) lru_free_slots(c);
         dev_free(ctx, c->item_slots, (size_t)c->aligned_total * 4);
         dev_free(ctx, c->new_ids, (size_t)(total ? total : 1) * 4);
-        dev_free(ctx, c->status, c->status_words * 8);
-        dev_free(ctx, c->sort_counts, sort_count_bytes(ctx));
+        dev_free(ctx, c->status, lru_status_bytes(c));
         dev_free(ctx, c->q, sizeof(QueryState));
         if (c->h_q) cudaFreeHost(c->h_q);
         delete c;
@@ -344,10 +344,9 @@ static void lru_delete(bcmc_lru* c)
     lru_free_slots(c);
     dev_free(ctx, c->item_slots, (size_t)c->aligned_total * 4);
     dev_free(ctx, c->new_ids, (size_t)(c->total ? c->total : 1) * 4);
-    dev_free(ctx, c->status, c->status_words * 8);
+    dev_free(ctx, c->status, lru_status_bytes(c));
     dev_free(ctx, c->age_hist, (size_t)kAgeBins * 4);
     dev_free(ctx, c->age_rank, (size_t)kAgeBins);
-    dev_free(ctx, c->sort_counts, sort_count_bytes(ctx));
     dev_free(ctx, c->q, sizeof(QueryState));
     if (c->h_q) cudaFreeHost(c->h_q);
     delete c;
@@ -403,12 +402,13 @@ struct bcmc_vol {
     uint64_t nwords = 0;
     size_t compressed_bytes = 0;
     float* ranges = nullptr;
-    void* flag_words = nullptr;  // k_query_flags' words (flag_bytes)
     uint32_t* active = nullptr;
     uint32_t* active_ids = nullptr;
-    uint32_t *live_ids = nullptr, *live_at = nullptr;  // the active blocks that can have vertices
     uint32_t* with_verts = nullptr;
     uint32_t* vert_offsets = nullptr;
+    // one allocation (vol_work_bytes), as each takes some 20 us of a volume's load
+    void* flag_words = nullptr;  // k_query_flags' words (flag_bytes)
+    uint32_t *live_ids = nullptr, *live_at = nullptr;  // the active blocks that can have vertices
     uint32_t* block_counts = nullptr;
     uint2* verts = nullptr;
     uint32_t vert_capacity = 0;
@@ -446,6 +446,8 @@ struct bcmc_vol {
 // new blocks a query stages at most (32 MiB); k_assign decodes any beyond
 constexpr uint32_t kStageBlocksMax = 1u << 17;
 
+static size_t vol_work_bytes(uint64_t total) { return flag_bytes(total) + (size_t)total * 12u; }
+
 static void vol_free(bcmc_vol* v)
 {
     if (!v) return;
@@ -453,14 +455,11 @@ static void vol_free(bcmc_vol* v)
     cudaStreamSynchronize(ctx->stream);
     dev_free(ctx, v->words, v->nwords * 8);
     dev_free(ctx, v->ranges, (size_t)v->total * 8);
-    dev_free(ctx, v->flag_words, flag_bytes(v->total));
+    dev_free(ctx, v->flag_words, vol_work_bytes(v->total));
     dev_free(ctx, v->active, (size_t)v->total * 4);
     dev_free(ctx, v->active_ids, (size_t)v->total * 4);
-    dev_free(ctx, v->live_ids, (size_t)v->total * 4);
-    dev_free(ctx, v->live_at, (size_t)v->total * 4);
     dev_free(ctx, v->with_verts, (size_t)v->total * 4);
     dev_free(ctx, v->vert_offsets, (size_t)v->total * 4);
-    dev_free(ctx, v->block_counts, (size_t)v->total * 4);
     if (v->copy) cudaStreamSynchronize(v->copy);
     dev_free(ctx, v->verts, (size_t)v->vert_capacity * 8);
     for (int r = 0; r < kVertRing; ++r)
@@ -533,14 +532,14 @@ static bcmc_status vol_create_common(bcmc_ctx* ctx, const void* src, bool src_de
             BCMC_CUDA(cudaMemsetAsync(v->words, 0, v->nwords * 8, s));
             BCMC_CUDA(cudaMemcpyAsync(v->words, src, len, src_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
             v->ranges = (float*)dev_alloc(ctx, (size_t)total * 8);
-            v->flag_words = dev_alloc(ctx, flag_bytes(total));
             v->active = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
             v->active_ids = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
-            v->live_ids = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
-            v->live_at = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
             v->with_verts = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
             v->vert_offsets = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
-            v->block_counts = (uint32_t*)dev_alloc(ctx, (size_t)total * 4);
+            v->flag_words = dev_alloc(ctx, vol_work_bytes(total));
+            v->live_ids = (uint32_t*)((char*)v->flag_words + flag_bytes(total));
+            v->live_at = v->live_ids + total;
+            v->block_counts = v->live_at + total;
             const uint32_t init_slots =
                 (uint32_t)std::min<double>((double)total, std::ceil((double)total * ctx->opts.initial_cache_fraction));
             v->lru = lru_new(ctx, init_slots, 256u, (uint32_t)total);
