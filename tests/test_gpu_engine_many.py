@@ -1,5 +1,6 @@
 """Batches whose queries take one, two and three rounds to find a tile's query among
-(32 to a round), over volumes of one tile and of several: the same counts and meshes
+(32 to a round), and batches of one group of eight tiles (whose entries k_bactive
+makes) and of more, over volumes of one tile and of two: the same counts and meshes
 as in batches of a few."""
 import numpy as np
 import pytest
@@ -10,8 +11,8 @@ from bcmc import datasets as D
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n", [31, 32, 33, 1024, 1025, 2100])
-def test_batch_equals_its_parts(ctx, oracle, n):
+@pytest.mark.parametrize("n,part", [(7, 3), (8, 5), (9, 8), (31, 8), (32, 16), (33, 16), (1024, 16), (1025, 16), (2100, 16)])
+def test_batch_equals_its_parts(ctx, oracle, n, part):
     eng = bcmc.Engine(ctx, max_batch=4096)
     for dims in ((12, 8, 8), (56, 44, 40)):
         eng.addVolume(oracle.zfp_encode(D.make_field("blobs", dims, 3), 8), 8, dims)
@@ -19,9 +20,9 @@ def test_batch_equals_its_parts(ctx, oracle, n):
     qs = [(int(v), float(np.float32(i))) for v, i in zip(rng.random(n) < 0.1, rng.uniform(0.05, 1.0, n))]
     res = eng.run(qs)
     mesh = eng.copyVertices()
-    for a in range(0, n, 16):
-        part = eng.run(qs[a: a + 16])
-        assert np.array_equal(part["num_vertices"], res["num_vertices"][a: a + 16])
-        assert np.array_equal(part["num_active_blocks"], res["num_active_blocks"][a: a + 16])
+    for a in range(0, n, part):
+        got = eng.run(qs[a: a + part])
+        assert np.array_equal(got["num_vertices"], res["num_vertices"][a: a + part])
+        assert np.array_equal(got["num_active_blocks"], res["num_active_blocks"][a: a + part])
         first = int(res["vertex_offset"][a])
-        assert np.array_equal(eng.copyVertices(), mesh[first: first + int(part["num_vertices"].sum())])
+        assert np.array_equal(eng.copyVertices(), mesh[first: first + int(got["num_vertices"].sum())])
