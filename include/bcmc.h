@@ -416,7 +416,10 @@ bcmc_status bcmc_engine_stats_get(bcmc_engine* eng, bcmc_engine_stats* out);
  * from the defaults), and times a decode probe over up to 2^18 blocks of the
  * largest volume for the decode kernel's threads per CTA and CTAs per SM.  The
  * MC kernel's CTA size (mc_blocks_per_tile: 8, 16 or 32, 16 threads to each; a
- * compiled instance of the kernel per size) is tuned first, then its CTAs per SM.  The chosen
+ * compiled instance of the kernel per size) is tuned first, then its CTAs per SM
+ * (mc_ctas_per_sm: 4, 5 or 6 at 16 blocks, and as many threads at the other
+ * sizes) as far as the SM holds them: 4 at 16 blocks, so that today the three
+ * values give one grid and are not timed apart.  The chosen
  * parameters are used (and captured into that bucket's graph) from then on.
  * The engine has no sort (its pool hands out free slots instead of the LRU's
  * age order), so no radix digit width is tuned here. */

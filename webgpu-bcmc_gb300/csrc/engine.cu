@@ -35,6 +35,7 @@
 
 #include "active_test.cuh"
 #include "bcmc_impl.h"
+#include "engine_tuning.h"
 #include "mc_common.cuh"
 #include "zfp_device.cuh"
 
@@ -46,8 +47,7 @@ constexpr uint32_t kEngTile = 1024;  // blocks per active tile (4 per thread)
 // k_bmc CTAs of 8, 16 or 32 "tile blocks", 16 threads to each; 1024 threads per
 // SM resident whatever the tile (4 CTAs of 16)
 constexpr int kBmcThreadsPerSm = 1024;
-constexpr int kBmcPerSm = 6;        // CTAs per SM that a configuration may ask for at 16 blocks
-constexpr int kBmcMaxPerSm = 12;    // of the 8-block tile: sizes the MC status words
+constexpr int kBmcMaxPerSm = 2 * kBmcPerSm;  // CTAs per SM asked for at 8 blocks: sizes the MC status words
 constexpr uint32_t kMaxVolumes = 4096;
 
 struct EngVolDev {
@@ -819,17 +819,6 @@ struct EngVolume {
     BlockGrid grid;
 };
 
-// Launch parameters the autotuner chooses per batch-size bucket (the kernels'
-// tile shapes are compile-time; these are the runtime knobs).
-struct EngConfig {
-    int act_per_sm = 8;      // k_bactive and k_bentries CTAs per SM
-    int dec_threads = 128;   // k_bdecode threads per CTA (64, 128, 256)
-    int dec_per_sm = 16;     // k_bdecode CTAs per SM
-    int mc_per_sm = kBmcPerSm;  // k_bmc CTAs per SM of the 16-block tile (<= its residency, 6); scaled
-                                // by 16 / mc_blocks for the other tiles
-    int mc_blocks = 32;         // k_bmc "tile blocks", 16 threads each (8, 16, 32)
-};
-
 // The buffers of one batch in flight.  Two lanes let the server keep two
 // batches on the device at once: the next batch's active test, claims and
 // decode (phase 1) run while the current batch's marching cubes (phase 2) do.
@@ -919,13 +908,11 @@ int bmc_resident()
     }();
     return n;
 }
-int eng_grid_mc(bcmc_engine* e)
+int bmc_resident(int mc_blocks)
 {
-    const int kb = e->cfg.mc_blocks;
-    const int resident = kb == 8 ? bmc_resident<8>() : (kb == 32 ? bmc_resident<32>() : bmc_resident<16>());
-    const int per_sm = std::min(std::min(e->cfg.mc_per_sm, kBmcPerSm) * 16 / kb, resident);
-    return e->ctx->num_sms * std::max(per_sm, 1);
+    return mc_blocks == 8 ? bmc_resident<8>() : (mc_blocks == 32 ? bmc_resident<32>() : bmc_resident<16>());
 }
+int eng_grid_mc(bcmc_engine* e) { return e->ctx->num_sms * mc_ctas(e->cfg, bmc_resident(e->cfg.mc_blocks)); }
 int eng_grid_act(bcmc_engine* e) { return e->ctx->num_sms * e->cfg.act_per_sm; }
 int eng_grid_dec(bcmc_engine* e) { return e->ctx->num_sms * e->cfg.dec_per_sm; }
 
@@ -1679,27 +1666,21 @@ extern "C" bcmc_status bcmc_engine_autotune(bcmc_engine* e, const bcmc_query* qu
         double t_best = eng_time_sequence(e, queries, m, res.data());
         out->batch_ms_default = t_best;
         // coordinate descent over the sequence's launch parameters
-        for (int mb : {8, 32}) {  // MC tile: active blocks per CTA tile
-            EngConfig c = best;
-            c.mc_blocks = mb;
-            e->tuned[bucket] = c;
-            const double t = eng_time_sequence(e, queries, m, res.data());
-            if (t < t_best) best = c, t_best = t;
+        const auto take_faster = [&](const std::vector<EngConfig>& others) {
+            for (const EngConfig& c : others) {
+                e->tuned[bucket] = c;
+                const double t = eng_time_sequence(e, queries, m, res.data());
+                if (t < t_best) best = c, t_best = t;
+            }
+        };
+        take_faster(other_mc_sizes(best));
+        take_faster(other_mc_ctas(best, bmc_resident(best.mc_blocks)));
+        std::vector<EngConfig> acts;
+        for (int act : {4, 16}) {
+            acts.push_back(best);
+            acts.back().act_per_sm = act;
         }
-        for (int mc : {4, 5}) {
-            EngConfig c = best;
-            c.mc_per_sm = mc;
-            e->tuned[bucket] = c;
-            const double t = eng_time_sequence(e, queries, m, res.data());
-            if (t < t_best) best = c, t_best = t;
-        }
-        for (int act : {4, 8, 16}) {
-            EngConfig c = best;
-            c.act_per_sm = act;
-            e->tuned[bucket] = c;
-            const double t = eng_time_sequence(e, queries, m, res.data());
-            if (t < t_best) best = c, t_best = t;
-        }
+        take_faster(acts);
         out->batch_ms_tuned = t_best;
         // decode: a probe over (up to 2^18) blocks of the largest volume
         const EngVolume* big = &e->vols[0];
