@@ -996,8 +996,10 @@ bcmc_status bcmc_memory_report(bcmc_vol* v, bcmc_memory* m)
     m->cache = (uint64_t)c->capacity * c->element_size;
     m->cachedItemSlots = (uint64_t)c->aligned_total * 4;
     m->slotData = (uint64_t)c->capacity * 12;
-    m->scratch = (uint64_t)c->capacity * 4 * 6 + c->status_words * 8 + (uint64_t)c->total * 4 + sizeof(QueryState) +
-                 (uint64_t)v->stage_blocks * 256u + flag_bytes(v->total);
+    m->scratch = (uint64_t)c->capacity * 4 * 6 + lru_status_bytes(c) + (uint64_t)c->total * 4 + sizeof(QueryState) +
+                 (uint64_t)kAgeBins * 5 + (uint64_t)v->stage_blocks * 256u + vol_work_bytes(v->total);
+    for (int r = 0; r < kVertRing; ++r)
+        if (r != v->cur) m->scratch += (uint64_t)v->ring_cap[r] * 8;
     m->deviceTotal = m->compressedData + m->vertexBuffer + m->blockActive + m->blockRanges + m->activeBlockIDs +
                      m->blocksWithVertices + m->blockVertexOffsets + m->cache + m->cachedItemSlots + m->slotData +
                      m->scratch;
