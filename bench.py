@@ -496,6 +496,43 @@ SERVED = dict(workload="1024x1024x1080 uint16-range value noise (~60% background
               server_max_batch=1)
 
 
+def plain_open_loop(lat_ms, rate_qps: float, n: int = 2000, seed: int = 0) -> dict:
+    """The plain path as a FIFO single server under open-loop Poisson arrivals,
+    from its measured per-query service times: request i starts at
+    max(arrival_i, finish_{i-1}).  Exact for one FIFO server."""
+    g = np.random.default_rng(seed)
+    arrive = np.cumsum(g.exponential(1.0 / rate_qps, size=n))
+    svc = np.asarray(lat_ms)[np.arange(n) % len(lat_ms)] / 1000.0
+    finish = np.empty(n)
+    t = 0.0
+    for i in range(n):
+        t = max(t, arrive[i]) + svc[i]
+        finish[i] = t
+    l_ms = 1000.0 * (finish - arrive)
+    return {"offered_qps": rate_qps, "achieved_qps": n / (finish[-1] - arrive[0]),
+            "p50_ms": float(np.percentile(l_ms, 50)), "p99_ms": float(np.percentile(l_ms, 99))}
+
+
+def plain_rate_at(lat_ms, p99_ms: float, plain_qps: float):
+    """Highest offered rate, from one query a second up, that the plain path
+    sustains with p99 <= p99_ms; None when it does so at no rate."""
+
+    def sustains(rate):
+        r = plain_open_loop(lat_ms, rate)
+        return r["p99_ms"] <= p99_ms and r["achieved_qps"] >= 0.95 * rate
+
+    lo, hi = 1.0, plain_qps
+    if not sustains(lo):
+        return None
+    for _ in range(30):
+        mid = 0.5 * (lo + hi)
+        if sustains(mid):
+            lo = mid
+        else:
+            hi = mid
+    return lo
+
+
 def served_bench() -> dict:
     """The continuous-batching server on the served mix against the plain
     per-query path: plain = one query at a time, back to back; served = open-loop
@@ -575,44 +612,16 @@ def served_bench() -> dict:
     st = eng.stats()
     p99_plain = float(np.percentile(lat, 99))
 
-    def plain_open_loop(rate_qps, n=2000, seed=0):
-        """The plain path as a FIFO single server under the same open-loop
-        Poisson arrivals, from its measured per-query service times: request i
-        starts at max(arrival_i, finish_{i-1}).  Exact for one FIFO server."""
-        g = np.random.default_rng(seed)
-        arrive = np.cumsum(g.exponential(1.0 / rate_qps, size=n))
-        svc = np.asarray(lat)[np.arange(n) % len(lat)] / 1000.0
-        finish = np.empty(n)
-        t = 0.0
-        for i in range(n):
-            t = max(t, arrive[i]) + svc[i]
-            finish[i] = t
-        l_ms = 1000.0 * (finish - arrive)
-        return {"offered_qps": rate_qps, "achieved_qps": n / (finish[-1] - arrive[0]),
-                "p50_ms": float(np.percentile(l_ms, 50)), "p99_ms": float(np.percentile(l_ms, 99))}
-
-    plain_sweep = [plain_open_loop(s["offered_qps"]) for s in sweeps]
-
-    def plain_rate_at(p99_ms):
-        """Highest offered rate the plain path sustains with p99 <= p99_ms."""
-        lo, hi = 1.0, plain_qps
-        for _ in range(30):
-            mid = 0.5 * (lo + hi)
-            r = plain_open_loop(mid)
-            if r["p99_ms"] <= p99_ms and r["achieved_qps"] >= 0.95 * mid:
-                lo = mid
-            else:
-                hi = mid
-        return lo
+    plain_sweep = [plain_open_loop(lat, s["offered_qps"]) for s in sweeps]
 
     ratios = []
     for sv in sweeps:
         if sv["achieved_qps"] >= 0.95 * sv["offered_qps"]:
             ratios.append({"served_qps": sv["achieved_qps"], "p99_ms": sv["p99_ms"],
-                           "plain_qps_at_same_p99": plain_rate_at(sv["p99_ms"])})
-    for r in ratios:
-        r["ratio"] = r["served_qps"] / r["plain_qps_at_same_p99"]
-    best = max(ratios, key=lambda r: r["ratio"]) if ratios else None
+                           "plain_qps_at_same_p99": plain_rate_at(lat, sv["p99_ms"], plain_qps)})
+    for r in ratios:  # none where the plain path has that p99 at no rate
+        r["ratio"] = r["served_qps"] / r["plain_qps_at_same_p99"] if r["plain_qps_at_same_p99"] else None
+    best = max((r for r in ratios if r["ratio"]), key=lambda r: r["ratio"], default=None)
     return {"workload": SERVED["workload"],
             "plain": {"queries_per_s": plain_qps, "p50_ms": float(np.percentile(lat, 50)), "p99_ms": p99_plain,
                       "what": "back to back, one query at a time (service times)"},
@@ -673,7 +682,7 @@ def _served_summary(sv):
     return {"plain_queries_per_s": sv["plain"]["queries_per_s"], "plain_p99_ms": sv["plain"]["p99_ms"],
             "max_sustained_qps": top["achieved_qps"] if top else None, "p99_ms_at_max": top["p99_ms"] if top else None,
             "best_ratio_at_equal_p99": sv["best_ratio_at_equal_p99"],
-            "ratios_at_equal_p99": [round(r["ratio"], 3) for r in sv["served_vs_plain_at_equal_p99"]],
+            "ratios_at_equal_p99": [r["ratio"] and round(r["ratio"], 3) for r in sv["served_vs_plain_at_equal_p99"]],
             "overlapped_batches": sv["overlapped_batches"],
             "max_speedup_if_only_mc_remains": sv["plain_mc"]["max_speedup_if_only_mc_remains"]}
 
