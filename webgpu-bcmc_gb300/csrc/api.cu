@@ -679,7 +679,7 @@ static void vol_enqueue_query(bcmc_vol* v, cudaStream_t s, float iso, int from_s
     aa.live_at = v->live_at;
     aa.status_l = c->st_active_l;
     aa.sound = sound_ranges(v->dims, grid, zfp_ranged_blocks(ctx, v->dims));
-    McArgs ma{v->active, v->active_ids, v->live_ids, v->live_at, c->item_slots, reinterpret_cast<const float*>(c->cache), nb, grid,
+    McArgs ma{v->active, v->active_ids, v->live_ids, v->live_at, c->item_slots, reinterpret_cast<const float*>(c->cache), grid,
               v->with_verts, v->vert_offsets, v->block_counts, out, c->st_mc_v, c->st_mc_b, out != v->verts ? 1u : 0u};
     SlotArgs sa{v->active,  c->slot_age, c->slot_avail, c->slot_item, c->avail_ids, c->avail_keys, c->st_slots, 1u, 1u,
                 c->age_hist, c->age_rank};
@@ -769,7 +769,7 @@ static bcmc_status vol_query(bcmc_vol* v, float iso, bcmc_perf* perf, uint32_t* 
         for (int attempt = 0;; ++attempt) {
             vol_ensure_graph(v, mode, host_out);
             lru_epoch_tick(c, s);
-            *v->h_in = QueryInputs{iso, c->capacity, out_cap, 0u, ctx->debug_drop_tile};
+            *v->h_in = QueryInputs{iso, c->capacity, out_cap, ctx->debug_drop_tile};
             BCMC_CUDA(cudaGraphLaunch(v->graph[graph_slot(v, mode)], s));
             count_launches(v->graph_kernels);
             BCMC_CUDA(cudaStreamSynchronize(s));
@@ -790,7 +790,7 @@ static bcmc_status vol_query(bcmc_vol* v, float iso, bcmc_perf* perf, uint32_t* 
             break;
         }
         const uint3 nb = make_uint3(v->nb[0], v->nb[1], v->nb[2]);
-        McArgs ma{v->active, v->active_ids, v->live_ids, v->live_at, c->item_slots, reinterpret_cast<const float*>(c->cache), nb,
+        McArgs ma{v->active, v->active_ids, v->live_ids, v->live_at, c->item_slots, reinterpret_cast<const float*>(c->cache),
                   make_block_grid(nb), v->with_verts, v->vert_offsets, v->block_counts, v->verts, c->st_mc_v,
                   c->st_mc_b};
         QueryState& h = *c->h_q;

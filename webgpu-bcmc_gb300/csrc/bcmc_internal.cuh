@@ -24,7 +24,6 @@ struct QueryInputs {
     float isovalue;
     uint32_t capacity;
     uint32_t vert_capacity;
-    uint32_t mc_only;
     uint32_t debug_drop_tile;  // test hook (bcmc_debug_drop_tile): 0, or tile + 1
 };
 
@@ -333,9 +332,10 @@ struct CtaCount {
 // The sums over the CTAs before `rank` of kN counts that each published in its
 // status words (aggregates of this epoch; `drop`: this CTA publishes nothing, the
 // test hook's case).  Every thread takes a share of the predecessors, so all
-// are read in one round trip; the wait is for the slowest of them.
+// are read in one round trip; the wait is for the slowest of them.  True when this
+// thread's wait timed out.
 template <int kThreads, int kN>
-__device__ __forceinline__ void cta_prefix_sums(const CtaCount (&c)[kN], uint32_t rank, uint32_t epoch, uint32_t* err,
+__device__ __forceinline__ bool cta_prefix_sums(const CtaCount (&c)[kN], uint32_t rank, uint32_t epoch, uint32_t* err,
                                                 bool drop = false)
 {
     if (threadIdx.x == 0 && !drop) {
@@ -343,6 +343,7 @@ __device__ __forceinline__ void cta_prefix_sums(const CtaCount (&c)[kN], uint32_
         for (int i = 0; i < kN; ++i) lb_store(c[i].status + rank, lb_pack(epoch, kFlagAggregate, c[i].count));
     }
     uint32_t sum[kN] = {};
+    bool timed_out = false;
     for (uint32_t p = threadIdx.x; p < rank; p += kThreads) {
         uint64_t v[kN];
         uint32_t spins = 0;
@@ -355,6 +356,7 @@ __device__ __forceinline__ void cta_prefix_sums(const CtaCount (&c)[kN], uint32_
             if (!late) break;
             if (++spins > kSpinLimit) {
                 atomicCAS(err, 0u, late);
+                timed_out = true;
                 break;
             }
             if (spins > 8) __nanosleep(100);
@@ -367,34 +369,7 @@ __device__ __forceinline__ void cta_prefix_sums(const CtaCount (&c)[kN], uint32_
         sum[i] = __reduce_add_sync(0xffffffffu, sum[i]);
         if ((threadIdx.x & 31u) == 0u && sum[i]) atomicAdd(c[i].sum, sum[i]);
     }
-}
-
-// The same for one count; true when this thread's wait timed out.
-template <int kThreads>
-__device__ __forceinline__ bool cta_prefix_sum(uint64_t* status, uint32_t rank, uint32_t a, uint32_t epoch, uint32_t* err,
-                                               uint32_t site, uint32_t* sum, bool drop = false)
-{
-    if (threadIdx.x == 0 && !drop) lb_store(status + rank, lb_pack(epoch, kFlagAggregate, a));
-    uint32_t sa = 0;
-    bool late = false;
-    for (uint32_t p = threadIdx.x; p < rank; p += kThreads) {
-        uint64_t v;
-        uint32_t spins = 0;
-        for (;;) {
-            v = lb_load(status + p);
-            if ((uint32_t)(v >> 34) == epoch) break;
-            if (++spins > kSpinLimit) {
-                atomicCAS(err, 0u, site);
-                late = true;
-                break;
-            }
-            if (spins > 8) __nanosleep(100);
-        }
-        sa += (uint32_t)v;
-    }
-    sa = __reduce_add_sync(0xffffffffu, sa);
-    if ((threadIdx.x & 31u) == 0u && sa) atomicAdd(sum, sa);
-    return late;
+    return timed_out;
 }
 
 // The radix sort's pass plan, made by the last of the CTAs that accumulated

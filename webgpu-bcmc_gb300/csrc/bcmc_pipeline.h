@@ -105,7 +105,6 @@ struct McArgs {
     const uint32_t* live_at;
     const int32_t* item_slots;
     const float* cache;
-    uint3 nb;
     BlockGrid grid;
     uint32_t* with_verts;
     uint32_t* vert_offsets;

@@ -554,7 +554,7 @@ __device__ __forceinline__ void update_slots(QueryState* q, const SlotArgs& a)
         count = __reduce_add_sync(0xffffffffu, count);
         if (lane == 0 && count) atomicAdd(&s_sum, count);
         __syncthreads();
-        cta_prefix_sum<kActThreads>(a.status, s_rank, s_sum, q->epoch, &q->error, 32u, &s_prefix);
+        cta_prefix_sums<kActThreads>({{a.status, s_sum, 32u, &s_prefix}}, s_rank, q->epoch, &q->error);
         __syncthreads();
         uint32_t run = s_prefix;
         for (uint32_t base = first; base < end; base += kSlotChunk) {

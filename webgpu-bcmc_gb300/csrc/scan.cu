@@ -107,15 +107,15 @@ __global__ void __launch_bounds__(kRangeThreads, kRangePerSm) k_scan(QueryState*
         load_items<kWide>(in, (uint64_t)tile * kRangeTile + 128u * kRangeGroups * warp, n, v);
 #pragma unroll
         for (uint32_t j = 0; j < kRangeGroups; ++j) {
-                const uint4 x = addends<kSelect>(v[j]);
+            const uint4 x = addends<kSelect>(v[j]);
             all += x.x + x.y + x.z + x.w;
         }
     }
     all = __reduce_add_sync(0xffffffffu, all);
     if ((t & 31u) == 0u && all) atomicAdd(&s_sum, all);
     __syncthreads();
-    const bool late = cta_prefix_sum<kRangeThreads>(status, rank, s_sum, status_tag(q), &q->error, kSelect ? 2u : 1u,
-                                                    &s_prefix, lb_dropped(q, rank));
+    const bool late = cta_prefix_sums<kRangeThreads>({{status, s_sum, kSelect ? 2u : 1u, &s_prefix}}, rank, status_tag(q),
+                                                     &q->error, lb_dropped(q, rank));
     if (late && tot.host) tot.host[1] = 1u;
     __syncthreads();
     uint32_t run = s_prefix;
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kRangeThreads, kRangePerSm) k_scan(QueryState*
         uint32_t before[kRangeGroups], sum = 0;  // of the warp's elements
 #pragma unroll
         for (uint32_t j = 0; j < kRangeGroups; ++j) {
-                const uint4 x = addends<kSelect>(v[j]);
+            const uint4 x = addends<kSelect>(v[j]);
             const uint32_t mine = x.x + x.y + x.z + x.w, inc = warp_inclusive_scan(mine);
             before[j] = sum + inc - mine;
             sum += __shfl_sync(0xffffffffu, inc, 31);
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kRangeThreads, kRangePerSm) k_scan(QueryState*
         run += total;
 #pragma unroll
         for (uint32_t j = 0; j < kRangeGroups; ++j) {
-                const uint64_t i = base + 128u * j + 4u * lane;
+            const uint64_t i = base + 128u * j + 4u * lane;
             const uint4 x = addends<kSelect>(v[j]);
             uint4 p;
             p.x = start + before[j];

@@ -1,6 +1,7 @@
 // scan_noalloc.cu -- exclusive scan that allocates nothing.
 //
-// Same result as bcmc_scan_exclusive_u32_async (the scan by ranges of scan.cu), for callers that must not allocate device memory on the call:
+// Same result as bcmc_scan_exclusive_u32_async (the scan by ranges of scan.cu),
+// for callers that must not allocate device memory on the call:
 // a host runtime that owns every device byte through its own pool and forbids
 // cudaMalloc/cudaFree outside it, code running between a stream's enqueue and
 // its synchronisation where an allocation's implicit device synchronisation
