@@ -786,7 +786,11 @@ constexpr int kMcPerSm = 2;  // resident CTAs per SM (the grid: one launch, all 
 // their own CTA; longer ones go through a grid barrier and an even share-out.
 constexpr uint32_t kMcOwnRange = kMcWarps * kMcBlocks;
 // Ranges longer than this are counted by all CTAs together, which costs a barrier.
-constexpr uint32_t kMcSharedRange = 1024;
+// The same queries both ways, 76 isovalues of 224^3 to 1024 x 1024 x 1080 voxels: up
+// to 2,000 active blocks to a CTA the barrier costs 2 to 4 us (512^3 82 -> 84, 256^3 47
+// -> 49), to 5,000 neither way is faster by more than 1 %, above that sharing gains 0.2
+// to 1.2 % (800^3 653 -> 649 us, 640^3 1,026 -> 1,018, 1024 x 1024 x 1080 1,753 -> 1,733).
+constexpr uint32_t kMcSharedRange = 4096;
 
 // Marching cubes over the active blocks, one cooperative launch (every CTA
 // resident), all of its block work done by single warps (mc_common.cuh):
@@ -795,8 +799,7 @@ constexpr uint32_t kMcSharedRange = 1024;
 //     block totals are kept.  Each CTA counts its own range of the blocks, or,
 //     when the ranges are long, its share of batches from the whole grid, with a
 //     barrier after it: a batch's cost depends on whether the surface passes
-//     through it (512^3: 878 -> 867 us, 1024 x 1024 x 1080: 636 -> 612 us, but
-//     256^3: 59 -> 63 us, where the barrier costs more than the balance saves);
+//     through it (kMcSharedRange);
 //   each CTA publishes its range's totals and adds up those of the CTAs before
 //     it: its vertex offset and its place in the blocks-with-vertices list;
 //   it writes its entries of that list and their vertex offsets, then a grid
