@@ -26,3 +26,21 @@ def test_batch_equals_its_parts(ctx, oracle, n, part):
         assert np.array_equal(got["num_active_blocks"], res["num_active_blocks"][a: a + part])
         first = int(res["vertex_offset"][a])
         assert np.array_equal(eng.copyVertices(), mesh[first: first + int(got["num_vertices"].sum())])
+
+
+def test_one_group_with_a_full_pool(ctx, oracle):
+    """Batches of one group whose blocks do not fit the pool beside the last batch's:
+    claims run out, slots are evicted, and the batch runs again."""
+    dims = (40, 36, 36)  # 810 blocks, one tile
+    words = [oracle.zfp_encode(D.make_field("turbulence", dims, s), 6) for s in range(3)]
+    small, large = bcmc.Engine(ctx, pool_slots=820), bcmc.Engine(ctx)
+    for w in words:
+        small.addVolume(w, 6, dims)
+        large.addVolume(w, 6, dims)
+    for i in range(9):
+        q = [(i % 3, 0.05 * (i - 4))] * (1 + i % 2)
+        a, b = small.run(q), large.run(q)
+        assert np.array_equal(a["num_vertices"], b["num_vertices"]) and a["num_vertices"][0] > 0
+        assert np.array_equal(a["num_active_blocks"], b["num_active_blocks"])
+        assert np.array_equal(small.copyVertices(), large.copyVertices())
+    assert small.stats()["evicted_blocks"] > 0 and large.stats()["evicted_blocks"] == 0
