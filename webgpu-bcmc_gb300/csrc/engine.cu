@@ -847,6 +847,7 @@ struct EngLane {
         cudaGraphExec_t exec = nullptr;        // the whole sequence on one stream
         cudaGraphExec_t front = nullptr;       // phase 1 (pipelined runs)
         cudaGraphExec_t back = nullptr;        // phase 2 (pipelined runs)
+        uint32_t kernels = 0, split_kernels = 0;  // in exec, in front and back
         uint64_t generation = 0, split_generation = 0;
         int cfg_key = -1, split_cfg_key = -1;  // the launch parameters they were captured with
     };
@@ -1131,8 +1132,8 @@ void eng_lane_free(bcmc_engine* e, EngLane& l)
 
 // The launch sequence of one batch (also what a graph captures).
 // Phase 1 of a batch: inputs in, active test, claims, decode of the claimed
-// blocks into their slots.
-void eng_enqueue_front(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
+// blocks into their slots.  Returns the kernels it launches, as the others do.
+uint32_t eng_enqueue_front(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
 {
     const BatchArgs a = eng_args(e);
     BCMC_CUDA(cudaMemcpyAsync(e->L->d_queries, e->L->h_queries, bucket * sizeof(EngQuery), cudaMemcpyHostToDevice, s));
@@ -1155,8 +1156,8 @@ void eng_enqueue_front(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
         allow_smem(k_bdecode<128>, smem);
         k_bdecode<128><<<eng_grid_dec(e), 128, smem, s>>>(a, r);
     }
-    count_launches(4);
     BCMC_CUDA(cudaGetLastError());
+    return 4;
 }
 
 template <int kB>
@@ -1168,7 +1169,7 @@ void bmc_launch(cudaLaunchConfig_t cfg, const BatchArgs& a)
 }
 
 // Phase 2: marching cubes over the batch's entries, per-query results, state out.
-void eng_enqueue_back(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
+uint32_t eng_enqueue_back(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
 {
     const BatchArgs a = eng_args(e);
     // cooperative: k_bmc's grid barrier needs every CTA resident
@@ -1185,18 +1186,17 @@ void eng_enqueue_back(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
     else if (e->cfg.mc_blocks == 32) bmc_launch<32>(cfg, a);
     else bmc_launch<16>(cfg, a);
     k_bfinish<<<1, kFinThreads, 0, s>>>(a);
-    count_launches(2);
     BCMC_CUDA(cudaGetLastError());
     BCMC_CUDA(cudaEventRecordWithFlags(e->L->ev1, s, cudaEventRecordExternal));
     BCMC_CUDA(cudaMemcpyAsync(e->L->h_st, e->L->d_st, sizeof(EngState), cudaMemcpyDeviceToHost, s));
     BCMC_CUDA(cudaMemcpyAsync(e->L->h_results, e->L->d_results, bucket * sizeof(EngResult), cudaMemcpyDeviceToHost, s));
+    return 2;
 }
 
-// The launch sequence of one batch on one stream (also what a graph captures).
-void eng_enqueue(bcmc_engine* e, uint32_t bucket)
+// The launch sequence of one batch on one stream (what a graph captures).
+uint32_t eng_enqueue(bcmc_engine* e, uint32_t bucket)
 {
-    eng_enqueue_front(e, bucket, e->stream);
-    eng_enqueue_back(e, bucket, e->stream);
+    return eng_enqueue_front(e, bucket, e->stream) + eng_enqueue_back(e, bucket, e->stream);
 }
 
 int eng_cfg_key(const EngConfig& c)
@@ -1205,22 +1205,20 @@ int eng_cfg_key(const EngConfig& c)
     return c.act_per_sm | (c.dec_threads << 8) | (c.dec_per_sm << 18) | (c.mc_per_sm << 24) | (log_blocks << 27);
 }
 
-// Captures what `enqueue` issues on stream s into a graph.
+// Captures what `enqueue` issues on stream s into a graph; adds its kernels to *kernels.
 template <typename F>
-cudaGraphExec_t eng_capture(cudaStream_t s, F&& enqueue)
+cudaGraphExec_t eng_capture(cudaStream_t s, uint32_t* kernels, F&& enqueue)
 {
     cudaGraph_t graph = nullptr;
-    const uint64_t before = g_kernel_launches.load();
     BCMC_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     try {
-        enqueue();
+        *kernels += enqueue();
     } catch (...) {
         cudaStreamEndCapture(s, &graph);
         if (graph) cudaGraphDestroy(graph);
         throw;
     }
     BCMC_CUDA(cudaStreamEndCapture(s, &graph));
-    g_kernel_launches.store(before);  // captured, not launched
     cudaGraphExec_t exec = nullptr;
     const cudaError_t err = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
@@ -1237,12 +1235,13 @@ void eng_launch(bcmc_engine* e, uint32_t bucket)
     if (!g.exec || g.generation != e->L->generation || g.cfg_key != key) {
         if (g.exec) cudaGraphExecDestroy(g.exec);
         g.exec = nullptr;
-        g.exec = eng_capture(e->stream, [&] { eng_enqueue(e, bucket); });
+        g.kernels = 0;
+        g.exec = eng_capture(e->stream, &g.kernels, [&] { return eng_enqueue(e, bucket); });
         g.generation = e->L->generation;
         g.cfg_key = key;
     }
     BCMC_CUDA(cudaGraphLaunch(g.exec, e->stream));
-    count_launches(5);
+    count_launches(g.kernels);
 }
 
 // Pipelined launch: phase 1 on the front stream, phase 2 on the back stream
@@ -1258,8 +1257,9 @@ void eng_launch_split(bcmc_engine* e, uint32_t bucket)
         if (g.front) cudaGraphExecDestroy(g.front);
         if (g.back) cudaGraphExecDestroy(g.back);
         g.front = g.back = nullptr;
-        g.front = eng_capture(e->stream, [&] { eng_enqueue_front(e, bucket, e->stream); });
-        g.back = eng_capture(e->stream_back, [&] { eng_enqueue_back(e, bucket, e->stream_back); });
+        g.split_kernels = 0;
+        g.front = eng_capture(e->stream, &g.split_kernels, [&] { return eng_enqueue_front(e, bucket, e->stream); });
+        g.back = eng_capture(e->stream_back, &g.split_kernels, [&] { return eng_enqueue_back(e, bucket, e->stream_back); });
         g.split_generation = e->L->generation;
         g.split_cfg_key = key;
     }
@@ -1267,7 +1267,7 @@ void eng_launch_split(bcmc_engine* e, uint32_t bucket)
     BCMC_CUDA(cudaEventRecord(e->L->ev_front, e->stream));
     BCMC_CUDA(cudaStreamWaitEvent(e->stream_back, e->L->ev_front, 0));
     BCMC_CUDA(cudaGraphLaunch(g.back, e->stream_back));
-    count_launches(5);
+    count_launches(g.split_kernels);
 }
 
 uint32_t bucket_of(uint32_t n)
