@@ -8,7 +8,8 @@
 //              A tile whose extended value range (its blocks and their 26
 //              neighbours, from volume load) excludes the isovalue is skipped
 //              whole.  Active bits go to a per-query bitmap, counts to the tiles
-//   k_bentries (query, block) entries of the active blocks that can have vertices
+//   k_bentries (not for a batch of up to eight tiles, whose entries k_bactive makes)
+//              (query, block) entries of the active blocks that can have vertices
 //              in query-major, block-ascending order from the tiles' counts;
 //              active blocks no slot holds are claimed
 //              (one claim per block across the batch) and given a slot from
@@ -404,9 +405,10 @@ __device__ __forceinline__ void tile_entries(const BatchArgs& a, uint32_t qi, co
 }
 
 // A batch of one group of tiles is one CTA's: its warps have the words and the counts
-// at hand and go on to the entries themselves (with the runs' missing words left out
-// and the words without active blocks passed over, single queries on 8^3 volumes 40.7
-// -> 32.0 us on the device, on 32^3 41.7 -> 37.5).
+// at hand and go on to the entries themselves, and k_bentries is not launched.  With
+// the runs' missing words left out and the words without active blocks passed over,
+// single queries on 8^3 volumes 40.7 -> 31.9 us on the device, on 48^3 44.0 -> 39.8,
+// four on 32^3 42.7 -> 38.3.
 __global__ void __launch_bounds__(kEngThreads, 3) k_bactive(BatchArgs a)
 {
     __shared__ RunWords s_run[kGroup];
@@ -459,8 +461,8 @@ __global__ void __launch_bounds__(kEngThreads, 3) k_bactive(BatchArgs a)
 //
 // A CTA owns a contiguous range of groups of tiles.  Every count is known, so
 // it adds up those of the groups before its range and waits for nobody; a warp
-// takes a tile of a group, whose words' bits say where each entry goes.  (The
-// entries of a batch of one group k_bactive has made itself.)
+// takes a tile of a group, whose words' bits say where each entry goes.  (Not
+// launched for a batch of one group, whose entries k_bactive makes.)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kEngThreads) k_bentries(BatchArgs a)
 {
@@ -469,7 +471,7 @@ __global__ void __launch_bounds__(kEngThreads) k_bentries(BatchArgs a)
     const uint32_t ntiles = st->ntiles, nq = st->nq, cap = st->entry_capacity, use_epoch = st->use_epoch;
     const uint32_t ngroups = div_up(ntiles, kGroup), per = div_up(ngroups, gridDim.x);
     const uint32_t first = blockIdx.x * per, end = min(ngroups, first + per);
-    if (ngroups <= 1u || first >= ngroups) return;
+    if (first >= ngroups) return;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t* groups = group_counts(a, ntiles);
     if (threadIdx.x == 0) s_sum = 0;
@@ -842,7 +844,8 @@ struct EngLane {
     uint64_t status_a_words = 0;
     uint64_t epoch_calls = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    // one graph per batch-size bucket, rebuilt when buffers move
+    // one graph per batch-size bucket and number of tile groups, one or more (graph_key),
+    // rebuilt when buffers move
     struct Graph {
         cudaGraphExec_t exec = nullptr;        // the whole sequence on one stream
         cudaGraphExec_t front = nullptr;       // phase 1 (pipelined runs)
@@ -1133,15 +1136,16 @@ void eng_lane_free(bcmc_engine* e, EngLane& l)
 // The launch sequence of one batch (also what a graph captures).
 // Phase 1 of a batch: inputs in, active test, claims, decode of the claimed
 // blocks into their slots.  Returns the kernels it launches, as the others do.
-uint32_t eng_enqueue_front(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
+uint32_t eng_enqueue_front(bcmc_engine* e, uint32_t bucket, bool one_group, cudaStream_t s)
 {
     const BatchArgs a = eng_args(e);
     BCMC_CUDA(cudaMemcpyAsync(e->L->d_queries, e->L->h_queries, bucket * sizeof(EngQuery), cudaMemcpyHostToDevice, s));
     BCMC_CUDA(cudaMemcpyAsync(e->L->d_st, e->L->h_st, offsetof(EngState, epoch), cudaMemcpyHostToDevice, s));
     BCMC_CUDA(cudaEventRecordWithFlags(e->L->ev0, s, cudaEventRecordExternal));
     k_bbegin<<<1, 1024, 0, s>>>(e->L->d_st, e->L->q_nverts, e->L->q_nactive, bucket);
-    k_bactive<<<eng_grid_act(e), kEngThreads, 0, s>>>(a);
-    k_bentries<<<eng_grid_act(e), kEngThreads, 0, s>>>(a);
+    // one group: one CTA's work, entries included
+    k_bactive<<<one_group ? 1 : eng_grid_act(e), kEngThreads, 0, s>>>(a);
+    if (!one_group) k_bentries<<<eng_grid_act(e), kEngThreads, 0, s>>>(a);
     const uint32_t r = e->max_rate;
     if (e->cfg.dec_threads == 64) {
         const size_t smem = zfp_stage_smem(64, r);
@@ -1157,7 +1161,7 @@ uint32_t eng_enqueue_front(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
         k_bdecode<128><<<eng_grid_dec(e), 128, smem, s>>>(a, r);
     }
     BCMC_CUDA(cudaGetLastError());
-    return 4;
+    return one_group ? 3 : 4;
 }
 
 template <int kB>
@@ -1194,9 +1198,9 @@ uint32_t eng_enqueue_back(bcmc_engine* e, uint32_t bucket, cudaStream_t s)
 }
 
 // The launch sequence of one batch on one stream (what a graph captures).
-uint32_t eng_enqueue(bcmc_engine* e, uint32_t bucket)
+uint32_t eng_enqueue(bcmc_engine* e, uint32_t bucket, bool one_group)
 {
-    return eng_enqueue_front(e, bucket, e->stream) + eng_enqueue_back(e, bucket, e->stream);
+    return eng_enqueue_front(e, bucket, one_group, e->stream) + eng_enqueue_back(e, bucket, e->stream);
 }
 
 int eng_cfg_key(const EngConfig& c)
@@ -1226,17 +1230,26 @@ cudaGraphExec_t eng_capture(cudaStream_t s, uint32_t* kernels, F&& enqueue)
     return exec;
 }
 
-void eng_launch(bcmc_engine* e, uint32_t bucket)
+// A batch as it is launched: its batch-size bucket, tiles and bitmap words.
+struct SeqShape {
+    uint32_t bucket;
+    uint64_t tiles, words;
+
+    bool one_group() const { return tiles <= kGroup; }
+    uint32_t graph_key() const { return 2u * bucket + (one_group() ? 1u : 0u); }
+};
+
+void eng_launch(bcmc_engine* e, const SeqShape& sh)
 {
-    auto it = e->tuned.find(bucket);
+    auto it = e->tuned.find(sh.bucket);
     e->cfg = it != e->tuned.end() ? it->second : EngConfig{};
-    auto& g = e->L->graphs[bucket];
+    auto& g = e->L->graphs[sh.graph_key()];
     const int key = eng_cfg_key(e->cfg);
     if (!g.exec || g.generation != e->L->generation || g.cfg_key != key) {
         if (g.exec) cudaGraphExecDestroy(g.exec);
         g.exec = nullptr;
         g.kernels = 0;
-        g.exec = eng_capture(e->stream, &g.kernels, [&] { return eng_enqueue(e, bucket); });
+        g.exec = eng_capture(e->stream, &g.kernels, [&] { return eng_enqueue(e, sh.bucket, sh.one_group()); });
         g.generation = e->L->generation;
         g.cfg_key = key;
     }
@@ -1247,19 +1260,19 @@ void eng_launch(bcmc_engine* e, uint32_t bucket)
 // Pipelined launch: phase 1 on the front stream, phase 2 on the back stream
 // after it.  The next batch's phase 1 (front stream) can then run while this
 // batch's phase 2 does.
-void eng_launch_split(bcmc_engine* e, uint32_t bucket)
+void eng_launch_split(bcmc_engine* e, const SeqShape& sh)
 {
-    auto it = e->tuned.find(bucket);
+    auto it = e->tuned.find(sh.bucket);
     e->cfg = it != e->tuned.end() ? it->second : EngConfig{};
-    auto& g = e->L->graphs[bucket];
+    auto& g = e->L->graphs[sh.graph_key()];
     const int key = eng_cfg_key(e->cfg);
     if (!g.front || g.split_generation != e->L->generation || g.split_cfg_key != key) {
         if (g.front) cudaGraphExecDestroy(g.front);
         if (g.back) cudaGraphExecDestroy(g.back);
         g.front = g.back = nullptr;
         g.split_kernels = 0;
-        g.front = eng_capture(e->stream, &g.split_kernels, [&] { return eng_enqueue_front(e, bucket, e->stream); });
-        g.back = eng_capture(e->stream_back, &g.split_kernels, [&] { return eng_enqueue_back(e, bucket, e->stream_back); });
+        g.front = eng_capture(e->stream, &g.split_kernels, [&] { return eng_enqueue_front(e, sh.bucket, sh.one_group(), e->stream); });
+        g.back = eng_capture(e->stream_back, &g.split_kernels, [&] { return eng_enqueue_back(e, sh.bucket, e->stream_back); });
         g.split_generation = e->L->generation;
         g.split_cfg_key = key;
     }
@@ -1282,13 +1295,6 @@ uint32_t bucket_of(uint32_t n)
 struct AdmitPrefix : std::length_error {
     uint32_t fit;
     explicit AdmitPrefix(uint32_t f) : std::length_error("batch above the vertex budget"), fit(f) {}
-};
-
-// Runs queries[0..n) (n <= max_batch) as one launch sequence; results go to out.
-// Throws std::length_error when the pool cannot hold the sequence's active blocks.
-struct SeqShape {
-    uint32_t bucket;
-    uint64_t tiles, words;
 };
 
 // The current lane's query table for queries[0..n), padded to the batch-size
@@ -1360,7 +1366,7 @@ void eng_run_sequence(bcmc_engine* e, const bcmc_query* queries, uint32_t n, bcm
         EngState& st = *e->L->h_st;
         eng_set_inputs(e, sh);
         eng_epoch_tick(e);
-        eng_launch(e, bucket);
+        eng_launch(e, sh);
         BCMC_CUDA(cudaStreamSynchronize(e->stream));
         ++e->stats.launch_sequences;
         if (st.error) throw std::runtime_error("device wait timed out in the batched engine");
@@ -1834,7 +1840,7 @@ bcmc_status engine_submit(bcmc_engine* e, int k, const bcmc_query* queries, uint
         eng_ensure_verts(e, 1);
         eng_set_inputs(e, sh);
         eng_epoch_tick(e);
-        eng_launch_split(e, sh.bucket);
+        eng_launch_split(e, sh);
         BCMC_CUDA(cudaEventRecord(me.ev_done, e->stream_back));
         if (on_done) BCMC_CUDA(cudaLaunchHostFunc(e->stream_back, on_done, arg));
         me.in_flight = true;
